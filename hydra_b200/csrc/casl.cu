@@ -14,6 +14,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
 #include <map>
 #include <string>
 #include <vector>
@@ -347,25 +348,23 @@ struct LoadQC {
   }
 };
 
-// Advection product -u*fx - v*(fy [+ beta]) of evolution.f90:449,456-461,
-// read from physical arrays ([ix][iy]); b = 0 for qd, 1 for qs.
 // Two adjacent elements of an FP64 or FP32 field, as FP64.
 __device__ __forceinline__ double2 ld2(const double *p) { return *reinterpret_cast<const double2 *>(p); }
 __device__ __forceinline__ double2 ld2(const float *p) {
   const float2 f = *reinterpret_cast<const float2 *>(p);
   return make_double2((double)f.x, (double)f.y);
 }
-template <class T>
-struct LoadAdvectT {
-  __host__ double bytes() const { return 4.0 * sizeof(T); }
-  const T *uu, *vv;
-  const T *fx[2], *fy[2];
+// Advection product -u*fx - v*(fy [+ beta]) of evolution.f90:449,456-461,
+// read from FP32 physical arrays ([ix][iy]); b = 0 for qd, 1 for qs (the
+// FP32-inversion mode).
+struct LoadAdvectF {
+  const float *uu, *vv;
+  const float *fx[2], *fy[2];
   double betab[2];  // beta added to fy for the qs term when beffect
   int n;
-  long long ms = 0;  // ensemble: entry b is term b % 2 of member b / 2, fields ms apart
   __device__ __forceinline__ double operator()(int b, int v /*ix*/, int j /*iy*/) const {
     const int e = b & 1;
-    long long k = (long long)(b >> 1) * ms + (long long)v * n + j;
+    long long k = (long long)v * n + j;
     const double bb = pick(betab, e);
     double gx = (double)pick(fx, e)[k], gy = (double)pick(fy, e)[k];
     if (bb != 0.0) gy = gy + bb;
@@ -373,7 +372,7 @@ struct LoadAdvectT {
   }
   __device__ __forceinline__ double2 pair(int b, int v, int j) const {
     const int e = b & 1;
-    long long k = (long long)(b >> 1) * ms + (long long)v * n + j;
+    long long k = (long long)v * n + j;
     const double bb = pick(betab, e);
     const double2 gx = ld2(pick(fx, e) + k);
     double2 gy = ld2(pick(fy, e) + k);
@@ -386,17 +385,14 @@ struct LoadAdvectT {
     return make_double2(-u.x * gx.x - w.x * gy.x, -u.y * gx.y - w.y * gy.y);
   }
 };
-using LoadAdvect = LoadAdvectT<double>;
 
 // Store of the source terms after ptospc pass B (evolution.f90:466-487):
 // b = 0 -> sqd with damping and the integrating factor, b = 1 -> sqs.
 struct StoreSource {
-  __host__ double bytes() const { return 8.0 + 0.5 * 24.0; }  // sqd reads qq, pp, epq
   double *sqd, *sqs;
   const double *qq, *pp, *epq;
   double rekman, kdsq, therm;
   int heating, friction, lev, n;
-  long long ms = 0;  // ensemble: entry b is term b % 2 of member b / 2
   __device__ __forceinline__ double damped(double x, double p, double q, double e) const {
     double t;
     if (heating) {
@@ -414,7 +410,7 @@ struct StoreSource {
     return t;
   }
   __device__ __forceinline__ void operator()(int b, int v /*ky*/, int k /*kx*/, double x) const {
-    const long long idx = (long long)(b >> 1) * ms + (long long)v * n + k;
+    const long long idx = (long long)v * n + k;
     if (b & 1) {
       sqs[idx] = x;
       return;
@@ -422,7 +418,7 @@ struct StoreSource {
     sqd[idx] = damped(x, pp[idx], qq[idx], lev ? epq[idx] : 0.0);
   }
   __device__ __forceinline__ void pair(int b, int v, int k, double2 x) const {
-    const long long i = (long long)(b >> 1) * ms + (long long)v * n + k;
+    const long long i = (long long)v * n + k;
     if (b & 1) {
       *reinterpret_cast<double2 *>(sqs + i) = x;
       return;
@@ -478,7 +474,6 @@ using LoadBatch = LoadBatchT<false>;
 // the kernel's arithmetic stays FP64 in registers; the intermediate and the
 // physical outputs are rounded to FP32 once, when stored.
 struct StoreStridedF {
-  __host__ double bytes() const { return 4.0; }
   float *p;
   long long bs, vs, es;
   __device__ __forceinline__ void operator()(int b, int v, int k, double x) const {
@@ -495,7 +490,6 @@ struct StoreStridedF {
   }
 };
 struct LoadBatchF {
-  __host__ double bytes() const { return 4.0; }
   const float *p[6];
   long long vs, es;
   __device__ __forceinline__ double operator()(int b, int v, int j) const {
@@ -503,7 +497,6 @@ struct LoadBatchF {
   }
 };
 struct StoreScaledF {
-  __host__ double bytes() const { return 4.0; }
   float *p[6];
   double scale[6];
   int n;
@@ -521,14 +514,12 @@ struct StoreScaledF {
 
 // Load qq + kdsq*pp (adapt, evolution.f90:541-547).
 struct LoadVort {
-  __host__ double bytes() const { return btropic ? 8.0 : 16.0; }
   const double *qq, *pp;
   double kdsq;
   int btropic, n;
-  long long ms = 0;  // ensemble: entry b = member b, fields ms apart
   // first pass of an inverse transform: vector v = ky, element j = kx
-  __device__ __forceinline__ double operator()(int b, int v, int j) const {
-    long long k = (long long)b * ms + (long long)v * n + j;
+  __device__ __forceinline__ double operator()(int, int v, int j) const {
+    long long k = (long long)v * n + j;
     return btropic ? qq[k] : qq[k] + kdsq * pp[k];
   }
 };
@@ -1012,11 +1003,14 @@ int con2grid_dev(casl_handle *h, bool want_levels) {
     unsigned long long *JW = reinterpret_cast<unsigned long long *>(h->fineJ);
     const C2GMembers mb{h->M > 1 ? h->mnode : nullptr, h->M, (long long)c.nxf * n, c.nxf,
                         (int)(sizeof(Scalars) / 8)};
-    {
+    // zero words and bottom jumps: inside a step the stage that used them
+    // last has cleared them (k_fs_cols)
+    if (h->jw_dirty) {
       const FillJob z[2] = {{JW, 2LL * c.nxf * n * h->M, 0u},
                             {h->ljx, (long long)c.nxf * h->M, 0u}};
       if (int rc = fill_words(h->stream, z, 2)) return rc;
     }
+    h->jw_dirty = 1;
     // with no nodes the scatter still runs (its first block clears the sums)
     CASL_K(k_c2g_scatter<true>, grid_for(h->nptq > 0 ? h->nptq : 1), 256, 0, h->stream)(
         h->xq, h->yq, h->nextq, h->scal, nullptr, JW, h->ljx, c, err, csum, mb);
@@ -1036,6 +1030,7 @@ int con2grid_dev(casl_handle *h, bool want_levels) {
   // the fine-grid levels themselves are wanted: crossings onto the fine
   // grid, bottom row, scan in place, then coarsen
   size_t fine = (size_t)c.nxf * c.nyf;
+  h->jw_dirty = 1;
   CASL_CUDA_TRY(cudaMemsetAsync(h->fineJ, 0, fine * sizeof(int), h->stream));
   CASL_CUDA_TRY(cudaMemsetAsync(h->ljx, 0, (size_t)c.nxf * sizeof(int), h->stream));
   if (h->nptq > 0) {
@@ -1212,18 +1207,11 @@ __global__ void k_combine(double *__restrict__ qs, double *__restrict__ qd,
 // adapt (evolution.f90:524-608): deterministic two-level reductions
 // ---------------------------------------------------------------------------
 #define RED_BLOCKS 296
-template <class T>
-__global__ void k_reduce_adapt(const double *__restrict__ zz, const T *__restrict__ uu,
-                               const T *__restrict__ vv, double *__restrict__ part,
+#define MAX_PARTS 512  // adapt's partials: one per k_fs_prod block, n/4 of them at n = 2048
+__global__ void k_reduce_adapt(const double *__restrict__ zz, const float *__restrict__ uu,
+                               const float *__restrict__ vv, double *__restrict__ part,
                                long long nn) {
   CASL_PDL_ENTRY();
-  {  // ensemble member blockIdx.y: its fields and its gridDim.x partials
-    const long long m = blockIdx.y;
-    zz += m * nn;
-    uu += m * nn;
-    vv += m * nn;
-    part += m * 3 * gridDim.x;
-  }
   double sum = 0.0, zmax = 0.0, umax = 0.0;
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < nn;
        k += (long long)gridDim.x * blockDim.x) {
@@ -1305,14 +1293,12 @@ __global__ void k_adapt_final(const double *__restrict__ part, int nparts, Scala
 }
 
 __global__ void k_epq(const double *__restrict__ qdiss, double *__restrict__ epq,
-                      double *__restrict__ emq, const Scalars *__restrict__ s, long long nn,
-                      long long tot) {
+                      double *__restrict__ emq, const Scalars *__restrict__ s, long long nn) {
   CASL_PDL_ENTRY();
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < tot;
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < nn;
        k += (long long)gridDim.x * blockDim.x) {
-    const Scalars &sm = s[k / nn];  // ensemble member of element k
-    const double dfac = sm.dt2 * sm.zzrms;
-    double e = exp(dfac * qdiss[k & (nn - 1)]);
+    const double dfac = s->dt2 * s->zzrms;
+    double e = exp(dfac * qdiss[k]);
     epq[k] = e;
     emq[k] = 1.0 / e;
   }
@@ -1325,17 +1311,15 @@ __device__ __forceinline__ void spec_rk_body(int bid, int nbk, double *__restric
                           double *__restrict__ qsi, double *__restrict__ qsf,
                           double *__restrict__ qdi, double *__restrict__ qdf,
                           const double *__restrict__ sqs, const double *__restrict__ sqd,
-                          double *__restrict__ emq, const Scalars *__restrict__ s, long long nn,
-                          long long tot) {
+                          double *__restrict__ emq, const Scalars *__restrict__ s, long long nn) {
   auto L = [](const double *p, long long k) { return *reinterpret_cast<const double2 *>(p + k); };
   auto S = [](double *p, long long k, double x, double y) {
     *reinterpret_cast<double2 *>(p + k) = make_double2(x, y);
   };
-  for (long long k2 = bid * (long long)blockDim.x + threadIdx.x; k2 < tot / 2;
+  for (long long k2 = bid * (long long)blockDim.x + threadIdx.x; k2 < nn / 2;
        k2 += (long long)nbk * blockDim.x) {
     const long long k = 2 * k2;
-    const Scalars &sm = s[tot == nn ? 0 : k / nn];  // ensemble member of element k
-    const double dt = sm.dt, dt2 = sm.dt2, dt3 = sm.dt3, dt6 = sm.dt6;
+    const double dt = s->dt, dt2 = s->dt2, dt3 = s->dt3, dt6 = s->dt6;
     const double2 a = L(sqs, k), b = L(sqd, k);
     if (STAGE == 1) {
       const double2 si = L(qs, k), di = L(qd, k), e = L(emq, k);
@@ -1368,9 +1352,7 @@ __device__ __forceinline__ void spec_rk_body(int bid, int nbk, double *__restric
   }
 }
 
-// The end of an RK4 stage in one launch: blocks below nbn move the nodes
-// (velint + node update), the rest update the spectral fields; the two
-// parts touch disjoint data and read only dt from the scalars.
+// The node update's arguments.
 template <class T>
 struct NodeRkArgs {
   double *xq, *yq, *xqi, *yqi, *xqf, *yqf;
@@ -1379,14 +1361,17 @@ struct NodeRkArgs {
   int M;
   const double *du, *dv;  // learned closure: correction at every node (nullable)
 };
+// The end of an RK4 stage in the FP32-inversion mode, one launch: blocks below
+// nbn move the nodes (velint + node update), the rest update the spectral
+// fields; the two parts touch disjoint data and read only dt from the scalars.
 struct SpecRkArgs {
   double *qs, *qd, *qsi, *qsf, *qdi, *qdf;
   const double *sqs, *sqd;
   double *emq;
-  long long nn, tot;  // tot = M*nn
+  long long nn;
 };
-template <int STAGE, class T>
-__global__ void k_stage_rk(NodeRkArgs<T> a, SpecRkArgs b, Scalars *__restrict__ s, Consts c,
+template <int STAGE>
+__global__ void k_stage_rk(NodeRkArgs<float> a, SpecRkArgs b, Scalars *__restrict__ s, Consts c,
                            int nbn) {
   CASL_PDL_ENTRY();
   // the half-step time advance that opens stages 2 and 4 (nothing reads t
@@ -1394,13 +1379,18 @@ __global__ void k_stage_rk(NodeRkArgs<T> a, SpecRkArgs b, Scalars *__restrict__ 
   if ((STAGE == 1 || STAGE == 3) && blockIdx.x == 0)
     for (int m = threadIdx.x; m < a.M; m += blockDim.x) s[m].t = s[m].t + s[m].dt2;
   if ((int)blockIdx.x < nbn)
-    nodes_rk_body<STAGE, T>(blockIdx.x, nbn, a.xq, a.yq, a.xqi, a.yqi, a.xqf, a.yqf, a.uu, a.vv, s, c,
+    nodes_rk_body<STAGE, float>(blockIdx.x, nbn, a.xq, a.yq, a.xqi, a.yqi, a.xqf, a.yqf, a.uu, a.vv, s, c,
                             a.mnode, a.M, a.du, a.dv);
   else
     spec_rk_body<STAGE>(blockIdx.x - nbn, gridDim.x - nbn, b.qs, b.qd, b.qsi, b.qsf, b.qdi,
-                        b.qdf, b.sqs, b.sqd, b.emq, s, b.nn, b.tot);
+                        b.qdf, b.sqs, b.sqd, b.emq, s, b.nn);
 }
 
+}  // namespace casl
+
+#include "stage.cuh"
+
+namespace casl {
 
 __global__ void k_twist_sub(Scalars *s, double twistmax, int M) {
   CASL_PDL_ENTRY();
@@ -1478,48 +1468,27 @@ static int main_invert_dev(casl_handle *h) {
   return h->M > 1 ? main_invert_t<true>(h) : main_invert_t<false>(h);
 }
 
-// main_invert and the four gradients of source (evolution.f90:432-490,
-// spectral.f90:304-366) as one batch-6 inverse transform pair: vv, uu from
-// green*qq, and the x/y derivatives of qd (into w[4], w[5]) and of qs (into
-// sqs, sqd, as scratch for the advection products).  One batch of six fills
-// the SMs better than a batch of two beside a batch of four.  Scratch:
-// gtmp (6 fields).
-template <bool MB>
-static int invert_and_gradients_t(casl_handle *h) {
-  long long nn = (long long)h->n * h->n, n = h->n;
-  const int M = h->M;  // ensemble: six entries per member
-  LoadDerivT<MB> ld{};
-  const double *src[6] = {h->qq, h->qq, h->qd, h->qd, h->qs, h->qs};
-  for (int b = 0; b < 6; b++) {
-    ld.f[b] = src[b];
-    ld.dir[b] = b & 1;
-    ld.wg[b] = b < 2;
-  }
-  ld.green = h->green; ld.hrkx = h->hrkx; ld.hrky = h->hrky; ld.n = h->n;
-  ld.err = &h->scal->error;
-  ld.nb = 6; ld.ms = nn;
-  double *tmp = h->gtmp;  // 6M contiguous fields
-  int rc = RFFT_DISPATCH(false, false, false, ld, (StoreStrided{tmp, nn, n, 1}), 6 * M);
+int inversion_dev(casl_handle *h) {
+  int rc = inversion_qq(h, false);
   if (rc) return rc;
-  LoadBatchT<MB> lb{};
-  for (int b = 0; b < 6; b++) lb.p[b] = tmp + b * nn;
-  lb.vs = 1; lb.es = n;
-  lb.nb = 6; lb.ms = 6 * nn;
-  StoreScaledT<MB> st{};
-  double *dst[6] = {h->vv, h->uu, h->w[4], h->w[5], h->sqs, h->sqd};
-  for (int b = 0; b < 6; b++) {
-    st.p[b] = dst[b];
-    st.scale[b] = b == 1 ? -1.0 : 1.0;
-  }
-  st.n = h->n;
-  st.nb = 6; st.ms = nn;
-  return RFFT_DISPATCH(false, true, false, lb, st, 6 * M);
-}
-static int invert_and_gradients(casl_handle *h) {
-  return h->M > 1 ? invert_and_gradients_t<true>(h) : invert_and_gradients_t<false>(h);
+  h->uv_fp32 = 0;
+  return main_invert_dev(h);
 }
 
-// The same batch-6 inverse pair with FP32 storage (CASL_PREC_FP32_INVERSION):
+
+// ---------------------------------------------------------------------------
+// The FP32-inversion mode's stage
+// ---------------------------------------------------------------------------
+// One launch per transform and axis, in the transforms' own order of
+// operations, rather than stage.cuh's.  Rounding the inverse transforms'
+// intermediate to FP32 turns a difference in the last FP64 bit into one of
+// 6e-8 wherever a value lies next to a rounding boundary; over five steps at
+// 2048^2 stage.cuh's order moved qd by 2.5e-9 (and the FP64 mode's by 1e-14),
+// so runs in this mode keep the order they have been made with.
+// main_invert and the four gradients of source (evolution.f90:432-490,
+// spectral.f90:304-366) as one batch-6 inverse transform pair with FP32
+// storage (CASL_PREC_FP32_INVERSION): u, v from green*qq and the x/y
+// derivatives of qd and qs;
 // the intermediate in gtmp as floats, the outputs in f32 = [u, v, dqd/dx,
 // dqd/dy, dqs/dx, dqs/dy].
 static int invert_and_gradients32(casl_handle *h) {
@@ -1550,127 +1519,224 @@ static int invert_and_gradients32(casl_handle *h) {
   return RFFT_DISPATCH(false, true, false, lb, st, 6);
 }
 
-int inversion_dev(casl_handle *h, bool reset) {
-  int rc = inversion_qq(h, reset);
-  if (rc) return rc;
-  h->uv_fp32 = 0;
-  return main_invert_dev(h);
-}
-
-static int adapt_dev(casl_handle *h) {
+static int adapt32(casl_handle *h) {
   long long nn = (long long)h->n * h->n, n = h->n;
-  const int M = h->M;  // ensemble: one entry, one reduction and one dt per member
   LoadVort lv{h->qq, h->pp, h->c.kdsq, h->c.btropic, h->n};
-  lv.ms = nn;
-  int rc = RFFT_DISPATCH(false, false, false, lv, (StoreStrided{h->w[0], nn, n, 1}), M);
+  int rc = RFFT_DISPATCH(false, false, false, lv, (StoreStrided{h->w[0], nn, n, 1}), 1);
   if (rc) return rc;
   rc = RFFT_DISPATCH(false, true, false, (LoadStrided{h->w[0], nn, 1, n}),
-                     (StoreStrided{h->w[1], nn, n, 1}), M);
+                     (StoreStrided{h->w[1], nn, n, 1}), 1);
   if (rc) return rc;
-  if (h->prec == CASL_PREC_FP32_INVERSION)
-    CASL_K(k_reduce_adapt<float>, RED_BLOCKS, 256, 0, h->stream)(h->w[1], h->f32, h->f32 + nn,
-                                                                 h->part, nn);
-  else
-    CASL_K(k_reduce_adapt<double>, dim3(RED_BLOCKS, M), 256, 0, h->stream)(h->w[1], h->uu, h->vv,
-                                                                           h->part, nn);
-  CASL_K(k_adapt_final, M, 256, 0, h->stream)(h->part, RED_BLOCKS, h->scal, h->c, h->p.fixed_dt);
-  CASL_K(k_epq, grid_for(M * nn), 256, 0, h->stream)(h->qdiss, h->epq, h->emq, h->scal, nn,
-                                                     M * nn);
+  CASL_K(k_reduce_adapt, RED_BLOCKS, 256, 0, h->stream)(h->w[1], h->f32, h->f32 + nn, h->part, nn);
+  CASL_K(k_adapt_final, 1, 256, 0, h->stream)(h->part, RED_BLOCKS, h->scal, h->c, h->p.fixed_dt);
+  CASL_K(k_epq, grid_for(nn), 256, 0, h->stream)(h->qdiss, h->epq, h->emq, h->scal, nn);
   return check_launch(h);
 }
 
-// source (evolution.f90:432-490) after its gradients (invert_and_gradients):
+// source (evolution.f90:432-490) after its gradients (invert_and_gradients32):
 // the advection products fused into ptospc's first pass, damping and the
 // integrating factor into its store.
-static int source_prod(casl_handle *h, int stage) {
+static int source32(casl_handle *h, int stage) {
   const int lev = stage == 1 ? 0 : (stage == 4 ? 2 : 1);
   long long nn = (long long)h->n * h->n, n = h->n;
   double *tmp = h->w[0];  // w[0..1]
   int rc;
   // products -> ptospc's first pass into tmp, its second pass with the source store
-  if (h->prec == CASL_PREC_FP32_INVERSION) {
-    const float *f = h->f32;
-    LoadAdvectT<float> la{};
-    la.uu = f; la.vv = f + nn;
-    la.fx[0] = f + 2 * nn; la.fy[0] = f + 3 * nn;
-    la.fx[1] = f + 4 * nn; la.fy[1] = f + 5 * nn;
-    la.betab[0] = 0.0; la.betab[1] = h->c.beffect ? h->c.beta : 0.0;
-    la.n = h->n;
-    rc = RFFT_DISPATCH(true, false, true, la, (StoreStrided{tmp, nn, 1, n}), 2);
-  } else {
-    LoadAdvect la{};
-    la.uu = h->uu; la.vv = h->vv;
-    la.fx[0] = h->w[4]; la.fy[0] = h->w[5];
-    la.fx[1] = h->sqs; la.fy[1] = h->sqd;
-    la.betab[0] = 0.0; la.betab[1] = h->c.beffect ? h->c.beta : 0.0;
-    la.n = h->n;
-    la.ms = nn;
-    // ensemble: two entries per member; tmp (w[0..1]) is 2M fields long
-    rc = RFFT_DISPATCH(true, false, true, la, (StoreStrided{tmp, nn, 1, n}), 2 * h->M);
-  }
+  const float *f = h->f32;
+  LoadAdvectF la{};
+  la.uu = f; la.vv = f + nn;
+  la.fx[0] = f + 2 * nn; la.fy[0] = f + 3 * nn;
+  la.fx[1] = f + 4 * nn; la.fy[1] = f + 5 * nn;
+  la.betab[0] = 0.0; la.betab[1] = h->c.beffect ? h->c.beta : 0.0;
+  la.n = h->n;
+  rc = RFFT_DISPATCH(true, false, true, la, (StoreStrided{tmp, nn, 1, n}), 2);
   if (rc) return rc;
   StoreSource ss{};
   ss.sqd = h->sqd; ss.sqs = h->sqs; ss.qq = h->qq; ss.pp = h->pp; ss.epq = h->epq;
   ss.rekman = h->p.rekman; ss.kdsq = h->c.kdsq; ss.therm = h->c.therm;
   ss.heating = h->c.heating; ss.friction = h->c.friction; ss.lev = lev; ss.n = h->n;
-  ss.ms = nn;
-  return RFFT_DISPATCH(true, false, false, (LoadRow{tmp, nn, n, (int)n, &h->scal->error}), ss, 2 * h->M);
+  return RFFT_DISPATCH(true, false, false, (LoadRow{tmp, nn, n, (int)n, &h->scal->error}), ss, 2);
 }
 
-}  // namespace casl
-
 // node update and spectral RK update of a stage, one launch; velint reads
-// the velocity fields u, v (FP64, or FP32 in the FP32-inversion mode)
-template <class T>
-static int stage_update(casl_handle *h, int stage, const T *u, const T *v, const double *du,
-                        const double *dv) {
-  const long long nn = (long long)h->n * h->n, tot = h->M * nn;
+// the FP32 velocity
+static int update32(casl_handle *h, int stage, const double *du, const double *dv) {
+  const long long nn = (long long)h->n * h->n;
   const int nbn = h->contex ? grid_for(h->nptq > 0 ? h->nptq : 1) : 0;
-  const int g = nbn + grid_for(tot / 2);
-  const NodeRkArgs<T> a{h->xq, h->yq, h->xqi, h->yqi, h->xqf, h->yqf, u, v,
-                        h->M > 1 ? h->mnode : nullptr, h->M, du, dv};
-  const SpecRkArgs b{h->qs, h->qd, h->qsi, h->qsf, h->qdi, h->qdf, h->sqs, h->sqd, h->emq,
-                     nn, tot};
+  const int g = nbn + grid_for(nn / 2);
+  const NodeRkArgs<float> a{h->xq, h->yq, h->xqi, h->yqi, h->xqf, h->yqf, h->f32, h->f32 + nn,
+                            nullptr, 1, du, dv};
+  const SpecRkArgs b{h->qs, h->qd, h->qsi, h->qsf, h->qdi, h->qdf, h->sqs, h->sqd, h->emq, nn};
   cudaStream_t st = h->stream;
   switch (stage) {
-    case 1: CASL_K((k_stage_rk<1, T>), g, 256, 0, st)(a, b, h->scal, h->c, nbn); break;
-    case 2: CASL_K((k_stage_rk<2, T>), g, 256, 0, st)(a, b, h->scal, h->c, nbn); break;
-    case 3: CASL_K((k_stage_rk<3, T>), g, 256, 0, st)(a, b, h->scal, h->c, nbn); break;
-    default: CASL_K((k_stage_rk<4, T>), g, 256, 0, st)(a, b, h->scal, h->c, nbn); break;
+    case 1: CASL_K(k_stage_rk<1>, g, 256, 0, st)(a, b, h->scal, h->c, nbn); break;
+    case 2: CASL_K(k_stage_rk<2>, g, 256, 0, st)(a, b, h->scal, h->c, nbn); break;
+    case 3: CASL_K(k_stage_rk<3>, g, 256, 0, st)(a, b, h->scal, h->c, nbn); break;
+    default: CASL_K(k_stage_rk<4>, g, 256, 0, st)(a, b, h->scal, h->c, nbn); break;
+  }
+  return check_launch(h);
+}
+static int stage32(casl_handle *h, int stage) {
+  int rc;
+  // stage 1: the reset inside the filter combination rewrites qs and qd
+  // before the gradients read them
+  if ((rc = inversion_qq(h, stage == 1))) return rc;
+  if ((rc = invert_and_gradients32(h))) return rc;
+  if (stage == 1 && (rc = adapt32(h))) return rc;
+  if ((rc = source32(h, stage))) return rc;
+  const double *du = nullptr, *dv = nullptr;
+  const long long nn = (long long)h->n * h->n;
+  if (h->closure && (rc = closure_stage32(h, h->f32, h->f32 + nn, &du, &dv))) return rc;
+  return update32(h, stage, du, dv);
+}
+
+// One launch of a stage kernel (stage.cuh); `bytes` > 0 counts it as a
+// transform pass of that many algorithmic bytes.
+template <auto KERN, class... A>
+static int fs_launch(casl_handle *h, const char *what, dim3 grid, int nt, size_t smem, double bytes,
+                     A... args) {
+  static std::atomic<unsigned long long> configured{0};  // per kernel, a bit per device
+  const unsigned long long bit = 1ULL << (h->device & 63);
+  if (smem > 48 * 1024 && !(configured.load() & bit)) {
+    CASL_CUDA_TRY(cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    configured.fetch_or(bit);
+  }
+  const bool prof = bytes > 0.0 && h->prof_class == CASL_PROF_FFT && h->prof_ev &&
+                    h->prof_n < CASL_PROF_MAX;
+  if (prof) cudaEventRecord(h->prof_ev[2 * h->prof_n], h->stream);
+  for (bool once = kt_begin(what, grid, nt, smem, h->stream); once; once = kt_end())
+    launch_of(KERN, grid, dim3(nt), smem, h->stream)(args...);
+  if (prof) {
+    cudaEventRecord(h->prof_ev[2 * h->prof_n + 1], h->stream);
+    h->prof_n++;
+    h->prof_bytes += bytes;
   }
   return check_launch(h);
 }
 
-// advance (evolution.f90:166-326): four RK4 stages, each con2grid + the
-// filter combination, the batched inversion + source gradients, (stage 1)
-// adapt, source, the node update and the spectral RK update.
-static int advance_dev(casl_handle *h) {
+// One RK4 stage after con2grid's integer part (evolution.f90:166-326): the
+// transforms, the filter combination, adapt in stage 1, the source terms, the
+// closure's correction and the update of fields and nodes.
+template <int LOGN, int STAGE>
+static int stage_t(casl_handle *h) {
+  constexpr int N = 1 << LOGN;
+  constexpr long long nn = (long long)N * N;
+  constexpr bool FIRST = STAGE == 1;
+  const int M = h->M;
+  const double field = 8.0 * (double)nn * M;  // a pass reads or writes half of 16 B per element
+  double *tqc = h->w[4], *tzz = h->w[5], *tp = h->w[0];
+  const int have = h->nptq > 0;
   int rc;
+  if (have) {
+    using C = FsCols<LOGN>;
+    LoadQC ld{h->coarseC, h->scal, h->c.beffect ? h->betac : nullptr, nn,
+              1.0 / (256.0 * (double)N * (double)N), N};
+    const int ncol = N / 4 / C::TPC;
+    ClearJob clr{reinterpret_cast<uint4 *>(h->fineJ), 2 * nn * M, h->ljx, (long long)h->c.nxf * M};
+    // enough blocks to keep the stores of two per SM in flight
+    const int extra = (int)std::max(1LL, std::min(2 * nn * M / (8 * C::NT), 296LL) / M);
+    rc = fs_launch<k_fs_cols<LOGN>>(h, "k_fs_cols", dim3(ncol + extra, M), C::NT, C::smem, field, ld,
+                                    tqc, (const double2 *)h->tw, ncol, clr);
+    if (rc) return rc;
+    h->jw_dirty = 0;
+  }
+  {
+    using R = FsRows<LOGN>;
+    FsRowArgs a{};
+    a.tqc = tqc;
+    a.qs = h->qs; a.qd = h->qd; a.qc = h->qc; a.qq = h->qq; a.pp = h->pp;
+    a.flo = h->flo; a.fhi = h->fhi; a.green = h->green; a.hrkx = h->hrkx; a.hrky = h->hrky;
+    a.t6 = h->gtmp;
+    a.tzz = tzz;
+    a.kdsq = h->c.kdsq;
+    a.btropic = h->c.btropic;
+    a.have = have;
+    // qc, qq and pp are the state's after a step (stage 4); stage 1's and the
+    // damping terms read them inside it
+    a.keep = STAGE == 1 || STAGE == 4 || h->c.heating || h->c.friction;
+    a.err = &h->scal->error;
+    rc = fs_launch<k_fs_rows<LOGN, FIRST>>(h, "k_fs_rows", dim3(N / 2 / R::P, M), R::NT, R::smem,
+                                              (FIRST ? 8 : 7) * field, a, (const double2 *)h->tw);
+    if (rc) return rc;
+  }
+  {
+    using P = FsProd<LOGN>;
+    FsProdArgs a{};
+    a.t6 = h->gtmp;
+    a.tzz = tzz;
+    a.uu = h->uu; a.vv = h->vv;
+    a.tp = tp;
+    a.part = h->part;
+    a.betab = h->c.beffect ? h->c.beta : 0.0;
+    a.err = &h->scal->error;
+    const int nb = N / 4 / P::TPC;
+    static_assert(N / 4 / P::TPC <= MAX_PARTS, "adapt's partials");
+    rc = fs_launch<k_fs_prod<LOGN, FIRST>>(h, "k_fs_prod", dim3(nb, M), P::NT, P::smem,
+                                              (FIRST ? 9 : 8) * field, a, (const double2 *)h->tw);
+    if (rc) return rc;
+    if (FIRST)
+      CASL_K(k_adapt_final, M, 256, 0, h->stream)(h->part, nb, h->scal, h->c, h->p.fixed_dt);
+  }
+  // the learned closure's correction at the nodes (null without it)
+  const double *du = nullptr, *dv = nullptr;
+  if (h->closure && (rc = closure_stage(h, &du, &dv))) return rc;
+  using E = FsEnd<LOGN>;
+  FsEndArgs a{};
+  a.tp = tp;
+  a.qs = h->qs; a.qd = h->qd; a.qsi = h->qsi; a.qsf = h->qsf; a.qdi = h->qdi; a.qdf = h->qdf;
+  a.emq = h->emq; a.epq = h->epq; a.qq = h->qq; a.pp = h->pp; a.qdiss = h->qdiss;
+  a.rekman = h->p.rekman; a.kdsq = h->c.kdsq; a.therm = h->c.therm;
+  a.heating = h->c.heating; a.friction = h->c.friction;
+  const NodeRkArgs<double> nd{h->xq, h->yq, h->xqi, h->yqi, h->xqf, h->yqf, h->uu, h->vv,
+                              M > 1 ? h->mnode : nullptr, M, du, dv};
+  const long long npt = h->contex ? (h->nptq > 0 ? h->nptq : 1) : 0;
+  // Nodes beyond what the row kernel's half occupancy holds at once move in a
+  // launch of their own at full occupancy
+  const bool apart = npt > FS_NODES_TOGETHER;
+  if (apart)
+    CASL_K(k_nodes_rk<STAGE>, grid_for(npt), 256, 0, h->stream)(nd, h->scal, h->c);
+  const int nbn = apart || !npt ? 0 : grid_for(npt, E::NT);
+  return fs_launch<k_fs_end<LOGN, STAGE>>(h, "k_fs_end", dim3(E::ROWB * M + nbn), E::NT, E::smem,
+                                             0.0, a, nd, h->scal, h->c, nbn, (const double2 *)h->tw);
+}
+template <int STAGE>
+static int stage_dispatch(casl_handle *h) {
+  switch (h->n) {
+    case 32: return stage_t<5, STAGE>(h);
+    case 64: return stage_t<6, STAGE>(h);
+    case 128: return stage_t<7, STAGE>(h);
+    case 256: return stage_t<8, STAGE>(h);
+    case 512: return stage_t<9, STAGE>(h);
+    case 1024: return stage_t<10, STAGE>(h);
+    case 2048: return stage_t<11, STAGE>(h);
+    default: return CASL_EINVAL;
+  }
+}
+
+}  // namespace casl
+
+// advance (evolution.f90:166-326): four RK4 stages, each con2grid and the
+// stage's spectral work and updates
+static int advance_dev(casl_handle *h) {
+  h->uv_fp32 = h->prec == CASL_PREC_FP32_INVERSION;
   Trace tr;
   tr.begin(h->stream, "advance");
   for (int stage = 1; stage <= 4; stage++) {
-    // stage 1: the reset inside the filter combination rewrites qs and qd
-    // before the gradients read them
-    if ((rc = inversion_qq(h, stage == 1))) return rc;
-    tr.point("con2grid+qq");
-    const bool f32 = h->prec == CASL_PREC_FP32_INVERSION;
-    if ((rc = f32 ? invert_and_gradients32(h) : invert_and_gradients(h))) return rc;
-    tr.point("invert");
-    if (stage == 1 && (rc = adapt_dev(h))) return rc;
-    if ((rc = source_prod(h, stage))) return rc;
-    tr.point("adapt+source");
-    // the learned closure's correction at the nodes (null without it)
-    const double *du = nullptr, *dv = nullptr;
-    if (f32) {
-      const long long nn = (long long)h->n * h->n;
-      const float *u = h->f32, *v = h->f32 + nn;
-      if (h->closure && (rc = closure_stage32(h, u, v, &du, &dv))) return rc;
-      if ((rc = stage_update<float>(h, stage, u, v, du, dv))) return rc;
+    int rc;
+    if (h->uv_fp32) {
+      rc = stage32(h, stage);
     } else {
-      if (h->closure && (rc = closure_stage(h, &du, &dv))) return rc;
-      if ((rc = stage_update<double>(h, stage, h->uu, h->vv, du, dv))) return rc;
+      if (h->nptq > 0 && (rc = con2grid_dev(h, false))) return rc;
+      tr.point("con2grid");
+      switch (stage) {
+        case 1: rc = stage_dispatch<1>(h); break;
+        case 2: rc = stage_dispatch<2>(h); break;
+        case 3: rc = stage_dispatch<3>(h); break;
+        default: rc = stage_dispatch<4>(h); break;
+      }
     }
-    tr.point("stage update");
+    if (rc) return rc;
+    tr.point("spectral + update");
     static const char *const names[4] = {"RK4 stage 1", "RK4 stage 2", "RK4 stage 3",
                                          "RK4 stage 4"};
     if ((rc = debug_check(h, names[stage - 1]))) return rc;
@@ -1730,7 +1796,7 @@ int judge_velocity(casl_handle *h, casl_handle *hf, double *uJ, double *vJ, doub
   const int npt = h->nptq, nq = h->nq;
   if (npt > hf->npm || nq > hf->nm) return CASL_ECAPACITY;
   // the coarse inversion: qq, qc (spectral), uu, vv of h
-  if ((rc = inversion_dev(h, false))) return rc;
+  if ((rc = inversion_dev(h))) return rc;
   if (uP && npt)
     CASL_K(k_velint, grid_for(npt), 256, 0, h->stream)(h->xq, h->yq, npt, h->uu, h->vv, uP, vP,
                                                      h->c);
@@ -2253,7 +2319,7 @@ static int alloc_all(casl_handle *h) {
   for (auto pp : cont) CASL_CUDA_TRY(cudaMalloc(pp, (size_t)nm * sizeof(int)));
   // per-member fields (M stacked), then the shared tables
   double **fields[] = {&h->qr, &h->qs, &h->qd, &h->qc, &h->qq, &h->pp, &h->uu, &h->vv, &h->emq,
-                       &h->epq, &h->qspre, &h->sqs, &h->sqd, &h->qsi, &h->qsf, &h->qdi, &h->qdf};
+                       &h->epq, &h->qspre, &h->qsi, &h->qsf, &h->qdi, &h->qdf};
   for (auto pp : fields) {
     CASL_CUDA_TRY(cudaMalloc(pp, (size_t)(M * nn) * sizeof(double)));
     CASL_CUDA_TRY(cudaMemset(*pp, 0, (size_t)(M * nn) * sizeof(double)));
@@ -2284,8 +2350,9 @@ static int alloc_all(casl_handle *h) {
   size_t fine = M == 1 ? (size_t)h->c.nxf * h->c.nyf : (size_t)(M * 8 * nn);
   CASL_CUDA_TRY(cudaMalloc(&h->fineJ, fine * sizeof(int)));
   CASL_CUDA_TRY(cudaMalloc(&h->ljx, (size_t)(M * h->c.nxf) * sizeof(int)));
+  h->jw_dirty = 1;
   CASL_CUDA_TRY(cudaMalloc(&h->coarseC, (size_t)(M * nn) * sizeof(int)));
-  CASL_CUDA_TRY(cudaMalloc(&h->part, (size_t)(3 * RED_BLOCKS * M) * sizeof(double)));
+  CASL_CUDA_TRY(cudaMalloc(&h->part, (size_t)(3 * MAX_PARTS * M) * sizeof(double)));
   CASL_CUDA_TRY(cudaMalloc(&h->scal, (size_t)M * sizeof(Scalars)));
   CASL_CUDA_TRY(cudaMemset(h->scal, 0, (size_t)M * sizeof(Scalars)));
   CASL_CUDA_TRY(cudaMallocHost(&h->hscal, (size_t)M * sizeof(Scalars)));
@@ -2306,7 +2373,7 @@ static int alloc_all(casl_handle *h) {
 static void free_all(casl_handle *h) {
   void *ptrs[] = {h->xq, h->yq, h->xqi, h->yqi, h->xqf, h->yqf, h->uq, h->vq, h->nextq, h->i1q,
                   h->i2q, h->npq, h->indq, h->qr, h->qs, h->qd, h->qc, h->qq, h->pp, h->uu,
-                  h->vv, h->emq, h->epq, h->qspre, h->sqs, h->sqd, h->qsi, h->qsf, h->qdi,
+                  h->vv, h->emq, h->epq, h->qspre, h->qsi, h->qsf, h->qdi,
                   h->qdf, h->green, h->flo, h->fhi, h->qdiss, h->w[0], h->hrkx, h->hrky,
                   h->bety, h->betac, h->tw, h->fineJ, h->ljx, h->coarseC, h->part, h->scal,
                   h->sx, h->sx2, h->sxe, h->shell_idx, h->shell_off, h->rkxf, h->rkyf, h->gtmp};
@@ -2414,6 +2481,8 @@ void casl_destroy(casl_handle *h) {
   forcing_release(h);
   ensemble_release(h);
   cudaFree(h->f32);
+  cudaFree(h->sqs);
+  cudaFree(h->sqd);
   free_all(h);
   if (h->prof_ev) {
     for (int i = 0; i < 2 * CASL_PROF_MAX; i++) cudaEventDestroy(h->prof_ev[i]);
@@ -2782,7 +2851,7 @@ int casl_gradient(casl_handle *h, const double *ff, double *ffx, double *ffy) {
 
 int casl_inversion(casl_handle *h) {
   if (!h) return CASL_EINVAL;
-  int rc = inversion_dev(h, false);
+  int rc = inversion_dev(h);
   if (rc) return rc;
   CASL_CUDA_TRY(cudaStreamSynchronize(h->stream));
   return sync_counts(h);
@@ -3003,10 +3072,17 @@ int casl_set_precision(casl_handle *h, int mode) {
   if (!h || (mode != CASL_PREC_FP64 && mode != CASL_PREC_FP32_INVERSION)) return CASL_EINVAL;
   if (h->M > 1 && mode != CASL_PREC_FP64) return CASL_EUNSUPPORTED;
   cudaSetDevice(h->device);
-  if (mode == CASL_PREC_FP32_INVERSION && !h->f32) {
+  if (mode == CASL_PREC_FP32_INVERSION && !h->sqd) {
+    cudaFree(h->f32);
+    cudaFree(h->sqs);
+    h->f32 = nullptr;
+    h->sqs = nullptr;
     const size_t bytes = (size_t)6 * h->n * h->n * sizeof(float);
     CASL_CUDA_TRY(cudaMalloc(&h->f32, bytes));
     CASL_CUDA_TRY(cudaMemset(h->f32, 0, bytes));
+    const size_t src = (size_t)h->n * h->n * sizeof(double);
+    CASL_CUDA_TRY(cudaMalloc(&h->sqs, src));
+    CASL_CUDA_TRY(cudaMalloc(&h->sqd, src));
   }
   h->prec = mode;
   return CASL_OK;

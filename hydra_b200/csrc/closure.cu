@@ -1375,7 +1375,7 @@ int casl_closure_correction(casl_handle *h, casl_net *net, double *du, double *d
   const int npt = h->nptq;
   if (npt == 0) return CASL_OK;
   if ((rc = casl::cs_grow(cs, npt))) return rc;
-  if ((rc = casl::inversion_dev(h, false))) return rc;  // con2grid writes the sub-cell levels
+  if ((rc = casl::inversion_dev(h))) return rc;  // con2grid writes the sub-cell levels
   if ((rc = casl::net_run_t<double>(h, net, h->uu, h->vv, false))) return rc;
   cudaStream_t st = h->stream;
   CASL_K(casl::net::k_corr_nodes, casl::gsz(npt), 256, 0, st)(h->xq, h->yq, npt, net->fout,
@@ -1396,7 +1396,7 @@ int casl_closure_features(casl_handle *h, casl_net *net, float *x) {
   cudaSetDevice(h->device);
   int rc;
   if (!casl::cs_get(h, &rc)) return rc;
-  if ((rc = casl::inversion_dev(h, false))) return rc;
+  if ((rc = casl::inversion_dev(h))) return rc;
   const long long nn = (long long)h->n * h->n;
   cudaStream_t st = h->stream;
   CASL_K(casl::net::k_features<double>, casl::gsz(nn), 256, 0, st)(

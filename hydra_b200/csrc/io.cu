@@ -456,7 +456,7 @@ int casl_savecont(casl_handle *h, const char *dir, int icrec) {
   const double t = h->hscal->t, qjump = h->hscal->qjump;
   cudaStream_t st = h->stream;
   // residual qq - qc after an inversion (evolution.f90:87, 749-751)
-  rc = inversion_dev(h, false);
+  rc = inversion_dev(h);
   if (rc) return rc;
   CASL_K(k_io_sub, 1184, 256, 0, st)(h->qq, h->qc, h->w[4], nn);
   rc = spctop_dev(h, h->w[4], h->w[5], h->w[0]);
@@ -584,7 +584,7 @@ int casl_savegrid(casl_handle *h, const char *dir, int irec) {
   rc = get_scalars(h);
   if (rc) return rc;
   const double t = h->hscal->t;
-  rc = inversion_dev(h, false);
+  rc = inversion_dev(h);
   if (rc) return rc;
   double diag[4];
   rc = casl_diagnostics(h, diag);  // energy (evolution.f90:612-644)
@@ -720,7 +720,7 @@ int saves_before_advance(casl_handle *h) {
   bool have = false;  // an inversion of this state and its energies in diag
   if (s->gpend) {
     if ((rc = io_join(h))) return rc;
-    if ((rc = inversion_dev(h, false))) return rc;
+    if ((rc = inversion_dev(h))) return rc;
     if ((rc = casl_diagnostics(h, diag))) return rc;
     have = true;
     // weights for time interpolation (evolution.f90:665-677)
@@ -744,7 +744,7 @@ int saves_before_advance(casl_handle *h) {
   s->snap = s->tgsave > 0.0 && t + dtmax >= s->tgrid;
   if (s->snap) {
     if (!have) {
-      if ((rc = inversion_dev(h, false))) return rc;
+      if ((rc = inversion_dev(h))) return rc;
       if ((rc = casl_diagnostics(h, diag))) return rc;
     }
     // qspre = qs after the reset, the same values as qq (evolution.f90:592)

@@ -38,7 +38,8 @@ struct casl_handle {
 
   // fields, n*n doubles each
   double *qr, *qs, *qd, *qc, *qq, *pp, *uu, *vv, *emq, *epq, *qspre;
-  double *sqs, *sqd, *qsi, *qsf, *qdi, *qdf;
+  double *qsi, *qsf, *qdi, *qdf;
+  double *sqs, *sqd;     // FP32-inversion mode: source terms, allocated with f32
   double *w[6];          // work fields
   // tables
   double *green, *flo, *fhi, *qdiss, *hrkx, *hrky, *bety, *betac;
@@ -53,6 +54,7 @@ struct casl_handle {
   // con2grid scratch
   int *fineJ;            // (nyf, nxf): row 0 = bottom level, rows 1.. = jump counts
   int *ljx;              // (nxf)
+  int jw_dirty;          // the packed jumps (or ljx) are not zero: clear before a scatter
   int *coarseC;          // (n*n) coarse integer cells
   // reductions
   double *part;          // per-block partials
@@ -126,7 +128,7 @@ int sync_counts(casl_handle *h);    // device counts -> host copies
 int debug_check(casl_handle *h, const char *phase);  // CASL_CHECK=1: node sanity after a phase
 int get_scalars(casl_handle *h);    // device scalars -> hscal
 int put_scalars(casl_handle *h);    // hscal -> device scalars
-int inversion_dev(casl_handle *h, bool reset);  // evolution.f90:494-520
+int inversion_dev(casl_handle *h);  // evolution.f90:494-520
 int evo_init(casl_handle *h);       // evolution.f90:96-131 (qc, qd, qspre)
 int spec1d_dev(casl_handle *h, const double *ss, double *dspec);
 void io_release(casl_handle *h);    // joins the output writer, frees its staging
