@@ -4,14 +4,13 @@
 //    (con2ugrid, congen.f90:338-441) plus the bilinear residual
 //    (congen.f90:45-61), or the bilinear field alone when there are no
 //    contours (congen.f90:63-95).
-// 2. Every grid-line crossing of every level is enumerated in the
-//    reference's numbering order (x lines: ix outer / iy inner, then y lines:
-//    iy outer / ix inner, congen.f90:200-254), then stably sorted by level.
-// 3. The per-box crossing tables (noctab/icrtab) become a hash on
-//    (level, box).  A crossing's successor is the out-crossing of the box it
-//    enters; only boxes with two out-crossings (saddles) depend on the order
-//    of the reference's traversal, so those few are resolved by a short
-//    exact simulation of that traversal over chains.
+// 2. Crossings are numbered by edge in the reference's order (x lines: ix outer
+//    / iy inner, then y lines: iy outer / ix inner, congen.f90:200-254), from
+//    per-edge counts, and contours are followed box by box inside tiles of
+//    the grid (trace.cuh); the pieces are linked and ranked.
+// 3. Only boxes with two out-crossings of a level (saddles) depend on the
+//    order of the reference's traversal, so those few are resolved by a short
+//    exact simulation of that traversal over the lists between them.
 // 4. Each contour starts at its lowest-numbered crossing (the reference's
 //    `free` loop); contours are ordered by level then by that crossing,
 //    gathered into walk order and renoded three times (congen.f90:295-310).
@@ -28,6 +27,7 @@
 #include <stdlib.h>
 
 #include <algorithm>
+#include <atomic>
 #include <vector>
 
 #include "renode.cuh"
@@ -296,142 +296,6 @@ __global__ void __launch_bounds__(256, 4) k_u_field(const int *__restrict__ L, c
 }
 
 // ---------------------------------------------------------------------------
-// Crossings
-// ---------------------------------------------------------------------------
-constexpr int EDGES_PER_THREAD = 16;
-
-// Crossings are counted and emitted per chunk of 16 consecutive edges in the
-// reference's numbering: x-line edges (ix, iy)-(ix, iy+1) are numbered
-// e = ix*nyu + iy, y-line edges (ix, iy)-(ix+1, iy) e = NE + iy*nxu + ix.
-// One CTA takes two tiles of CB = 16 columns x RB = 64 rows of level codes,
-// each staged in shared memory with the next row and column (periodic):
-// each column's 64 codes are 8 16-byte loads, so a tile with its halo is one
-// load per thread of its half of the CTA.  An edge whose ends have codes
-// ca, cb crosses exactly the levels min(ca, cb) < l <= max(ca, cb) (none
-// when they are equal, which takes in equal end values).  Each thread owns
-// one chunk of its tile (64 chunks of 16 rows of a column, then 64 chunks of
-// 16 columns of a row) and walks its 17 codes: COUNT writes the chunk's
-// number of crossings, EMIT writes its crossings (edge, level) from the
-// chunk's offset on, edge by edge and level by level, which is the
-// reference's order within a chunk.
-constexpr int CR_CB = 16, CR_RB = 64;
-
-template <bool EMIT>
-__global__ void __launch_bounds__(256) k_cr_tile(const unsigned short *__restrict__ lc, LevInfo li,
-                                                 int nxu, int nyu, int *__restrict__ cnt,
-                                                 const int *__restrict__ off,
-                                                 unsigned long long *__restrict__ redge,
-                                                 int *__restrict__ rlev) {
-  CASL_PDL_ENTRY();
-  __shared__ int Cl[2][CR_CB + 1][CR_RB + 1];  // row length 65
-  const int half = threadIdx.x >> 7, t = threadIdx.x & 127;
-  const int ntx = nxu / CR_CB, nty = nyu / CR_RB;
-  const long long tile = 2LL * blockIdx.x + half;
-  const bool live = tile < (long long)ntx * nty;
-  const int ix0 = live ? (int)(tile % ntx) * CR_CB : 0, iy0 = live ? (int)(tile / ntx) * CR_RB : 0;
-  int(*C)[CR_RB + 1] = Cl[half];
-  if (live) {
-    for (int q = t; q < (CR_CB + 1) * 9; q += 128) {
-      if (q < (CR_CB + 1) * 8) {  // 17 columns x 8 vectors of 8 codes
-        const int cc = q >> 3, part = q & 7;
-        int ix = ix0 + cc;
-        if (ix >= nxu) ix -= nxu;
-        const uint4 v = *reinterpret_cast<const uint4 *>(lc + (long long)ix * nyu + iy0 + 8 * part);
-        const unsigned int w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-          C[cc][8 * part + 2 * j] = (int)(w[j] & 0xffffu);
-          C[cc][8 * part + 2 * j + 1] = (int)(w[j] >> 16);
-        }
-      } else {  // the row after the tile, periodic
-        const int cc = q - (CR_CB + 1) * 8;
-        int ix = ix0 + cc, iy = iy0 + CR_RB;
-        if (ix >= nxu) ix -= nxu;
-        if (iy >= nyu) iy -= nyu;
-        C[cc][CR_RB] = lc[(long long)ix * nyu + iy];
-      }
-    }
-  }
-  __syncthreads();
-  if (!live) return;
-  const long long NE = (long long)nxu * nyu;
-  // chunk t: x-line chunks 0..63 (column t>>2, rows 16*(t&3)...), then
-  // y-line chunks 64..127 (row t-64, columns 0..15)
-  const bool xl = t < 64;
-  const int cc0 = xl ? t >> 2 : 0, r0 = xl ? 16 * (t & 3) : t - 64;
-  const long long e0 = xl ? (long long)(ix0 + cc0) * nyu + (iy0 + r0)
-                          : NE + (long long)(iy0 + r0) * nxu + ix0;
-  const long long chunk_id = e0 / EDGES_PER_THREAD;
-  int pos = EMIT ? off[chunk_id] : 0, total = 0;
-  int ca = xl ? C[cc0][r0] : C[0][r0];
-#pragma unroll 4
-  for (int i = 0; i < 16; i++) {
-    const int cb = xl ? C[cc0][r0 + i + 1] : C[i + 1][r0];
-    const int l1 = max(min(ca, cb) + 1, li.levbeg), l2 = min(max(ca, cb), li.levend);
-    if (!EMIT) {
-      total += l2 >= l1 ? l2 - l1 + 1 : 0;
-    } else {
-      for (int l = l1; l <= l2; l++) {
-        redge[pos] = (unsigned long long)(e0 + i);
-        rlev[pos] = l - li.levbeg;
-        pos++;
-      }
-    }
-    ca = cb;
-  }
-  if (!EMIT) cnt[chunk_id] = total;
-}
-
-// Position and box transitions of every crossing (congen.f90:211-252).
-// The end values are the ultra-fine field recomputed at the edge's two
-// points, bit for bit the values the level codes were taken from.
-__global__ void k_cr_geom(UField uf, const unsigned long long *__restrict__ redge,
-                          const int *__restrict__ rlev, long long ncr, LevInfo li, Consts c,
-                          double *__restrict__ xcr, double *__restrict__ ycr,
-                          unsigned int *__restrict__ kib, unsigned int *__restrict__ kob) {
-  CASL_PDL_ENTRY();
-  const int nxu = c.nxu, nyu = c.nyu;
-  const long long NE = (long long)nxu * nyu;
-  const double qavg = ufield_qavg(uf.lsum, uf.qjump, uf.have, nxu, nyu);
-  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < ncr;
-       r += (long long)gridDim.x * blockDim.x) {
-    long long e = (long long)redge[r];
-    double qtmp = qtmp_of(rlev[r] + li.levbeg, li);
-    if (e < NE) {
-      int ix = (int)(e / nyu) + 1, iy = (int)(e % nyu) + 1;
-      double q0 = ufield_at(uf, qavg, ix, iy, c) - qtmp;
-      double q1 = ufield_at(uf, qavg, ix, iy == nyu ? 1 : iy + 1, c) - qtmp;
-      int isy = (int)f_sign1(q0);
-      int inc = (1 - isy) / 2;
-      long long kaa = (long long)(iy - 1) * nxu + 1;
-      int j1 = ix + inc, j2 = ix + 1 - inc;
-      long long bx1 = j1 == 1 ? nxu - 1 : j1 - 2, bx2 = j2 == 1 ? nxu - 1 : j2 - 2;
-      kib[r] = (unsigned int)(kaa + bx1);
-      kob[r] = (unsigned int)(kaa + bx2);
-      xcr[r] = c.xmin + c.glxu * (double)(ix - 1);
-      double ygu = c.ymin + c.glyu * (double)(iy - 1);
-      double yy = ygu - c.glyu * q0 / (q1 - q0);
-      ycr[r] = c.oms * (yy - c.elly * f_dint(yy * c.hlyi));
-    } else {
-      long long f = e - NE;
-      int iy = (int)(f / nxu) + 1, ix = (int)(f % nxu) + 1;
-      double q0 = ufield_at(uf, qavg, ix, iy, c) - qtmp;
-      double q1 = ufield_at(uf, qavg, ix == nxu ? 1 : ix + 1, iy, c) - qtmp;
-      int isx = (int)f_sign1(q0);
-      int inc = (1 - isx) / 2;
-      int j1 = iy + 1 - inc, j2 = iy + inc;
-      long long by1 = j1 == 1 ? nyu - 1 : j1 - 2, by2 = j2 == 1 ? nyu - 1 : j2 - 2;
-      kib[r] = (unsigned int)((long long)nxu * by1 + ix);
-      kob[r] = (unsigned int)((long long)nxu * by2 + ix);
-      ycr[r] = c.ymin + c.glyu * (double)(iy - 1);
-      double xgu = c.xmin + c.glxu * (double)(ix - 1);
-      double xx = xgu - c.glxu * q0 / (q1 - q0);
-      xcr[r] = c.oms * (xx - c.ellx * f_dint(xx * c.hlxi));
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
 // beta != 0 (econgen.f90:27-488): the grid extended in y
 // ---------------------------------------------------------------------------
 // PV on a beta-plane is not periodic in y: the periodic image of row iy0 one
@@ -442,20 +306,10 @@ __global__ void k_cr_geom(UField uf, const unsigned long long *__restrict__ redg
 struct ExtGrid {
   int iymin, iymax, nby;       // nby: boxes below the basic one (econgen.f90:217)
   double bfac;
-  const unsigned short *lc;    // basic rows' level codes, [ix][iy]
-  const unsigned short *lcb;   // rows iymin..0, [ix][iy - iymin]
-  const unsigned short *lca;   // rows nyu+1..iymax, [ix][iy - nyu - 1]
 };
 __device__ __forceinline__ int ext_row0(const ExtGrid &g, int iy, int nyu) {
   return iy < 1 ? 1 + (g.nby * nyu + iy - 1) % nyu : (iy > nyu ? 1 + (iy - 1) % nyu : iy);
 }
-// level code of the 1-based point (ix, iy) of the extended grid
-__device__ __forceinline__ int ext_code(const ExtGrid &g, int ix, int iy, int nyu) {
-  if (iy < 1) return g.lcb[(long long)(ix - 1) * (1 - g.iymin) + (iy - g.iymin)];
-  if (iy > nyu) return g.lca[(long long)(ix - 1) * (g.iymax - nyu) + (iy - nyu - 1)];
-  return g.lc[(long long)(ix - 1) * nyu + iy - 1];
-}
-
 // Minimum and maximum of the field along every basic row (econgen.f90:
 // 114-129): one block per 16 rows, threads over the columns.
 __global__ void __launch_bounds__(256) k_u_rowmm(UField uf, Consts c, double *__restrict__ rmin,
@@ -504,144 +358,52 @@ __global__ void __launch_bounds__(256) k_u_rowmm(UField uf, Consts c, double *__
   }
 }
 
-// Level codes of the extension rows: the level index of qa(iy0) +
-// bfac*(iy - iy0), the value rounded once as the reference's x-line scan
-// forms it (econgen.f90:247-258).
-__global__ void k_u_ext(UField uf, ExtGrid g, LevInfo li, Consts c, unsigned short *__restrict__ lcb,
-                        unsigned short *__restrict__ lca) {
+// Level codes of the extended grid, column by column (ld codes each), rows
+// iymin..iymax: the basic rows' codes, and in the extension the level index
+// of qa(iy0) + bfac*(iy - iy0), the value rounded once as the reference's
+// x-line scan forms it (econgen.f90:247-258).
+__global__ void k_u_ext(UField uf, ExtGrid g, LevInfo li, Consts c,
+                        const unsigned short *__restrict__ lc, long long ld,
+                        unsigned short *__restrict__ le) {
   CASL_PDL_ENTRY();
-  const int nxu = c.nxu, nyu = c.nyu;
-  const int nb = 1 - g.iymin, na = g.iymax - nyu, nr = nb + na;
+  const int nxu = c.nxu, nyu = c.nyu, nr = g.iymax - g.iymin + 1;
   const double qavg = ufield_qavg(uf.lsum, uf.qjump, uf.have, nxu, nyu);
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < (long long)nxu * nr;
        t += (long long)gridDim.x * blockDim.x) {
-    const int ix = (int)(t / nr) + 1, r = (int)(t % nr);
-    const int iy = r < nb ? g.iymin + r : nyu + 1 + (r - nb);
-    const int iy0 = ext_row0(g, iy, nyu);
-    const double v = ufield_at(uf, qavg, ix, iy0, c) + g.bfac * (double)(iy - iy0);
-    const unsigned short code = (unsigned short)min(max(level_index(v, li), 0), 65535);
-    if (r < nb) lcb[(long long)(ix - 1) * nb + r] = code;
-    else lca[(long long)(ix - 1) * na + (r - nb)] = code;
-  }
-}
-
-// Crossings of the extended grid, counted or emitted per chunk of 16 edges
-// in the reference's numbering (econgen.f90:238-348): x-line edges (ix, iy)
-// -(ix, iy+1) for iy = iymin..iymax-1, e = (ix-1)(nye-1) + iy - iymin; then
-// y-line edges (ix, iy)-(ix+1, iy) for iy = iymin+1..iymax-1,
-// e = NEX + (iy-iymin-1) nxu + ix-1.  An edge crosses the levels between its
-// ends' codes (the y lines of the extension use the same once-rounded
-// values; the reference adds (offset - qtmp) there, which can differ from
-// them only when qa lies within an ulp of a level).
-template <bool EMIT>
-__global__ void k_cre(ExtGrid g, LevInfo li, int nxu, int nyu, long long nedge, long long nex,
-                      int *__restrict__ cnt, const int *__restrict__ off,
-                      unsigned long long *__restrict__ redge, int *__restrict__ rlev) {
-  CASL_PDL_ENTRY();
-  const int nye = g.iymax - g.iymin + 1;
-  const long long nchunks = (nedge + EDGES_PER_THREAD - 1) / EDGES_PER_THREAD;
-  for (long long ch = blockIdx.x * (long long)blockDim.x + threadIdx.x; ch < nchunks;
-       ch += (long long)gridDim.x * blockDim.x) {
-    const long long e0 = ch * EDGES_PER_THREAD;
-    const long long e1 = e0 + EDGES_PER_THREAD < nedge ? e0 + EDGES_PER_THREAD : nedge;
-    int pos = EMIT ? off[ch] : 0, total = 0;
-    for (long long e = e0; e < e1; e++) {
-      int ca, cb;
-      if (e < nex) {
-        const int ix = (int)(e / (nye - 1)) + 1, iy = g.iymin + (int)(e % (nye - 1));
-        ca = ext_code(g, ix, iy, nyu);
-        cb = ext_code(g, ix, iy + 1, nyu);
-      } else {
-        const long long f = e - nex;
-        const int iy = g.iymin + 1 + (int)(f / nxu), ix = (int)(f % nxu) + 1;
-        ca = ext_code(g, ix, iy, nyu);
-        cb = ext_code(g, ix == nxu ? 1 : ix + 1, iy, nyu);
-      }
-      const int l1 = max(min(ca, cb) + 1, li.levbeg), l2 = min(max(ca, cb), li.levend);
-      if (!EMIT) {
-        total += l2 >= l1 ? l2 - l1 + 1 : 0;
-      } else {
-        for (int l = l1; l <= l2; l++) {
-          redge[pos] = (unsigned long long)e;
-          rlev[pos] = l - li.levbeg;
-          pos++;
-        }
-      }
-    }
-    if (!EMIT) cnt[ch] = total;
-  }
-}
-
-// Position and box transitions of every crossing of the extended grid
-// (econgen.f90:238-348): y is not folded here; boxes are numbered over the
-// extended grid, row by row from iymin (1-based, as the reference's).
-__global__ void k_cre_geom(UField uf, ExtGrid g, const unsigned long long *__restrict__ redge,
-                           const int *__restrict__ rlev, long long ncr, long long nex, LevInfo li,
-                           Consts c, double *__restrict__ xcr, double *__restrict__ ycr,
-                           unsigned int *__restrict__ kib, unsigned int *__restrict__ kob) {
-  CASL_PDL_ENTRY();
-  const int nxu = c.nxu, nyu = c.nyu, nye = g.iymax - g.iymin + 1;
-  const double qavg = ufield_qavg(uf.lsum, uf.qjump, uf.have, nxu, nyu);
-  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < ncr;
-       r += (long long)gridDim.x * blockDim.x) {
-    const long long e = (long long)redge[r];
-    const double qtmp = qtmp_of(rlev[r] + li.levbeg, li);
-    if (e < nex) {
-      const int ix = (int)(e / (nye - 1)) + 1, iy = g.iymin + (int)(e % (nye - 1));
-      double q[2];
-#pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const int yy = iy + h, y0 = ext_row0(g, yy, nyu);
-        const double v = (yy >= 1 && yy <= nyu)
-                             ? ufield_at(uf, qavg, ix, yy, c)
-                             : ufield_at(uf, qavg, ix, y0, c) + g.bfac * (double)(yy - y0);
-        q[h] = v - qtmp;
-      }
-      const int isy = (int)f_sign1(q[0]);
-      const int inc = (1 - isy) / 2;
-      const long long kaa = (long long)(iy - g.iymin) * nxu + 1;
-      const int j1 = ix + inc, j2 = ix + 1 - inc;
-      const long long bx1 = j1 == 1 ? nxu - 1 : j1 - 2, bx2 = j2 == 1 ? nxu - 1 : j2 - 2;
-      kib[r] = (unsigned int)(kaa + bx1);
-      kob[r] = (unsigned int)(kaa + bx2);
-      xcr[r] = c.xmin + c.glxu * (double)(ix - 1);
-      ycr[r] = (c.glyu * (double)(iy - 1) + c.ymin) - c.glyu * q[0] / (q[1] - q[0]);
+    const int ix = (int)(t / nr) + 1, r = (int)(t % nr), iy = g.iymin + r;
+    unsigned short code;
+    if (iy >= 1 && iy <= nyu) {
+      code = lc[(long long)(ix - 1) * nyu + iy - 1];
     } else {
-      const long long f = e - nex;
-      const int iy = g.iymin + 1 + (int)(f / nxu), ix = (int)(f % nxu) + 1;
-      const int y0 = ext_row0(g, iy, nyu);
-      const bool basic = iy >= 1 && iy <= nyu;
-      const double qadd = g.bfac * (double)(iy - y0) - qtmp;
-      double q[2];
-#pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const int xx = h == 0 ? ix : (ix == nxu ? 1 : ix + 1);
-        q[h] = basic ? ufield_at(uf, qavg, xx, iy, c) - qtmp : ufield_at(uf, qavg, xx, y0, c) + qadd;
-      }
-      const int isx = (int)f_sign1(q[0]);
-      const int inc = (1 - isx) / 2;
-      const long long kaa = (long long)(iy - 1 - g.iymin) * nxu + ix;
-      kib[r] = (unsigned int)(kaa + (long long)(1 - inc) * nxu);
-      kob[r] = (unsigned int)(kaa + (long long)inc * nxu);
-      ycr[r] = c.glyu * (double)(iy - 1) + c.ymin;
-      const double xgu = c.xmin + c.glxu * (double)(ix - 1);
-      const double xx = xgu - c.glxu * q[0] / (q[1] - q[0]);
-      xcr[r] = c.oms * (xx - c.ellx * f_dint(xx * c.hlxi));
+      const int iy0 = ext_row0(g, iy, nyu);
+      const double v = ufield_at(uf, qavg, ix, iy0, c) + g.bfac * (double)(iy - iy0);
+      code = (unsigned short)min(max(level_index(v, li), 0), 65535);
     }
+    le[(long long)(ix - 1) * ld + r] = code;
   }
 }
 
 // One periodic image per contour (econgen.f90:238-246): bit 0 of flags[k]
 // is set when a crossing of contour k lies below ymin, bit 1 when one lies
 // below ymax; k is kept when bit 0 is clear and bit 1 set.
+// (A contour's crossings are consecutive: a warp that lies in one contour
+// combines its bits, and bits already there are not set again; an atomic per
+// crossing took 435 us at 256^2, this 40.)
 __global__ void k_ec_flags(const double *__restrict__ yw, const int *__restrict__ cidw, long long N,
                            Consts c, int *__restrict__ flags) {
   CASL_PDL_ENTRY();
-  for (long long w = blockIdx.x * (long long)blockDim.x + threadIdx.x; w < N;
-       w += (long long)gridDim.x * blockDim.x) {
-    const double y = yw[w];
-    const int f = (y < c.ymin ? 1 : 0) | (y < c.ymax ? 2 : 0);
-    if (f) atomicOr(&flags[cidw[w]], f);
+  for (long long b = blockIdx.x * (long long)blockDim.x; b < N; b += (long long)gridDim.x * blockDim.x) {
+    const long long w = b + threadIdx.x;
+    const bool in = w < N;
+    const double y = in ? yw[w] : 0.0;
+    const int k = in ? cidw[w] : -1;
+    int f = in ? (y < c.ymin ? 1 : 0) | (y < c.ymax ? 2 : 0) : 0;
+    const int k0 = __shfl_sync(0xffffffffu, k, 0);
+    if (__all_sync(0xffffffffu, k == k0)) {
+      f = __reduce_or_sync(0xffffffffu, f);
+      if (threadIdx.x & 31) f = 0;
+    }
+    if (f && (__ldcg(&flags[k]) & f) != f) atomicOr(&flags[k], f);
   }
 }
 __global__ void k_ec_keep(const int *__restrict__ flags, const int *__restrict__ clen, int C,
@@ -686,211 +448,6 @@ __global__ void k_ec_contours(const int *__restrict__ clen, const int *__restric
   }
 }
 
-// ---------------------------------------------------------------------------
-// (level, box) -> out-crossings hash (the reference's noctab/icrtab)
-// ---------------------------------------------------------------------------
-constexpr unsigned long long HEMPTY = ~0ull;
-
-__device__ __forceinline__ unsigned long long hkey(int lev, unsigned int box) {
-  return ((unsigned long long)(unsigned int)lev << 32) | box;
-}
-__device__ __forceinline__ unsigned long long hmix(unsigned long long k) {
-  k ^= k >> 33;
-  k *= 0xff51afd7ed558ccdULL;
-  k ^= k >> 33;
-  k *= 0xc4ceb9fe1a85ec53ULL;
-  k ^= k >> 33;
-  return k;
-}
-
-// One bucket per (level, box) key: the key and its (at most two) out-
-// crossings share 16 bytes, so a probe touches one sector.  The two slots
-// are filled in arrival order; readers that need them ordered take min/max.
-struct __align__(16) HBucket {
-  unsigned long long key;
-  int s0, s1;
-};
-
-// Crossings [0, n) of a batch of consecutive levels; slots store the global
-// crossing index base + r.
-__global__ void k_h_insert(const int *__restrict__ rlev, const unsigned int *__restrict__ kob,
-                           long long n, int base, HBucket *__restrict__ hb,
-                           unsigned long long mask, int *__restrict__ err) {
-  CASL_PDL_ENTRY();
-  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < n;
-       r += (long long)gridDim.x * blockDim.x) {
-    unsigned long long k = hkey(rlev[r], kob[r]);
-    unsigned long long p = hmix(k) & mask;
-    const int slot = base + (int)r;
-    bool inserted = false;
-    for (unsigned long long probe = 0; probe <= mask; probe++) {
-      unsigned long long prev = atomicCAS(&hb[p].key, HEMPTY, k);
-      if (prev == HEMPTY || prev == k) {
-        if (atomicCAS(&hb[p].s0, -1, slot) != -1)
-          if (atomicCAS(&hb[p].s1, -1, slot) != -1) atomicExch(err, CASL_ECAPACITY);
-        inserted = true;
-        break;
-      }
-      p = (p + 1) & mask;
-    }
-    // a full table would leave this crossing out of the (level, box) table
-    if (!inserted) atomicExch(err, CASL_ECAPACITY);
-  }
-}
-
-// Successor of each crossing of the batch.  A crossing that enters a saddle
-// box (two out-crossings) gets succ = -1 and, in sadslot, the box's two
-// out-crossings packed as (lower << 32) | higher: the pair names the box
-// once the table has been reused for the next batch.  -1 elsewhere.
-__global__ void k_h_succ(const int *__restrict__ rlev, const unsigned int *__restrict__ kib,
-                         long long n, const HBucket *__restrict__ hb, unsigned long long mask,
-                         int *__restrict__ succ, long long *__restrict__ sadslot,
-                         int *__restrict__ err) {
-  CASL_PDL_ENTRY();
-  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < n;
-       r += (long long)gridDim.x * blockDim.x) {
-    const unsigned long long k = hkey(rlev[r], kib[r]);
-    unsigned long long p = hmix(k) & mask;
-    bool found = false;
-    HBucket v;
-    for (unsigned long long probe = 0; probe <= mask; probe++) {
-      v = hb[p];
-      if (v.key == k) {
-        found = true;
-        break;
-      }
-      if (v.key == HEMPTY) break;
-      p = (p + 1) & mask;
-    }
-    if (!found) {
-      atomicExch(err, CASL_EINVAL);
-      succ[r] = -1;
-      sadslot[r] = -1;
-      continue;
-    }
-    if (v.s1 < 0) {
-      succ[r] = v.s0;
-      sadslot[r] = -1;
-    } else {
-      succ[r] = -1;
-      sadslot[r] = (long long)(((unsigned long long)min(v.s0, v.s1) << 32) |
-                               (unsigned int)max(v.s0, v.s1));
-    }
-  }
-}
-
-// first crossing of each level (crossings are sorted by level); lstart[nlev] = n
-__global__ void k_lev_starts(const int *__restrict__ rlev, long long n, int nlev,
-                             long long *__restrict__ lstart) {
-  CASL_PDL_ENTRY();
-  for (int l = blockIdx.x * blockDim.x + threadIdx.x; l <= nlev; l += gridDim.x * blockDim.x) {
-    long long lo = 0, hi = n;
-    while (lo < hi) {
-      const long long mid = (lo + hi) >> 1;
-      if (rlev[mid] < l) lo = mid + 1; else hi = mid;
-    }
-    lstart[l] = lo;
-  }
-}
-
-// contour start flags and lengths for plain cycles (start = cycle minimum)
-__global__ void k_ct_plain(const int *__restrict__ lab, const int *__restrict__ term,
-                           const int *__restrict__ val, long long ncr, int *__restrict__ startf,
-                           int *__restrict__ clenr) {
-  CASL_PDL_ENTRY();
-  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < ncr;
-       r += (long long)gridDim.x * blockDim.x) {
-    bool st = !term[r] && lab[r] == (int)r;
-    startf[r] = st;
-    clenr[r] = st ? val[r] : 0;
-  }
-}
-
-// A crossing in walk layout: its position and contour in one 32-byte record,
-// so that the scattered store of each crossing fills one whole sector (a
-// partial sector costs a read of the sector as well); k_walk_split then
-// turns the records into the walk arrays with coalesced accesses.
-struct __align__(32) WalkRec {
-  double x, y;
-  int cid, pad[3];
-};
-__device__ __forceinline__ void put_rec(WalkRec *__restrict__ rec, long long pos, double x,
-                                        double y, int cid) {
-  double2 *p = reinterpret_cast<double2 *>(rec + pos);
-  p[0] = make_double2(x, y);
-  reinterpret_cast<int4 *>(p + 1)[0] = make_int4(cid, 0, 0, 0);
-}
-__global__ void k_walk_split(const WalkRec *__restrict__ rec, long long ncr,
-                             double *__restrict__ xw, double *__restrict__ yw,
-                             int *__restrict__ cidw) {
-  CASL_PDL_ENTRY();
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < ncr;
-       p += (long long)gridDim.x * blockDim.x) {
-    const double2 v = reinterpret_cast<const double2 *>(rec + p)[0];
-    xw[p] = v.x;
-    yw[p] = v.y;
-    cidw[p] = rec[p].cid;  // the contour of every walk position, for the first renode
-  }
-}
-
-// positions of plain-cycle crossings in walk layout
-__global__ void k_ct_gather_plain(const int *__restrict__ lab, const int *__restrict__ term,
-                                  const int *__restrict__ val, const int *__restrict__ cidx,
-                                  const int *__restrict__ coff, const int *__restrict__ clen,
-                                  const double *__restrict__ xcr, const double *__restrict__ ycr,
-                                  long long ncr, WalkRec *__restrict__ rec) {
-  CASL_PDL_ENTRY();
-  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < ncr;
-       r += (long long)gridDim.x * blockDim.x) {
-    if (term[r]) continue;
-    int s = lab[r];
-    int c = cidx[s];
-    long long pos = (long long)coff[c] + (clen[c] - val[r]);
-    put_rec(rec, pos, xcr[r], ycr[r], c);
-  }
-}
-
-// chain crossings: position from the per-chain placement of the simulation
-__global__ void k_ct_gather_chain(const int *__restrict__ term, const int *__restrict__ ep,
-                                  const int *__restrict__ val, const int *__restrict__ chain_of_end,
-                                  const long long *__restrict__ chpos, const int *__restrict__ chlen,
-                                  const int *__restrict__ chrot, const int *__restrict__ chclen,
-                                  const int *__restrict__ chcont, const double *__restrict__ xcr,
-                                  const double *__restrict__ ycr, long long ncr,
-                                  WalkRec *__restrict__ rec) {
-  CASL_PDL_ENTRY();
-  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < ncr;
-       r += (long long)gridDim.x * blockDim.x) {
-    if (!term[r]) continue;
-    int ch = chain_of_end[ep[r]];
-    if (ch < 0) continue;
-    int local = chlen[ch] - val[r];          // position from the chain start
-    long long pos;
-    int rot = chrot[ch];
-    if (rot < 0) {
-      pos = chpos[ch] + local;
-    } else {
-      // first chain of a contour started mid-chain at local index rot
-      int L = chclen[ch];
-      int rel = local >= rot ? local - rot : L - rot + local;
-      pos = chpos[ch] + rel;
-    }
-    put_rec(rec, pos, xcr[r], ycr[r], chcont[ch]);
-  }
-}
-
-__global__ void k_lev_of_contour(const int *__restrict__ startf, const int *__restrict__ rlev,
-                                 const int *__restrict__ cidx, long long ncr, LevInfo li,
-                                 int nlevm, int *__restrict__ clevt) {
-  CASL_PDL_ENTRY();
-  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < ncr;
-       r += (long long)gridDim.x * blockDim.x) {
-    if (!startf[r]) continue;
-    int lev = rlev[r] + li.levbeg;
-    clevt[cidx[r]] = lev - nlevm + (lev - 1) / nlevm - 1;
-  }
-}
-
 __global__ void k_set_counts2(Scalars *s, const int *cnt) {
   CASL_PDL_ENTRY();
   s->nq = cnt[0];
@@ -918,309 +475,11 @@ __global__ void k_out_links(const int *__restrict__ ocs, const int *__restrict__
 }
 
 
-// ---------------------------------------------------------------------------
-// List ranking of the crossing successor graph with splitters.
-// Splitters: every K-th crossing and every chain start (a crossing no one
-// points to); each walks its segment up to the next splitter.  Cycles that
-// hold no sampled crossing get every crossing as a splitter in a second
-// round.  Pointer jumping then runs on the (few) splitters only, and the
-// result expands back to: term (on a chain), lab (cycle minimum / chain
-// minimum at chain starts), val (cycles: crossings from here to the end of
-// the walk that starts at the cycle minimum; chains: to the chain end,
-// inclusive) and ep (chain end).
-// ---------------------------------------------------------------------------
-__global__ void k_sp_pred(const int *__restrict__ succ, long long N, int *__restrict__ pred) {
-  CASL_PDL_ENTRY();
-  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < N;
-       r += (long long)gridDim.x * blockDim.x) {
-    int s = succ[r];
-    if (s >= 0) pred[s] = (int)r;
-  }
-}
-// A walk step reads the next node's successor and splitter flag (sf, one
-// 8-byte load) and writes the node's (owner, offset) pair (own, one 8-byte
-// store): two random accesses per step.  isspl keeps the flags as a plain
-// array for the scan.  The sampled crossings are those whose index hashes
-// to 0 mod K, not every K-th index: along a contour the indices often step
-// by a constant (parallel contours put the same number of crossings in
-// every row), and an arithmetic sample can then miss a whole contour.  All
-// splitters (sampled ones and chain starts) are appended to xlist, so the
-// walks run one thread per splitter with no idle lanes.
-__device__ __forceinline__ unsigned int sp_hash(unsigned int x) {
-  x ^= x >> 16;
-  x *= 0x7feb352dU;
-  x ^= x >> 15;
-  x *= 0x846ca68bU;
-  x ^= x >> 16;
-  return x;
-}
-// Appends go through one atomic per block and tile of the crossings: the
-// block's flags are counted by ballots, so the list keeps index order within
-// a block.
-__device__ __forceinline__ void sp_append(bool f, int r, int *__restrict__ xlist,
-                                          int *__restrict__ nx, int *wtot, int *wbase) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const unsigned m = __ballot_sync(0xffffffffu, f);
-  if (lane == 0) wtot[w] = __popc(m);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int t = 0;
-    for (int i = 0; i < nw; i++) {
-      const int c = wtot[i];
-      wtot[i] = t;
-      t += c;
-    }
-    *wbase = t ? atomicAdd(nx, t) : 0;
-  }
-  __syncthreads();
-  if (f) xlist[*wbase + wtot[w] + __popc(m & ((1u << lane) - 1))] = r;
-  __syncthreads();
-}
-__global__ void k_sp_flag(const int *__restrict__ pred, const int *__restrict__ succ, long long N,
-                          int K, int *__restrict__ isspl, int2 *__restrict__ sf,
-                          int2 *__restrict__ own, int *__restrict__ xlist,
-                          int *__restrict__ nx) {
-  CASL_PDL_ENTRY();
-  __shared__ int wtot[32], wbase;
-  for (long long b0 = blockIdx.x * (long long)blockDim.x; b0 < N;
-       b0 += (long long)gridDim.x * blockDim.x) {
-    const long long r = b0 + threadIdx.x;
-    int f = 0;
-    if (r < N) {
-      f = sp_hash((unsigned int)r) % (unsigned int)K == 0 || pred[r] < 0;
-      isspl[r] = f;
-      sf[r] = make_int2(succ[r], f);
-      own[r] = make_int2(-1, 0);
-    }
-    sp_append(f != 0, (int)r, xlist, nx, wtot, &wbase);
-  }
-}
-// Walks from the splitters xlist[0 .. *nx) up to the next splitter, one
-// thread per splitter.  A walk longer than N steps (impossible for a
-// successor graph) sets err and ends.
-__global__ void k_sp_walk(const int2 *__restrict__ sf, long long N, const int *__restrict__ xlist,
-                          const int *__restrict__ nx, int2 *__restrict__ own,
-                          int *__restrict__ nexts_c, int *__restrict__ seglen_c,
-                          int *__restrict__ segmin_c, int *__restrict__ segend_c,
-                          int *__restrict__ err) {
-  CASL_PDL_ENTRY();
-  const int total = *nx;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-    const int s = xlist[t];
-    int v = s, k = 0, mn = s, nxt = -1;
-    own[s] = make_int2(s, 0);
-    int n = sf[s].x;
-    for (long long guard = 0; guard < N; guard++) {
-      if (n < 0) { nxt = -1; break; }
-      const int2 q = sf[n];  // successor and flag of the next node
-      if (q.y) { nxt = n; break; }
-      v = n;
-      n = q.x;
-      k++;
-      own[v] = make_int2(s, k);
-      mn = min(mn, v);
-      if (guard == N - 1) atomicExch(err, CASL_EINVAL);
-    }
-    nexts_c[s] = nxt;
-    seglen_c[s] = k + 1;
-    segmin_c[s] = mn;
-    segend_c[s] = v;
-  }
-}
-// crossings on cycles that hold no splitter: every one becomes a splitter
-// (its walk ends at once, the successor being one too)
-__global__ void k_sp_unowned(long long N, const int2 *__restrict__ own, int *__restrict__ isspl,
-                             int2 *__restrict__ sf, int *__restrict__ xlist,
-                             int *__restrict__ nx) {
-  CASL_PDL_ENTRY();
-  __shared__ int wtot[32], wbase;
-  for (long long b0 = blockIdx.x * (long long)blockDim.x; b0 < N;
-       b0 += (long long)gridDim.x * blockDim.x) {
-    const long long r = b0 + threadIdx.x;
-    bool f = false;
-    if (r < N && own[r].x < 0) {
-      f = true;
-      isspl[r] = 1;
-      sf[r].y = 1;
-    }
-    sp_append(f, (int)r, xlist, nx, wtot, &wbase);
-  }
-}
-__global__ void k_sp_compact(const int *__restrict__ isspl, const int *__restrict__ srank, long long N,
-                             const int *__restrict__ nexts_c, const int *__restrict__ seglen_c,
-                             const int *__restrict__ segmin_c, const int *__restrict__ segend_c,
-                             int *__restrict__ nexts, int *__restrict__ seglen,
-                             int *__restrict__ segmin, int *__restrict__ segend) {
-  CASL_PDL_ENTRY();
-  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < N;
-       r += (long long)gridDim.x * blockDim.x) {
-    if (!isspl[r]) continue;
-    int k = srank[r];
-    int nx = nexts_c[r];
-    nexts[k] = nx < 0 ? -1 : srank[nx];
-    seglen[k] = seglen_c[r];
-    segmin[k] = segmin_c[r];
-    segend[k] = segend_c[r];
-  }
-}
-// Pointer jumping over the splitters.  Each splitter's jump state is one
-// 16-byte record (next, minimum, terminal flag, last), so that a round
-// gathers two records (at next and at last) instead of four separate words.
-__global__ void k_sp_init(const int *__restrict__ nexts, const int *__restrict__ segmin, int S,
-                          int4 *__restrict__ J) {
-  CASL_PDL_ENTRY();
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < S; k += gridDim.x * blockDim.x) {
-    const int n = nexts[k];
-    J[k] = make_int4(n < 0 ? k : n, segmin[k], n < 0, n < 0 ? k : n);
-  }
-}
-__global__ void k_sp_jump1(const int4 *__restrict__ J, int S, int4 *__restrict__ J2) {
-  CASL_PDL_ENTRY();
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < S; k += gridDim.x * blockDim.x) {
-    const int4 a = J[k];
-    const int4 b = J[a.x];
-    J2[k] = make_int4(b.x, min(a.y, b.y), a.z | b.z, J[a.w].w);
-  }
-}
-// the jump results as the separate arrays the later passes read
-__global__ void k_sp_unpack1(const int4 *__restrict__ J, int S, int *__restrict__ mn,
-                             int *__restrict__ tm, int *__restrict__ lastp) {
-  CASL_PDL_ENTRY();
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < S; k += gridDim.x * blockDim.x) {
-    const int4 a = J[k];
-    mn[k] = a.y;
-    tm[k] = a.z;
-    lastp[k] = a.w;
-  }
-}
-// list for suffix sums: cycles are cut before the splitter holding the cycle
-// minimum; chains end at their last splitter
-// (link, suffix sum) of the suffix-sum jumps, one 16-byte record
-struct __align__(16) SlSuf {
-  long long suf;
-  int sl, pad;
-};
-__global__ void k_sp_list(const int *__restrict__ nexts, const int *__restrict__ mn,
-                          const int *__restrict__ tm, const int2 *__restrict__ own,
-                          const int *__restrict__ srank, const int *__restrict__ seglen, int S,
-                          SlSuf *__restrict__ L, int *__restrict__ head) {
-  CASL_PDL_ENTRY();
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < S; k += gridDim.x * blockDim.x) {
-    int n = nexts[k], sl;
-    if (tm[k]) {
-      sl = n;
-      head[k] = -1;
-    } else {
-      int h = srank[own[mn[k]].x];
-      head[k] = h;
-      sl = n == h ? -1 : n;
-    }
-    L[k] = SlSuf{(long long)seglen[k], sl, 0};
-  }
-}
-__global__ void k_sp_jump2(const SlSuf *__restrict__ L, int S, SlSuf *__restrict__ L2) {
-  CASL_PDL_ENTRY();
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < S; k += gridDim.x * blockDim.x) {
-    const SlSuf a = L[k];
-    if (a.sl >= 0) {
-      const SlSuf b = L[a.sl];
-      L2[k] = SlSuf{a.suf + b.suf, b.sl, 0};
-    } else {
-      L2[k] = a;
-    }
-  }
-}
-__global__ void k_sp_unpack2(const SlSuf *__restrict__ L, int S, long long *__restrict__ suf) {
-  CASL_PDL_ENTRY();
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < S; k += gridDim.x * blockDim.x)
-    suf[k] = L[k].suf;
-}
-__global__ void k_sp_expand(long long N, const int2 *__restrict__ own,
-                            const int *__restrict__ srank, const int *__restrict__ tm,
-                            const int *__restrict__ mn, const long long *__restrict__ suf,
-                            const int *__restrict__ head, const int *__restrict__ lastp,
-                            const int *__restrict__ segend, int *__restrict__ term,
-                            int *__restrict__ lab, int *__restrict__ val, int *__restrict__ ep) {
-  CASL_PDL_ENTRY();
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < N;
-       c += (long long)gridDim.x * blockDim.x) {
-    const int2 oc = own[c];
-    int k = srank[oc.x];
-    int o = oc.y;
-    if (tm[k]) {
-      term[c] = 1;
-      val[c] = (int)(suf[k] - o);
-      ep[c] = segend[lastp[k]];
-      lab[c] = o == 0 ? mn[k] : (int)c;
-    } else {
-      int m = mn[k];
-      long long L = suf[head[k]];
-      long long pos = (L - suf[k]) + o - own[m].y;
-      if (pos < 0) pos += L;
-      term[c] = 0;
-      val[c] = (int)(L - pos);
-      lab[c] = m;
-      ep[c] = (int)c;
-    }
-  }
-}
+}  // namespace casl
 
-// --- small device helpers for the saddle bookkeeping ------------------------
-__global__ void k_sd_endflag(const int *__restrict__ succ, long long ncr, int *__restrict__ flag) {
-  CASL_PDL_ENTRY();
-  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < ncr;
-       r += (long long)gridDim.x * blockDim.x)
-    flag[r] = succ[r] < 0;
-}
-__global__ void k_sd_compact(const int *__restrict__ flag, const int *__restrict__ pos,
-                             const long long *__restrict__ sadslot, long long ncr,
-                             int *__restrict__ oidx, long long *__restrict__ oslot) {
-  CASL_PDL_ENTRY();
-  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < ncr;
-       r += (long long)gridDim.x * blockDim.x)
-    if (flag[r]) {
-      oidx[pos[r]] = (int)r;
-      oslot[pos[r]] = sadslot[r];
-    }
-}
-__global__ void k_gather_i(const int *__restrict__ src, const int *__restrict__ idx, int m,
-                           int *__restrict__ dst) {
-  CASL_PDL_ENTRY();
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x)
-    dst[k] = src[idx[k]];
-}
-// three arrays gathered at the same indices: dst[j*m + k] = src_j[idx[k]]
-__global__ void k_gather3_i(const int *__restrict__ s0, const int *__restrict__ s1,
-                            const int *__restrict__ s2, const int *__restrict__ idx, int m,
-                            int *__restrict__ dst) {
-  CASL_PDL_ENTRY();
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x) {
-    const int i = idx[k];
-    dst[k] = s0[i];
-    dst[m + k] = s1[i];
-    dst[2 * m + k] = s2[i];
-  }
-}
-__global__ void k_ct_len(const int *__restrict__ startf, const int *__restrict__ clenr,
-                         const int *__restrict__ cidx, long long ncr, int *__restrict__ clen) {
-  CASL_PDL_ENTRY();
-  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < ncr;
-       r += (long long)gridDim.x * blockDim.x)
-    if (startf[r]) clen[cidx[r]] = clenr[r];
-}
-__global__ void k_chain_of_end(const int *__restrict__ ends, int nch, int *__restrict__ coe) {
-  CASL_PDL_ENTRY();
-  for (int ch = blockIdx.x * blockDim.x + threadIdx.x; ch < nch; ch += gridDim.x * blockDim.x)
-    coe[ends[ch]] = ch;
-}
-__global__ void k_set_starts(const int *__restrict__ st_idx, const int *__restrict__ st_len, int m,
-                             int *__restrict__ startf, int *__restrict__ clenr) {
-  CASL_PDL_ENTRY();
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x) {
-    startf[st_idx[k]] = 1;
-    clenr[st_idx[k]] = st_len[k];
-  }
-}
+#include "trace.cuh"
+
+namespace casl {
 
 static inline int gsz(long long work) {
   long long g = (work + 255) / 256;
@@ -1288,7 +547,7 @@ int recontour_dev(casl_handle *h, const double *qq) {
   }
   // Field memory: level codes + integer levels + per-chunk crossing counts;
   // kept for the whole call.
-  const long long nchunks_f = (2 * NU + EDGES_PER_THREAD - 1) / EDGES_PER_THREAD;
+  const long long nchunks_f = 2 * NU / 16;
   size_t need_field = (size_t)NU * 6 + (size_t)nchunks_f * 8 + (size_t)nxu * 4 +
                       (size_t)nyu * 16 + ((size_t)64 << 20);
   RC_TRY(ensure_scratch(h, need_field));
@@ -1374,7 +633,6 @@ int recontour_dev(casl_handle *h, const double *qq) {
     eg.iymax = iy;
     eg.nby = 1 - eg.iymin / nyu;
     eg.bfac = bfac;
-    eg.lc = lc;
     // box numbers of the extended grid are 32-bit
     if ((long long)nxu * (eg.iymax - eg.iymin + 2) >= (1LL << 32)) return CASL_ECAPACITY;
   }
@@ -1394,18 +652,28 @@ int recontour_dev(casl_handle *h, const double *qq) {
   const int nlev = li.levend - li.levbeg + 1;
 
   tr.point("levels");
-  // --- 3. crossings in reference order, stably sorted by level ----------------
-  // beta != 0: the extension rows' codes, then the extended grid's edges
+  // --- 3. crossings in reference order ----------------------------------------
+  // beta != 0: the extended grid's codes and edges
   const int nye = econ ? eg.iymax - eg.iymin + 1 : 0;
-  const long long nex = econ ? (long long)nxu * (nye - 1) : 0;
-  const long long NE2 = econ ? nex + (long long)nxu * (nye - 2) : 2 * NU;
-  const long long nchunks = (NE2 + EDGES_PER_THREAD - 1) / EDGES_PER_THREAD;
+  CrGrid cg{};
+  cg.nxu = nxu;
+  cg.periodic = !econ;
+  cg.nrow = econ ? nye : nyu;
+  cg.ner = cg.nbr = econ ? nye - 1 : nyu;
+  cg.nseg = (cg.ner + 15) / 16;
+  cg.ylo = econ ? 1 : 0;
+  cg.nyl = econ ? nye - 2 : nyu;
+  cg.ld = econ ? ((long long)nye + 255) / 256 * 256 : nyu;
+  cg.ncx = (long long)nxu * cg.nseg;
+  cg.cmin = li.levbeg - 1;
+  cg.cmax = li.levend;
+  cg.lc = lc;
+  const long long nchunks = cr_chunks(cg);
   int *ccnt, *coffs, *tmpi;
   if (econ) {
     // codes and chunk counts in a buffer of their own (the field arena is
     // sized before the extension is known)
-    const int nb = 1 - eg.iymin, na = eg.iymax - nyu;
-    const size_t bcodes = ((size_t)nxu * (nb + na) * 2 + 255) / 256 * 256;
+    const size_t bcodes = ((size_t)nxu * cg.ld * 2 + 255) / 256 * 256;
     const size_t need = bcodes + (size_t)nchunks * 8 + (size_t)(scan_tmp_elems(nchunks) + 4) * 4 +
                         ((size_t)1 << 20);
     if (h->sxe_bytes < need) {
@@ -1416,29 +684,24 @@ int recontour_dev(casl_handle *h, const double *qq) {
       h->sxe_bytes = need + need / 2;
     }
     Arena are{(char *)h->sxe, h->sxe_bytes, 0};
-    unsigned short *lcb = are.get<unsigned short>((long long)nxu * nb);
-    unsigned short *lca = are.get<unsigned short>((long long)nxu * na);
+    unsigned short *le = are.get<unsigned short>((size_t)nxu * cg.ld);
     ccnt = are.get<int>(nchunks);
-    coffs = are.get<int>(nchunks);
+    coffs = are.get<int>(nchunks + 1);
     tmpi = are.get<int>(scan_tmp_elems(nchunks) + 4);
     if (are.failed) return CASL_ENOMEM;
-    eg.lcb = lcb;
-    eg.lca = lca;
-    CASL_K(k_u_ext, gsz((long long)nxu * (nb + na)), 256, 0, st)(uf, eg, li, c, lcb, lca);
-    CASL_K(k_cre<false>, gsz(nchunks), 256, 0, st)(eg, li, nxu, nyu, NE2, nex, ccnt, nullptr,
-                                                   nullptr, nullptr);
+    cg.lc = le;
+    CASL_K(k_u_ext, gsz((long long)nxu * nye), 256, 0, st)(uf, eg, li, c, lc, cg.ld, le);
   } else {
     ccnt = ar.get<int>(nchunks);
-    coffs = ar.get<int>(nchunks);
+    coffs = ar.get<int>(nchunks + 1);
     tmpi = ar.get<int>(scan_tmp_elems(nchunks) + 4);
     if (ar.failed) return CASL_ENOMEM;
   }
-  const long long ntile = (long long)(nxu / CR_CB) * (nyu / CR_RB);
-  const int tgrid = (int)((ntile + 1) / 2);
-  if (!econ)
-    CASL_K(k_cr_tile<false>, tgrid, 256, 0, st)(lc, li, nxu, nyu, ccnt, nullptr, nullptr, nullptr);
+  CASL_K(k_cr_count, (int)((nxu / 128) * (cg.ld / 256)), 256, 0, st)(cg, ccnt);
   tr.point("cr_count");
   exclusive_scan<int>(st, ccnt, coffs, nchunks, tmpi, dtot);
+  // the offset after the last chunk
+  CASL_CUDA_TRY(cudaMemcpyAsync(coffs + nchunks, dtot, sizeof(int), cudaMemcpyDeviceToDevice, st));
   int ncr_i = 0;
   CASL_CUDA_TRY(cudaMemcpyAsync(&ncr_i, dtot, sizeof(int), cudaMemcpyDeviceToHost, st));
   CASL_CUDA_TRY(cudaStreamSynchronize(st));
@@ -1447,249 +710,120 @@ int recontour_dev(casl_handle *h, const double *qq) {
   if (ncr == 0) return set_empty();
   // Per-crossing storage lives in a second arena sized from the count, so
   // that the ultra-fine field in the first one is kept.
-  int endbit = 1;
-  while ((1 << endbit) < nlev + 1) endbit++;
-  size_t sort_bytes = 0;
-  cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, (int *)nullptr, (int *)nullptr,
-                                  (unsigned long long *)nullptr, (unsigned long long *)nullptr,
-                                  (int)ncr, 0, endbit, st);
   {
-    unsigned long long capb = 1;
-    while (capb < (unsigned long long)(2 * ncr)) capb <<= 1;
-    long long capn = std::max<long long>(ncr * 2, h->npm);
-    size_t need2 = (size_t)ncr * 640 + (size_t)capb * 16 + (size_t)capn * 32 + sort_bytes +
-                   ((size_t)64 << 20);
-    RC_TRY(ensure_scratch2(h, need2));
+    const long long capn = std::max<long long>(ncr * 2, h->npm);
+    RC_TRY(ensure_scratch2(h, (size_t)ncr * 448 + (size_t)capn * 32 + ((size_t)64 << 20)));
   }
   Arena ar2{(char *)h->sx2, h->sx2_bytes, 0};
-  unsigned long long *redge = ar2.get<unsigned long long>(ncr), *redge2 = ar2.get<unsigned long long>(ncr);
-  int *rlev = ar2.get<int>(ncr), *rlev2 = ar2.get<int>(ncr);
-  int *tmpi2 = ar2.get<int>(scan_tmp_elems(ncr) + 4);
-  void *sort_tmp = ar2.get<char>(sort_bytes + 16);
+  TrArgs ta{};
+  ta.g = cg;
+  ta.off = coffs;
+  ta.own = ar2.get<int2>(ncr);
+  ta.chain = ar2.get<int4>(ncr);
+  ta.clev = ar2.get<int>(ncr);
+  ta.eidx = ar2.get<int>(ncr);
+  ta.eslot = ar2.get<long long>(ncr);
+  ta.nchain = dtot + 2;
+  ta.nend = dtot + 3;
+  ta.cap = (int)ncr;
+  ta.err = &h->scal->error;
   if (ar2.failed) return CASL_ENOMEM;
   tr.point("cr_alloc");
-  if (econ)
-    CASL_K(k_cre<true>, gsz(nchunks), 256, 0, st)(eg, li, nxu, nyu, NE2, nex, nullptr, coffs,
-                                                  redge, rlev);
-  else
-    CASL_K(k_cr_tile<true>, tgrid, 256, 0, st)(lc, li, nxu, nyu, nullptr, coffs, redge, rlev);
-  tr.point("cr_emit");
-  CASL_CUDA_TRY(cub::DeviceRadixSort::SortPairs(sort_tmp, sort_bytes, rlev, rlev2, redge, redge2,
-                                                (int)ncr, 0, endbit, st));
-  std::swap(rlev, rlev2);
-  std::swap(redge, redge2);
-  tr.point("cr_sort");
-  double *xcr = ar2.get<double>(ncr), *ycr = ar2.get<double>(ncr);
-  unsigned int *kib = ar2.get<unsigned int>(ncr), *kob = ar2.get<unsigned int>(ncr);
-  if (ar2.failed) return CASL_ENOMEM;
-  if (econ)
-    CASL_K(k_cre_geom, gsz(ncr), 256, 0, st)(uf, eg, redge, rlev, ncr, nex, li, c, xcr, ycr, kib,
-                                             kob);
-  else
-    CASL_K(k_cr_geom, gsz(ncr), 256, 0, st)(uf, redge, rlev, ncr, li, c, xcr, ycr, kib, kob);
-  RC_TRY(check_launch(h));
-
-  tr.point("crossings");
-  // --- 4. box tables: hash (level, box) -> two out-crossing slots ------------
-  // Levels go through the table in batches of about HB_BATCH crossings (2M:
-  // a 64 MB table; 1M batches measured 20 % slower), so that the table (16
-  // bytes per bucket, load <= 1/2) stays in L2 while the
-  // batch's inserts and look-ups run; the keys carry the level, so a batch of
-  // several levels shares one table.  CASL_HASH_BATCH=<crossings> overrides
-  // the batch size (a test forces one level per batch with it).
-  long long HB_BATCH = 1 << 21;
-  if (const char *e = getenv("CASL_HASH_BATCH"))
-    if (atoll(e) > 0) HB_BATCH = atoll(e);
-  long long *lstart = ar2.get<long long>(nlev + 1);
-  if (ar2.failed) return CASL_ENOMEM;
-  std::vector<long long> hl(nlev + 1);
-  CASL_K(k_lev_starts, 1, 128, 0, st)(rlev, ncr, nlev, lstart);
-  CASL_CUDA_TRY(cudaMemcpyAsync(hl.data(), lstart, (nlev + 1) * sizeof(long long),
-                                cudaMemcpyDeviceToHost, st));
-  CASL_CUDA_TRY(cudaStreamSynchronize(st));
-  tr.point("hash_levels");
-  std::vector<std::pair<long long, long long>> batches;  // [r0, r1)
-  for (int l = 0; l < nlev;) {
-    int l2 = l + 1;
-    while (l2 < nlev && hl[l2 + 1] - hl[l] <= HB_BATCH) l2++;
-    batches.push_back({hl[l], hl[l2]});
-    l = l2;
+  // --- 4. contours followed inside tiles ----------------------------------------
+  {
+    const FillJob z[1] = {{ta.nchain, 2, 0u}};
+    RC_TRY(fill_words(st, z, 1));
   }
-  long long bmax = 0;
-  for (auto &b : batches) bmax = std::max(bmax, b.second - b.first);
-  unsigned long long cap = 1;
-  while (cap < (unsigned long long)(2 * bmax)) cap <<= 1;
-  HBucket *hb = ar2.get<HBucket>(cap);
-  int *succ = ar2.get<int>(ncr);
-  long long *sadslot = ar2.get<long long>(ncr);
-  if (ar2.failed) return CASL_ENOMEM;
-  for (auto &b : batches) {
-    const long long nb = b.second - b.first;
-    if (nb <= 0) continue;
-    unsigned long long cb = 1;
-    while (cb < (unsigned long long)(2 * nb)) cb <<= 1;
-    CASL_CUDA_TRY(cudaMemsetAsync(hb, 0xff, cb * sizeof(HBucket), st));  // empty key, slots -1
-    CASL_K(k_h_insert, gsz(nb), 256, 0, st)(rlev + b.first, kob + b.first, nb, (int)b.first, hb,
-                                           cb - 1, &h->scal->error);
-    CASL_K(k_h_succ, gsz(nb), 256, 0, st)(rlev + b.first, kib + b.first, nb, hb, cb - 1,
-                                         succ + b.first, sadslot + b.first, &h->scal->error);
+  const int ntile = (nxu / TX) * ((cg.nbr + TY - 1) / TY);
+  {
+    static std::atomic<unsigned long long> configured{0};  // a bit per device
+    const unsigned long long bit = 1ULL << (h->device & 63);
+    if (!(configured.load() & bit)) {
+      CASL_CUDA_TRY(cudaFuncSetAttribute(k_tr_walk, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)sizeof(TrSmem)));
+      configured.fetch_or(bit);
+    }
   }
+  CASL_K(k_tr_walk, ntile, TR_NT, sizeof(TrSmem), st)(ta);
   RC_TRY(check_launch(h));
+  int cnts[2] = {0, 0};
+  CASL_CUDA_TRY(cudaMemcpyAsync(cnts, ta.nchain, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
   RC_TRY(fetch_err(h));
-  if (tr.on)
-    fprintf(stderr, "[casl trace] hash: %zu level batches, table %llu buckets\n", batches.size(),
-            cap);
-
-  tr.point("hash");
-  // --- 5. list ranking over crossings (splitters) ------------------------------
-  int *lab = ar2.get<int>(ncr), *term = ar2.get<int>(ncr), *val = ar2.get<int>(ncr),
-      *ep = ar2.get<int>(ncr);
-  int *pred = ar2.get<int>(ncr), *isspl = ar2.get<int>(ncr), *srank = ar2.get<int>(ncr);
-  int2 *sf = ar2.get<int2>(ncr), *own = ar2.get<int2>(ncr);
-  int *nexts_c = ar2.get<int>(ncr), *seglen_c = ar2.get<int>(ncr), *segmin_c = ar2.get<int>(ncr),
-      *segend_c = ar2.get<int>(ncr);
-  if (ar2.failed) return CASL_ENOMEM;
-  int g = gsz(ncr);
-  CASL_CUDA_TRY(cudaMemsetAsync(pred, 0xff, ncr * sizeof(int), st));
-  CASL_K(k_sp_pred, g, 256, 0, st)(succ, ncr, pred);
-  tr.point("rk_pred");
-  // term and val are written only by the expansion at the end: until then
-  // they hold the lists of splitters
-  const int K = 16;
-  int *xl1 = term, *xl2 = val, *nx1 = dtot + 10, *nx2 = dtot + 11;
-  CASL_CUDA_TRY(cudaMemsetAsync(nx1, 0, 2 * sizeof(int), st));
-  CASL_K(k_sp_flag, g, 256, 0, st)(pred, succ, ncr, K, isspl, sf, own, xl1, nx1);
-  tr.point("rk_flag");
-  CASL_K(k_sp_walk, gsz(ncr / K + 1), 256, 0, st)(sf, ncr, xl1, nx1, own, nexts_c, seglen_c,
-                                                  segmin_c, segend_c, &h->scal->error);
-  tr.point("rk_walk1");
-  CASL_K(k_sp_unowned, g, 256, 0, st)(ncr, own, isspl, sf, xl2, nx2);
-  CASL_K(k_sp_walk, g, 256, 0, st)(sf, ncr, xl2, nx2, own, nexts_c, seglen_c, segmin_c,
-                                   segend_c, &h->scal->error);
-  tr.point("rk_walk2");
-  exclusive_scan<int>(st, isspl, srank, ncr, tmpi2, dtot + 6);
-  int S = 0;
-  CASL_CUDA_TRY(cudaMemcpyAsync(&S, dtot + 6, sizeof(int), cudaMemcpyDeviceToHost, st));
-  CASL_CUDA_TRY(cudaStreamSynchronize(st));
+  const int S = cnts[0], nends = cnts[1];
   if (S <= 0) return CASL_EINVAL;
-  int *nexts = ar2.get<int>(S), *seglen = ar2.get<int>(S), *segmin = ar2.get<int>(S),
-      *segend = ar2.get<int>(S);
-  int *smn = ar2.get<int>(S), *stm = ar2.get<int>(S), *slp = ar2.get<int>(S),
-      *shead = ar2.get<int>(S);
-  long long *ssuf = ar2.get<long long>(S);
+  if (tr.on)
+    fprintf(stderr, "[casl trace] tracing: %d chains, %.1f crossings each, %d saddle entries\n", S,
+            (double)ncr / S, nends);
+  tr.point("trace");
+  // --- 5. ranking over the chains -------------------------------------------------
+  int *nexts = ar2.get<int>(S), *head = ar2.get<int>(S), *cslot = ar2.get<int>(S);
   int4 *jA = ar2.get<int4>(S), *jB = ar2.get<int4>(S);
   SlSuf *lA = ar2.get<SlSuf>(S), *lB = ar2.get<SlSuf>(S);
+  const long long ccap = (long long)S + 2LL * nends;  // contours: cycles and those through saddles
+  unsigned long long *key = ar2.get<unsigned long long>(ccap), *key2 = ar2.get<unsigned long long>(ccap);
+  int *slot = ar2.get<int>(ccap), *slot2 = ar2.get<int>(ccap), *slen = ar2.get<int>(ccap);
   if (ar2.failed) return CASL_ENOMEM;
-  tr.point("rk_scan");
-  CASL_K(k_sp_compact, g, 256, 0, st)(isspl, srank, ncr, nexts_c, seglen_c, segmin_c, segend_c,
-                                      nexts, seglen, segmin, segend);
-  int gsS = gsz(S);
+  constexpr int MAXR = 18;  // 4^17 windows cover any int count of chains, and one launch to see it
+  int *flag = ar2.get<int>(2 * MAXR);
+  if (ar2.failed) return CASL_ENOMEM;
+  const int gsS = gsz(S);
   int rounds = 1;
-  while ((1LL << rounds) < S) rounds++;
+  while (rounds < MAXR - 1 && (1LL << (2 * rounds)) < S) rounds++;
   rounds++;
-  CASL_K(k_sp_init, gsS, 256, 0, st)(nexts, segmin, S, jA);
+  {
+    const FillJob z[2] = {{flag, 2 * MAXR, 0u}, {dtot + 4, 1, 0u}};
+    RC_TRY(fill_words(st, z, 2));
+  }
+  CASL_K(k_ch_init, gsS, 256, 0, st)(ta.chain, ta.own, S, nexts, jA, ta.err);
   for (int it = 0; it < rounds; it++) {
-    CASL_K(k_sp_jump1, gsS, 256, 0, st)(jA, S, jB);
+    CASL_K(k_ch_jump1, gsS, 256, 0, st)(jA, S, jB, it, flag);
     std::swap(jA, jB);
   }
-  CASL_K(k_sp_unpack1, gsS, 256, 0, st)(jA, S, smn, stm, slp);
-  CASL_K(k_sp_list, gsS, 256, 0, st)(nexts, smn, stm, own, srank, seglen, S, lA, shead);
+  CASL_K(k_ch_list, gsS, 256, 0, st)(nexts, jA, ta.own, ta.chain, S, lA, head);
   for (int it = 0; it < rounds; it++) {
-    CASL_K(k_sp_jump2, gsS, 256, 0, st)(lA, S, lB);
+    CASL_K(k_ch_jump2, gsS, 256, 0, st)(lA, S, lB, it, flag + MAXR);
     std::swap(lA, lB);
   }
-  CASL_K(k_sp_unpack2, gsS, 256, 0, st)(lA, S, ssuf);
-  tr.point("rk_jump");
-  CASL_K(k_sp_expand, g, 256, 0, st)(ncr, own, srank, stm, smn, ssuf, shead, slp, segend,
-                                     term, lab, val, ep);
+  CASL_K(k_ch_heads, gsS, 256, 0, st)(head, jA, lA, ta.clev, S, key, slot, slen, cslot, dtot + 4);
   RC_TRY(check_launch(h));
-  if (tr.on) {
-    std::vector<int> sl(S);
-    CASL_CUDA_TRY(cudaMemcpyAsync(sl.data(), seglen, S * sizeof(int), cudaMemcpyDeviceToHost, st));
-    CASL_CUDA_TRY(cudaStreamSynchronize(st));
-    long long tot = 0;
-    int mx = 0;
-    for (int x : sl) {
-      tot += x;
-      mx = std::max(mx, x);
-    }
-    fprintf(stderr, "[casl trace] ranking: %d splitters, %d jump rounds; segment length mean %.2f, max %d\n",
-            S, rounds, (double)tot / S, mx);
-  }
-
-  tr.point("rk_expand");
-  // --- 6. saddle chains: exact simulation of the reference traversal ----------
-  // Only the crossings entering saddle boxes and the chain starts come to the
-  // host; everything of size ncr stays on the device.
-  int *endflag = ar2.get<int>(ncr), *endpos = ar2.get<int>(ncr);
-  if (ar2.failed) return CASL_ENOMEM;
-  CASL_K(k_sd_endflag, g, 256, 0, st)(succ, ncr, endflag);
-  exclusive_scan<int>(st, endflag, endpos, ncr, tmpi2, dtot + 3);
-  int nends = 0;
-  CASL_CUDA_TRY(cudaMemcpyAsync(&nends, dtot + 3, sizeof(int), cudaMemcpyDeviceToHost, st));
-  CASL_CUDA_TRY(cudaStreamSynchronize(st));
-  // gather src[idx[k]] for a host index list
-  int *gidx = nullptr, *gout = nullptr;
-  long long gcap = 0;
-  auto gather = [&](const int *src, const std::vector<int> &idx, std::vector<int> &out) -> int {
-    int m = (int)idx.size();
-    out.assign(m, 0);
-    if (m == 0) return CASL_OK;
-    if (m > gcap) {
-      gidx = ar2.get<int>(m);
-      gout = ar2.get<int>(m);
-      gcap = m;
-      if (ar2.failed) return CASL_ENOMEM;
-    }
-    CASL_CUDA_TRY(cudaMemcpyAsync(gidx, idx.data(), m * sizeof(int), cudaMemcpyHostToDevice, st));
-    CASL_K(k_gather_i, gsz(m), 256, 0, st)(src, gidx, m, gout);
-    CASL_CUDA_TRY(cudaMemcpyAsync(out.data(), gout, m * sizeof(int), cudaMemcpyDeviceToHost, st));
-    CASL_CUDA_TRY(cudaStreamSynchronize(st));
-    return CASL_OK;
-  };
-  int nsad_contours = 0;
-  std::vector<int> sad_start;      // start crossing of each saddle contour
-  std::vector<int> sad_len;        // its length
-  std::vector<int> ch_end, ch_len, ch_rot, ch_clen, ch_cont;
-  std::vector<long long> ch_pos;   // position relative to the contour start (set later)
+  int C0 = 0;
+  std::vector<int> eidx(nends);
+  std::vector<long long> eslot(nends);
   if (nends > 0) {
-    int *d_eidx = ar2.get<int>(nends);
-    long long *d_eslot = ar2.get<long long>(nends);
-    if (ar2.failed) return CASL_ENOMEM;
-    CASL_K(k_sd_compact, g, 256, 0, st)(endflag, endpos, sadslot, ncr, d_eidx, d_eslot);
-    std::vector<int> eidx(nends);
-    std::vector<long long> eslot(nends);
-    CASL_CUDA_TRY(cudaMemcpyAsync(eidx.data(), d_eidx, nends * sizeof(int), cudaMemcpyDeviceToHost, st));
-    CASL_CUDA_TRY(cudaMemcpyAsync(eslot.data(), d_eslot, nends * sizeof(long long), cudaMemcpyDeviceToHost, st));
-    CASL_CUDA_TRY(cudaStreamSynchronize(st));
+    CASL_CUDA_TRY(cudaMemcpyAsync(eidx.data(), ta.eidx, nends * sizeof(int), cudaMemcpyDeviceToHost, st));
+    CASL_CUDA_TRY(cudaMemcpyAsync(eslot.data(), ta.eslot, nends * sizeof(long long), cudaMemcpyDeviceToHost, st));
+  }
+  CASL_CUDA_TRY(cudaMemcpyAsync(&C0, dtot + 4, sizeof(int), cudaMemcpyDeviceToHost, st));
+  RC_TRY(fetch_err(h));
+  tr.point("ranking");
+  // --- 6. lists between saddles: exact simulation of the reference traversal -------
+  // Only the crossings entering saddle boxes and the list starts come to the
+  // host; everything of size ncr stays on the device.
+  int nsad_contours = 0;
+  int *listof = nullptr, *d_ladd = nullptr, *d_lslot = nullptr;
+  if (nends > 0) {
     std::vector<long long> sad_p(eslot);
     std::sort(sad_p.begin(), sad_p.end());
     sad_p.erase(std::unique(sad_p.begin(), sad_p.end()), sad_p.end());
-    int nsb = (int)sad_p.size();
+    const int nsb = (int)sad_p.size();
     // each saddle box is named by its two out-crossings, lower index first
-    std::vector<int> slot2(2 * nsb);
+    std::vector<int> slot2h(2 * nsb);
     for (int b = 0; b < nsb; b++) {
-      slot2[2 * b] = (int)((unsigned long long)sad_p[b] >> 32);
-      slot2[2 * b + 1] = (int)((unsigned long long)sad_p[b] & 0xffffffffull);
+      slot2h[2 * b] = (int)((unsigned long long)sad_p[b] >> 32);
+      slot2h[2 * b + 1] = (int)((unsigned long long)sad_p[b] & 0xffffffffull);
     }
-    // chain starts (the saddle out-crossings) and their ends, lengths, minima
-    int nch = 2 * nsb;
-    std::vector<int> cstart(slot2), cend(nch), clen(nch), cmin(nch);
-    {
-      // ends, lengths and minima at the chain starts: one gather, one copy
-      int *d_idx = ar2.get<int>(nch), *d_out = ar2.get<int>(3LL * nch);
-      if (ar2.failed) return CASL_ENOMEM;
-      std::vector<int> h_out(3 * (size_t)nch);
-      CASL_CUDA_TRY(cudaMemcpyAsync(d_idx, cstart.data(), nch * sizeof(int), cudaMemcpyHostToDevice, st));
-      CASL_K(k_gather3_i, gsz(nch), 256, 0, st)(ep, val, lab, d_idx, nch, d_out);
-      CASL_CUDA_TRY(cudaMemcpyAsync(h_out.data(), d_out, h_out.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
-      CASL_CUDA_TRY(cudaStreamSynchronize(st));
-      std::copy(h_out.begin(), h_out.begin() + nch, cend.begin());
-      std::copy(h_out.begin() + nch, h_out.begin() + 2 * nch, clen.begin());
-      std::copy(h_out.begin() + 2 * nch, h_out.end(), cmin.begin());
-    }
-    std::vector<int> val_at_min;
-    RC_TRY(gather(val, cmin, val_at_min));
+    // list starts (the saddle out-crossings) and their ends, lengths, minima
+    const int nch = 2 * nsb;
+    std::vector<int> cstart(slot2h), q(6 * (size_t)nch);
+    int *d_idx = ar2.get<int>(nch), *d_out = ar2.get<int>(6LL * nch);
+    if (ar2.failed) return CASL_ENOMEM;
+    CASL_CUDA_TRY(cudaMemcpyAsync(d_idx, cstart.data(), nch * sizeof(int), cudaMemcpyHostToDevice, st));
+    CASL_K(k_ch_query, gsz(nch), 256, 0, st)(d_idx, nch, ta.own, jA, lA, ta.chain, ta.clev, d_out);
+    CASL_CUDA_TRY(cudaMemcpyAsync(q.data(), d_out, q.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
+    CASL_CUDA_TRY(cudaStreamSynchronize(st));
+    const int *cend = &q[0], *clen = &q[nch], *cmin = &q[2 * (size_t)nch],
+              *val_at_min = &q[3 * (size_t)nch], *clev = &q[4 * (size_t)nch],
+              *clast = &q[5 * (size_t)nch];
     std::vector<std::pair<int, int>> start2ch;
     for (int ch = 0; ch < nch; ch++) start2ch.push_back({cstart[ch], ch});
     std::sort(start2ch.begin(), start2ch.end());
@@ -1697,7 +831,7 @@ int recontour_dev(casl_handle *h, const double *qq) {
       auto it = std::lower_bound(start2ch.begin(), start2ch.end(), std::make_pair(s, -1));
       return (it != start2ch.end() && it->first == s) ? it->second : -1;
     };
-    // saddle box entered by each chain end
+    // saddle box entered by each list's end
     std::vector<std::pair<int, long long>> end_slot(nends);
     for (int k = 0; k < nends; k++) end_slot[k] = {eidx[k], eslot[k]};
     std::sort(end_slot.begin(), end_slot.end());
@@ -1709,122 +843,102 @@ int recontour_dev(casl_handle *h, const double *qq) {
     }
     std::vector<int> noc(nsb, 2);
     std::vector<char> used(nch, 0);
-    ch_end = cend;
-    ch_len = clen;
-    ch_rot.assign(nch, -1);
-    ch_clen.assign(nch, 0);
-    ch_cont.assign(nch, -1);
-    ch_pos.assign(nch, 0);
-    // chains in order of their smallest crossing: contour starts
+    std::vector<int> ladd(nch, 0), lslot(nch, -1);
+    std::vector<unsigned long long> skey;
+    std::vector<int> sslot, sad_len;
+    // lists in order of their smallest crossing: contour starts
     std::vector<int> order(nch);
     for (int k = 0; k < nch; k++) order[k] = k;
     std::sort(order.begin(), order.end(), [&](int a, int b) { return cmin[a] < cmin[b]; });
     for (int oc : order) {
       if (used[oc]) continue;
-      int icr = cmin[oc];            // the contour's first crossing
-      std::vector<int> seq;          // chains in traversal order
+      const int icr = cmin[oc];      // the contour's first crossing
+      std::vector<int> seq;          // lists in traversal order
       int ch = oc;
       used[ch] = 1;
       seq.push_back(ch);
       int guard = 0;
       while (true) {
-        int b = box_of_end[ch];
-        int k = noc[b];
+        const int b = box_of_end[ch];
+        const int k = noc[b];
         if (k < 1 || k > 2) return CASL_EINVAL;
-        int icrn = slot2[2 * b + k - 1];
+        const int icrn = slot2h[2 * b + k - 1];
         if (icrn == icr) break;      // closes at the start (no decrement)
         noc[b] = k - 1;
-        int nxt = chain_starting_at(icrn);
+        const int nxt = chain_starting_at(icrn);
         if (nxt < 0) return CASL_EINVAL;
-        if (nxt == oc) break;        // back into the first chain, which holds icr
+        if (nxt == oc) break;        // back into the first list, which holds icr
         if (used[nxt]) return CASL_EINVAL;
         used[nxt] = 1;
         seq.push_back(nxt);
         ch = nxt;
         if (++guard > nch + 2) return CASL_EINVAL;
       }
-      // lay out: first chain rotated to start at icr, then the others
+      // lay out: first list rotated to start at icr, its head wrapping to the
+      // end of the contour, then the others
       int L = 0;
-      for (int q : seq) L += clen[q];
-      int cont = nsad_contours++;
-      sad_start.push_back(icr);
+      for (int x : seq) L += clen[x];
+      const int at = C0 + nsad_contours++;
+      skey.push_back((unsigned long long)(unsigned)clev[oc] << 32 | (unsigned)icr);
+      sslot.push_back(at);
       sad_len.push_back(L);
-      int first = seq[0];
-      int rot = clen[first] - val_at_min[oc];  // local index of icr in its chain
-      ch_rot[first] = rot;
-      ch_clen[first] = clen[first];
-      ch_cont[first] = cont;
-      ch_pos[first] = 0;
-      long long off = clen[first] - rot;   // crossings from icr to the chain end
-      for (size_t q = 1; q < seq.size(); q++) {
-        ch_cont[seq[q]] = cont;
-        ch_pos[seq[q]] = off;
-        off += clen[seq[q]];
+      const int rot = clen[oc] - val_at_min[oc];  // place of icr in its list
+      ladd[oc] = clen[oc] - rot;
+      lslot[oc] = at;
+      int off = clen[oc] - rot;      // crossings from icr to the list's end
+      for (size_t x = 1; x < seq.size(); x++) {
+        ladd[seq[x]] = clen[seq[x]] + off;
+        lslot[seq[x]] = at;
+        off += clen[seq[x]];
       }
     }
+    for (int ch = 0; ch < nch; ch++)
+      if (lslot[ch] < 0) return CASL_EINVAL;
+    listof = ar2.get<int>(S);
+    int *d_last = ar2.get<int>(nch);
+    d_ladd = ar2.get<int>(nch);
+    d_lslot = ar2.get<int>(nch);
+    if (ar2.failed || C0 + nsad_contours > ccap) return CASL_ENOMEM;
+    CASL_CUDA_TRY(cudaMemsetAsync(listof, 0xff, (size_t)S * sizeof(int), st));
+    CASL_CUDA_TRY(cudaMemcpyAsync(d_last, clast, nch * sizeof(int), cudaMemcpyHostToDevice, st));
+    CASL_CUDA_TRY(cudaMemcpyAsync(d_ladd, ladd.data(), nch * sizeof(int), cudaMemcpyHostToDevice, st));
+    CASL_CUDA_TRY(cudaMemcpyAsync(d_lslot, lslot.data(), nch * sizeof(int), cudaMemcpyHostToDevice, st));
+    CASL_CUDA_TRY(cudaMemcpyAsync(key + C0, skey.data(), nsad_contours * sizeof(skey[0]), cudaMemcpyHostToDevice, st));
+    CASL_CUDA_TRY(cudaMemcpyAsync(slot + C0, sslot.data(), nsad_contours * sizeof(int), cudaMemcpyHostToDevice, st));
+    CASL_CUDA_TRY(cudaMemcpyAsync(slen + C0, sad_len.data(), nsad_contours * sizeof(int), cudaMemcpyHostToDevice, st));
+    CASL_K(k_list_of, gsz(nch), 256, 0, st)(d_last, nch, listof);
+    // the host vectors must outlive their copies
+    CASL_CUDA_TRY(cudaStreamSynchronize(st));
   }
-
   tr.point("saddles");
   // --- 7. contour order and walk layout ---------------------------------------
-  int *startf = ar2.get<int>(ncr), *clenr = ar2.get<int>(ncr), *cidx = ar2.get<int>(ncr);
-  if (ar2.failed) return CASL_ENOMEM;
-  CASL_K(k_ct_plain, g, 256, 0, st)(lab, term, val, ncr, startf, clenr);
-  if (nsad_contours > 0) {
-    int *d_si = ar2.get<int>(nsad_contours), *d_sl = ar2.get<int>(nsad_contours);
-    if (ar2.failed) return CASL_ENOMEM;
-    CASL_CUDA_TRY(cudaMemcpyAsync(d_si, sad_start.data(), nsad_contours * sizeof(int), cudaMemcpyHostToDevice, st));
-    CASL_CUDA_TRY(cudaMemcpyAsync(d_sl, sad_len.data(), nsad_contours * sizeof(int), cudaMemcpyHostToDevice, st));
-    CASL_K(k_set_starts, gsz(nsad_contours), 256, 0, st)(d_si, d_sl, nsad_contours, startf, clenr);
-  }
-  exclusive_scan<int>(st, startf, cidx, ncr, tmpi2, dtot + 1);
-  int C = 0;
-  CASL_CUDA_TRY(cudaMemcpyAsync(&C, dtot + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-  CASL_CUDA_TRY(cudaStreamSynchronize(st));
+  const int C = C0 + nsad_contours;
   if (C == 0) return set_empty();
-  int *clen = ar2.get<int>(C), *coff = ar2.get<int>(C), *clevt = ar2.get<int>(C);
+  {
+    int lb = 1;
+    while ((1 << lb) <= li.levend) lb++;
+    size_t sort_bytes = 0;
+    cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, key, key2, slot, slot2, C, 0, 32 + lb, st);
+    void *sort_tmp = ar2.get<char>(sort_bytes + 16);
+    if (ar2.failed) return CASL_ENOMEM;
+    CASL_CUDA_TRY(cub::DeviceRadixSort::SortPairs(sort_tmp, sort_bytes, key, key2, slot, slot2, C, 0,
+                                                  32 + lb, st));
+  }
+  int *clen = ar2.get<int>(C), *coff = ar2.get<int>(C), *clevt = ar2.get<int>(C), *place = ar2.get<int>(C);
+  int *tmpi2 = ar2.get<int>(scan_tmp_elems(C) + 4);
+  int4 *R = ar2.get<int4>(S);
   double *xw = ar2.get<double>(ncr), *yw = ar2.get<double>(ncr);
   int *cidw = ar2.get<int>(ncr);
-  WalkRec *rec = ar2.get<WalkRec>(ncr);
   if (ar2.failed) return CASL_ENOMEM;
-  // contour lengths in contour order, and their offsets
-  CASL_K(k_ct_len, g, 256, 0, st)(startf, clenr, cidx, ncr, clen);
-  exclusive_scan<int>(st, clen, coff, C, tmpi2, dtot + 2);
-  CASL_K(k_ct_gather_plain, g, 256, 0, st)(lab, term, val, cidx, coff, clen, xcr, ycr, ncr, rec);
-  int nch = (int)ch_end.size();
-  if (nch > 0) {
-    // absolute position of every chain; the first chain of a contour is
-    // rotated to begin at the contour's first crossing, its head wrapping
-    // to the end of the contour
-    std::vector<int> sad_cidx, sad_off;
-    RC_TRY(gather(cidx, sad_start, sad_cidx));
-    RC_TRY(gather(coff, sad_cidx, sad_off));
-    std::vector<long long> abs_pos(nch);
-    std::vector<int> rotlen(nch, 0), chc(nch);
-    for (int ch = 0; ch < nch; ch++) {
-      int cont = ch_cont[ch];
-      if (cont < 0) return CASL_EINVAL;
-      abs_pos[ch] = sad_off[cont] + ch_pos[ch];
-      if (ch_rot[ch] >= 0) rotlen[ch] = sad_len[cont];
-      chc[ch] = sad_cidx[cont];
-    }
-    long long *d_pos = ar2.get<long long>(nch);
-    int *d_len = ar2.get<int>(nch), *d_rot = ar2.get<int>(nch), *d_cl = ar2.get<int>(nch);
-    int *d_ends = ar2.get<int>(nch), *d_cc = ar2.get<int>(nch);
-    int *chain_of_end = ar2.get<int>(ncr);
-    if (ar2.failed) return CASL_ENOMEM;
-    CASL_CUDA_TRY(cudaMemcpyAsync(d_pos, abs_pos.data(), nch * sizeof(long long), cudaMemcpyHostToDevice, st));
-    CASL_CUDA_TRY(cudaMemcpyAsync(d_len, ch_len.data(), nch * sizeof(int), cudaMemcpyHostToDevice, st));
-    CASL_CUDA_TRY(cudaMemcpyAsync(d_rot, ch_rot.data(), nch * sizeof(int), cudaMemcpyHostToDevice, st));
-    CASL_CUDA_TRY(cudaMemcpyAsync(d_cl, rotlen.data(), nch * sizeof(int), cudaMemcpyHostToDevice, st));
-    CASL_CUDA_TRY(cudaMemcpyAsync(d_ends, ch_end.data(), nch * sizeof(int), cudaMemcpyHostToDevice, st));
-    CASL_CUDA_TRY(cudaMemcpyAsync(d_cc, chc.data(), nch * sizeof(int), cudaMemcpyHostToDevice, st));
-    CASL_CUDA_TRY(cudaMemsetAsync(chain_of_end, 0xff, ncr * sizeof(int), st));
-    CASL_K(k_chain_of_end, gsz(nch), 256, 0, st)(d_ends, nch, chain_of_end);
-    CASL_K(k_ct_gather_chain, g, 256, 0, st)(term, ep, val, chain_of_end, d_pos, d_len, d_rot, d_cl,
-                                             d_cc, xcr, ycr, ncr, rec);
-  }
-  CASL_K(k_walk_split, g, 256, 0, st)(rec, ncr, xw, yw, cidw);
-  CASL_K(k_lev_of_contour, g, 256, 0, st)(startf, rlev, cidx, ncr, li, h->p.nlevm, clevt);
+  CASL_K(k_ct_order, gsz(C), 256, 0, st)(key2, slot2, slen, C, h->p.nlevm, clen, clevt, place);
+  exclusive_scan<int>(st, clen, coff, C, tmpi2, dtot + 5);
+  CASL_K(k_ch_place, gsS, 256, 0, st)(head, jA, lA, ta.own, cslot, place, coff, clen, listof, d_ladd,
+                                      d_lslot, S, R);
+  const PlArgs pl{cg, li, uf, eg, c, coffs, ta.own, R, xw, yw, cidw};
+  if (econ)
+    CASL_K(k_tr_place<true>, ntile, TR_NT, 0, st)(pl);
+  else
+    CASL_K(k_tr_place<false>, ntile, TR_NT, 0, st)(pl);
   RC_TRY(check_launch(h));
 
   tr.point("layout");
@@ -1838,16 +952,16 @@ int recontour_dev(casl_handle *h, const double *qq) {
     int *cidw2 = ar2.get<int>(ncr);
     if (ar2.failed) return CASL_ENOMEM;
     CASL_CUDA_TRY(cudaMemsetAsync(flags, 0, (size_t)C * sizeof(int), st));
-    CASL_K(k_ec_flags, g, 256, 0, st)(yw, cidw, ncr, c, flags);
+    CASL_K(k_ec_flags, gsz(ncr), 256, 0, st)(yw, cidw, ncr, c, flags);
     CASL_K(k_ec_keep, gsz(C), 256, 0, st)(flags, clen, C, klen, kone);
-    exclusive_scan<int>(st, klen, koff, C, tmpi2, dtot + 4);
-    exclusive_scan<int>(st, kone, kidx, C, tmpi2, dtot + 5);
+    exclusive_scan<int>(st, klen, koff, C, tmpi2, dtot + 6);
+    exclusive_scan<int>(st, kone, kidx, C, tmpi2, dtot + 7);
     int kc[2] = {0, 0};
-    CASL_CUDA_TRY(cudaMemcpyAsync(kc, dtot + 4, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+    CASL_CUDA_TRY(cudaMemcpyAsync(kc, dtot + 6, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
     CASL_CUDA_TRY(cudaStreamSynchronize(st));
     if (kc[1] == 0) return set_empty();
     const double yoff = c.hly + c.elly * (double)eg.nby;
-    CASL_K(k_ec_compact, g, 256, 0, st)(xw, yw, cidw, ncr, coff, klen, koff, kidx, c, yoff, xw2,
+    CASL_K(k_ec_compact, gsz(ncr), 256, 0, st)(xw, yw, cidw, ncr, coff, klen, koff, kidx, c, yoff, xw2,
                                         yw2, cidw2);
     CASL_K(k_ec_contours, gsz(C), 256, 0, st)(clen, clevt, C, klen, koff, kidx, cs2, len2, lev2);
     RC_TRY(check_launch(h));
