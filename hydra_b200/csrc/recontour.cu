@@ -468,9 +468,12 @@ __global__ void k_out_contours(const int *__restrict__ ocs, const int *__restric
 __global__ void k_out_links(const int *__restrict__ ocs, const int *__restrict__ olen, int nq,
                             int npt, int *__restrict__ nextq) {
   CASL_PDL_ENTRY();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npt; i += gridDim.x * blockDim.x) {
-    int j = contour_of(ocs, nq, i);
-    nextq[i] = i + 1 < ocs[j] + olen[j] ? i + 1 : ocs[j];
+  for (long long b = blockIdx.x * (long long)CC_CHUNK; b < npt; b += (long long)gridDim.x * CC_CHUNK) {
+    chunk_contours(ocs, nq, b);
+    for (int i = (int)b + threadIdx.x; i < min((long long)npt, b + CC_CHUNK); i += blockDim.x) {
+      const int j = chunk_contour_of(ocs, nq, i);
+      nextq[i] = i + 1 < ocs[j] + olen[j] ? i + 1 : ocs[j];
+    }
   }
 }
 

@@ -1,6 +1,8 @@
 // Parallel renode of many contours (contours.f90:687-933); see renode.cuh.
 #include <math.h>
 
+#include <algorithm>
+
 #include "renode.cuh"
 
 namespace casl {
@@ -12,13 +14,14 @@ __device__ __forceinline__ long long wprev(long long w, long long cs, long long 
   return w > cs ? w - 1 : cs + L - 1;
 }
 
-__global__ void k_rn_cid(RenodeIn in, long long N, int *__restrict__ cid) {
+__global__ void __launch_bounds__(256) k_rn_cid(RenodeIn in, long long N, int *__restrict__ cid) {
   CASL_PDL_ENTRY();
   const int C = contours_in(in);
-  const int *cs = in.cs;
-  for (long long w = blockIdx.x * (long long)blockDim.x + threadIdx.x; w < N;
-       w += (long long)gridDim.x * blockDim.x)
-    cid[w] = contour_of(cs, C, w);
+  for (long long b = blockIdx.x * (long long)CC_CHUNK; b < N; b += (long long)gridDim.x * CC_CHUNK) {
+    chunk_contours(in.cs, C, b);
+    for (long long w = b + threadIdx.x; w < min(N, b + CC_CHUNK); w += blockDim.x)
+      cid[w] = chunk_contour_of(in.cs, C, w);
+  }
 }
 
 // The node densities of renode (contours.f90:718-796) for node w: dx, dy,
@@ -31,7 +34,7 @@ __global__ void k_rn_cid(RenodeIn in, long long N, int *__restrict__ cid) {
 // it to the neighbouring lanes, with rn_node for the warps whose nodes come
 // near a contour's end.  Both use the same expressions in the same order.
 __device__ __forceinline__ void rn_node(const RenodeIn &in, const RenodeScratch &s, const Consts &c,
-                                        long long w) {
+                                        long long w, double &eout, int &cout) {
   const double f12 = 0.5, f13 = 1.0 / 3.0, f16 = 1.0 / 6.0;
   const int k = s.cid[w];
   const long long cs = in.cs[k], L = in.len[k];
@@ -96,15 +99,17 @@ __device__ __forceinline__ void rn_node(const RenodeIn &in, const RenodeScratch 
   const double t = c.densf * sqrt(uu) + uu;
   s.dx[w] = dx[2];
   s.dy[w] = dy[2];
-  s.e[w] = e1[2] * fmin(c.dmi, t);
+  s.e[w] = eout = e1[2] * fmin(c.dmi, t);
   s.A[w] = A;
   s.B[w] = B;
   s.Cc[w] = Cc;
-  s.corner[w] = corner2;
-  s.head[w] = (w == cs);
+  cout = corner2;
   if (corner2) red_add_s32(&s.ccnt[k], 1);
 }
 
+// Densities, their sums along each contour and the corners' ranks, in one
+// pass: a tile of RN_IT x 224 nodes per block.
+//
 // One warp covers nodes base-2 .. base+29 (lane L holds node base-2+L) and
 // writes nodes base .. base+27 (lanes 2..29): the segment quantities (rn1)
 // of lane L, its curvature (rn2), its cubic and density terms (rn3) and its
@@ -112,18 +117,32 @@ __device__ __forceinline__ void rn_node(const RenodeIn &in, const RenodeScratch 
 // upper neighbour's from lane L+1.  Valid while every written node's
 // stencil w-2..w+3 lies inside its contour without wrapping; otherwise the
 // warp takes rn_node.
-constexpr int RN_OUT = 28;
-__global__ void __launch_bounds__(256, 4) k_rn_stencil(RenodeIn in, RenodeScratch s, Consts c) {
+//
+// The densities and flags stay in shared memory for the tile's scans; tiles
+// look back at earlier ones for the corners before them (any order: integers)
+// and, to the last contour start before the tile, for the densities, whose
+// tile sums are added from left to right (the same on every run).
+constexpr int RN_OUT = 28, RN_WARPS = 8, RN_STEP = RN_OUT * RN_WARPS;
+template <int RN_IT>
+__global__ void __launch_bounds__(256, 3) k_rn_nodes(RenodeIn in, RenodeScratch s, Consts c) {
   CASL_PDL_ENTRY();
   const double f12 = 0.5, f13 = 1.0 / 3.0, f16 = 1.0 / 6.0;
   const unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
+  constexpr int RN_TILE = RN_STEP * RN_IT;
+  __shared__ double te[RN_TILE];
+  __shared__ unsigned char tf[RN_TILE];  // 1: contour start, 2: corner
+  __shared__ SegPair total;
+  __shared__ unsigned int ctot, cbefore;
+  __shared__ double carry;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const long long N = in.N;
-  const long long nwin = (N + RN_OUT - 1) / RN_OUT;
-  const long long wstride = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long wi = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); wi < nwin;
-       wi += wstride) {
-    const long long base = wi * RN_OUT;
+  const int tile = lb_ticket(&s.tick[0]);
+  const long long t0 = (long long)tile * RN_TILE;
+  if (t0 >= N) return;
+#pragma unroll 1
+  for (int it = 0; it < RN_IT; it++) {
+    const long long base = t0 + (long long)(it * RN_WARPS + wid) * RN_OUT;
+    if (base >= N) break;
     const long long o = base - 2 + lane;  // this lane's node
     const bool out = lane >= 2 && lane < 2 + RN_OUT && o < N;
     int k = 0;
@@ -135,8 +154,14 @@ __global__ void __launch_bounds__(256, 4) k_rn_stencil(RenodeIn in, RenodeScratc
       L = in.len[k];
       lin = o - 2 >= cs && o + 3 <= cs + L - 1;
     }
+    double e = 0.0;
+    int corner = 0;
     if (!__all_sync(FULL, lin)) {
-      if (out) rn_node(in, s, c, o);
+      if (out) {
+        rn_node(in, s, c, o, e, corner);
+        te[o - t0] = e;
+        tf[o - t0] = (unsigned char)((o == cs) | corner << 1);
+      }
       continue;
     }
     // coordinates of this lane's node and of the next one
@@ -164,7 +189,7 @@ __global__ void __launch_bounds__(256, 4) k_rn_stencil(RenodeIn in, RenodeScratc
     // rn2 at this node, from the previous segment
     const double up = __shfl_up_sync(FULL, v, 1);
     const double a = -__shfl_up_sync(FULL, dx, 1), ccp = -__shfl_up_sync(FULL, dy, 1);
-    const int corner = dx * a + dy * ccp > 0.0;
+    corner = dx * a + dy * ccp > 0.0;
     double b;
     if (corner) {
       b = 0.0;
@@ -190,25 +215,89 @@ __global__ void __launch_bounds__(256, 4) k_rn_stencil(RenodeIn in, RenodeScratc
       // rn5
       const double uu = 0.5 * (d + dn);
       const double t = c.densf * sqrt(uu) + uu;
+      e = e1 * fmin(c.dmi, t);
       s.dx[o] = dx;
       s.dy[o] = dy;
-      s.e[o] = e1 * fmin(c.dmi, t);
+      s.e[o] = e;
       s.A[o] = A;
       s.B[o] = B;
       s.Cc[o] = Cc;
-      s.corner[o] = corner;
-      s.head[o] = (o == cs);
+      te[o - t0] = e;
+      tf[o - t0] = (unsigned char)((o == cs) | corner << 1);
       if (corner) red_add_s32(&s.ccnt[k], 1);
     }
   }
-}
-
-__global__ void k_rn_cornerpos(const int *__restrict__ corner, const int *__restrict__ crank,
-                               int *__restrict__ pos, long long N) {
-  CASL_PDL_ENTRY();
-  for (long long w = blockIdx.x * (long long)blockDim.x + threadIdx.x; w < N;
-       w += (long long)gridDim.x * blockDim.x)
-    if (corner[w]) pos[crank[w]] = (int)w;
+  __syncthreads();
+  // the tile's scans, PT nodes per thread
+  constexpr int PT = (RN_TILE + 255) / 256;
+  const int n = (int)min((long long)RN_TILE, N - t0), i0 = PT * threadIdx.x;
+  SegPair acc{0.0, 0};
+  int nc = 0;
+#pragma unroll
+  for (int q = 0; q < PT; q++)
+    if (i0 + q < n) {
+      acc = seg_op(acc, SegPair{te[i0 + q], tf[i0 + q] & 1});
+      nc += tf[i0 + q] >> 1;
+    }
+  SegPair run = block_seg_excl(acc, &total);
+  const unsigned int before = block_excl_scan_any<unsigned int>((unsigned)nc, &ctot);
+  if (wid == 0) {
+    if (lane == 0) {
+      s.tilev[tile] = total.v;
+      s.tilef[tile] = total.f;
+      __threadfence();
+    }
+    __syncwarp();
+    const unsigned long long pre = lb_prefix(s.nstat, tile, ctot, s.err);
+    if (lane == 0) cbefore = (unsigned)pre;
+    // The densities from the last contour start up to this tile.  Every tile
+    // whose sum is needed has published it before its status word; one that
+    // the corners' look-back did not reach is waited for here.
+    auto ready = [&](int t) {
+      const long long c0 = clock64();
+      while (lb_load(&s.nstat[t]) == 0)
+        if (clock64() - c0 > 2000000000LL) {
+          atomicExch(s.err, CASL_ETIMEOUT);
+          break;
+        }
+    };
+    double v = 0.0;
+    if (tile > 0 && !(tf[0] & 1)) {
+      int j = tile - 1;  // the tile of that start
+      for (;; j -= 32) {
+        const int t = j - lane;
+        bool f = t <= 0;
+        if (t >= 0) {
+          ready(t);
+          f = f || __ldcg(&s.tilef[t]) != 0;
+        }
+        const unsigned m = __ballot_sync(FULL, f);
+        if (m) {
+          j -= __ffs(m) - 1;
+          break;
+        }
+      }
+      j = max(j, 0);
+      for (; j < tile; j += 32) {
+        const int t = j + lane;
+        const double x = t < tile ? __ldcg(&s.tilev[t]) : 0.0;
+        for (int q = 0; q < min(32, tile - j); q++) v = v + __shfl_sync(FULL, x, q);
+      }
+    }
+    if (lane == 0) carry = v;
+  }
+  __syncthreads();
+  int rank = (int)(cbefore + before);
+#pragma unroll
+  for (int q = 0; q < PT; q++)
+    if (i0 + q < n) {
+      const int f = tf[i0 + q];
+      run = seg_op(run, SegPair{te[i0 + q], f & 1});
+      const long long o = t0 + i0 + q;
+      s.S[o] = run.f ? run.v : run.v + carry;
+      s.cc[o] = 2 * rank + (f >> 1);
+      if (f & 2) s.cornerpos[rank++] = (int)o;
+    }
 }
 
 // Sum of e over `m` nodes of contour [cs, cs+L) starting at walk index st.
@@ -244,48 +333,45 @@ __device__ double seq_sum(const double *__restrict__ e, long long cs, long long 
   return t;
 }
 
-// Per contour: node count, pieces (contours.f90:799-809, 813-930), and
-// where its pieces are stored (block by block from a running total in
-// d_tot[1]; piece storage order is free, the output order comes from the
-// contour scan).
-__global__ void k_rn_count(RenodeIn in, RenodeScratch s, Consts c, int mode) {
+// Per contour: node count and pieces (contours.f90:799-809, 813-930), and where
+// its nodes go in the output: tiles of 256 contours, whose kept nodes and
+// contours are scanned by looking back (packed as nodes * 2^31 + contours).
+// Pieces are stored block by block from a running total; their order is free.
+__global__ void __launch_bounds__(256) k_rn_contours(RenodeIn in, RenodeScratch s, RenodeOut out,
+                                                     Consts c, int mode) {
   CASL_PDL_ENTRY();
-  __shared__ int btot, bbase;
-  const int Ce = contours_in(in);
-  for (int base = blockIdx.x * blockDim.x; base < Ce; base += gridDim.x * blockDim.x) {
-    const int k = base + threadIdx.x;
-    int np = 0;
+  __shared__ int ptot, pbase;
+  __shared__ unsigned long long ntot, nbefore;
+  const int Ce = contours_in(in), ntile = (Ce + 255) / 256;
+  while (true) {
+    const int tile = lb_ticket(&s.tick[1]);
+    if (tile >= ntile) {
+      if (ntile == 0 && tile == 0 && threadIdx.x < 3) out.d_counts[threadIdx.x] = 0;
+      return;
+    }
+    const int k = tile * 256 + threadIdx.x;
+    int np = 0, nc = 0;
+    long long cs = 0, L = 0;
+    double total = 0.0;
     if (k < Ce) {
-      long long cs = in.cs[k], L = in.len[k];
-      double total = s.S[cs + L - 1];
+      cs = in.cs[k];
+      L = in.len[k];
+      nc = s.ccnt[k];
+      total = s.S[cs + L - 1];
       if (near_half(total)) total = seq_sum(s.e, cs, L, cs, L);
-      s.ctot[k] = total;
       if (!(mode == RENODE_SURGERY && L <= 3)) {
         int npr0 = nint_d(total) + 1;
-        if (npr0 >= 3) np = s.ccnt[k] > 1 ? s.ccnt[k] : 1;
+        if (npr0 >= 3) np = nc > 1 ? nc : 1;
       }
-      s.npiece[k] = np;
     }
-    const int ex = block_excl_scan_any<int>(np, &btot);
-    if (threadIdx.x == 0) bbase = atomicAdd(&s.d_tot[1], btot);
+    const int ex = block_excl_scan_any<int>(np, &ptot);
+    if (threadIdx.x == 0) pbase = ptot ? atomicAdd(&s.tick[2], ptot) : 0;
     __syncthreads();
-    if (k < Ce) s.poff[k] = bbase + ex;
-    __syncthreads();
-  }
-}
-
-__global__ void k_rn_fill(RenodeIn in, RenodeScratch s, Consts c, int mode) {
-  CASL_PDL_ENTRY();
-  const int Ce = contours_in(in);
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < Ce; k += gridDim.x * blockDim.x) {
-    long long cs = in.cs[k], L = in.len[k];
-    int np = s.npiece[k];
+    const int p0 = pbase + ex;
     int npr = 0;
-    double total = s.ctot[k];
-    int nc = s.ccnt[k];
-    int cfirst = s.crank[cs];
+    const int cfirst = np ? s.cc[cs] >> 1 : 0;
     for (int q = 0; q < np; q++) {
-      int p = s.poff[k] + q;
+      const int p = p0 + q;
       long long st, pl;
       double sum;
       int n;
@@ -303,36 +389,45 @@ __global__ void k_rn_fill(RenodeIn in, RenodeScratch s, Consts c, int mode) {
         if (near_half(sum)) sum = seq_sum(s.e, cs, L, st, pl);
         n = sum > c.small ? nint_d(sum) + 1 : 0;
       }
-      s.pc[p] = k;
       s.pstart[p] = (int)st;
       s.plen[p] = (int)pl;
-      s.psum[p] = sum;
       s.pn[p] = n;
       s.pfac[p] = n > 0 ? (double)n / sum : 0.0;
       npr += n;
     }
-    int keep = mode == RENODE_SURGERY ? npr > 3 : npr > 0;
-    s.ckeep[k] = keep;
-    s.cnpr[k] = keep ? npr : 0;
-  }
-}
-
-__global__ void k_rn_pout(RenodeIn in, RenodeScratch s, RenodeOut out) {
-  CASL_PDL_ENTRY();
-  if (out.d_counts[2]) return;  // overflow: the caller reports it
-  const int Ce = contours_in(in);
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < Ce; k += gridDim.x * blockDim.x) {
-    if (!s.ckeep[k]) continue;
-    int base = s.cout[k];
-    for (int q = 0; q < s.npiece[k]; q++) {
-      int p = s.poff[k] + q;
-      s.pout[p] = base;
-      base += s.pn[p];
+    const bool keep = k < Ce && (mode == RENODE_SURGERY ? npr > 3 : npr > 0);
+    const unsigned long long mine = keep ? ((unsigned long long)npr << 31) + 1ull : 0ull;
+    unsigned long long at = block_excl_scan_any<unsigned long long>(mine, &ntot);
+    if (threadIdx.x < 32) {
+      const unsigned long long pre = lb_prefix(s.cstat, tile, ntot, s.err);
+      if (threadIdx.x == 0) nbefore = pre;
     }
-    int j = s.ckidx[k];
-    out.ocs[j] = s.cout[k];
-    out.olen[j] = s.cnpr[k];
-    out.olev[j] = in.levt ? in.levt[k] : 0;
+    __syncthreads();
+    at += nbefore;
+    if (k < Ce) {
+      s.npiece[k] = np;
+      s.poff[k] = p0;
+      s.ckeep[k] = keep;
+      if (keep) {
+        int base = (int)(at >> 31);
+        const int j = (int)(at & 0x7fffffffull);
+        s.ckidx[k] = j;
+        out.ocs[j] = base;
+        out.olen[j] = npr;
+        out.olev[j] = in.levt ? in.levt[k] : 0;
+        for (int q = 0; q < np; q++) {
+          s.pout[p0 + q] = base;
+          base += s.pn[p0 + q];
+        }
+      }
+    }
+    if (tile == ntile - 1 && threadIdx.x == 0) {
+      const unsigned long long all = nbefore + ntot;
+      const long long nodes = (long long)(all >> 31);
+      out.d_counts[0] = (int)(all & 0x7fffffffull);
+      out.d_counts[1] = (int)nodes;
+      out.d_counts[2] = nodes > out.cap;
+    }
   }
 }
 
@@ -347,7 +442,8 @@ __global__ void k_rn_place(RenodeIn in, RenodeScratch s, RenodeOut out, Consts c
     int nc = s.ccnt[k];
     int q = 0;
     if (nc >= 2) {
-      int inc = s.crank[w] - s.crank[cs] + s.corner[w];
+      const int cw = s.cc[w];
+      int inc = (cw >> 1) - (s.cc[cs] >> 1) + (cw & 1);
       q = inc - 1;
       if (q < 0) q = nc - 1;
     }
@@ -396,37 +492,6 @@ __global__ void k_rn_place(RenodeIn in, RenodeScratch s, RenodeOut out, Consts c
   }
 }
 
-// The kept contours' node counts and keep flags scanned (both over the
-// contours the device holds), then the output counts: one block.
-__global__ void __launch_bounds__(SCAN_BLOCK) k_rn_scan2_finish(RenodeIn in, RenodeScratch s,
-                                                                RenodeOut out) {
-  CASL_PDL_ENTRY();
-  __shared__ unsigned long long tot;
-  const long long n = contours_in(in);
-  // each thread takes a run of consecutive contours; both counts go through
-  // one scan, the node counts in the high word and the keep flags in the low
-  // word (each total stays below 2^31)
-  auto pack = [&](long long k) -> unsigned long long {
-    return ((unsigned long long)(unsigned)s.cnpr[k] << 32) | (unsigned)s.ckeep[k];
-  };
-  const long long per = (n + SCAN_BLOCK - 1) / SCAN_BLOCK;
-  const long long k0 = min(n, (long long)threadIdx.x * per), k1 = min(n, k0 + per);
-  unsigned long long sum = 0;
-  for (long long k = k0; k < k1; k++) sum += pack(k);
-  unsigned long long ex = block_excl_scan<unsigned long long>(sum, &tot);
-  for (long long k = k0; k < k1; k++) {
-    s.cout[k] = (int)(ex >> 32);
-    s.ckidx[k] = (int)(ex & 0xffffffffu);
-    ex += pack(k);
-  }
-  if (threadIdx.x == 0) {
-    const long long nodes = (long long)(tot >> 32);
-    out.d_counts[0] = (int)(tot & 0xffffffffu);
-    out.d_counts[1] = (int)nodes;
-    out.d_counts[2] = nodes > out.cap;
-  }
-}
-
 static inline int gsz(long long work) {
   long long g = (work + 255) / 256;
   if (g < 1) g = 1;
@@ -448,40 +513,45 @@ int renode_batch(casl_handle *h, Arena &ar, const RenodeIn &in, RenodeOut &out, 
   s.dx = ar.get<double>(N); s.dy = ar.get<double>(N);
   s.e = ar.get<double>(N); s.A = ar.get<double>(N);
   s.B = ar.get<double>(N); s.Cc = ar.get<double>(N); s.S = ar.get<double>(N);
-  s.corner = ar.get<int>(N); s.crank = ar.get<int>(N); s.head = ar.get<int>(N);
+  s.cc = ar.get<int>(N);
   s.cornerpos = ar.get<int>(N + 1);
-  s.ccnt = ar.get<int>(C); s.ctot = ar.get<double>(C);
+  s.ccnt = ar.get<int>(C);
   s.npiece = ar.get<int>(C); s.poff = ar.get<int>(C);
-  s.cnpr = ar.get<int>(C); s.cout = ar.get<int>(C); s.ckeep = ar.get<int>(C);
-  s.ckidx = ar.get<int>(C);
-  long long tmpn = scan_tmp_elems(N > C ? N : C) + 4;
-  s.tmpi = ar.get<int>(tmpn);
-  s.tmps = ar.get<SegPair>(tmpn);
-  s.d_tot = ar.get<int>(8);
+  s.ckeep = ar.get<int>(C); s.ckidx = ar.get<int>(C);
+  // Tiles of one step while that leaves no more blocks than fit on the SMs at
+  // once (a tile's steps run one after the other: 10k nodes 16 us with 1, 33
+  // with 8); larger ones above, where each further tile costs its scans (1.4M
+  // nodes 170, 101 and 87 us with 1, 3 and 8; 75k nodes 23, 24, 35).
+  const int rnit = N <= 148LL * 3 * RN_STEP ? 1 : (N <= 148LL * 3 * RN_STEP * 4 ? 3 : 8);
+  const long long nt = (N + rnit * RN_STEP - 1) / (rnit * RN_STEP), ct = (C + 255LL) / 256;
+  s.nstat = ar.get<unsigned long long>(nt + ct + 2);  // then the contours' words, then the tickets
+  s.cstat = s.nstat + nt;
+  s.tick = reinterpret_cast<int *>(s.cstat + ct);
+  s.tilev = ar.get<double>(nt);
+  s.tilef = ar.get<int>(nt);
+  s.err = &h->scal->error;
   // pieces: one per corner of a contour with >= 2 corners, else one per
   // contour, so at most N + C
   long long P = N + C;
-  s.pc = ar.get<int>(P); s.pstart = ar.get<int>(P); s.plen = ar.get<int>(P);
+  s.pstart = ar.get<int>(P); s.plen = ar.get<int>(P);
   s.pn = ar.get<int>(P); s.pout = ar.get<int>(P);
-  s.psum = ar.get<double>(P); s.pfac = ar.get<double>(P);
+  s.pfac = ar.get<double>(P);
   if (ar.failed) return CASL_ENOMEM;
   {
-    const FillJob z[2] = {{s.ccnt, C, 0u}, {s.d_tot + 1, 1, 0u}};
+    const FillJob z[2] = {{s.ccnt, C, 0u}, {s.nstat, 2 * (nt + ct + 2), 0u}};
     if (int rc = fill_words(st, z, 2)) return rc;
   }
   int g = gsz(N);
   if (!in.cid) CASL_K(k_rn_cid, g, 256, 0, st)(in, N, s.cid);
-  CASL_K(k_rn_stencil, g, 256, 0, st)(in, s, c);
-  segmented_scan(st, s.e, s.head, s.S, N, s.tmps);
-  exclusive_scan<int>(st, s.corner, s.crank, N, s.tmpi, s.d_tot + 0);
-  CASL_K(k_rn_cornerpos, g, 256, 0, st)(s.corner, s.crank, s.cornerpos, N);
-  // per-contour passes: C may be a capacity (surgery: the count is on the
-  // device), so the grids are sized for the usual counts and loop
-  int gc = gsz(C < (1 << 16) ? C : (1 << 16));
-  CASL_K(k_rn_count, gc, 256, 0, st)(in, s, c, mode);
-  CASL_K(k_rn_fill, gc, 256, 0, st)(in, s, c, mode);
-  CASL_K(k_rn_scan2_finish, 1, SCAN_BLOCK, 0, st)(in, s, out);
-  CASL_K(k_rn_pout, gc, 256, 0, st)(in, s, out);
+  if (rnit == 1)
+    CASL_K(k_rn_nodes<1>, (int)nt, 256, 0, st)(in, s, c);
+  else if (rnit == 3)
+    CASL_K(k_rn_nodes<3>, (int)nt, 256, 0, st)(in, s, c);
+  else
+    CASL_K(k_rn_nodes<8>, (int)nt, 256, 0, st)(in, s, c);
+  // (C may be a capacity, the count being on the device: the grid is sized
+  // for the usual counts and its blocks take tiles until there are none)
+  CASL_K(k_rn_contours, (int)std::min(ct, 2LL * 148), 256, 0, st)(in, s, out, c, mode);
   CASL_K(k_rn_place, g, 256, 0, st)(in, s, out, c);
   return check_launch(h);
 }

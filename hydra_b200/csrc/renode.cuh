@@ -47,21 +47,64 @@ __device__ __forceinline__ int contour_of(const int *__restrict__ cs, int C, lon
   return lo;
 }
 
+// The contour of every node of a chunk of CC_CHUNK nodes (a block's): one search
+// in memory for the first, the following starts staged in shared memory and
+// searched there (beyond them, in memory again).
+constexpr int CC_CHUNK = 1024, CC_STARTS = 256;
+struct ChunkContours {
+  int j0, st[CC_STARTS];
+};
+__device__ __forceinline__ ChunkContours &chunk_shared() {
+  __shared__ ChunkContours c;
+  return c;
+}
+__device__ __forceinline__ void chunk_contours(const int *__restrict__ cs, int C, long long w0) {
+  ChunkContours &c = chunk_shared();
+  __syncthreads();
+  if (threadIdx.x < 32) {  // 32-way search: the last contour starting at or before w0
+    int lo = 0, hi = C;    // cs[lo] <= w0, and w0 < cs[hi] (hi = C: none)
+    while (hi - lo > 1) {
+      const int step = (hi - lo + 31) / 32, at = lo + step * (int)threadIdx.x;
+      const unsigned m = __ballot_sync(0xffffffffu, at < hi && cs[at] <= w0);
+      const int last = 31 - __clz(m | 1u);
+      hi = min(hi, lo + step * (last + 1));
+      lo = lo + step * last;
+    }
+    if (threadIdx.x == 0) c.j0 = lo;
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < CC_STARTS; t += blockDim.x)
+    c.st[t] = c.j0 + t < C ? cs[c.j0 + t] : 0x7fffffff;
+  __syncthreads();
+}
+__device__ __forceinline__ int chunk_contour_of(const int *__restrict__ cs, int C, long long w) {
+  const ChunkContours &c = chunk_shared();
+  if (c.st[CC_STARTS - 1] <= w) return contour_of(cs, C, w);
+  int lo = 0, hi = CC_STARTS - 1;  // st[lo] <= w < st[hi]
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (c.st[mid] <= w) lo = mid; else hi = mid;
+  }
+  return c.j0 + lo;
+}
+
 struct RenodeScratch {
   int *cid;                  // contour of each walk node
   double *dx, *dy, *e, *A, *B, *Cc, *S;
-  int *corner, *crank, *head;
+  int *cc;                   // 2 * (corners before the node) + (the node is one)
   int *ccnt;                 // corners per contour
-  double *ctot;              // density sum per contour
   int *npiece, *poff;        // pieces per contour, offsets
-  int *pc, *pstart, *plen, *pn, *pout;  // per piece: contour, start w, length, count, out offset
-  double *psum, *pfac;
-  int *cnpr, *cout, *ckeep, *ckidx;     // per contour: kept npr, out offset, keep, kept index
+  int *pstart, *plen, *pn, *pout;  // per piece: start w, length, count, out offset
+  double *pfac;
+  int *ckeep, *ckidx;        // per contour: keep, kept index
   int *cornerpos;
-  int *tmpi;
-  SegPair *tmps;
-  int *d_tot;
-  long long maxpieces;
+  // tiles of the two scans: tickets, status words, and the node tiles'
+  // densities since their last contour start
+  int *tick;                 // [0] nodes, [1] contours, [2] pieces allotted
+  unsigned long long *nstat, *cstat;
+  double *tilev;
+  int *tilef;
+  int *err;
 };
 
 // Renodes every contour; issues no host synchronisation.  out.d_counts

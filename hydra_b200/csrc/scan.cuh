@@ -1,9 +1,9 @@
 // Device-wide scans and a bump allocator over the handle's scratch arena.
 //
-// Scans are three-phase (per-block scan, scan of block totals in one block,
-// carry add), deterministic, with 4096 elements per block.  Integer scans
-// are exact; the segmented double scan sums in a fixed order (the same on
-// every run), restarting at every head flag.
+// Integer scans of whole arrays are two- or three-phase with 4096 elements per
+// block.  Scans whose values and prefixes live in one kernel look back from
+// tile to tile instead (lb_prefix).  The segmented double scan sums in a fixed
+// order, the same on every run, restarting at every head.
 #pragma once
 
 #include "common.cuh"
@@ -282,8 +282,68 @@ int exclusive_scan(cudaStream_t st, const T *in, T *out, long long n, T *tmp, T 
 inline long long scan_tmp_elems(long long n) { return (n + SCAN_TILE - 1) / SCAN_TILE + 1; }
 
 // ---------------------------------------------------------------------------
-// Segmented inclusive scan of doubles: out[i] = sum of in[j] for j from the
-// last head at or before i through i.  head[i] != 0 starts a segment.
+// Scans inside a kernel: tiles in ticket order, each publishing its sum and
+// looking back at the sums before it, so that what produces the values, the
+// scan and what uses the prefixes are one launch and one pass over memory.
+// ---------------------------------------------------------------------------
+// Status word of a tile: 0 until its sum is known, then LB_SUM | sum, then
+// LB_PREFIX | sum of all tiles up to it.  Sums stay below 2^62; pairs of counts
+// are packed as hi * 2^31 + lo (each below 2^31).  A tile waits only for
+// tiles with lower tickets, which running blocks hold.
+constexpr unsigned long long LB_SUM = 1ull << 62, LB_PREFIX = 2ull << 62, LB_VALUE = LB_SUM - 1;
+__device__ __forceinline__ unsigned long long lb_load(const unsigned long long *p) {
+  unsigned long long v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(__cvta_generic_to_global(p)) : "memory");
+  return v;
+}
+__device__ __forceinline__ void lb_store(unsigned long long *p, unsigned long long v) {
+  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "l"(v) : "memory");
+}
+// By one whole warp: publishes the tile's sum and returns the sum of the tiles
+// before it.  Gives up after about a second (CASL_ETIMEOUT).
+__device__ __forceinline__ unsigned long long lb_prefix(unsigned long long *status, int tile,
+                                                        unsigned long long sum, int *err) {
+  const int lane = threadIdx.x & 31;
+  if (lane == 0) lb_store(&status[tile], (tile == 0 ? LB_PREFIX : LB_SUM) | sum);
+  if (tile == 0) return 0;
+  unsigned long long pre = 0;
+  const long long t0 = clock64();
+  for (int look = tile - 1; look >= 0; look -= 32) {
+    const int idx = look - lane;
+    unsigned long long w = LB_PREFIX;  // before the first tile: a prefix of 0
+    unsigned have;
+    bool wait;
+    do {
+      if (idx >= 0) w = lb_load(&status[idx]);
+      // only the tiles down to the nearest prefix are needed
+      have = __ballot_sync(0xffffffffu, w >= LB_PREFIX);
+      const unsigned need = have ? (have & (0u - have)) - 1u : 0xffffffffu;
+      wait = (__ballot_sync(0xffffffffu, w == 0) & need) != 0;
+      if (wait && __any_sync(0xffffffffu, clock64() - t0 > 2000000000LL)) {
+        if (lane == 0) atomicExch(err, CASL_ETIMEOUT);
+        wait = false;
+      }
+    } while (wait);
+    unsigned long long v = !have || lane < __ffs(have) ? w & LB_VALUE : 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    pre += v;
+    if (have) break;
+  }
+  if (lane == 0) lb_store(&status[tile], LB_PREFIX | (pre + sum));
+  return pre;
+}
+// A block's next tile (all threads).
+__device__ __forceinline__ int lb_ticket(int *ticket) {
+  __shared__ int t;
+  __syncthreads();
+  if (threadIdx.x == 0) t = atomicAdd(ticket, 1);
+  __syncthreads();
+  return t;
+}
+
+// ---------------------------------------------------------------------------
+// Segmented scan of doubles: sums restart at every flagged element.
 // ---------------------------------------------------------------------------
 struct SegPair {
   double v;
@@ -306,11 +366,12 @@ __device__ __forceinline__ SegPair warp_seg_incl(SegPair x) {
   }
   return x;
 }
-// Exclusive (prefix before this thread) segmented scan across the block.
-static __device__ SegPair block_seg_excl(SegPair x, SegPair *total) {
+// Exclusive (prefix before this thread) segmented scan across a block of at
+// most 32 warps, in a fixed order; the block's own result through *total.
+static __device__ __forceinline__ SegPair block_seg_excl(SegPair x, SegPair *total) {
   __shared__ double wv[32];
   __shared__ int wf[32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   SegPair incl = warp_seg_incl(x);
   SegPair ex;
   ex.v = __shfl_up_sync(0xffffffffu, incl.v, 1);
@@ -319,7 +380,7 @@ static __device__ SegPair block_seg_excl(SegPair x, SegPair *total) {
   if (lane == 31) { wv[wid] = incl.v; wf[wid] = incl.f; }
   __syncthreads();
   if (wid == 0) {
-    SegPair w{wv[lane], wf[lane]};
+    SegPair w{lane < nw ? wv[lane] : 0.0, lane < nw ? wf[lane] : 0};
     SegPair wi = warp_seg_incl(w);
     SegPair we;
     we.v = __shfl_up_sync(0xffffffffu, wi.v, 1);
@@ -336,6 +397,8 @@ static __device__ SegPair block_seg_excl(SegPair x, SegPair *total) {
   return r;
 }
 
+// out[i] = sum of in[j] for j from the last head at or before i through i, over a
+// whole array (three launches).
 static __global__ void __launch_bounds__(SCAN_BLOCK) k_segscan_tiles(const double *__restrict__ in,
                                                               const int *__restrict__ head,
                                                               double *__restrict__ out,

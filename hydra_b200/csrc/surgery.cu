@@ -622,41 +622,49 @@ __global__ void k_sg_replay(SurgState S, const LevelDesc *__restrict__ lev,
 // ---------------------------------------------------------------------------
 // Rebuild: cycles of nextq -> walk-ordered contours (contours.f90:621-663)
 // ---------------------------------------------------------------------------
-__global__ void k_rb_flags(const int *__restrict__ nextq, int npt, int *__restrict__ st,
-                           int *__restrict__ brk) {
+// Runs of consecutive links, numbered in node order: tiles of 2048 nodes, each
+// counting its runs and looking back for those before it.  rid: the run of
+// every node; rs, re: a run's first and last node; *R their number.
+constexpr int RB_TILE = 2048;
+__global__ void __launch_bounds__(256) k_rb_runs(const int *__restrict__ nextq, int npt,
+                                                 int *__restrict__ tick,
+                                                 unsigned long long *__restrict__ stat,
+                                                 int *__restrict__ rid, int *__restrict__ rs,
+                                                 int *__restrict__ re, int *__restrict__ R,
+                                                 int *__restrict__ err) {
   CASL_PDL_ENTRY();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npt; i += gridDim.x * blockDim.x) {
-    brk[i] = nextq[i] != i + 1;
-    st[i] = (i == 0) || (nextq[i - 1] != i);
+  __shared__ int tot, before;
+  const int tile = lb_ticket(tick);
+  const int i0 = tile * RB_TILE + 8 * (int)threadIdx.x;  // 8 consecutive nodes
+  unsigned st = 0, en = 0;
+  if (i0 < npt) {
+    int prev = i0 > 0 ? nextq[i0 - 1] : -1;
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+      if (i0 + k < npt) {
+        const int nx = nextq[i0 + k];
+        st |= (unsigned)(i0 + k == 0 || prev != i0 + k) << k;
+        en |= (unsigned)(nx != i0 + k + 1) << k;
+        prev = nx;
+      }
   }
+  int r = block_excl_scan_any<int>(__popc(st), &tot);
+  if (threadIdx.x < 32) {
+    const unsigned long long pre = lb_prefix(stat, tile, (unsigned)tot, err);
+    if (threadIdx.x == 0) before = (int)pre;
+  }
+  __syncthreads();
+  r += before - 1;
+#pragma unroll
+  for (int k = 0; k < 8; k++)
+    if (i0 + k < npt) {
+      if (st >> k & 1) rs[++r] = i0 + k;
+      rid[i0 + k] = r;
+      if (en >> k & 1) re[r] = i0 + k;
+    }
+  if ((tile + 1) * (long long)RB_TILE >= npt && threadIdx.x == 0) *R = before + tot;
 }
 
-__global__ void k_rb_runs(const int *__restrict__ st, const int *__restrict__ brk,
-                          const int *__restrict__ sx, int npt, int *__restrict__ rid,
-                          int *__restrict__ rs, int *__restrict__ re) {
-  CASL_PDL_ENTRY();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npt; i += gridDim.x * blockDim.x) {
-    int r = sx[i] + st[i] - 1;
-    rid[i] = r;
-    if (st[i]) rs[r] = i;
-    if (brk[i]) re[r] = i;
-  }
-}
-
-
-
-
-
-
-
-
-
-
-
-// All run-level cycle work in one block.  A contour no reconnection touched
-// is a single run that points to itself and is finished at once; pointer
-// jumping (min label, then list ranking) runs over the few remaining runs
-// only, rounds separated by block barriers.
 // Every run: its successor run; a run that closes on itself is a whole
 // contour (head, length); the others (the few runs surgery cut and joined)
 // go to the multi list for k_rb_cycles_block.  Grid-wide.
@@ -664,21 +672,19 @@ __global__ void k_rb_cycles_pre(const int *__restrict__ nextq, const int *__rest
                                 const int *__restrict__ rs, const int *__restrict__ re,
                                 const int *__restrict__ R_dev, int *__restrict__ nr,
                                 int *__restrict__ lab, int *__restrict__ nrj,
-                                int *__restrict__ hr, long long *__restrict__ val,
-                                long long *__restrict__ val2, int *__restrict__ ishead,
-                                int *__restrict__ multi, int *__restrict__ nmulti) {
+                                int *__restrict__ hr, int *__restrict__ val,
+                                int *__restrict__ ishead, int *__restrict__ multi, int *__restrict__ nmulti) {
   CASL_PDL_ENTRY();
   const int R = *R_dev;
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < R; r += gridDim.x * blockDim.x) {
     const int t = rid[nextq[re[r]]];
     nr[r] = t;
-    const long long len = re[r] - rs[r] + 1;
+    const int len = re[r] - rs[r] + 1;
     lab[r] = rs[r];
     if (t == r) {  // a whole contour
       hr[r] = r;
       ishead[r] = 1;
       val[r] = len;
-      val2[r] = len;
     } else {
       nrj[r] = t;
       multi[atomicAdd(nmulti, 1)] = r;
@@ -692,8 +698,8 @@ __global__ void __launch_bounds__(1024) k_rb_cycles_block(
     const int *__restrict__ nextq, const int *__restrict__ rid, const int *__restrict__ rs,
     const int *__restrict__ re, const int *__restrict__ R_dev, int *__restrict__ nr,
     int *lab, int *lab2, int *nrj, int *nrj2, int *__restrict__ hr, int *succ, int *succ2,
-    long long *val, long long *val2, int *__restrict__ ishead, int *__restrict__ multi,
-    long long **valout, const int *__restrict__ nmulti) {
+    int *val, int *val2, int *__restrict__ ishead, int *__restrict__ multi,
+    const int *__restrict__ nmulti) {
   CASL_PDL_ENTRY();
   const int M = *nmulti;
   int rounds = 1;
@@ -738,38 +744,61 @@ __global__ void __launch_bounds__(1024) k_rb_cycles_block(
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) *valout = val;
 }
 
-__global__ void k_rb_cycles2(const int *__restrict__ ishead, const int *__restrict__ cidx,
-                             long long *const *__restrict__ valp, const int *__restrict__ rs,
-                             const int *__restrict__ lvl, const LevelDesc *__restrict__ lev,
-                             const int *__restrict__ R_dev, int *__restrict__ clen,
-                             int *__restrict__ clev) {
+// The contours: the head runs in order, their first walk positions, lengths and
+// levels.  Tiles of 256 runs, scanned by looking back (contours * 2^31 +
+// nodes); cidx is written for head runs only.  *C the number of contours.
+__global__ void __launch_bounds__(256) k_rb_contours(const int *__restrict__ ishead,
+                                                     const int *__restrict__ val,
+                                                     const int *__restrict__ rs,
+                                                     const int *__restrict__ lvl,
+                                                     const LevelDesc *__restrict__ lev,
+                                                     const int *__restrict__ R_dev,
+                                                     int *__restrict__ tick,
+                                                     unsigned long long *__restrict__ stat,
+                                                     int *__restrict__ cidx, int *__restrict__ cst,
+                                                     int *__restrict__ clen, int *__restrict__ clev,
+                                                     int *__restrict__ C, int *__restrict__ err) {
   CASL_PDL_ENTRY();
-  const int R = *R_dev;
-  const long long *val = *valp;
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < R; r += gridDim.x * blockDim.x) {
-    if (!ishead[r]) continue;
-    int c = cidx[r];
-    clen[c] = (int)val[r];
-    clev[c] = lev[lvl[rs[r]]].levt;
+  __shared__ unsigned long long tot, before;
+  const int R = *R_dev, ntile = (R + 255) / 256;
+  while (true) {
+    const int tile = lb_ticket(tick);
+    if (tile >= ntile) return;
+    const int r = tile * 256 + threadIdx.x;
+    const bool f = r < R && ishead[r];
+    const int len = f ? val[r] : 0;
+    unsigned long long at =
+        block_excl_scan_any<unsigned long long>(f ? (1ull << 31) + (unsigned)len : 0ull, &tot);
+    if (threadIdx.x < 32) {
+      const unsigned long long pre = lb_prefix(stat, tile, tot, err);
+      if (threadIdx.x == 0) before = pre;
+    }
+    __syncthreads();
+    at += before;
+    if (f) {
+      const int c = (int)(at >> 31);
+      cidx[r] = c;
+      cst[c] = (int)(at & 0x7fffffffull);
+      clen[c] = len;
+      clev[c] = lev[lvl[rs[r]]].levt;
+    }
+    if (tile == ntile - 1 && threadIdx.x == 0) *C = (int)((before + tot) >> 31);
   }
 }
 
 __global__ void k_rb_gather2(const double *__restrict__ xq, const double *__restrict__ yq, int npt,
                              const int *__restrict__ rid, const int *__restrict__ rs,
                              const int *__restrict__ hr, const int *__restrict__ cidx,
-                             long long *const *__restrict__ valp, const int *__restrict__ cst,
+                             const int *__restrict__ val, const int *__restrict__ cst,
                              const int *__restrict__ clen, double *__restrict__ xw,
                              double *__restrict__ yw, int *__restrict__ cidw) {
   CASL_PDL_ENTRY();
-  const long long *val = *valp;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npt; i += gridDim.x * blockDim.x) {
-    int r = rid[i];
-    int c = cidx[hr[r]];
-    long long off = (long long)clen[c] - val[r];
-    long long pos = cst[c] + off + (i - rs[r]);
+    const int r = rid[i];
+    const int c = cidx[hr[r]];
+    const int pos = cst[c] + (clen[c] - val[r]) + (i - rs[r]);
     xw[pos] = xq[i];
     yw[pos] = yq[i];
     cidw[pos] = c;
@@ -798,11 +827,14 @@ __global__ void k_rb_writeback(const int *__restrict__ cnt, long long npm, long 
     npq[j] = olen[j];
     indq[j] = olev[j];
   }
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npt; i += gridDim.x * blockDim.x) {
-    xq[i] = xo[i];
-    yq[i] = yo[i];
-    int j = contour_of(ocs, nq, i);
-    nextq[i] = i + 1 < ocs[j] + olen[j] ? i + 1 : ocs[j];
+  for (long long b = blockIdx.x * (long long)CC_CHUNK; b < npt; b += (long long)gridDim.x * CC_CHUNK) {
+    chunk_contours(ocs, nq, b);
+    for (int i = (int)b + threadIdx.x; i < min((long long)npt, b + CC_CHUNK); i += blockDim.x) {
+      xq[i] = xo[i];
+      yq[i] = yo[i];
+      const int j = chunk_contour_of(ocs, nq, i);
+      nextq[i] = i + 1 < ocs[j] + olen[j] ? i + 1 : ocs[j];
+    }
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     s->nq = nq;
@@ -823,43 +855,42 @@ static inline int gs(long long work) {
 static int rebuild_and_renode(casl_handle *h, Arena &ar, int npt, const int *lvl,
                               const LevelDesc *dlev) {
   cudaStream_t st = h->stream;
-  int *stf = ar.get<int>(npt), *brk = ar.get<int>(npt), *sx = ar.get<int>(npt);
-  int *rid = ar.get<int>(npt), *tmpi = ar.get<int>(scan_tmp_elems(npt) + 4);
+  int *rid = ar.get<int>(npt);
   int *dtot = ar.get<int>(8);
   // run arrays (R <= npt)
   int *rs = ar.get<int>(npt), *re = ar.get<int>(npt), *nr = ar.get<int>(npt);
   int *lab = ar.get<int>(npt), *lab2 = ar.get<int>(npt), *nrj = ar.get<int>(npt);
   int *nrj2 = ar.get<int>(npt), *hr = ar.get<int>(npt), *succ = ar.get<int>(npt);
   int *succ2 = ar.get<int>(npt), *ishead = ar.get<int>(npt), *cidx = ar.get<int>(npt);
-  long long *val = ar.get<long long>(npt), *val2 = ar.get<long long>(npt);
-  long long **valp = ar.get<long long *>(1);
+  int *val = ar.get<int>(npt), *val2 = ar.get<int>(npt);
   int *multi = ar.get<int>(npt);
   // cycles (C <= R <= npt)
   int *clen = ar.get<int>(npt), *clev = ar.get<int>(npt), *cst = ar.get<int>(npt);
   double *xw = ar.get<double>(npt), *yw = ar.get<double>(npt);
   int *ocs = ar.get<int>(npt), *olen = ar.get<int>(npt), *olev = ar.get<int>(npt);
   int *cnt = ar.get<int>(4);
-  int *nmulti = ar.get<int>(4);
-  if (ar.failed) return CASL_ENOMEM;
-  const int g = gs(npt);
-  CASL_K(k_rb_flags, g, 256, 0, st)(h->nextq, npt, stf, brk);
-  exclusive_scan<int>(st, stf, sx, npt, tmpi, dtot);           // dtot[0] = R
-  CASL_K(k_rb_runs, g, 256, 0, st)(stf, brk, sx, npt, rid, rs, re);
-  {
-    const FillJob z[3] = {{ishead, npt, 0u}, {clen, npt, 0u}, {nmulti, 1, 0u}};
-    if (int rc = fill_words(st, z, 3)) return rc;
-  }
-  CASL_K(k_rb_cycles_pre, g, 256, 0, st)(h->nextq, rid, rs, re, dtot, nr, lab, nrj, hr, val, val2,
-                                         ishead, multi, nmulti);
-  CASL_K(k_rb_cycles_block, 1, 1024, 0, st)(h->nextq, rid, rs, re, dtot, nr, lab, lab2, nrj, nrj2,
-                                            hr, succ, succ2, val, val2, ishead, multi, valp,
-                                            nmulti);
-  exclusive_scan<int>(st, ishead, cidx, npt, tmpi, dtot + 1);  // dtot[1] = C
-  CASL_K(k_rb_cycles2, g, 256, 0, st)(ishead, cidx, valp, rs, lvl, dlev, dtot, clen, clev);
-  exclusive_scan<int>(st, clen, cst, npt, tmpi, dtot + 2);
   int *cidw = ar.get<int>(npt);
+  // status words of the runs' and the contours' tiles, then their tickets and
+  // the number of cut runs
+  const int rt = (npt + RB_TILE - 1) / RB_TILE, ct = (npt + 255) / 256;
+  unsigned long long *stat = ar.get<unsigned long long>(rt + ct + 2);
   if (ar.failed) return CASL_ENOMEM;
-  CASL_K(k_rb_gather2, g, 256, 0, st)(h->xq, h->yq, npt, rid, rs, hr, cidx, valp, cst, clen, xw, yw,
+  int *tick = reinterpret_cast<int *>(stat + rt + ct), *nmulti = tick + 2, *err = &h->scal->error;
+  const int g = gs(npt);
+  {
+    const FillJob z[1] = {{stat, 2LL * (rt + ct + 2), 0u}};
+    if (int rc = fill_words(st, z, 1)) return rc;
+  }
+  CASL_K(k_rb_runs, rt, 256, 0, st)(h->nextq, npt, tick, stat, rid, rs, re, dtot, err);  // dtot[0] = R
+  CASL_K(k_rb_cycles_pre, g, 256, 0, st)(h->nextq, rid, rs, re, dtot, nr, lab, nrj, hr, val, ishead,
+                                         multi, nmulti);
+  CASL_K(k_rb_cycles_block, 1, 1024, 0, st)(h->nextq, rid, rs, re, dtot, nr, lab, lab2, nrj, nrj2,
+                                            hr, succ, succ2, val, val2, ishead, multi, nmulti);
+  // (the run count is on the device: blocks take tiles until there are none)
+  CASL_K(k_rb_contours, std::min(ct, 2 * 148), 256, 0, st)(ishead, val, rs, lvl, dlev, dtot, tick + 1,
+                                                           stat + rt, cidx, cst, clen, clev,
+                                                           dtot + 1, err);  // dtot[1] = C
+  CASL_K(k_rb_gather2, g, 256, 0, st)(h->xq, h->yq, npt, rid, rs, hr, cidx, val, cst, clen, xw, yw,
                                       cidw);
   int rc = check_launch(h);
   if (rc) return rc;
