@@ -4,8 +4,8 @@
 // node positions and links as it goes, so later tests see earlier
 // reconnections.  The B200 version keeps that exact semantics:
 //   1. Box every segment of every level in parallel (the reference's
-//      nbx = nint(1.2 sqrt(N_lev)) boxes, its bwxi/bwyi scaling and its
-//      per-box list order, restored by sorting each box by node index).
+//      nbx = nint(1.2 sqrt(N_lev)) boxes, its bwxi/bwyi scaling), as linked
+//      lists in any order: a scan takes the lowest list index that passes.
 //   2. Test every node against the segments of its box in parallel on the
 //      unmodified state; nodes with a passing test are marked pending.
 //   3. One warp per level replays the reference loop in node order, but only
@@ -39,14 +39,20 @@ struct LevelDesc {
   double bwxi, bwyi;
 };
 
+// A segment in a box: the box's next entry, the segment's list index (the node
+// before its first) and its first node.  isb < 0: no segment, only the node of
+// list index -2 - isb, which lies in this box (see k_sg_link).
+struct __align__(16) BoxEntry {
+  int next, isb, is, pad;
+};
 struct SurgState {
-  double *xq, *yq, *dx, *dy, *dsq;     // mutable
+  double *xq, *yq, *dx, *dy;           // mutable
   int *nextq;                          // mutable
-  const double *x0, *y0, *dx0, *dy0;   // original
+  const double4 *g0;                   // original x, y, dx, dy of every node
   const int *nq0, *prev0, *lvl;
-  const int *kb1, *bcnt, *bnode;       // segment lists per box
-  const int *bnq;                      // nq0 of each bnode entry
-  const int *nb1, *nbcnt, *nbnode;     // nodes located per box
+  const int *bhead;                    // segments listed per box: first entry (-1: none)
+  const BoxEntry *ent;
+  const int *nbox_of;                  // the box each list index's node lies in
   unsigned char *pending;
   // one bit per window of 512 nodes (a word per 16384) set wherever a
   // pending flag is set, so the replay skips empty windows a word at a time
@@ -96,73 +102,68 @@ __device__ __forceinline__ int node_box(double x, double y, const LevelDesc &L, 
 
 // --- levels (contours.f90:374-394) and box counts (contours.f90:429-454) ----
 // A new level starts where indq increases; contours arrive sorted by level.
-
-
-
-
-// The level table in one block (levels are few, contours ~1e4): level
-// starts where indq increases, their ranks, each level's node range, box
-// counts nint(1.2 sqrt(N_lev)) per side (contours.f90:403-416) and the
-// levels' first global boxes; and endnext, each contour's last node linked
-// to its first (the rest of endnext is -1 on entry).  dtot[0] = levels,
-// dtot[1] = boxes.
+//
+// The level table: level starts, their ranks and node ranges, and endnext,
+// each contour's last node linked to its first (the rest of endnext is -1 on
+// entry).  A thread per contour; a block counts the starts before its own
+// contours itself (coalesced reads of a few thousand words), where one block
+// over all contours took 27 us for 13k of them and 158 us for 53k (an
+// ensemble).  The block that finishes last sizes the boxes: nint(1.2
+// sqrt(N_lev)) per side (contours.f90:403-416) and the levels' first global
+// boxes.  dtot[0] = levels, dtot[1] = boxes; dtot[6] = 0 on entry.
 __global__ void __launch_bounds__(SCAN_BLOCK) k_lv_all(const int *__restrict__ i1q,
                                                        const int *__restrict__ i2q,
                                                        const int *__restrict__ indq, int nq,
-                                                       int npt, Consts c,
-                                                       LevelDesc *__restrict__ lev,
-                                                       int *__restrict__ lidx,
+                                                       int npt, Consts c, LevelDesc *lev,
                                                        int *__restrict__ endnext,
                                                        int *__restrict__ dtot,
                                                        long long nbox_cap,
                                                        int *__restrict__ err) {
   CASL_PDL_ENTRY();
-  __shared__ int tot, carry;
-  const int tid = threadIdx.x;
-  // each thread takes a run of consecutive contours: it counts the level
-  // starts in its run, one block scan numbers them, and a second pass over
-  // the run writes the levels (two rounds of loads instead of one per
-  // 1024 contours)
-  const int per = (nq + SCAN_BLOCK - 1) / SCAN_BLOCK;
-  const int j0 = min(nq, tid * per), j1 = min(nq, j0 + per);
-  int cnt = 0;
-  {
-    int prev = j0 > 0 ? indq[j0 - 1] : 0;
-    for (int j = j0; j < j1; j++) {
-      const int v = indq[j];
-      cnt += j == 0 || v > prev;
-      if (j > 0 && v < prev) atomicExch(err, CASL_EINVAL);
-      prev = v;
-    }
+  __shared__ int tot, carry, last;
+  const int tid = threadIdx.x, b0 = blockIdx.x * SCAN_BLOCK, j = b0 + tid;
+  int before = 0;
+  for (int k = tid; k < b0; k += SCAN_BLOCK) before += k == 0 || indq[k] > indq[k - 1];
+  block_excl_scan<int>(before, &tot);
+  before = tot;
+  __syncthreads();
+  int v = 0, first = 0;
+  if (j < nq) {
+    v = indq[j];
+    const int prev = j > 0 ? indq[j - 1] : 0;
+    first = j == 0 || v > prev;
+    if (j > 0 && v < prev) atomicExch(err, CASL_EINVAL);
   }
-  int lv = block_excl_scan<int>(cnt, &tot) - 1;
-  const int nlev = tot;
-  {
-    int prev = j0 > 0 ? indq[j0 - 1] : 0;
-    for (int j = j0; j < j1; j++) {
-      const int v = indq[j], a = i1q[j], b = i2q[j];
-      const bool first = j == 0 || v > prev;
-      lv += first;
-      lidx[j] = lv;  // the level of contour j
-      endnext[b] = a;  // a contour's last node links back to its first
-      if (first) {
-        lev[lv].ibeg = a;
-        lev[lv].levt = v;
-      }
-      if (j == nq - 1 || indq[j + 1] > v) lev[lv].iend = b;
-      prev = v;
+  const int lv = before + block_excl_scan<int>(first, &tot) + first - 1;
+  if (j < nq) {
+    const int a = i1q[j], b = i2q[j];
+    endnext[b] = a;  // a contour's last node links back to its first
+    if (first) {
+      lev[lv].ibeg = a;
+      lev[lv].levt = v;
     }
+    if (j == nq - 1 || indq[j + 1] > v) lev[lv].iend = b;
+    if (j == nq - 1) dtot[0] = lv + 1;
+  }
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) {
+    last = atomicAdd(&dtot[6], 1) == (int)gridDim.x - 1;
+    carry = 0;
   }
   __syncthreads();
-  if (tid == 0) carry = 0;
-  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const int nlev = __ldcg(&dtot[0]);
   for (int base = 0; base < nlev; base += SCAN_BLOCK) {
     const int L = base + tid;
     int nb = 0;
     LevelDesc d{};
     bool ok = false;
     if (L < nlev) {
-      d = lev[L];
+      d.ibeg = __ldcg(&lev[L].ibeg);
+      d.iend = __ldcg(&lev[L].iend);
+      d.levt = __ldcg(&lev[L].levt);
       if (d.ibeg < 0 || d.iend >= npt || d.iend < d.ibeg) {
         atomicExch(err, CASL_EINVAL);
       } else {
@@ -191,19 +192,17 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_lv_all(const int *__restrict__ i
     __syncthreads();
   }
   if (tid == 0) {
-    dtot[0] = nlev;
     dtot[1] = carry;
     if ((long long)carry > nbox_cap) atomicExch(err, CASL_ECAPACITY);
   }
 }
 
-
-
-// work arrays dx, dy, dsq (contours.f90:397-415) and the original copies
+// work arrays dx, dy (contours.f90:397-415; dsq is dx*dx + dy*dy throughout)
+// and the original state, one 32-byte record per node
 __global__ void k_sg_init(const double *__restrict__ xq, const double *__restrict__ yq,
                           const int *__restrict__ nextq, const int *__restrict__ endnext, int npt,
-                          double *dx, double *dy, double *dsq, double *x0, double *y0,
-                          double *dx0, double *dy0, int *nq0, int *prev0, unsigned char *pending,
+                          double *dx, double *dy, double4 *g0, int *nq0, int *prev0,
+                          unsigned char *pending,
                           const LevelDesc *__restrict__ lev, const int *__restrict__ nlev_dev,
                           int *__restrict__ lvl, Consts c, int *err) {
   CASL_PDL_ENTRY();
@@ -226,9 +225,11 @@ __global__ void k_sg_init(const double *__restrict__ xq, const double *__restric
     double ddx = xx - c.ellx * f_dint(xx * c.hlxi);
     double yy = yq[a] - yi;
     double ddy = yy - c.elly * f_dint(yy * c.hlyi);
-    dx[i] = ddx; dy[i] = ddy; dsq[i] = ddx * ddx + ddy * ddy;
-    dx0[i] = ddx; dy0[i] = ddy;
-    x0[i] = xi; y0[i] = yi;
+    dx[i] = ddx;
+    dy[i] = ddy;
+    double2 *g = reinterpret_cast<double2 *>(g0 + i);
+    g[0] = make_double2(xi, yi);
+    g[1] = make_double2(ddx, ddy);
     int nx = nextq[i];
     if (nx < 0 || nx >= npt) { atomicExch(err, CASL_EINVAL); nx = i; }
     nq0[i] = nx;
@@ -237,149 +238,65 @@ __global__ void k_sg_init(const double *__restrict__ xq, const double *__restric
   }
 }
 
-// Per segment: the number of box entries it makes, and where they start
-// relative to its block's share of the entries.  Block b takes the nodes
-// [b*chunk, (b+1)*chunk) in steps of blockDim.x with a running carry, then
-// takes its share of the entry array with one atomic on the running total
-// (bbase[b]); the entries' order in memory is free, since every box list is
-// read as a set.
-__global__ void k_sg_count_entries(SurgState S, const LevelDesc *__restrict__ lev, int npt,
-                                   int chunk, int *__restrict__ ecount, int *__restrict__ eoff,
-                                   int *__restrict__ bbase, int *__restrict__ ne_tot,
-                                   int *__restrict__ nbox_of, int *__restrict__ nbcnt, Consts c) {
-  CASL_PDL_ENTRY();
-  __shared__ int btot;
-  const int b0 = blockIdx.x * chunk, b1 = min(npt, b0 + chunk);
-  int carry = 0;
-  for (int base = b0; base < b1; base += blockDim.x) {
-    const int ib = base + threadIdx.x;
-    int cnt = 0;
-    if (ib < b1) {
-      LevelDesc L = lev[S.lvl[ib]];
-      int i = S.nq0[ib];
-      int mbx1, mbx2, mby1, mby2;
-      seg_boxes(S.x0[i], S.y0[i], S.dx0[i], S.dy0[i], L, c, mbx1, mbx2, mby1, mby2);
-      cnt = (mbx2 - mbx1 + 1) * (mby2 - mby1 + 1);
-      ecount[ib] = cnt;
-      int nb = node_box(S.x0[i], S.y0[i], L, c);
-      nbox_of[ib] = nb;
-      red_add_s32(&nbcnt[nb], 1);
-    }
-    const int ex = block_excl_scan_any<int>(cnt, &btot);
-    if (ib < b1) eoff[ib] = carry + ex;
-    carry += btot;
-  }
-  if (threadIdx.x == 0) bbase[blockIdx.x] = atomicAdd(ne_tot, carry);
+__device__ __forceinline__ double4 ld_g0(const double4 *p) {
+  const double2 a = reinterpret_cast<const double2 *>(p)[0], b = reinterpret_cast<const double2 *>(p)[1];
+  return make_double4(a.x, a.y, b.x, b.y);
 }
 
-// Start of every box's segment list and of its node list.  Block b takes
-// the boxes [b*chunk, (b+1)*chunk): it sums their counts, takes its share
-// of both lists with one atomic each (box order in memory is free), then
-// scans the counts again (from L2) and writes each start twice, the start
-// itself and the placement cursor.
-__global__ void __launch_bounds__(1024) k_sg_box_alloc(const int *__restrict__ bcnt,
-                                                       const int *__restrict__ nbcnt,
-                                                       const int *__restrict__ nbox_dev,
-                                                       long long nbox_cap, long long chunk,
-                                                       int *__restrict__ kb1,
-                                                       int *__restrict__ cb,
-                                                       int *__restrict__ nb1,
-                                                       int *__restrict__ cn,
-                                                       int *__restrict__ tot) {
-  CASL_PDL_ENTRY();
-  __shared__ unsigned long long btot;
-  __shared__ int bb[2];
-  const long long nbox = *nbox_dev < nbox_cap ? (long long)*nbox_dev : nbox_cap;
-  const long long g0 = (long long)blockIdx.x * chunk;
-  const long long g1 = g0 + chunk < nbox ? g0 + chunk : nbox;
-  if (g0 >= g1) return;
-  // both counts in one word: segment entries in the high half, nodes in the
-  // low half (each total stays below 2^31)
-  auto pack = [&](long long gb) -> unsigned long long {
-    return gb < g1 ? ((unsigned long long)bcnt[gb] << 32) | (unsigned)nbcnt[gb] : 0ull;
-  };
-  unsigned long long sum = 0;
-  for (long long gb = g0 + threadIdx.x; gb < g1; gb += blockDim.x) sum += pack(gb);
-  block_excl_scan_any<unsigned long long>(sum, &btot);
-  if (threadIdx.x == 0) {
-    bb[0] = atomicAdd(&tot[0], (int)(btot >> 32));
-    bb[1] = atomicAdd(&tot[1], (int)(btot & 0xffffffffu));
-  }
-  __syncthreads();
-  unsigned long long carry = ((unsigned long long)(unsigned)bb[0] << 32) | (unsigned)bb[1];
-  for (long long base = g0; base < g1; base += blockDim.x) {
-    const long long gb = base + threadIdx.x;
-    const unsigned long long ex = block_excl_scan_any<unsigned long long>(pack(gb), &btot) + carry;
-    if (gb < g1) {
-      const int k = (int)(ex >> 32), m = (int)(ex & 0xffffffffu);
-      kb1[gb] = k;
-      cb[gb] = k;
-      nb1[gb] = m;
-      cn[gb] = m;
-    }
-    carry += btot;
-  }
-}
-
-__global__ void k_sg_emit(SurgState S, const LevelDesc *__restrict__ lev, int npt,
-                          const int *__restrict__ eoff, const int *__restrict__ bbase, int chunk,
-                          const int *__restrict__ ecount,
-                          long long ne_cap, int *__restrict__ ebox, int *__restrict__ eib,
-                          int *__restrict__ bcnt, Consts c, int *__restrict__ err) {
+// Lists every segment in every box it spans, as linked lists: their order is
+// free (every box list is read as a set) and they hold about two entries, so
+// one exchange on the box's head per entry replaces
+// counting, allotting and placing (at 1.4M nodes five launches of 128 us
+// together, here one of 42; the replay, which now follows the links, went from
+// 26 to 42).  Entry q of segment ib is number q*npt + ib for q < SG_OWN;
+// further ones (a segment over more boxes than that) are taken from a running
+// total.  Past its capacity nothing is written (CASL_ECAPACITY is raised).
+// A box's nodes are found through the segments that start in it.  The box a
+// node is tested in and the first of its segment's are rounded apart, so a
+// node on a box's edge can be in neither: it gets an entry of its own.
+constexpr int SG_OWN = 4;
+__global__ void k_sg_link(const double4 *__restrict__ g0, const int *__restrict__ nq0,
+                          const int *__restrict__ lvl, const LevelDesc *__restrict__ lev, int npt,
+                          long long ne_cap, int *__restrict__ bhead, BoxEntry *__restrict__ ent,
+                          int *__restrict__ nbox_of,
+                          int *__restrict__ extra, Consts c, int *__restrict__ err) {
   CASL_PDL_ENTRY();
   for (int ib = blockIdx.x * blockDim.x + threadIdx.x; ib < npt; ib += gridDim.x * blockDim.x) {
-    LevelDesc L = lev[S.lvl[ib]];
-    int i = S.nq0[ib];
+    const LevelDesc L = lev[lvl[ib]];
+    const int i = nq0[ib];
+    const double4 g = ld_g0(g0 + i);
     int mbx1, mbx2, mby1, mby2;
-    seg_boxes(S.x0[i], S.y0[i], S.dx0[i], S.dy0[i], L, c, mbx1, mbx2, mby1, mby2);
-    long long e = (long long)eoff[ib] + bbase[ib / chunk];
-    // Past the capacity nothing is written (CASL_ECAPACITY is raised): the
-    // offsets tile [0, total) densely, so every entry below the capacity is
-    // written, and the box counts count exactly the entries written.
-    if (e + ecount[ib] > ne_cap) atomicExch(err, CASL_ECAPACITY);
+    seg_boxes(g.x, g.y, g.z, g.w, L, c, mbx1, mbx2, mby1, mby2);
+    const int cnt = (mbx2 - mbx1 + 1) * (mby2 - mby1 + 1);
+    const int nb = node_box(g.x, g.y, L, c);
+    nbox_of[ib] = nb;
+    long long far = 0;  // where this segment's entries beyond SG_OWN start
+    bool own = false;    // the node's own box is among its segment's
+    if (cnt > SG_OWN) {
+      far = (long long)SG_OWN * npt + atomicAdd(extra, cnt - SG_OWN);
+      if (far + cnt - SG_OWN > ne_cap) atomicExch(err, CASL_ECAPACITY);
+    }
+    int q = 0;
     for (int mbx = mbx1; mbx <= mbx2; mbx++) {
-      int mmbx = mbx % L.nbx;
-      for (int mby = mby1; mby <= mby2; mby++) {
-        int gb = L.boxbase + L.nby * mmbx + mby % L.nby;
-        if (e < ne_cap) {
-          ebox[e] = gb;
-          eib[e] = ib;
-          red_add_s32(&bcnt[gb], 1);
-        }
-        e++;
+      const int mmbx = mbx % L.nbx;
+      for (int mby = mby1; mby <= mby2; mby++, q++) {
+        const int gb = L.boxbase + L.nby * mmbx + mby % L.nby;
+        const long long e = q < SG_OWN ? (long long)q * npt + ib : far + q - SG_OWN;
+        own |= gb == nb;
+        if (e < ne_cap)
+          reinterpret_cast<int4 *>(ent)[e] = make_int4(atomicExch(&bhead[gb], (int)e), ib, i, 0);
       }
     }
+    if (!own) {
+      const long long e = (long long)SG_OWN * npt + atomicAdd(extra, 1);
+      if (e < ne_cap)
+        reinterpret_cast<int4 *>(ent)[e] = make_int4(atomicExch(&bhead[nb], (int)e), -2 - ib, i, 0);
+      else
+        atomicExch(err, CASL_ECAPACITY);
+    }
   }
 }
 
-__global__ void k_sg_place(const int *__restrict__ ebox, const int *__restrict__ eib,
-                           const int *__restrict__ ne_dev, long long ne_cap,
-                           int *__restrict__ cursor, const int *__restrict__ nq0,
-                           int *__restrict__ bnode, int *__restrict__ bnq) {
-  CASL_PDL_ENTRY();
-  // the emit pass wrote the entries below the capacity only
-  const long long ne = *ne_dev < ne_cap ? (long long)*ne_dev : ne_cap;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < ne;
-       e += (long long)gridDim.x * blockDim.x) {
-    int gb = ebox[e];
-    int pos = atomicAdd(&cursor[gb], 1);  // starts at the box's list start
-    const int isb = eib[e];
-    bnode[pos] = isb;
-    bnq[pos] = nq0[isb];  // the candidate search reads the segment's end node directly
-  }
-}
-
-__global__ void k_sg_place_nodes(const int *__restrict__ nbox_of, int npt,
-                                 int *__restrict__ cursor,
-                                 int *__restrict__ nbnode) {
-  CASL_PDL_ENTRY();
-  for (int ib = blockIdx.x * blockDim.x + threadIdx.x; ib < npt; ib += gridDim.x * blockDim.x) {
-    int gb = nbox_of[ib];
-    nbnode[atomicAdd(&cursor[gb], 1)] = ib;  // cursor starts at the box's list start
-  }
-}
-
-// Restore the reference's per-box order (ascending node before the segment).
 // The two tests of contours.f90:542-563.
 __device__ __forceinline__ bool surg_test(double xi, double yi, double xs, double ys, double dxs,
                                           double dys, double dsqs, const Consts &c) {
@@ -403,17 +320,19 @@ __global__ void k_sg_candidates(SurgState S, const LevelDesc *__restrict__ lev, 
   for (int ib = blockIdx.x * blockDim.x + threadIdx.x; ib < npt; ib += gridDim.x * blockDim.x) {
     int i = S.nq0[ib];
     int mb = nbox_of[ib];
-    double xi = S.x0[i], yi = S.y0[i];
-    int k0 = S.kb1[mb], k1 = k0 + S.bcnt[mb];
+    const double2 xy = *reinterpret_cast<const double2 *>(S.g0 + i);
+    const double xi = xy.x, yi = xy.y;
     bool hit = false;
-    // the next entry's node index is loaded while this one is tested
-    int isn = k0 < k1 ? S.bnq[k0] : 0;
-    for (int k = k0; k < k1 && !hit; k++) {
-      const int is = isn;
-      if (k + 1 < k1) isn = S.bnq[k + 1];
+    // the next entry is loaded while this one is tested
+    int e = S.bhead[mb];
+    int4 r = e >= 0 ? reinterpret_cast<const int4 *>(S.ent)[e] : make_int4(-1, 0, 0, 0);
+    while (e >= 0 && !hit) {
+      const int is = r.y < 0 ? i : r.z;
+      e = r.x;
+      if (e >= 0) r = reinterpret_cast<const int4 *>(S.ent)[e];
       if (is == ib || is == i) continue;
-      const double dxs = S.dx0[is], dys = S.dy0[is];
-      hit = surg_test(xi, yi, S.x0[is], S.y0[is], dxs, dys, dxs * dxs + dys * dys, c);
+      const double4 g = ld_g0(S.g0 + is);
+      hit = surg_test(xi, yi, g.x, g.y, g.z, g.w, g.z * g.z + g.w * g.w, c);
     }
     S.pending[ib] = hit ? 1 : 0;
     if (hit) atomicOr(&S.wsum[ib >> 14], 1u << ((ib >> 9) & 31));
@@ -436,13 +355,23 @@ __device__ void mark_affected(SurgState &S, const LevelDesc &L, int j, int ib, c
     // boxes listing the segment whose list entry is e
     int i = S.nq0[e];
     int mbx1, mbx2, mby1, mby2;
-    seg_boxes(S.x0[i], S.y0[i], S.dx0[i], S.dy0[i], L, c, mbx1, mbx2, mby1, mby2);
+    const double4 g = ld_g0(S.g0 + i);
+    seg_boxes(g.x, g.y, g.z, g.w, L, c, mbx1, mbx2, mby1, mby2);
     for (int mbx = mbx1; mbx <= mbx2; mbx++) {
       int mmbx = mbx % L.nbx;
       for (int mby = mby1; mby <= mby2; mby++) {
-        int gb = L.boxbase + L.nby * mmbx + mby % L.nby;
-        int s = S.nb1[gb], n = S.nbcnt[gb];
-        for (int k = lane; k < n; k += 32) mark(S, S.nbnode[s + k], ib, L.iend);
+        // the nodes in this box are among the first nodes of its segments
+        const int gb = L.boxbase + L.nby * mmbx + mby % L.nby;
+        for (int e = S.bhead[gb]; e >= 0;) {  // 32 entries at a time, one per lane
+          int my = -1;
+          for (int k = 0; k < 32 && e >= 0; k++) {
+            const int2 r = *reinterpret_cast<const int2 *>(S.ent + e);
+            if (lane == k) my = r.y;
+            e = r.x;
+          }
+          if (my < -1) my = -2 - my;
+          if (my >= 0 && S.nbox_of[my] == gb) mark(S, my, ib, L.iend);
+        }
       }
     }
   }
@@ -462,7 +391,7 @@ __global__ void k_sg_replay(SurgState S, const LevelDesc *__restrict__ lev,
   // other lanes through this SM's L1 after __syncwarp(), and plain cached
   // loads are coherent here.
   const unsigned char *pend = S.pending;
-  double *xq = S.xq, *yq = S.yq, *dx = S.dx, *dy = S.dy, *dsq = S.dsq;
+  double *xq = S.xq, *yq = S.yq, *dx = S.dx, *dy = S.dy;
   int *nextq = S.nextq;
   const double f12 = 0.5;
   int count = 0, npend = 0;
@@ -534,8 +463,7 @@ __global__ void k_sg_replay(SurgState S, const LevelDesc *__restrict__ lev,
     int i = nextq[ib];
     double xi = xq[i], yi = yq[i];
     int mb = node_box(xi, yi, L, c);
-    const int kbeg = S.kb1[mb];
-    const int kend = kbeg + S.bcnt[mb];
+    const int ehead = S.bhead[mb];
     // The reference walks the box's segments in list order and continues
     // after each reconnection with the moved node.  The box list is stored
     // unordered, so each round takes the passing segment with the smallest
@@ -543,12 +471,19 @@ __global__ void k_sg_replay(SurgState S, const LevelDesc *__restrict__ lev,
     int thr = -1;
     while (true) {
       int best = INT_MAX;
-      for (int kk = kbeg + lane; kk < kend; kk += 32) {
-        int isb = S.bnode[kk];
+      for (int e = ehead; e >= 0;) {  // 32 entries of the list at a time, one per lane
+        int isb = -1;
+        for (int k = 0; k < 32 && e >= 0; k++) {
+          const int2 r = *reinterpret_cast<const int2 *>(S.ent + e);
+          if (lane == k) isb = r.y;
+          e = r.x;
+        }
         if (isb > thr && isb < best) {
-          int is = nextq[isb];
-          if (!(is == ib || is == i) && surg_test(xi, yi, xq[is], yq[is], dx[is], dy[is], dsq[is], c))
-            best = isb;
+          const int is = nextq[isb];
+          if (!(is == ib || is == i)) {
+            const double ex = dx[is], ey = dy[is];
+            if (surg_test(xi, yi, xq[is], yq[is], ex, ey, ex * ex + ey * ey, c)) best = isb;
+          }
         }
       }
       for (int o = 16; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
@@ -563,7 +498,7 @@ __global__ void k_sg_replay(SurgState S, const LevelDesc *__restrict__ lev,
         double dely = yy - c.elly * f_dint(yy * c.hlyi);
         double aa = delx * dx[is] + dely * dy[is];
         double dxa, dya;
-        if (dsq[is] + 2.0 * aa < 0.0) {
+        if (dx[is] * dx[is] + dy[is] * dy[is] + 2.0 * aa < 0.0) {
           dxa = f12 * (delx + dx[is]);
           dya = f12 * (dely + dy[is]);
           isb = is;
@@ -578,20 +513,16 @@ __global__ void k_sg_replay(SurgState S, const LevelDesc *__restrict__ lev,
         yq[i] = wrapp(yy, c.elly, c.hlyi, c.oms);
         dx[i] = dx[i] - dxa;
         dy[i] = dy[i] - dya;
-        dsq[i] = dx[i] * dx[i] + dy[i] * dy[i];
         nextq[isb] = i;
         dx[isb] = dx[isb] - dxa;
         dy[isb] = dy[isb] - dya;
-        dsq[isb] = dx[isb] * dx[isb] + dy[isb] * dy[isb];
         xq[is] = xq[i];
         yq[is] = yq[i];
         dx[is] = dx[is] + dxa;
         dy[is] = dy[is] + dya;
-        dsq[is] = dx[is] * dx[is] + dy[is] * dy[is];
         nextq[ib] = is;
         dx[ib] = dx[ib] + dxa;
         dy[ib] = dy[ib] + dya;
-        dsq[ib] = dx[ib] * dx[ib] + dy[ib] * dy[ib];
         tsb = isb;
         inew = is;
         count++;
@@ -915,7 +846,7 @@ int surgery_dev(casl_handle *h) {
   const Consts &c = h->c;
   const int nq = h->nq, npt = h->nptq;
   const long long nbox_cap = 2LL * npt + nq + 64;
-  const long long ne_cap = 16LL * npt + 64;
+  const long long ne_cap = std::min((16LL + SG_OWN) * npt + 64, (long long)INT_MAX);
   size_t need = (size_t)npt * 760 + (size_t)nq * 96 + (size_t)nbox_cap * 24 +
                 (size_t)ne_cap * 16 + ((size_t)64 << 20);
   int rc = ensure_scratch(h, need);
@@ -925,60 +856,38 @@ int surgery_dev(casl_handle *h) {
   Trace tr;
   tr.begin(st, "start");
   // levels and boxes, on the device
-  int *lex = ar.get<int>(nq);
   LevelDesc *dlev = ar.get<LevelDesc>(nq);
-  // [0] nlev, [1] nbox, [2] ne, [3] nsurg, [4] box segment entries, [5] box nodes
+  // [0] nlev, [1] nbox, [2] entries beyond the segments' own, [3] nsurg, [6] blocks done
   int *dtot = ar.get<int>(16);
   int *endnext = ar.get<int>(npt), *lvl = ar.get<int>(npt);
-  double *dx = ar.get<double>(npt), *dy = ar.get<double>(npt), *dsq = ar.get<double>(npt);
-  double *x0 = ar.get<double>(npt), *y0 = ar.get<double>(npt);
-  double *dx0 = ar.get<double>(npt), *dy0 = ar.get<double>(npt);
+  double *dx = ar.get<double>(npt), *dy = ar.get<double>(npt);
+  double4 *g0 = ar.get<double4>(npt);
   int *nq0 = ar.get<int>(npt), *prev0 = ar.get<int>(npt);
   unsigned char *pending = ar.get<unsigned char>(npt + 16);
   unsigned int *wsum = ar.get<unsigned int>((npt >> 14) + 2);
-  int *ecount = ar.get<int>(npt), *eoff = ar.get<int>(npt), *nbox_of = ar.get<int>(npt);
-  int *bcnt = ar.get<int>(nbox_cap), *kb1 = ar.get<int>(nbox_cap), *cursor = ar.get<int>(nbox_cap);
-  int *nbcnt = ar.get<int>(nbox_cap), *nb1 = ar.get<int>(nbox_cap), *nbnode = ar.get<int>(npt);
-  int *ncursor = ar.get<int>(nbox_cap), *bbase = ar.get<int>(148 * 16 + 1);
-  int *ebox = ar.get<int>(ne_cap), *eib = ar.get<int>(ne_cap), *bnode = ar.get<int>(ne_cap);
-  int *bnq = ar.get<int>(ne_cap);
+  int *nbox_of = ar.get<int>(npt), *bhead = ar.get<int>(nbox_cap);
+  BoxEntry *ent = ar.get<BoxEntry>(ne_cap);
   if (ar.failed) return CASL_ENOMEM;
-  const int g = gs(npt), gb = gs(nbox_cap);
+  const int g = gs(npt);
   {
-    const FillJob z[5] = {{endnext, npt, 0xffffffffu},
-                          {bcnt, nbox_cap, 0u},
-                          {nbcnt, nbox_cap, 0u},
+    const FillJob z[4] = {{endnext, npt, 0xffffffffu},
+                          {bhead, nbox_cap, 0xffffffffu},
                           {wsum, (npt >> 14) + 2, 0u},
-                          {dtot + 2, 4, 0u}};
-    if (int rc = fill_words(st, z, 5)) return rc;
+                          {dtot + 2, 5, 0u}};
+    if (int rc = fill_words(st, z, 4)) return rc;
   }
-  CASL_K(k_lv_all, 1, SCAN_BLOCK, 0, st)(h->i1q, h->i2q, h->indq, nq, npt, c, dlev, lex, endnext,
-                                         dtot, nbox_cap, err);
-  CASL_K(k_sg_init, g, 256, 0, st)(h->xq, h->yq, h->nextq, endnext, npt, dx, dy, dsq, x0, y0, dx0,
-                                   dy0, nq0, prev0, pending, dlev, dtot, lvl, c, err);
+  CASL_K(k_lv_all, (nq + SCAN_BLOCK - 1) / SCAN_BLOCK, SCAN_BLOCK, 0, st)(
+      h->i1q, h->i2q, h->indq, nq, npt, c, dlev, endnext, dtot, nbox_cap, err);
+  CASL_K(k_sg_init, g, 256, 0, st)(h->xq, h->yq, h->nextq, endnext, npt, dx, dy, g0, nq0, prev0,
+                                   pending, dlev, dtot, lvl, c, err);
+  CASL_K(k_sg_link, g, 256, 0, st)(g0, nq0, lvl, dlev, npt, ne_cap, bhead, ent, nbox_of, dtot + 2, c,
+                                   err);
   SurgState S{};
-  S.xq = h->xq; S.yq = h->yq; S.dx = dx; S.dy = dy; S.dsq = dsq; S.nextq = h->nextq;
-  S.x0 = x0; S.y0 = y0; S.dx0 = dx0; S.dy0 = dy0; S.nq0 = nq0; S.prev0 = prev0; S.lvl = lvl;
+  S.xq = h->xq; S.yq = h->yq; S.dx = dx; S.dy = dy; S.nextq = h->nextq;
+  S.g0 = g0; S.nq0 = nq0; S.prev0 = prev0; S.lvl = lvl;
+  S.bhead = bhead; S.ent = ent; S.nbox_of = nbox_of;
   S.pending = pending;
   S.wsum = wsum;
-  // count_entries: at most 148*16 blocks, each a whole number of 256-node steps
-  const int echunk = (int)((((long long)npt + g - 1) / g + 255) / 256 * 256);
-  const int eg = (int)(((long long)npt + echunk - 1) / echunk);
-  CASL_K(k_sg_count_entries, eg, 256, 0, st)(S, dlev, npt, echunk, ecount, eoff, bbase, dtot + 2,
-                                             nbox_of, nbcnt, c);
-  CASL_K(k_sg_emit, g, 256, 0, st)(S, dlev, npt, eoff, bbase, echunk, ecount, ne_cap, ebox, eib,
-                                   bcnt, c, err);
-  {
-    // boxes in 296 chunks (two blocks of 1024 per SM), each a whole number
-    // of 1024-box steps
-    const long long bchunk = ((nbox_cap + 295) / 296 + 1023) / 1024 * 1024;
-    const int bg = (int)((nbox_cap + bchunk - 1) / bchunk);
-    CASL_K(k_sg_box_alloc, bg, 1024, 0, st)(bcnt, nbcnt, dtot + 1, nbox_cap, bchunk, kb1, cursor,
-                                            nb1, ncursor, dtot + 4);
-  }
-  CASL_K(k_sg_place, gs(ne_cap), 256, 0, st)(ebox, eib, dtot + 2, ne_cap, cursor, nq0, bnode, bnq);
-  CASL_K(k_sg_place_nodes, g, 256, 0, st)(nbox_of, npt, ncursor, nbnode);
-  S.kb1 = kb1; S.bcnt = bcnt; S.bnode = bnode; S.bnq = bnq; S.nb1 = nb1; S.nbcnt = nbcnt; S.nbnode = nbnode;
   tr.point("binning");
   CASL_K(k_sg_candidates, g, 256, 0, st)(S, dlev, npt, nbox_of, c);
   tr.point("candidates");
