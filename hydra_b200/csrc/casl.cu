@@ -551,6 +551,13 @@ __device__ __forceinline__ void c2g_decode(unsigned long long w, int &c0, int &c
   v = (v - c2) >> 16;
   c3 = (int)v;
 }
+// The same four rows as four 32-bit counts.
+__device__ __forceinline__ void c2g_decode(int4 w, int &c0, int &c1, int &c2, int &c3) {
+  c0 = w.x;
+  c1 = w.y;
+  c2 = w.z;
+  c3 = w.w;
+}
 
 // Member of node i in an ensemble (mnode[m] <= i < mnode[m+1]; members
 // without nodes have equal bounds and are skipped); 0 without an ensemble.
@@ -785,7 +792,8 @@ __global__ void k_c2g_coarsen(const int *__restrict__ L, int *__restrict__ C,
 // levels L(4cy-3 .. 4cy+3) follow: L(4cy-1) = lbot + ex, one count taken or
 // added per row on either side.  G passes through shared memory to the
 // 7-tap along x.  Coarse row 0 wraps to the top rows and is formed last.
-// Requires n % RPS == 0.
+// Requires n % RPS == 0.  W: four rows' counts in 64 bits, or as an int4 where
+// the caller's levels have no bound (c2g_sum32).
 #define C2G_CW 7
 #define C2G_FC (4 * C2G_CW + 3)
 
@@ -817,8 +825,8 @@ __device__ __forceinline__ void c2g_feature(int *__restrict__ F, int n, int cx0,
   }
 }
 
-template <int U>
-__global__ void __launch_bounds__(1024) k_c2g_packed_sum(const unsigned long long *__restrict__ JW,
+template <int U, class W = unsigned long long>
+__global__ void __launch_bounds__(1024) k_c2g_packed_sum(const W *__restrict__ JW,
                                                          const int *__restrict__ ljx,
                                                          int *__restrict__ C,
                                                          unsigned long long *__restrict__ csum,
@@ -843,9 +851,9 @@ __global__ void __launch_bounds__(1024) k_c2g_packed_sum(const unsigned long lon
   int col = 4 * cx0 - 3 + warp;  // this warp's fine column (0-based), wrapped
   if (col < 0) col += nf;
   if (col >= nf) col -= nf;
-  const unsigned long long *cp = JW + (long long)col * n + lane;
+  const W *cp = JW + (long long)col * n + lane;
   const int nsteps = n / RPS;
-  unsigned long long v[U];
+  W v[U];
   if (warp < C2G_FC) {
 #pragma unroll
     for (int u = 0; u < U; u++) v[u] = __ldcs(cp + u * 32);
@@ -985,6 +993,21 @@ static int grid_for(long long work, int block = 256) {
   if (g < 1) g = 1;
   if (g > 148 * 16) g = 148 * 16;
   return (int)g;
+}
+
+// Coarse cells and their sum from 32-bit jump counts (row 0 of every fine
+// column zero) and bottom-row jumps; *csum must be zero.  n a power of two,
+// 32 or more.
+void c2g_sum32(cudaStream_t st, const int4 *J4, const int *ljx, int *C, unsigned long long *csum,
+               int n) {
+  const C2GMembers mb{nullptr, 1, 0, 0, 0};
+  const int nblk = (n + C2G_CW - 1) / C2G_CW, nf = 4 * n;
+  if (n >= 128)
+    CASL_K((k_c2g_packed_sum<4, int4>), nblk, 1024, 0, st)(J4, ljx, C, csum, n, nf, mb, nullptr);
+  else if (n == 64)
+    CASL_K((k_c2g_packed_sum<2, int4>), nblk, 1024, 0, st)(J4, ljx, C, csum, n, nf, mb, nullptr);
+  else
+    CASL_K((k_c2g_packed_sum<1, int4>), nblk, 1024, 0, st)(J4, ljx, C, csum, n, nf, mb, nullptr);
 }
 
 int con2grid_dev(casl_handle *h, bool want_levels) {

@@ -327,9 +327,10 @@ int casl_genfg(casl_handle *h, int ix1v, int nxv, int iy1v, int nyv, int stride,
  * that context only, and not across a cudaDeviceReset.  An error the caller
  * left pending in the runtime (cudaPeekAtLastError) makes the call return
  * CASL_ECUDA at once and is left in place for the caller.
- * All calls on a device share the array and it keeps the last call's
- * contents (the call clears what must start at zero), so calls that overlap
- * on the GPU (e.g. on two streams at once) race.  `stream` is a cudaStream_t
+ * All calls on a device share the array (a call that succeeds leaves its
+ * counts cleared for the next; after one that did not, or that overlapped
+ * another, the next call clears them), so calls that overlap on the GPU (e.g.
+ * on two streams at once) race.  `stream` is a cudaStream_t
  * (NULL = default stream); the call synchronises it before returning. */
 int casl_con2grid_noalloc(int n, double ellx, double elly, int nptq, double qjump,
                           const double *xq_dev, const double *yq_dev, const int *nextq_dev,
