@@ -2410,6 +2410,7 @@ static void free_all(casl_handle *h) {
   free(h->spmf_h);
   free(h->alk_h);
   if (h->hscal) cudaFreeHost(h->hscal);
+  if (h->hpin) cudaFreeHost(h->hpin);
 }
 
 int casl_create(const casl_params *p, int device, casl_handle **out) {

@@ -7,6 +7,7 @@
 // outcomes (crossing cells, box indices, surgery decisions) are reproduced.
 #pragma once
 
+#include <string.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -112,6 +113,20 @@ __device__ __forceinline__ void red_add_u64(unsigned long long *p, unsigned long
 __device__ __forceinline__ void red_add_s32(int *p, int v) {
   asm volatile("red.relaxed.gpu.global.add.s32 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "r"(v)
                : "memory");
+}
+
+// Doubles as words of the same order (no NaN), for integer maxima; 0 lies
+// below every one of them.
+__host__ __device__ __forceinline__ unsigned long long ordered_word(double x) {
+  unsigned long long b;
+  memcpy(&b, &x, 8);
+  return b >> 63 ? ~b : b | 1ULL << 63;
+}
+__host__ __device__ __forceinline__ double from_ordered(unsigned long long w) {
+  const unsigned long long b = w >> 63 ? w & ~(1ULL << 63) : ~w;
+  double x;
+  memcpy(&x, &b, 8);
+  return x;
 }
 
 // Device-resident scalars of one simulation (variables.f90 and adapt()).

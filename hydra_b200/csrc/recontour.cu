@@ -146,11 +146,16 @@ __device__ __forceinline__ double qtmp_of(int lev, const LevInfo &li) {
 // <= v.  qtmp is increasing in l (also as rounded), so an edge with end
 // values lo < hi crosses exactly the levels c(lo) < l <= c(hi): those where
 // the reference's sign(qa - qtmp) differs at the two ends (congen.f90:205-212).
-__device__ __forceinline__ int level_index(double v, const LevInfo &li) {
-  int l = (int)floor((v + li.qoff) * li.qjumpi + 0.5);
-  while (qtmp_of(l + 1, li) <= v) l++;
-  while (qtmp_of(l, li) > v) l--;
+// The index is wanted within 0..65535 (the caller clips it), so the steps stop
+// beyond both ends: they end for a qjump of zero or a value that is not finite.
+__device__ __forceinline__ int level_steps(int l, double v, const LevInfo &li) {
+  l = min(max(l, -1), 65536);
+  while (l < 65536 && qtmp_of(l + 1, li) <= v) l++;
+  while (l >= 0 && qtmp_of(l, li) > v) l--;
   return l;
+}
+__device__ __forceinline__ int level_index(double v, const LevInfo &li) {
+  return level_steps((int)floor((v + li.qoff) * li.qjumpi + 0.5), v, li);
 }
 
 // level_index with the exact checks only near a level boundary: the
@@ -161,11 +166,9 @@ __device__ __forceinline__ int level_index(double v, const LevInfo &li) {
 __device__ __forceinline__ int level_index_fast(double v, const LevInfo &li) {
   const double x = (v + li.qoff) * li.qjumpi + 0.5;
   const double fl = floor(x), fr = x - fl;
-  int l = (int)fl;
+  const int l = (int)fl;
   if (fr > 1.0e-6 && fr < 1.0 - 1.0e-6) return l;
-  while (qtmp_of(l + 1, li) <= v) l++;
-  while (qtmp_of(l, li) > v) l--;
-  return l;
+  return level_steps(l, v, li);
 }
 
 // One element of the ultra-fine field: (L*qjump - qavg) + bilinear residual,
@@ -225,12 +228,12 @@ __device__ __forceinline__ double ufield_at(const UField &u, double qavg, int ix
 __global__ void __launch_bounds__(256, 4) k_u_field(const int *__restrict__ L, const unsigned long long *__restrict__ lsum,
                           const double *__restrict__ qq, double qjump, int have_contours,
                           LevInfo lq, double *__restrict__ qa, unsigned short *__restrict__ lc,
-                          double *__restrict__ part, Consts c, double bnc) {
+                          unsigned long long *__restrict__ ext, Consts c, double bnc) {
   CASL_PDL_ENTRY();
   const int nxu = c.nxu, nyu = c.nyu, n = c.nx;
   const long long nruns = (long long)nxu * (nyu / 16);
   const double qavg = ufield_qavg(lsum, qjump, have_contours, nxu, nyu);
-  double mx = -1.0e308, mn = 1.0e308;
+  double mx = -1.0e308, mn = 1.0e308, l1 = 0.0;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < nruns;
        t += (long long)gridDim.x * blockDim.x) {
     const int iyy = (int)(t % (nyu / 16)), ix = (int)(t / (nyu / 16)) + 1;
@@ -239,6 +242,7 @@ __global__ void __launch_bounds__(256, 4) k_u_field(const int *__restrict__ L, c
     const int iy0 = 1 + iyy, iy1 = 2 + iyy - n * (iy0 / n);
     const double q00 = qq[(long long)(ix0 - 1) * n + iy0 - 1], q10 = qq[(long long)(ix0 - 1) * n + iy1 - 1];
     const double q01 = qq[(long long)(ix1 - 1) * n + iy0 - 1], q11 = qq[(long long)(ix1 - 1) * n + iy1 - 1];
+    if (ixf == 1) l1 += fabs(q00);  // every residual point once
     const long long base = (long long)(ix - 1) * nyu + 16LL * iyy;
     // the run in two halves of 8 points (fewer live registers)
 #pragma unroll 1
@@ -278,20 +282,30 @@ __global__ void __launch_bounds__(256, 4) k_u_field(const int *__restrict__ L, c
         reinterpret_cast<uint4 *>(lc + base)[hf] = make_uint4(code[0], code[1], code[2], code[3]);
     }
   }
-  __shared__ double a[256], b[256];
-  a[threadIdx.x] = mx;
-  b[threadIdx.x] = mn;
-  __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if (threadIdx.x < o) {
-      a[threadIdx.x] = fmax(a[threadIdx.x], a[threadIdx.x + o]);
-      b[threadIdx.x] = fmin(b[threadIdx.x], b[threadIdx.x + o]);
-    }
-    __syncthreads();
+  // extremes and sum of |residual|: ext[0] the largest value's ordered word,
+  // ext[1] the complement of the smallest's, ext[2] the sum (a double), all 0
+  // on entry
+  __shared__ double a[8], b[8], w[8];
+  for (int o = 16; o > 0; o >>= 1) {
+    mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+    l1 += __shfl_xor_sync(0xffffffffu, l1, o);
   }
+  if ((threadIdx.x & 31) == 0) {
+    a[threadIdx.x >> 5] = mx;
+    b[threadIdx.x >> 5] = mn;
+    w[threadIdx.x >> 5] = l1;
+  }
+  __syncthreads();
   if (threadIdx.x == 0) {
-    part[2 * blockIdx.x] = a[0];
-    part[2 * blockIdx.x + 1] = b[0];
+    for (int k = 1; k < 8; k++) {
+      mx = fmax(mx, a[k]);
+      mn = fmin(mn, b[k]);
+      l1 += w[k];
+    }
+    atomicMax(&ext[0], ordered_word(mx));
+    atomicMax(&ext[1], ~ordered_word(mn));
+    if (!have_contours) atomicAdd(reinterpret_cast<double *>(ext + 2), l1);
   }
 }
 
@@ -497,12 +511,53 @@ static inline int gsz(long long work) {
     if (_r) return _r;   \
   } while (0)
 
-static int fetch_err(casl_handle *h) {
-  int e = 0;
-  cudaMemcpyAsync(&e, &h->scal->error, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
-  cudaError_t ce = cudaStreamSynchronize(h->stream);
-  if (ce != cudaSuccess) return set_cuda_error(h, ce);
-  return e;
+// Small device results for the host: all of them, and the error word, land in
+// pinned memory behind one wait.  Copies to the caller's own variables are
+// staged by the driver one after the other, 20 us each.  What does not fit
+// goes to its destination directly.  Returns the error word.
+struct ReadItem {
+  void *dst;
+  const void *src;
+  size_t bytes;
+};
+static int read_back(casl_handle *h, std::initializer_list<ReadItem> items) {
+  constexpr size_t cap = 256 << 10;
+  cudaStream_t st = h->stream;
+  if (!h->hpin && cudaMallocHost(&h->hpin, cap) != cudaSuccess) {
+    cudaGetLastError();
+    h->hpin = nullptr;
+  }
+  int err = 0;
+  size_t off = 16;  // the error word lies first
+  std::vector<size_t> at;
+  for (const ReadItem &r : items) {
+    const bool fits = h->hpin && off + r.bytes <= cap;
+    at.push_back(fits && r.bytes ? off : 0);
+    if (!r.bytes) continue;
+    CASL_CUDA_TRY(cudaMemcpyAsync(fits ? h->hpin + off : r.dst, r.src, r.bytes,
+                                  cudaMemcpyDeviceToHost, st));
+    if (fits) off += (r.bytes + 15) / 16 * 16;
+  }
+  CASL_CUDA_TRY(cudaMemcpyAsync(h->hpin ? (void *)h->hpin : &err, &h->scal->error, sizeof(int),
+                                cudaMemcpyDeviceToHost, st));
+  CASL_CUDA_TRY(cudaStreamSynchronize(st));
+  if (h->hpin) memcpy(&err, h->hpin, sizeof(int));
+  size_t k = 0;
+  for (const ReadItem &r : items) {
+    if (at[k]) memcpy(r.dst, h->hpin + at[k], r.bytes);
+    k++;
+  }
+  return err;
+}
+
+// l1norm (generic.f90:180-194) of the residual, summed as the reference does
+static int l1_host(casl_handle *h, const double *qq, double *l1) {
+  std::vector<double> hq((size_t)h->c.nx * h->c.ny);
+  CASL_CUDA_TRY(cudaMemcpyAsync(hq.data(), qq, hq.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+  CASL_CUDA_TRY(cudaStreamSynchronize(h->stream));
+  *l1 = 0.0;
+  for (double v : hq) *l1 += fabs(v);
+  return CASL_OK;
 }
 
 int recontour_dev(casl_handle *h, const double *qq) {
@@ -531,42 +586,46 @@ int recontour_dev(casl_handle *h, const double *qq) {
   } flush_at_exit{tr};
 
   // --- 1. ultra-fine field ---------------------------------------------------
-  if (!have && !econ) {
-    // l1norm (generic.f90:180-194) of the full field: nothing to contour if ~0
-    std::vector<double> hq((size_t)c.nx * c.ny);
-    CASL_CUDA_TRY(cudaMemcpyAsync(hq.data(), qq, hq.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+  auto set_empty = [&]() -> int {
+    h->nq = h->nptq = 0;
+    h->hscal->nq = h->hscal->nptq = 0;
+    int z[2] = {0, 0};
+    CASL_CUDA_TRY(cudaMemcpyAsync(&h->scal->nq, z, 2 * sizeof(int), cudaMemcpyHostToDevice, st));
     CASL_CUDA_TRY(cudaStreamSynchronize(st));
+    return CASL_OK;
+  };
+  // nothing to contour if l1norm (generic.f90:180-194) of the full field is
+  // ~0.  k_u_field sums it beside the level codes; with no interval to speak
+  // of (a field of zeros has none) the codes mean nothing and the host sums.
+  if (!have && !econ && !(qjump > 1.0e-200)) {
     double l1 = 0.0;
-    for (double v : hq) l1 += fabs(v);
-    if (c.garea * l1 < c.small) {
-      h->nq = h->nptq = 0;
-      h->hscal->nq = h->hscal->nptq = 0;
-      int z[2] = {0, 0};
-      int *dz = &h->scal->nq;
-      CASL_CUDA_TRY(cudaMemcpyAsync(dz, z, 2 * sizeof(int), cudaMemcpyHostToDevice, st));
-      CASL_CUDA_TRY(cudaStreamSynchronize(st));
-      return CASL_OK;
-    }
+    RC_TRY(l1_host(h, qq, &l1));
+    if (c.garea * l1 < c.small) return set_empty();
   }
   // Field memory: level codes + integer levels + per-chunk crossing counts;
   // kept for the whole call.
   const long long nchunks_f = 2 * NU / 16;
   size_t need_field = (size_t)NU * 6 + (size_t)nchunks_f * 8 + (size_t)nxu * 4 +
                       (size_t)nyu * 16 + ((size_t)64 << 20);
-  RC_TRY(ensure_scratch(h, need_field));
+  if (int rc = ensure_scratch(h, need_field)) {
+    // a field of zeros needs no memory
+    double l1 = 1.0;
+    if (!have && !econ) RC_TRY(l1_host(h, qq, &l1));
+    if (c.garea * l1 < c.small) return set_empty();
+    return rc;
+  }
   Arena ar{(char *)h->sx, h->sx_bytes, 0};
   unsigned short *lc = ar.get<unsigned short>(NU);
   int *Lu = ar.get<int>(NU);
   int *ljx = ar.get<int>(nxu);
-  unsigned long long *lsum = ar.get<unsigned long long>(4);
-  double *part = ar.get<double>(2 * 4096);
+  unsigned long long *lsum = ar.get<unsigned long long>(4);  // level sum; k_u_field's results
   double *rmn = ar.get<double>(nyu), *rmx = ar.get<double>(nyu);
   int *dtot = ar.get<int>(16);
   if (ar.failed) return CASL_ENOMEM;
+  CASL_CUDA_TRY(cudaMemsetAsync(lsum, 0, 4 * sizeof(unsigned long long), st));
   if (have) {
     CASL_CUDA_TRY(cudaMemsetAsync(Lu, 0, (size_t)NU * sizeof(int), st));
     CASL_CUDA_TRY(cudaMemsetAsync(ljx, 0, (size_t)nxu * sizeof(int), st));
-    CASL_CUDA_TRY(cudaMemsetAsync(lsum, 0, sizeof(unsigned long long), st));
     tr.point("u_memset");
     CASL_K(k_u_scatter, gsz(h->nptq), 256, 0, st)(h->xq, h->yq, h->nextq, h->nptq, qjump, Lu, ljx, c,
                                               &h->scal->error);
@@ -581,17 +640,21 @@ int recontour_dev(casl_handle *h, const double *qq) {
   li.qjumpi = 1.0 / qjump;
   li.qoff = qjump * (double)h->p.nlevm;
   li.levbeg = li.levend = 0;
-  const int fb = 4096;
-  CASL_K(k_u_field, fb, 256, 0, st)(Lu, lsum, qq, qjump, have, li, nullptr, lc, part, c, bnc);
+  CASL_K(k_u_field, 4096, 256, 0, st)(Lu, lsum, qq, qjump, have, li, nullptr, lc, lsum + 1, c, bnc);
   RC_TRY(check_launch(h));
-  RC_TRY(fetch_err(h));
-  std::vector<double> hp(2 * fb);
-  CASL_CUDA_TRY(cudaMemcpyAsync(hp.data(), part, hp.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-  CASL_CUDA_TRY(cudaStreamSynchronize(st));
-  double qamax = hp[0], qamin = hp[1];
-  for (int b = 1; b < fb; b++) {
-    qamax = std::max(qamax, hp[2 * b]);
-    qamin = std::min(qamin, hp[2 * b + 1]);
+  double qamax = 0.0, qamin = 0.0;
+  if (!econ) {
+    unsigned long long ext[3];
+    RC_TRY(read_back(h, {{ext, lsum + 1, sizeof(ext)}}));
+    qamax = from_ordered(ext[0]);
+    qamin = from_ordered(~ext[1]);
+    if (!have) {
+      // the device sums in another order: close to the line the host decides
+      double l1;
+      memcpy(&l1, &ext[2], 8);
+      if (fabs(c.garea * l1 - c.small) <= 1.0e-9 * c.small) RC_TRY(l1_host(h, qq, &l1));
+      if (c.garea * l1 < c.small) return set_empty();
+    }
   }
   tr.point("field");
   const UField uf{have ? Lu : nullptr, lsum, qq, qjump, have, bnc};
@@ -601,9 +664,8 @@ int recontour_dev(casl_handle *h, const double *qq) {
   if (econ) {
     CASL_K(k_u_rowmm, nyu / 16, 256, 0, st)(uf, c, rmn, rmx);
     std::vector<double> qqmin(nyu + 2), qqmax(nyu + 2);
-    CASL_CUDA_TRY(cudaMemcpyAsync(qqmin.data() + 1, rmn, nyu * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CASL_CUDA_TRY(cudaMemcpyAsync(qqmax.data() + 1, rmx, nyu * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CASL_CUDA_TRY(cudaStreamSynchronize(st));
+    RC_TRY(read_back(h, {{qqmin.data() + 1, rmn, nyu * sizeof(double)},
+                         {qqmax.data() + 1, rmx, nyu * sizeof(double)}}));
     qqmin[nyu + 1] = qqmin[1] + ppvdif;
     qqmax[nyu + 1] = qqmax[1] + ppvdif;
     qamin = qqmin[1];
@@ -644,13 +706,6 @@ int recontour_dev(casl_handle *h, const double *qq) {
   li.levend = (int)((li.qoff + qamax) * li.qjumpi + 0.5);
   // the level codes hold 0..65535: levels must lie inside
   if (li.levbeg <= li.levend && (li.levbeg < 1 || li.levend > 65534)) return CASL_ECAPACITY;
-  auto set_empty = [&]() -> int {
-    h->nq = h->nptq = 0;
-    int z[2] = {0, 0};
-    CASL_CUDA_TRY(cudaMemcpyAsync(&h->scal->nq, z, 2 * sizeof(int), cudaMemcpyHostToDevice, st));
-    CASL_CUDA_TRY(cudaStreamSynchronize(st));
-    return CASL_OK;
-  };
   if (li.levbeg > li.levend) return set_empty();
   const int nlev = li.levend - li.levbeg + 1;
 
@@ -706,8 +761,7 @@ int recontour_dev(casl_handle *h, const double *qq) {
   // the offset after the last chunk
   CASL_CUDA_TRY(cudaMemcpyAsync(coffs + nchunks, dtot, sizeof(int), cudaMemcpyDeviceToDevice, st));
   int ncr_i = 0;
-  CASL_CUDA_TRY(cudaMemcpyAsync(&ncr_i, dtot, sizeof(int), cudaMemcpyDeviceToHost, st));
-  CASL_CUDA_TRY(cudaStreamSynchronize(st));
+  RC_TRY(read_back(h, {{&ncr_i, dtot, sizeof(int)}}));
   const long long ncr = ncr_i;
   if (tr.on) fprintf(stderr, "[casl trace] recontour: %lld crossings on %d levels\n", ncr, nlev);
   if (ncr == 0) return set_empty();
@@ -750,8 +804,7 @@ int recontour_dev(casl_handle *h, const double *qq) {
   CASL_K(k_tr_walk, ntile, TR_NT, sizeof(TrSmem), st)(ta);
   RC_TRY(check_launch(h));
   int cnts[2] = {0, 0};
-  CASL_CUDA_TRY(cudaMemcpyAsync(cnts, ta.nchain, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
-  RC_TRY(fetch_err(h));
+  RC_TRY(read_back(h, {{cnts, ta.nchain, 2 * sizeof(int)}}));
   const int S = cnts[0], nends = cnts[1];
   if (S <= 0) return CASL_EINVAL;
   if (tr.on)
@@ -792,12 +845,9 @@ int recontour_dev(casl_handle *h, const double *qq) {
   int C0 = 0;
   std::vector<int> eidx(nends);
   std::vector<long long> eslot(nends);
-  if (nends > 0) {
-    CASL_CUDA_TRY(cudaMemcpyAsync(eidx.data(), ta.eidx, nends * sizeof(int), cudaMemcpyDeviceToHost, st));
-    CASL_CUDA_TRY(cudaMemcpyAsync(eslot.data(), ta.eslot, nends * sizeof(long long), cudaMemcpyDeviceToHost, st));
-  }
-  CASL_CUDA_TRY(cudaMemcpyAsync(&C0, dtot + 4, sizeof(int), cudaMemcpyDeviceToHost, st));
-  RC_TRY(fetch_err(h));
+  RC_TRY(read_back(h, {{&C0, dtot + 4, sizeof(int)},
+                       {eidx.data(), ta.eidx, nends * sizeof(int)},
+                       {eslot.data(), ta.eslot, nends * sizeof(long long)}}));
   tr.point("ranking");
   // --- 6. lists between saddles: exact simulation of the reference traversal -------
   // Only the crossings entering saddle boxes and the list starts come to the
@@ -822,8 +872,7 @@ int recontour_dev(casl_handle *h, const double *qq) {
     if (ar2.failed) return CASL_ENOMEM;
     CASL_CUDA_TRY(cudaMemcpyAsync(d_idx, cstart.data(), nch * sizeof(int), cudaMemcpyHostToDevice, st));
     CASL_K(k_ch_query, gsz(nch), 256, 0, st)(d_idx, nch, ta.own, jA, lA, ta.chain, ta.clev, d_out);
-    CASL_CUDA_TRY(cudaMemcpyAsync(q.data(), d_out, q.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
-    CASL_CUDA_TRY(cudaStreamSynchronize(st));
+    RC_TRY(read_back(h, {{q.data(), d_out, q.size() * sizeof(int)}}));
     const int *cend = &q[0], *clen = &q[nch], *cmin = &q[2 * (size_t)nch],
               *val_at_min = &q[3 * (size_t)nch], *clev = &q[4 * (size_t)nch],
               *clast = &q[5 * (size_t)nch];
@@ -960,8 +1009,7 @@ int recontour_dev(casl_handle *h, const double *qq) {
     exclusive_scan<int>(st, klen, koff, C, tmpi2, dtot + 6);
     exclusive_scan<int>(st, kone, kidx, C, tmpi2, dtot + 7);
     int kc[2] = {0, 0};
-    CASL_CUDA_TRY(cudaMemcpyAsync(kc, dtot + 6, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
-    CASL_CUDA_TRY(cudaStreamSynchronize(st));
+    RC_TRY(read_back(h, {{kc, dtot + 6, 2 * sizeof(int)}}));
     if (kc[1] == 0) return set_empty();
     const double yoff = c.hly + c.elly * (double)eg.nby;
     CASL_K(k_ec_compact, gsz(ncr), 256, 0, st)(xw, yw, cidw, ncr, coff, klen, koff, kidx, c, yoff, xw2,
@@ -992,8 +1040,7 @@ int recontour_dev(casl_handle *h, const double *qq) {
     size_t mark = ar2.off;
     RC_TRY(renode_batch(h, ar2, cur, out, RENODE_PLAIN));
     ar2.off = mark;
-    CASL_CUDA_TRY(cudaMemcpyAsync(hc, cnt, 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
-    CASL_CUDA_TRY(cudaStreamSynchronize(st));
+    RC_TRY(read_back(h, {{hc, cnt, 3 * sizeof(int)}}));
     if (hc[2]) return CASL_ECAPACITY;
     if (hc[0] == 0) return set_empty();
     cur = RenodeIn{out.xo, out.yo, out.ocs, out.olen, out.olev, hc[0], hc[1]};
@@ -1060,24 +1107,22 @@ extern "C" int casl_genfg(casl_handle *h, int ix1v, int nxv, int iy1v, int nyv, 
   int *Lu = ar.get<int>(NU);
   int *ljx = ar.get<int>(nxu);
   unsigned long long *lsum = ar.get<unsigned long long>(4);
-  double *part = ar.get<double>(2 * 4096);
   float *img = ar.get<float>(m);
   if (ar.failed) return CASL_ENOMEM;
   // con2ugrid (congen.f90:338-441), always called by genfg, then the
   // bilinear residual qr (genfg.f90:95-109)
   CASL_CUDA_TRY(cudaMemsetAsync(Lu, 0, (size_t)NU * sizeof(int), st));
   CASL_CUDA_TRY(cudaMemsetAsync(ljx, 0, (size_t)nxu * sizeof(int), st));
-  CASL_CUDA_TRY(cudaMemsetAsync(lsum, 0, sizeof(unsigned long long), st));
+  CASL_CUDA_TRY(cudaMemsetAsync(lsum, 0, 4 * sizeof(unsigned long long), st));
   if (h->nptq > 0)
     CASL_K(k_u_scatter, gsz(h->nptq), 256, 0, st)(h->xq, h->yq, h->nextq, h->nptq, h->qjump, Lu,
                                               ljx, c, &h->scal->error);
   CASL_K(k_u_lbot, 1, 1024, 0, st)(ljx, Lu, nxu, nyu);
   CASL_K(k_u_colscan, (nxu * 32 + 255) / 256, 256, 0, st)(Lu, nxu, nyu, lsum);
   LevInfo lq{0, 0, h->qjump, 0.0, 1.0};
-  CASL_K(k_u_field, 4096, 256, 0, st)(Lu, lsum, h->qr, h->qjump, 1, lq, qa, nullptr, part, c, 0.0);
+  CASL_K(k_u_field, 4096, 256, 0, st)(Lu, lsum, h->qr, h->qjump, 1, lq, qa, nullptr, lsum + 1, c, 0.0);
   CASL_K(k_gf_gather, gsz(m), 256, 0, st)(qa, nxu, nyu, ix1v - 1, nxv, iy1v - 1, nyv, stride, img);
   RC_TRY(check_launch(h));
   CASL_CUDA_TRY(cudaMemcpyAsync(out, img, (size_t)m * sizeof(float), cudaMemcpyDeviceToHost, st));
-  CASL_CUDA_TRY(cudaStreamSynchronize(st));
-  return fetch_err(h);
+  return read_back(h, {});
 }

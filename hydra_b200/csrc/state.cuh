@@ -60,6 +60,7 @@ struct casl_handle {
   double *part;          // per-block partials
   casl::Scalars *scal;   // device scalars
   casl::Scalars *hscal;  // pinned host mirror
+  char *hpin;            // pinned landing place of small reads (read_back), on first use
 
   // surgery / renode / recontour scratch (allocated on first use)
   void *sx;
