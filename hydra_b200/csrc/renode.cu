@@ -25,17 +25,16 @@ __global__ void __launch_bounds__(256) k_rn_cid(RenodeIn in, long long N, int *_
 }
 
 // The node densities of renode (contours.f90:718-796) for node w: dx, dy,
-// |d| to the next node; corners and curvature b; the cubic coefficients and
-// spherical-curvature densities; node curvature as a weighted average; the
-// fractional node count.  Only the results the placement reads (dx, dy, the
-// final e, A, B, Cc, corner) go to memory.  rn_node recomputes every
-// quantity node w needs from the coordinates of nodes w-2..w+3 (cyclic in
-// the contour); k_rn_stencil computes each quantity once per node and passes
-// it to the neighbouring lanes, with rn_node for the warps whose nodes come
-// near a contour's end.  Both use the same expressions in the same order.
+// |d| to the next node; corners and curvature b; spherical-curvature
+// densities; node curvature as a weighted average; the fractional node count.
+// Only the density e and the corner flag are kept (the placement forms the
+// cubic of a segment again where it puts nodes).  rn_node recomputes every
+// quantity node w needs from the coordinates of nodes w-2..w+3 (cyclic in the
+// contour); k_rn_nodes computes each quantity once per node and passes it to
+// the neighbouring lanes, with rn_node for the warps whose nodes come near a
+// contour's end.  Both use the same expressions in the same order.
 __device__ __forceinline__ void rn_node(const RenodeIn &in, const RenodeScratch &s, const Consts &c,
                                         long long w, double &eout, int &cout) {
-  const double f12 = 0.5, f13 = 1.0 / 3.0, f16 = 1.0 / 6.0;
   const int k = s.cid[w];
   const long long cs = in.cs[k], L = in.len[k];
   long long j[6];
@@ -77,17 +76,11 @@ __device__ __forceinline__ void rn_node(const RenodeIn &in, const RenodeScratch 
       b[m] = (dx[m] * cc - a * dy[m]) / sqrt(t1 * t1 + t2 * t2 + c.small3);
     }
   }
-  // rn3 at nodes m = 1..3 (the cubic coefficients only at m = 2)
-  double u2[4], v2[4], A = 0.0, B = 0.0, Cc = 0.0;
+  // rn3 at nodes m = 1..3
+  double u2[4], v2[4];
 #pragma unroll
   for (int m = 1; m < 4; m++) {
     double u = e1[m] * (b[m + 1] + b[m]);
-    double cc = e1[m] * (b[m + 1] - b[m]);
-    if (m == 2) {
-      A = f16 * cc - f12 * u;
-      B = f12 * (u - cc);
-      Cc = f13 * cc;
-    }
     double ww = 1.0 / (v[m] + c.dmsq);
     u2[m] = ww * sqrt(c.elf * v[m] + u * u);
     v2[m] = ww * e1[m];
@@ -97,12 +90,7 @@ __device__ __forceinline__ void rn_node(const RenodeIn &in, const RenodeScratch 
   const double d3 = (u2[2] + u2[3]) / (v2[2] + v2[3] + c.small);
   const double uu = 0.5 * (d2 + d3);
   const double t = c.densf * sqrt(uu) + uu;
-  s.dx[w] = dx[2];
-  s.dy[w] = dy[2];
   s.e[w] = eout = e1[2] * fmin(c.dmi, t);
-  s.A[w] = A;
-  s.B[w] = B;
-  s.Cc[w] = Cc;
   cout = corner2;
   if (corner2) red_add_s32(&s.ccnt[k], 1);
 }
@@ -115,21 +103,28 @@ __device__ __forceinline__ void rn_node(const RenodeIn &in, const RenodeScratch 
 // of lane L, its curvature (rn2), its cubic and density terms (rn3) and its
 // rn4 average each take the lower neighbour's value from lane L-1 and the
 // upper neighbour's from lane L+1.  Valid while every written node's
-// stencil w-2..w+3 lies inside its contour without wrapping; otherwise the
-// warp takes rn_node.
+// stencil w-2..w+3 lies inside its contour without wrapping, which the first
+// and last node of the warp's stencils tell (a contour's nodes are
+// consecutive); otherwise the warp takes rn_node.
 //
 // The densities and flags stay in shared memory for the tile's scans; tiles
 // look back at earlier ones for the corners before them (any order: integers)
 // and, to the last contour start before the tile, for the densities, whose
 // tile sums are added from left to right (the same on every run).
+//
+// Bound by the latency of a step's chain (three square roots and three
+// divisions one after the other, 24 warps an SM): the next step's nodes are
+// loaded before it, and the sums and ranks leave through shared memory (a
+// thread's 7 consecutive nodes would write 4 sectors for 1).  24M nodes 1036 us
+// before, with the cubic's five coefficients stored as well, and 630 so.
 constexpr int RN_OUT = 28, RN_WARPS = 8, RN_STEP = RN_OUT * RN_WARPS;
 template <int RN_IT>
 __global__ void __launch_bounds__(256, 3) k_rn_nodes(RenodeIn in, RenodeScratch s, Consts c) {
   CASL_PDL_ENTRY();
-  const double f12 = 0.5, f13 = 1.0 / 3.0, f16 = 1.0 / 6.0;
   const unsigned FULL = 0xffffffffu;
   constexpr int RN_TILE = RN_STEP * RN_IT;
   __shared__ double te[RN_TILE];
+  __shared__ int tc[RN_TILE];
   __shared__ unsigned char tf[RN_TILE];  // 1: contour start, 2: corner
   __shared__ SegPair total;
   __shared__ unsigned int ctot, cbefore;
@@ -139,40 +134,44 @@ __global__ void __launch_bounds__(256, 3) k_rn_nodes(RenodeIn in, RenodeScratch 
   const int tile = lb_ticket(&s.tick[0]);
   const long long t0 = (long long)tile * RN_TILE;
   if (t0 >= N) return;
+  // this lane's node of a step and, in lane 31, the one after: coordinates, contours
+  double pX, pY, pX1, pY1;
+  int pk, pk1;
+  auto fetch = [&](int it) {
+    const long long o = t0 + (long long)(it * RN_WARPS + wid) * RN_OUT - 2 + lane;
+    pX = pY = pX1 = pY1 = 0.0;
+    pk = pk1 = 0;
+    if (o >= 0 && o < N) {
+      pX = in.xw[o];
+      pY = in.yw[o];
+      pk = s.cid[o];
+    }
+    if (lane == 31 && o + 1 < N) {
+      pX1 = in.xw[o + 1];
+      pY1 = in.yw[o + 1];
+      pk1 = s.cid[o + 1];
+    }
+  };
+  fetch(0);
 #pragma unroll 1
   for (int it = 0; it < RN_IT; it++) {
     const long long base = t0 + (long long)(it * RN_WARPS + wid) * RN_OUT;
     if (base >= N) break;
+    const double X = pX, Y = pY, X1 = pX1, Y1 = pY1;
+    const int k = pk, k1 = pk1;
+    if (it + 1 < RN_IT) fetch(it + 1);
     const long long o = base - 2 + lane;  // this lane's node
     const bool out = lane >= 2 && lane < 2 + RN_OUT && o < N;
-    int k = 0;
-    long long cs = 0, L = 0;
-    bool lin = true;
-    if (out) {
-      k = s.cid[o];
-      cs = in.cs[k];
-      L = in.len[k];
-      lin = o - 2 >= cs && o + 3 <= cs + L - 1;
-    }
     double e = 0.0;
     int corner = 0;
-    if (!__all_sync(FULL, lin)) {
+    const int kf = __shfl_sync(FULL, k, 0), kl = __shfl_sync(FULL, k1, 31);
+    if (base < 2 || base + RN_OUT + 2 >= N || kf != kl) {
       if (out) {
         rn_node(in, s, c, o, e, corner);
         te[o - t0] = e;
-        tf[o - t0] = (unsigned char)((o == cs) | corner << 1);
+        tf[o - t0] = (unsigned char)((o == in.cs[k]) | corner << 1);
       }
       continue;
-    }
-    // coordinates of this lane's node and of the next one
-    double X = 0.0, Y = 0.0, X1 = 0.0, Y1 = 0.0;
-    if (o >= 0 && o < N) {
-      X = in.xw[o];
-      Y = in.yw[o];
-    }
-    if (lane == 31 && o + 1 < N) {
-      X1 = in.xw[o + 1];
-      Y1 = in.yw[o + 1];
     }
     double Xn = __shfl_down_sync(FULL, X, 1), Yn = __shfl_down_sync(FULL, Y, 1);
     if (lane == 31) {
@@ -200,10 +199,6 @@ __global__ void __launch_bounds__(256, 3) k_rn_nodes(RenodeIn in, RenodeScratch 
     // rn3 at this node, with the next node's curvature
     const double bn = __shfl_down_sync(FULL, b, 1);
     const double u = e1 * (bn + b);
-    const double cc = e1 * (bn - b);
-    const double A = f16 * cc - f12 * u;
-    const double B = f12 * (u - cc);
-    const double Cc = f13 * cc;
     const double ww = 1.0 / (v + c.dmsq);
     const double u2 = ww * sqrt(c.elf * v + u * u);
     const double v2 = ww * e1;
@@ -216,14 +211,9 @@ __global__ void __launch_bounds__(256, 3) k_rn_nodes(RenodeIn in, RenodeScratch 
       const double uu = 0.5 * (d + dn);
       const double t = c.densf * sqrt(uu) + uu;
       e = e1 * fmin(c.dmi, t);
-      s.dx[o] = dx;
-      s.dy[o] = dy;
       s.e[o] = e;
-      s.A[o] = A;
-      s.B[o] = B;
-      s.Cc[o] = Cc;
       te[o - t0] = e;
-      tf[o - t0] = (unsigned char)((o == cs) | corner << 1);
+      tf[o - t0] = (unsigned char)(corner << 1);
       if (corner) red_add_s32(&s.ccnt[k], 1);
     }
   }
@@ -293,11 +283,15 @@ __global__ void __launch_bounds__(256, 3) k_rn_nodes(RenodeIn in, RenodeScratch 
     if (i0 + q < n) {
       const int f = tf[i0 + q];
       run = seg_op(run, SegPair{te[i0 + q], f & 1});
-      const long long o = t0 + i0 + q;
-      s.S[o] = run.f ? run.v : run.v + carry;
-      s.cc[o] = 2 * rank + (f >> 1);
-      if (f & 2) s.cornerpos[rank++] = (int)o;
+      te[i0 + q] = run.f ? run.v : run.v + carry;
+      tc[i0 + q] = 2 * rank + (f >> 1);
+      if (f & 2) s.cornerpos[rank++] = (int)(t0 + i0 + q);
     }
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += 256) {
+    s.S[t0 + i] = te[i];
+    s.cc[t0 + i] = tc[i];
+  }
 }
 
 // Sum of e over `m` nodes of contour [cs, cs+L) starting at walk index st.
@@ -389,10 +383,9 @@ __global__ void __launch_bounds__(256) k_rn_contours(RenodeIn in, RenodeScratch 
         if (near_half(sum)) sum = seq_sum(s.e, cs, L, st, pl);
         n = sum > c.small ? nint_d(sum) + 1 : 0;
       }
-      s.pstart[p] = (int)st;
-      s.plen[p] = (int)pl;
-      s.pn[p] = n;
-      s.pfac[p] = n > 0 ? (double)n / sum : 0.0;
+      const double preA = st == cs ? 0.0 : s.S[st - 1];
+      s.piece[p] = RnPiece{(int)st, (int)pl, n, 0, n > 0 ? (double)n / sum : 0.0,
+                           preA, s.S[cs + L - 1] - preA, 0.0};
       npr += n;
     }
     const bool keep = k < Ce && (mode == RENODE_SURGERY ? npr > 3 : npr > 0);
@@ -405,19 +398,16 @@ __global__ void __launch_bounds__(256) k_rn_contours(RenodeIn in, RenodeScratch 
     __syncthreads();
     at += nbefore;
     if (k < Ce) {
-      s.npiece[k] = np;
-      s.poff[k] = p0;
-      s.ckeep[k] = keep;
+      s.poff[k] = keep ? p0 : -1;
       if (keep) {
         int base = (int)(at >> 31);
         const int j = (int)(at & 0x7fffffffull);
-        s.ckidx[k] = j;
         out.ocs[j] = base;
         out.olen[j] = npr;
         out.olev[j] = in.levt ? in.levt[k] : 0;
         for (int q = 0; q < np; q++) {
-          s.pout[p0 + q] = base;
-          base += s.pn[p0 + q];
+          s.piece[p0 + q].out = base;
+          base += s.piece[p0 + q].n;
         }
       }
     }
@@ -431,63 +421,175 @@ __global__ void __launch_bounds__(256) k_rn_contours(RenodeIn in, RenodeScratch 
   }
 }
 
-__global__ void k_rn_place(RenodeIn in, RenodeScratch s, RenodeOut out, Consts c) {
+// The new nodes: node t of a piece lies on the old segment whose cumulative
+// density reaches t (contours.f90:856-928).
+//
+// A block takes 128 * PU consecutive nodes.  First each one's cumulative
+// densities Ep, Ec at its two ends (in units of new nodes) say whether its
+// segment receives any; those that do (one in 18 of a recontouring's crossings,
+// most nodes of a state) are gathered in shared memory, so that the second half
+// runs on full warps: the segment's cubic from its four nodes, and the nodes.
+// A warp whose nodes lie in one piece of a contour, the usual case, reads its
+// data once and per node only the prefix sum.  24M crossings: 684 us with a
+// node a thread and its contour's data loaded for each, 287 so; 1.4M nodes 52
+// both ways.
+constexpr int PL_BT = 128;
+template <int PU>
+__global__ void __launch_bounds__(PL_BT, 8) k_rn_place(RenodeIn in, RenodeScratch s, RenodeOut out,
+                                                  Consts c) {
   CASL_PDL_ENTRY();
   if (out.d_counts[2]) return;  // overflow: the caller reports it
-  for (long long w = blockIdx.x * (long long)blockDim.x + threadIdx.x; w < in.N;
-       w += (long long)gridDim.x * blockDim.x) {
-    int k = s.cid[w];
-    if (!s.ckeep[k]) continue;
-    long long cs = in.cs[k], L = in.len[k];
-    int nc = s.ccnt[k];
-    int q = 0;
-    if (nc >= 2) {
-      const int cw = s.cc[w];
-      int inc = (cw >> 1) - (s.cc[cs] >> 1) + (cw & 1);
-      q = inc - 1;
-      if (q < 0) q = nc - 1;
+  constexpr int TILE = PL_BT * PU;
+  __shared__ double lEp[TILE], lEc[TILE];
+  __shared__ int lw[TILE], lp[TILE];
+  __shared__ int nl;
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const double f12 = 0.5, f13 = 1.0 / 3.0, f16 = 1.0 / 6.0;
+  for (long long b = blockIdx.x * (long long)TILE; b < in.N; b += (long long)gridDim.x * TILE) {
+    __syncthreads();  // the list of the tile before is done with
+    if (threadIdx.x == 0) nl = 0;
+    __syncthreads();
+    const long long wb = b + wid * 32 * PU, we = min(wb + 32 * PU, in.N) - 1;
+    if (wb <= we) {
+      double S[PU];
+#pragma unroll
+      for (int u = 0; u < PU; u++) S[u] = wb + 32 * u + lane <= we ? s.S[wb + 32 * u + lane] : 0.0;
+      double last = wb > 0 ? s.S[wb - 1] : 0.0;  // the sum before the warp's next 32 nodes
+      // the piece of node w of contour k, whose first node is cs (-1: not kept)
+      auto piece_of = [&](long long w, int k, long long cs) -> int {
+        const int nc = s.ccnt[k], p0 = s.poff[k];
+        if (nc < 2 || p0 < 0) return p0;
+        const int cw = s.cc[w];
+        const int q = (cw >> 1) - (s.cc[cs] >> 1) + (cw & 1) - 1;
+        return p0 + (q < 0 ? nc - 1 : q);
+      };
+      int k = s.cid[wb], p = -1;
+      long long cs = in.cs[k];
+      RnPiece pc{};
+      bool one = k == s.cid[we];
+      if (one) {
+        // the same piece at both ends, and both before or both after its
+        // first node (the last piece wraps), is the same between them
+        p = piece_of(wb, k, cs);
+        one = p == piece_of(we, k, cs);
+        if (one && p >= 0) {
+          pc = s.piece[p];
+          one = (wb < pc.st) == (we < pc.st);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < PU; u++) {
+        const long long w = wb + 32 * u + lane;
+        double P0 = __shfl_up_sync(FULL, S[u], 1);
+        if (lane == 0) P0 = last;
+        last = __shfl_sync(FULL, S[u], 31);
+        if (!one) {
+          p = -1;
+          if (w <= we) {
+            k = s.cid[w];
+            cs = in.cs[k];
+            p = piece_of(w, k, cs);
+            if (p >= 0) pc = s.piece[p];
+          }
+        }
+        int pw = w <= we ? p : -1;  // the node's piece, when it receives nodes
+        double Ep = 0.0, Ec = 0.0;
+        if (pw >= 0 && pc.n == 0) pw = -1;
+        if (pw >= 0) {
+          // sums of the piece's densities before and through w (sumrange's
+          // two cases, which agree where a range ends at the contour's end)
+          if (w == cs) P0 = 0.0;
+          Ep = pc.fac * (w < pc.st ? pc.preW + P0 : P0 - pc.preA);
+          Ec = pc.fac * (w < pc.st ? pc.preW + S[u] : S[u] - pc.preA);
+          if (w == pc.st) {
+            out.xo[pc.out] = in.xw[w];
+            out.yo[pc.out] = in.yw[w];
+          }
+        }
+        if (pw >= 0) {
+          long long t0 = (long long)floor(Ep) + 1, t1 = (long long)floor(Ec);
+          if (t1 > pc.n - 1) t1 = pc.n - 1;
+          if (t0 < 1) t0 = 1;
+          if (t1 < t0) pw = -1;
+        }
+        const unsigned m = __ballot_sync(FULL, pw >= 0);
+        if (m) {
+          int at = 0;
+          if (lane == 0) at = atomicAdd(&nl, __popc(m));
+          at = __shfl_sync(FULL, at, 0) + __popc(m & ((1u << lane) - 1u));
+          if (pw >= 0) {
+            lw[at] = (int)w;
+            lp[at] = pw;
+            lEp[at] = Ep;
+            lEc[at] = Ec;
+          }
+        }
+      }
     }
-    int p = s.poff[k] + q;
-    int n = s.pn[p];
-    if (n == 0) continue;
-    long long st = s.pstart[p];
-    // w and the piece start both lie in the contour [cs, cs+L)
-    long long rel = w - st;
-    if (rel < 0) rel += L;
-    if (rel >= s.plen[p]) continue;
-    long long o = s.pout[p];
-    if (rel == 0) {
-      out.xo[o] = in.xw[w];
-      out.yo[o] = in.yw[w];
-    }
-    double fac = s.pfac[p];
-    double Ep = fac * sumrange(s.S, cs, L, st, rel);
-    double Ec = fac * sumrange(s.S, cs, L, st, rel + 1);
-    long long t0 = (long long)floor(Ep) + 1;
-    long long t1 = (long long)floor(Ec);
-    if (t1 > n - 1) t1 = n - 1;
-    if (t0 < 1) t0 = 1;
-    if (t1 < t0) continue;
-    double ew = fac * s.e[w];
-    double xd = in.xw[w], yd = in.yw[w], dx = s.dx[w], dy = s.dy[w];
-    double A = s.A[w], B = s.B[w], Cc = s.Cc[w];
-    for (long long t = t0; t <= t1; t++) {
-      double acc = Ec - (double)t;
-      double pp = 1.0 - acc / ew;
-      // Targets are assigned by prefix sums, whose grouping rounds: a
-      // segment of density zero or at the rounding level (the zero-length
-      // segments that surgery leaves where it joins two nodes) can receive
-      // a target that the reference's running sum gives its neighbour, and
-      // 1 - acc/ew is then far outside [0, 1] or 0/0.  Such a target is
-      // placed by the prefix values that assigned it (Ep < t <= Ec, so the
-      // fraction lies in (0, 1]): the segment's start, within rounding of
-      // where the reference puts it.
-      if (!(pp >= -1e-9 && pp <= 1.0 + 1e-9)) pp = ((double)t - Ep) / (Ec - Ep);
-      double eta = pp * (A + pp * (B + pp * Cc));
-      double xx = xd + pp * dx - eta * dy;
-      double yy = yd + pp * dy + eta * dx;
-      out.xo[o + t] = wrapp(xx, c.ellx, c.hlxi, c.oms);
-      out.yo[o + t] = wrapp(yy, c.elly, c.hlyi, c.oms);
+    __syncthreads();
+    for (int i = threadIdx.x; i < nl; i += PL_BT) {
+      const long long w = lw[i];
+      const int k = s.cid[w];
+      const RnPiece &pc = s.piece[lp[i]];
+      const int n = pc.n;
+      const long long cs = in.cs[k], L = in.len[k], o = pc.out;
+      const double Ep = lEp[i], Ec = lEc[i];
+      const double ew = pc.fac * s.e[w];
+      // the segment's cubic (contours.f90:718-775), from nodes w-1 .. w+2
+      long long j[4];
+      j[0] = wprev(w, cs, L);
+      j[1] = w;
+      j[2] = wnext(w, cs, L);
+      j[3] = wnext(j[2], cs, L);
+      double X[4], Y[4], dx[3], dy[3], v[3], bb[2];
+#pragma unroll
+      for (int m = 0; m < 4; m++) {
+        X[m] = in.xw[j[m]];
+        Y[m] = in.yw[j[m]];
+      }
+#pragma unroll
+      for (int m = 0; m < 3; m++) {
+        const double xx = X[m + 1] - X[m];
+        dx[m] = xx - c.ellx * f_dint(xx * c.hlxi);
+        const double yy = Y[m + 1] - Y[m];
+        dy[m] = yy - c.elly * f_dint(yy * c.hlyi);
+        v[m] = dx[m] * dx[m] + dy[m] * dy[m];
+      }
+#pragma unroll
+      for (int m = 0; m < 2; m++) {
+        const double u = v[m], a = -dx[m], cc = -dy[m];
+        if (dx[m + 1] * a + dy[m + 1] * cc > 0.0) {
+          bb[m] = 0.0;
+        } else {
+          const double t1 = a * v[m + 1] - dx[m + 1] * u, t2 = cc * v[m + 1] - dy[m + 1] * u;
+          bb[m] = (dx[m + 1] * cc - a * dy[m + 1]) / sqrt(t1 * t1 + t2 * t2 + c.small3);
+        }
+      }
+      const double e1 = sqrt(v[1]);
+      const double u = e1 * (bb[1] + bb[0]), cc = e1 * (bb[1] - bb[0]);
+      const double A = f16 * cc - f12 * u, B = f12 * (u - cc), Cc = f13 * cc;
+      long long t0 = (long long)floor(Ep) + 1, t1 = (long long)floor(Ec);
+      if (t1 > n - 1) t1 = n - 1;
+      if (t0 < 1) t0 = 1;
+      for (long long t = t0; t <= t1; t++) {
+        const double acc = Ec - (double)t;
+        double pp = 1.0 - acc / ew;
+        // Targets are assigned by prefix sums, whose grouping rounds: a
+        // segment of density zero or at the rounding level (the zero-length
+        // segments that surgery leaves where it joins two nodes) can receive
+        // a target that the reference's running sum gives its neighbour, and
+        // 1 - acc/ew is then far outside [0, 1] or 0/0.  Such a target is
+        // placed by the prefix values that assigned it (Ep < t <= Ec, so the
+        // fraction lies in (0, 1]): the segment's start, within rounding of
+        // where the reference puts it.
+        if (!(pp >= -1e-9 && pp <= 1.0 + 1e-9)) pp = ((double)t - Ep) / (Ec - Ep);
+        const double eta = pp * (A + pp * (B + pp * Cc));
+        const double xx = X[1] + pp * dx[1] - eta * dy[1];
+        const double yy = Y[1] + pp * dy[1] + eta * dx[1];
+        out.xo[o + t] = wrapp(xx, c.ellx, c.hlxi, c.oms);
+        out.yo[o + t] = wrapp(yy, c.elly, c.hlyi, c.oms);
+      }
     }
   }
 }
@@ -510,19 +612,22 @@ int renode_batch(casl_handle *h, Arena &ar, const RenodeIn &in, RenodeOut &out, 
   }
   RenodeScratch s{};
   s.cid = in.cid ? const_cast<int *>(in.cid) : ar.get<int>(N);
-  s.dx = ar.get<double>(N); s.dy = ar.get<double>(N);
-  s.e = ar.get<double>(N); s.A = ar.get<double>(N);
-  s.B = ar.get<double>(N); s.Cc = ar.get<double>(N); s.S = ar.get<double>(N);
+  s.e = ar.get<double>(N);
+  s.S = ar.get<double>(N);
   s.cc = ar.get<int>(N);
   s.cornerpos = ar.get<int>(N + 1);
   s.ccnt = ar.get<int>(C);
-  s.npiece = ar.get<int>(C); s.poff = ar.get<int>(C);
-  s.ckeep = ar.get<int>(C); s.ckidx = ar.get<int>(C);
+  s.poff = ar.get<int>(C);
   // Tiles of one step while that leaves no more blocks than fit on the SMs at
   // once (a tile's steps run one after the other: 10k nodes 16 us with 1, 33
   // with 8); larger ones above, where each further tile costs its scans (1.4M
-  // nodes 170, 101 and 87 us with 1, 3 and 8; 75k nodes 23, 24, 35).
-  const int rnit = N <= 148LL * 3 * RN_STEP ? 1 : (N <= 148LL * 3 * RN_STEP * 4 ? 3 : 8);
+  // nodes 170, 101, 78 and 73 us with 1, 3, 8 and 16; 75k nodes 23, 24, 35 with
+  // 1, 3 and 8; 1.0M nodes 86 and 91 with 8 and 16), 16 once two blocks an SM
+  // are left.
+  const int rnit = N <= 148LL * 3 * RN_STEP       ? 1
+                   : N <= 148LL * 3 * RN_STEP * 4 ? 3
+                   : N <= 148LL * 2 * RN_STEP * 16 ? 8
+                                                   : 16;
   const long long nt = (N + rnit * RN_STEP - 1) / (rnit * RN_STEP), ct = (C + 255LL) / 256;
   s.nstat = ar.get<unsigned long long>(nt + ct + 2);  // then the contours' words, then the tickets
   s.cstat = s.nstat + nt;
@@ -533,9 +638,7 @@ int renode_batch(casl_handle *h, Arena &ar, const RenodeIn &in, RenodeOut &out, 
   // pieces: one per corner of a contour with >= 2 corners, else one per
   // contour, so at most N + C
   long long P = N + C;
-  s.pstart = ar.get<int>(P); s.plen = ar.get<int>(P);
-  s.pn = ar.get<int>(P); s.pout = ar.get<int>(P);
-  s.pfac = ar.get<double>(P);
+  s.piece = ar.get<RnPiece>(P);
   if (ar.failed) return CASL_ENOMEM;
   {
     const FillJob z[2] = {{s.ccnt, C, 0u}, {s.nstat, 2 * (nt + ct + 2), 0u}};
@@ -547,12 +650,20 @@ int renode_batch(casl_handle *h, Arena &ar, const RenodeIn &in, RenodeOut &out, 
     CASL_K(k_rn_nodes<1>, (int)nt, 256, 0, st)(in, s, c);
   else if (rnit == 3)
     CASL_K(k_rn_nodes<3>, (int)nt, 256, 0, st)(in, s, c);
-  else
+  else if (rnit == 8)
     CASL_K(k_rn_nodes<8>, (int)nt, 256, 0, st)(in, s, c);
+  else
+    CASL_K(k_rn_nodes<16>, (int)nt, 256, 0, st)(in, s, c);
   // (C may be a capacity, the count being on the device: the grid is sized
   // for the usual counts and its blocks take tiles until there are none)
   CASL_K(k_rn_contours, (int)std::min(ct, 2LL * 148), 256, 0, st)(in, s, out, c, mode);
-  CASL_K(k_rn_place, g, 256, 0, st)(in, s, out, c);
+  // four nodes a thread once that leaves every SM its blocks
+  const int pu = N <= 148LL * 16 * PL_BT ? 1 : 4;
+  const int gp = (int)std::min((N + pu * PL_BT - 1) / (pu * PL_BT), 148LL * 32);
+  if (pu == 1)
+    CASL_K(k_rn_place<1>, gp, PL_BT, 0, st)(in, s, out, c);
+  else
+    CASL_K(k_rn_place<4>, gp, PL_BT, 0, st)(in, s, out, c);
   return check_launch(h);
 }
 

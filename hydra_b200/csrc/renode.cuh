@@ -88,15 +88,20 @@ __device__ __forceinline__ int chunk_contour_of(const int *__restrict__ cs, int 
   return c.j0 + lo;
 }
 
+// A piece of a contour between corners (or all of it): first node, nodes, new
+// nodes, where those go; new nodes per density; the contour's prefix sum before
+// the first node, and the rest of its total.
+struct __align__(16) RnPiece {
+  int st, len, n, out;
+  double fac, preA, preW, pad;
+};
 struct RenodeScratch {
   int *cid;                  // contour of each walk node
-  double *dx, *dy, *e, *A, *B, *Cc, *S;
+  double *e, *S;              // node densities, and their sums along the contour
   int *cc;                   // 2 * (corners before the node) + (the node is one)
   int *ccnt;                 // corners per contour
-  int *npiece, *poff;        // pieces per contour, offsets
-  int *pstart, *plen, *pn, *pout;  // per piece: start w, length, count, out offset
-  double *pfac;
-  int *ckeep, *ckidx;        // per contour: keep, kept index
+  int *poff;                 // per contour: its first piece (-1: the contour is not kept)
+  RnPiece *piece;
   int *cornerpos;
   // tiles of the two scans: tickets, status words, and the node tiles'
   // densities since their last contour start
