@@ -784,8 +784,8 @@ __global__ void k_c2g_coarsen(const int *__restrict__ L, int *__restrict__ C,
 }
 
 
-// Packed con2grid, second half.  A CTA owns CW = 7 coarse columns and their
-// 4*CW+3 = 31 fine columns, one warp per column, RPS = 32U coarse rows per
+// Packed con2grid, second half.  A CTA owns CW = 7 or 3 coarse columns and
+// their 4*CW+3 = 31 or 15 fine columns, one warp per column, RPS = 32U coarse rows per
 // step with the next step's words in flight.  Lane cy decodes its word,
 // the warp scans the word totals (ex = jumps of all rows below 4cy), and
 // with the two top counts of the word below (rows 4cy-2, 4cy-1) the seven
@@ -794,8 +794,6 @@ __global__ void k_c2g_coarsen(const int *__restrict__ L, int *__restrict__ C,
 // 7-tap along x.  Coarse row 0 wraps to the top rows and is formed last.
 // Requires n % RPS == 0.  W: four rows' counts in 64 bits, or as an int4 where
 // the caller's levels have no bound (c2g_sum32).
-#define C2G_CW 7
-#define C2G_FC (4 * C2G_CW + 3)
 
 // The learned closure's sub-cell input: the fine levels at the 3 x 3 points
 // (4cx + 2a - 2, 4cy + 2b - 2), a, b = 0..2, of every coarse cell (cx, cy),
@@ -803,6 +801,7 @@ __global__ void k_c2g_coarsen(const int *__restrict__ L, int *__restrict__ C,
 // 4 cx0 - 3 + w: a column 4k+1 is the a = 0 sample of coarse column k and
 // the a = 2 sample of column k - 1, a column 4k+3 the a = 1 sample of k.
 // La, Lb, Lc are the levels at fine rows 4cy - 2, 4cy, 4cy + 2.
+template <int CW>
 __device__ __forceinline__ void c2g_feature(int *__restrict__ F, int n, int cx0, int w, int cy,
                                             int La, int Lb, int Lc) {
   const int r = w & 3, k = w >> 2;
@@ -812,7 +811,7 @@ __device__ __forceinline__ void c2g_feature(int *__restrict__ F, int n, int cx0,
   if (r == 3) {
     cxl[0] = k; aa[0] = 1; m = 1;
   } else {
-    if (k < C2G_CW) { cxl[m] = k; aa[m++] = 0; }
+    if (k < CW) { cxl[m] = k; aa[m++] = 0; }
     if (k >= 1) { cxl[m] = k - 1; aa[m++] = 2; }
   }
   for (int q = 0; q < m; q++) {
@@ -825,8 +824,8 @@ __device__ __forceinline__ void c2g_feature(int *__restrict__ F, int n, int cx0,
   }
 }
 
-template <int U, class W = unsigned long long>
-__global__ void __launch_bounds__(1024) k_c2g_packed_sum(const W *__restrict__ JW,
+template <int U, int CW, class W = unsigned long long>
+__global__ void __launch_bounds__(32 * (4 * CW + 4)) k_c2g_packed_sum(const W *__restrict__ JW,
                                                          const int *__restrict__ ljx,
                                                          int *__restrict__ C,
                                                          unsigned long long *__restrict__ csum,
@@ -840,21 +839,21 @@ __global__ void __launch_bounds__(1024) k_c2g_packed_sum(const W *__restrict__ J
     C += m * (long long)n * n;
     csum += m * mb.cs;
   }
-  constexpr int RPS = 32 * U;
-  __shared__ int G[RPS][C2G_FC + 2];  // row length 33: conflict-free both ways
-  __shared__ int G0[C2G_FC];
+  constexpr int RPS = 32 * U, FC = 4 * CW + 3, NW = 4 * CW + 4;
+  __shared__ int G[RPS][FC + 2];  // row length 33: conflict-free both ways
+  __shared__ int G0[FC];
   __shared__ long long red[32];
   const unsigned FULL = 0xffffffffu;
   const int w7[7] = {1, 2, 3, 4, 3, 2, 1};
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int cx0 = blockIdx.x * C2G_CW;
+  const int cx0 = blockIdx.x * CW;
   int col = 4 * cx0 - 3 + warp;  // this warp's fine column (0-based), wrapped
   if (col < 0) col += nf;
   if (col >= nf) col -= nf;
   const W *cp = JW + (long long)col * n + lane;
   const int nsteps = n / RPS;
   W v[U];
-  if (warp < C2G_FC) {
+  if (warp < FC) {
 #pragma unroll
     for (int u = 0; u < U; u++) v[u] = __ldcs(cp + u * 32);
   }
@@ -865,32 +864,32 @@ __global__ void __launch_bounds__(1024) k_c2g_packed_sum(const W *__restrict__ J
     __shared__ int ptot;
     const int c0 = 4 * cx0 - 3;
     int pcarry = 0;
-    for (int base = 0; base < nf; base += 4 * SCAN_BLOCK) {
+    for (int base = 0; base < nf; base += 4 * 32 * NW) {
       const int i0 = base + 4 * threadIdx.x;
       int a[4];
 #pragma unroll
       for (int k = 0; k < 4; k++) a[k] = i0 + k < nf ? ljx[i0 + k] : 0;
-      int pre = pcarry + block_excl_scan<int>(a[0] + a[1] + a[2] + a[3], &ptot);
+      int pre = pcarry + block_excl_scan_any<int>(a[0] + a[1] + a[2] + a[3], &ptot);
       int d = i0 - c0;  // this thread's first entry relative to the block's first column
       d = d < 0 ? d + nf : (d >= nf ? d - nf : d);
 #pragma unroll
       for (int k = 0; k < 4; k++) {
         int w = d + k;
         if (w >= nf) w -= nf;
-        if (i0 + k < nf && w < C2G_FC) G0[w] = pre;
+        if (i0 + k < nf && w < FC) G0[w] = pre;
         pre += a[k];
       }
       pcarry += ptot;
       __syncthreads();
     }
   }
-  const int lb = warp < C2G_FC ? G0[warp] : 0;
+  const int lb = warp < FC ? G0[warp] : 0;
   __syncthreads();  // G0 is reused for coarse row 0
   int carry = 0, q2 = 0, q3 = 0;       // running total; rows 4cy-2, 4cy-1 below lane 0
   int f0 = 0, f1 = 0, f2 = 0, f3 = 0;  // word 0 (rows 0..3), kept for coarse row 0
   long long local = 0;
   for (int s = 0; s < nsteps; s++) {
-    if (warp < C2G_FC) {
+    if (warp < FC) {
 #pragma unroll
       for (int u = 0; u < U; u++) {
         int c0, c1, c2, c3;
@@ -909,7 +908,7 @@ __global__ void __launch_bounds__(1024) k_c2g_packed_sum(const W *__restrict__ J
             w7[0] * L0 + w7[1] * L1 + w7[2] * L2 + w7[3] * L3 + w7[4] * L4 + w7[5] * L5 + w7[6] * L6;
         if (F) {
           const int cy = s * RPS + u * 32 + lane;
-          if (cy > 0) c2g_feature(F, n, cx0, warp, cy, L1, L3, L5);
+          if (cy > 0) c2g_feature<CW>(F, n, cx0, warp, cy, L1, L3, L5);
         }
         if (s == 0 && u == 0 && lane == 0) {
           f0 = c0; f1 = c1; f2 = c2; f3 = c3;
@@ -924,7 +923,7 @@ __global__ void __launch_bounds__(1024) k_c2g_packed_sum(const W *__restrict__ J
       }
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < C2G_CW * RPS; t += blockDim.x) {
+    for (int t = threadIdx.x; t < CW * RPS; t += blockDim.x) {
       const int cxl = t / RPS, rl = t % RPS;
       const int cx = cx0 + cxl, cy = s * RPS + rl;
       if (cx < n && cy > 0) {
@@ -939,15 +938,15 @@ __global__ void __launch_bounds__(1024) k_c2g_packed_sum(const W *__restrict__ J
   }
   // coarse row 0: fine rows nf-3, nf-2, nf-1 (the top word: q2, q3 are its
   // rows nf-2, nf-1; carry is the column total) and rows 0..3 (word 0)
-  if (warp < C2G_FC && lane == 0) {
+  if (warp < FC && lane == 0) {
     const int L2 = lb + carry, L1 = L2 - q3, L0 = L1 - q2;
     const int L3 = lb + f0, L4 = L3 + f1, L5 = L4 + f2, L6 = L5 + f3;
     G0[warp] = w7[0] * L0 + w7[1] * L1 + w7[2] * L2 + w7[3] * L3 + w7[4] * L4 + w7[5] * L5 +
                w7[6] * L6;
-    if (F) c2g_feature(F, n, cx0, warp, 0, L1, L3, L5);
+    if (F) c2g_feature<CW>(F, n, cx0, warp, 0, L1, L3, L5);
   }
   __syncthreads();
-  if (threadIdx.x < C2G_CW) {
+  if (threadIdx.x < CW) {
     const int cx = cx0 + threadIdx.x;
     if (cx < n) {
       int acc = 0;
@@ -961,7 +960,7 @@ __global__ void __launch_bounds__(1024) k_c2g_packed_sum(const W *__restrict__ J
   if (lane == 0) red[warp] = local;
   __syncthreads();
   if (warp == 0) {
-    long long x = red[lane];
+    long long x = lane < NW ? red[lane] : 0;
     for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(FULL, x, o);
     if (lane == 0) atomicAdd(csum, (unsigned long long)x);
   }
@@ -995,19 +994,41 @@ static int grid_for(long long work, int block = 256) {
   return (int)g;
 }
 
+// Second half of con2grid for M members from either kind of counts.  CTAs of 7
+// coarse columns read each fine column 31/28 times, of 3 columns 15/12 times,
+// but while those of 7 fill less than half the SMs, twice as many of half the
+// size are faster (64^2 9.5 and 8.7 us, 256^2 12.5 and 10.7, with 7 and 3; 512^2,
+// 74 CTAs of 7, 15.5 and 16.4; 1024^2 23 and 33).
+template <class W>
+static void c2g_sum(cudaStream_t st, const W *J, const int *ljx, int *C, unsigned long long *csum,
+                    int n, const C2GMembers &mb, int *feat) {
+  const bool wide = (long long)((n + 6) / 7) * mb.M * 2 >= 148;
+  const int cw = wide ? 7 : 3;
+  const dim3 g((n + cw - 1) / cw, mb.M);
+#define C2G_SUM(U)                                                                                   \
+  do {                                                                                               \
+    if (wide)                                                                                        \
+      CASL_K((k_c2g_packed_sum<U, 7, W>), g, 1024, 0, st)(J, ljx, C, csum, n, 4 * n, mb, feat); \
+    else                                                                                             \
+      CASL_K((k_c2g_packed_sum<U, 3, W>), g, 512, 0, st)(J, ljx, C, csum, n, 4 * n, mb, feat);  \
+  } while (0)
+  if (n % 256 == 0 && sizeof(W) == 8)
+    C2G_SUM(8);
+  else if (n % 128 == 0)
+    C2G_SUM(4);
+  else if (n % 64 == 0)
+    C2G_SUM(2);
+  else
+    C2G_SUM(1);
+#undef C2G_SUM
+}
+
 // Coarse cells and their sum from 32-bit jump counts (row 0 of every fine
 // column zero) and bottom-row jumps; *csum must be zero.  n a power of two,
 // 32 or more.
 void c2g_sum32(cudaStream_t st, const int4 *J4, const int *ljx, int *C, unsigned long long *csum,
                int n) {
-  const C2GMembers mb{nullptr, 1, 0, 0, 0};
-  const int nblk = (n + C2G_CW - 1) / C2G_CW, nf = 4 * n;
-  if (n >= 128)
-    CASL_K((k_c2g_packed_sum<4, int4>), nblk, 1024, 0, st)(J4, ljx, C, csum, n, nf, mb, nullptr);
-  else if (n == 64)
-    CASL_K((k_c2g_packed_sum<2, int4>), nblk, 1024, 0, st)(J4, ljx, C, csum, n, nf, mb, nullptr);
-  else
-    CASL_K((k_c2g_packed_sum<1, int4>), nblk, 1024, 0, st)(J4, ljx, C, csum, n, nf, mb, nullptr);
+  c2g_sum<int4>(st, J4, ljx, C, csum, n, C2GMembers{nullptr, 1, 0, 0, 0}, nullptr);
 }
 
 int con2grid_dev(casl_handle *h, bool want_levels) {
@@ -1015,12 +1036,12 @@ int con2grid_dev(casl_handle *h, bool want_levels) {
   int *err = &h->scal->error;
   unsigned long long *csum = (unsigned long long *)&h->scal->csum;
   const int n = h->n;
-  const int U = n % 256 == 0 ? 8 : (n % 128 == 0 ? 4 : (n % 64 == 0 ? 2 : (n % 32 == 0 ? 1 : 0)));
+  const bool rows32 = n % 32 == 0;
   // packed path while the 16-bit counts cannot overflow (one net crossing
   // per level and fine edge: levels well below 32767)
   // an ensemble always takes the packed path (its scratch holds only that)
-  if (h->M > 1 && (want_levels || U == 0 || h->p.ncontq >= 16384)) return CASL_EUNSUPPORTED;
-  if (!want_levels && c.nxf == c.nyf && U > 0 && h->p.ncontq < 16384) {
+  if (h->M > 1 && (want_levels || !rows32 || h->p.ncontq >= 16384)) return CASL_EUNSUPPORTED;
+  if (!want_levels && c.nxf == c.nyf && rows32 && h->p.ncontq < 16384) {
     // four fine rows of a column per 64-bit word, in the first half of the
     // fine-grid buffer (an ensemble: one such block per member)
     unsigned long long *JW = reinterpret_cast<unsigned long long *>(h->fineJ);
@@ -1037,17 +1058,9 @@ int con2grid_dev(casl_handle *h, bool want_levels) {
     // with no nodes the scatter still runs (its first block clears the sums)
     CASL_K(k_c2g_scatter<true>, grid_for(h->nptq > 0 ? h->nptq : 1), 256, 0, h->stream)(
         h->xq, h->yq, h->nextq, h->scal, nullptr, JW, h->ljx, c, err, csum, mb);
-    const dim3 nblk((n + C2G_CW - 1) / C2G_CW, h->M);
     // the learned closure's sub-cell levels, while it is attached (one simulation)
-    int *feat = h->M == 1 ? h->c2g_feat : nullptr;
-    if (U == 8)
-      CASL_K(k_c2g_packed_sum<8>, nblk, 1024, 0, h->stream)(JW, h->ljx, h->coarseC, csum, n, c.nxf, mb, feat);
-    else if (U == 4)
-      CASL_K(k_c2g_packed_sum<4>, nblk, 1024, 0, h->stream)(JW, h->ljx, h->coarseC, csum, n, c.nxf, mb, feat);
-    else if (U == 2)
-      CASL_K(k_c2g_packed_sum<2>, nblk, 1024, 0, h->stream)(JW, h->ljx, h->coarseC, csum, n, c.nxf, mb, feat);
-    else
-      CASL_K(k_c2g_packed_sum<1>, nblk, 1024, 0, h->stream)(JW, h->ljx, h->coarseC, csum, n, c.nxf, mb, feat);
+    c2g_sum<unsigned long long>(h->stream, JW, h->ljx, h->coarseC, csum, n, mb,
+                                h->M == 1 ? h->c2g_feat : nullptr);
     return check_launch(h);
   }
   // the fine-grid levels themselves are wanted: crossings onto the fine

@@ -40,3 +40,20 @@ def test_calls_in_a_row(gpu_lib, n):
         else:
             assert rc == 0 and np.array_equal(q, ref)
     g.close()
+
+
+@pytest.mark.parametrize("n", [32, 64, 128, 256, 512])
+def test_column_widths(oracle_mod, gpu_lib, n):
+    """The handle's con2grid with CTAs of 3 (up to 256) and 7 coarse columns
+    (512) against the oracle's: the same integers, whose mean the oracle takes
+    off in floating point."""
+    from hydra_b200.casl import CaslGPU
+    o = oracle_mod.Oracle(n, ncontq=20, dtmax=0.05)
+    o.initialise(random_pv(n, 4.0, n + 1))
+    ref = o.con2grid()
+    g = CaslGPU(n, ncontq=20)
+    g.set_contours(o.contours())
+    q = g.con2grid()
+    assert np.abs(q - ref).max() <= 1e-12 * np.abs(ref).max()
+    g.close()
+    o.close()
