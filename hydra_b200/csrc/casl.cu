@@ -63,9 +63,9 @@ bool kt_end() {
 }
 
 struct FillJobs {
-  unsigned int *p[6];
-  long long n[6];
-  unsigned int v[6];
+  unsigned int *p[8];
+  long long n[8];
+  unsigned int v[8];
   int nj;
 };
 __global__ void k_fill(FillJobs J) {
@@ -73,7 +73,7 @@ __global__ void k_fill(FillJobs J) {
   const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long stride = (long long)gridDim.x * blockDim.x;
 #pragma unroll
-  for (int j = 0; j < 6; j++) {
+  for (int j = 0; j < 8; j++) {
     if (j >= J.nj) break;
     unsigned int *p = J.p[j];
     const long long n = J.n[j];
@@ -90,7 +90,7 @@ __global__ void k_fill(FillJobs J) {
 }
 
 int fill_words(cudaStream_t st, const FillJob *jobs, int njobs) {
-  if (njobs < 1 || njobs > 6) return CASL_EINVAL;
+  if (njobs < 1 || njobs > 8) return CASL_EINVAL;
   FillJobs J{};
   long long most = 0;
   for (int j = 0; j < njobs; j++) {
