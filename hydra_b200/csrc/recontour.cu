@@ -158,39 +158,48 @@ __device__ __forceinline__ int level_index(double v, const LevInfo &li) {
   return level_steps((int)floor((v + li.qoff) * li.qjumpi + 0.5), v, li);
 }
 
-// level_index with the exact checks only near a level boundary: the
-// estimate x = (v + qoff)/qjump + 1/2 carries a rounding error of a few
-// units of 1e-16 relative (x is at most 65536 + nlevm), as do the qtmp
-// values, so a fractional part of x farther than 1e-6 from 0 and 1 fixes
-// the level; anything else (and a non-finite v) takes level_index's steps.
+// level_index with the exact checks only near a level boundary: the estimate
+// y = (v + qoff)/qjump carries a rounding error of a few units of 1e-16
+// relative (it is at most 65536 + nlevm), as do the qtmp values, so where y
+// lies farther than 1e-6 from a half-integer the nearest integer is the
+// level; anything else (and a non-finite v) takes level_index's steps.  The
+// nearest integer is the low word of y + 1.5 * 2^52: the conversions and the
+// floor it takes the place of run at a quarter of the FP64 rate.  (An y past
+// an int's range would give a wrong code; the levels' range is then refused.)
 __device__ __forceinline__ int level_index_fast(double v, const LevInfo &li) {
-  const double x = (v + li.qoff) * li.qjumpi + 0.5;
-  const double fl = floor(x), fr = x - fl;
-  const int l = (int)fl;
-  if (fr > 1.0e-6 && fr < 1.0 - 1.0e-6) return l;
-  return level_steps(l, v, li);
+  const double big = 6755399441055744.0;
+  const double y = (v + li.qoff) * li.qjumpi, t = y + big;
+  if (fabs(y - (t - big)) < 0.5 - 1.0e-6) return __double2loint(t);
+  return level_steps((int)floor(y + 0.5), v, li);
+}
+__device__ __forceinline__ unsigned int level_code(double v, const LevInfo &li) {
+  return (unsigned int)min(max(level_index_fast(v, li), 0), 65535);
+}
+// (double)i by an integer operation and one subtraction, exact
+__device__ __forceinline__ double int_as_double(int i) {
+  return __hiloint2double(0x43300000, i ^ (int)0x80000000) - 4503601774854144.0;
 }
 
 // One element of the ultra-fine field: (L*qjump - qavg) + bilinear residual,
-// or the bilinear residual alone; (ixf, iyf) is the point's 1-based place in
-// its coarse cell, q00..q11 the cell's corner values.  Per element the
+// or the bilinear residual alone; pxf, pyf is the point's place in its coarse
+// cell (cell_part), q00..q11 the cell's corner values.  Per element the
 // expression and its order are the reference's (congen.f90:45-61 on
 // con2ugrid's field).  The field kernel and the crossing geometry both
 // evaluate the field here, so the crossing positions are computed from the
 // very values the crossings were found on.
-__device__ __forceinline__ double ufield_elem(int lv, int ixf, int iyf, double q00, double q10,
+__device__ __forceinline__ double ufield_elem(int lv, double pxf, double pyf, double q00, double q10,
                                               double q01, double q11, double qjump, double qavg,
                                               int have_contours) {
-  const double fac = 1.0 / 16.0;
-  const double pxf = fac * (double)(ixf - 1), pxc = 1.0 - pxf;
-  const double pyf = fac * (double)(iyf - 1), pyc = 1.0 - pyf;
+  const double pxc = 1.0 - pxf, pyc = 1.0 - pyf;
   const double w00 = pyc * pxc, w10 = pyf * pxc, w01 = pyc * pxf, w11 = pyf * pxf;
   if (have_contours) {
-    double v = (double)lv * qjump - qavg;
+    double v = int_as_double(lv) * qjump - qavg;
     return v + w00 * q00 + w10 * q10 + w01 * q01 + w11 * q11;
   }
   return w00 * q00 + w10 * q10 + w01 * q01 + w11 * q11;
 }
+// a point's place in its coarse cell: (place - 1)/16, exact
+__device__ __forceinline__ double cell_part(int place) { return (1.0 / 16.0) * (double)(place - 1); }
 __device__ __forceinline__ double ufield_qavg(const unsigned long long *lsum, double qjump,
                                               int have_contours, int nxu, int nyu) {
   return have_contours ? qjump * ((double)(long long)(*lsum) / ((double)nxu * (double)nyu)) : 0.0;
@@ -215,7 +224,7 @@ __device__ __forceinline__ double ufield_at(const UField &u, double qavg, int ix
   const double q01 = u.qq[(long long)(ix1 - 1) * n + iy0 - 1];
   const double q11 = u.qq[(long long)(ix1 - 1) * n + iy1 - 1];
   const int lv = u.have ? u.L[(long long)(ix - 1) * c.nyu + iy - 1] : 0;
-  const double v = ufield_elem(lv, ixf, iyf, q00, q10, q01, q11, u.qjump, qavg, u.have);
+  const double v = ufield_elem(lv, cell_part(ixf), cell_part(iyf), q00, q10, q01, q11, u.qjump, qavg, u.have);
   return u.bnc != 0.0 ? v + u.bnc * (c.ymin + c.glyu * (double)(iy - 1)) : v;
 }
 
@@ -244,6 +253,7 @@ __global__ void __launch_bounds__(256, 4) k_u_field(const int *__restrict__ L, c
     const double q01 = qq[(long long)(ix1 - 1) * n + iy0 - 1], q11 = qq[(long long)(ix1 - 1) * n + iy1 - 1];
     if (ixf == 1) l1 += fabs(q00);  // every residual point once
     const long long base = (long long)(ix - 1) * nyu + 16LL * iyy;
+    const double pxf = cell_part(ixf);
     // the run in two halves of 8 points (fewer live registers)
 #pragma unroll 1
     for (int hf = 0; hf < 2; hf++) {
@@ -257,6 +267,7 @@ __global__ void __launch_bounds__(256, 4) k_u_field(const int *__restrict__ L, c
 #pragma unroll
         for (int k = 0; k < 8; k++) lv[k] = 0;
       }
+      const double pyh = 0.5 * hf;  // the half's first point
       unsigned int code[4];
 #pragma unroll
       for (int k = 0; k < 4; k++) {
@@ -264,18 +275,16 @@ __global__ void __launch_bounds__(256, 4) k_u_field(const int *__restrict__ L, c
 #pragma unroll
         for (int h = 0; h < 2; h++) {
           const int iyf = 8 * hf + 2 * k + h;  // 0-based place in the run
-          double v = ufield_elem(lv[2 * k + h], ixf, iyf + 1, q00, q10, q01, q11, qjump, qavg,
-                                 have_contours);
+          double v = ufield_elem(lv[2 * k + h], pxf, pyh + (2 * k + h) * (1.0 / 16.0), q00, q10, q01, q11,
+                                 qjump, qavg, have_contours);
           if (bnc != 0.0) v = v + bnc * (c.ymin + c.glyu * (double)(16 * iyy + iyf));
           out[h] = v;
-          mx = fmax(mx, v);
-          mn = fmin(mn, v);
+          mx = v > mx ? v : mx;  // (fmax and fmin take twice the instructions)
+          mn = v < mn ? v : mn;
         }
         if (qa) reinterpret_cast<double2 *>(qa + base)[4 * hf + k] = make_double2(out[0], out[1]);
         if (lc) {
-          const unsigned int c0 = (unsigned int)min(max(level_index_fast(out[0], lq), 0), 65535);
-          const unsigned int c1 = (unsigned int)min(max(level_index_fast(out[1], lq), 0), 65535);
-          code[k] = c0 | (c1 << 16);
+          code[k] = level_code(out[0], lq) | level_code(out[1], lq) << 16;
         }
       }
       if (lc)
@@ -325,75 +334,118 @@ __device__ __forceinline__ int ext_row0(const ExtGrid &g, int iy, int nyu) {
   return iy < 1 ? 1 + (g.nby * nyu + iy - 1) % nyu : (iy > nyu ? 1 + (iy - 1) % nyu : iy);
 }
 // Minimum and maximum of the field along every basic row (econgen.f90:
-// 114-129): one block per 16 rows, threads over the columns.
-__global__ void __launch_bounds__(256) k_u_rowmm(UField uf, Consts c, double *__restrict__ rmin,
-                                                 double *__restrict__ rmax) {
+// 114-129) as ordered words, the minimum's complemented, both 0 on entry: a
+// block takes 16 rows (one coarse cell) of 512 columns, a thread two columns'
+// runs of them.  (One block per 16 rows, all columns: 256 blocks at 256^2 and
+// the corner values read at every point, 74 us; so 48.)
+__global__ void __launch_bounds__(256) k_u_rowmm(UField uf, Consts c,
+                                                 unsigned long long *__restrict__ rmin,
+                                                 unsigned long long *__restrict__ rmax) {
   CASL_PDL_ENTRY();
-  const int nxu = c.nxu, nyu = c.nyu;
+  const int nxu = c.nxu, nyu = c.nyu, n = c.nx;
   const double qavg = ufield_qavg(uf.lsum, uf.qjump, uf.have, nxu, nyu);
-  const int r0 = 16 * blockIdx.x;
+  const int iyy = blockIdx.x, iy0 = 1 + iyy, iy1 = 2 + iyy - n * (iy0 / n);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   double mn[16], mx[16];
 #pragma unroll
   for (int k = 0; k < 16; k++) {
     mn[k] = 1.0e308;
     mx[k] = -1.0e308;
   }
-  for (int ix = threadIdx.x + 1; ix <= nxu; ix += blockDim.x) {
+#pragma unroll 1
+  for (int h = 0; h < 2; h++) {
+    const int ix = (2 * blockIdx.y + h) * 256 + threadIdx.x + 1, ixx = (ix - 1) / 16;
+    const int ix0 = 1 + ixx, ix1 = 2 + ixx - n * (ix0 / n);
+    const double *q0 = uf.qq + (long long)(ix0 - 1) * n, *q1 = uf.qq + (long long)(ix1 - 1) * n;
+    const double q00 = q0[iy0 - 1], q10 = q0[iy1 - 1], q01 = q1[iy0 - 1], q11 = q1[iy1 - 1];
+    const double pxf = cell_part(ix - 16 * ixx);
+    const int4 *l4 = reinterpret_cast<const int4 *>(uf.L + (long long)(ix - 1) * nyu + 16LL * iyy);
 #pragma unroll
     for (int k = 0; k < 16; k++) {
-      const double v = ufield_at(uf, qavg, ix, r0 + k + 1, c);
-      mn[k] = fmin(mn[k], v);
-      mx[k] = fmax(mx[k], v);
+      int4 l = make_int4(0, 0, 0, 0);
+      if (uf.have) l = l4[k / 4];
+      const int lv = k % 4 == 0 ? l.x : (k % 4 == 1 ? l.y : (k % 4 == 2 ? l.z : l.w));
+      double v = ufield_elem(lv, pxf, k * (1.0 / 16.0), q00, q10, q01, q11, uf.qjump, qavg, uf.have);
+      if (uf.bnc != 0.0) v = v + uf.bnc * (c.ymin + c.glyu * (double)(16 * iyy + k));
+      mn[k] = v < mn[k] ? v : mn[k];
+      mx[k] = v > mx[k] ? v : mx[k];
+    }
+  }
+  // across the warp, each step with half the rows: lanes 2k and 2k+1 end with
+  // row k
+#pragma unroll
+  for (int o = 16, m = 8; m >= 1; o >>= 1, m >>= 1) {
+    const bool hi = lane & o;
+#pragma unroll
+    for (int k = 0; k < m; k++) {
+      const double a = __shfl_xor_sync(0xffffffffu, hi ? mn[k] : mn[k + m], o);
+      const double b = __shfl_xor_sync(0xffffffffu, hi ? mx[k] : mx[k + m], o);
+      const double ka = hi ? mn[k + m] : mn[k], kb = hi ? mx[k + m] : mx[k];
+      mn[k] = a < ka ? a : ka;
+      mx[k] = b > kb ? b : kb;
     }
   }
   __shared__ double smn[8][16], smx[8][16];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < 16; k++) {
-    double a = mn[k], b = mx[k];
-    for (int o = 16; o > 0; o >>= 1) {
-      a = fmin(a, __shfl_xor_sync(0xffffffffu, a, o));
-      b = fmax(b, __shfl_xor_sync(0xffffffffu, b, o));
-    }
-    if (lane == 0) {
-      smn[w][k] = a;
-      smx[w][k] = b;
+  {
+    const double a = __shfl_xor_sync(0xffffffffu, mn[0], 1), b = __shfl_xor_sync(0xffffffffu, mx[0], 1);
+    if (!(lane & 1)) {
+      smn[w][lane >> 1] = a < mn[0] ? a : mn[0];
+      smx[w][lane >> 1] = b > mx[0] ? b : mx[0];
     }
   }
   __syncthreads();
-  if (threadIdx.x < 16 && r0 + threadIdx.x < nyu) {
-    double a = smn[0][threadIdx.x], b = smx[0][threadIdx.x];
-    for (int q = 1; q < (int)(blockDim.x >> 5); q++) {
-      a = fmin(a, smn[q][threadIdx.x]);
-      b = fmax(b, smx[q][threadIdx.x]);
+  if (threadIdx.x < 32) {
+    const int k = threadIdx.x & 15;
+    const bool up = threadIdx.x >= 16;
+    double a = up ? smx[0][k] : smn[0][k];
+    for (int q = 1; q < 8; q++) {
+      const double x = up ? smx[q][k] : smn[q][k];
+      a = up == (x > a) ? x : a;
     }
-    rmin[r0 + threadIdx.x] = a;
-    rmax[r0 + threadIdx.x] = b;
+    if (up)
+      atomicMax(&rmax[16 * iyy + k], ordered_word(a));
+    else
+      atomicMax(&rmin[16 * iyy + k], ~ordered_word(a));
   }
 }
 
 // Level codes of the extended grid, column by column (ld codes each), rows
 // iymin..iymax: the basic rows' codes, and in the extension the level index
 // of qa(iy0) + bfac*(iy - iy0), the value rounded once as the reference's
-// x-line scan forms it (econgen.f90:247-258).
-__global__ void k_u_ext(UField uf, ExtGrid g, LevInfo li, Consts c,
-                        const unsigned short *__restrict__ lc, long long ld,
-                        unsigned short *__restrict__ le) {
+// x-line scan forms it (econgen.f90:247-258).  A block takes 256 rows of the
+// 16 columns of one coarse cell, a thread one row: its corner values and
+// offset are formed once.  (A thread a point, with a 64-bit division, four
+// gathers and the full level search at each: 185 us at 256^2; so 50.)
+__global__ void __launch_bounds__(256) k_u_ext(UField uf, ExtGrid g, LevInfo li, Consts c,
+                                               const unsigned short *__restrict__ lc, long long ld,
+                                               unsigned short *__restrict__ le) {
   CASL_PDL_ENTRY();
-  const int nxu = c.nxu, nyu = c.nyu, nr = g.iymax - g.iymin + 1;
+  const int nxu = c.nxu, nyu = c.nyu, n = c.nx, nr = g.iymax - g.iymin + 1;
+  const int r = blockIdx.x * 256 + threadIdx.x, ixx = blockIdx.y;
+  if (r >= nr) return;
+  const int iy = g.iymin + r;
+  unsigned short *o = le + 16LL * ixx * ld + r;
+  if (iy >= 1 && iy <= nyu) {
+    const unsigned short *s = lc + 16LL * ixx * nyu + iy - 1;
+#pragma unroll
+    for (int k = 0; k < 16; k++) o[k * ld] = s[(long long)k * nyu];
+    return;
+  }
   const double qavg = ufield_qavg(uf.lsum, uf.qjump, uf.have, nxu, nyu);
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < (long long)nxu * nr;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int ix = (int)(t / nr) + 1, r = (int)(t % nr), iy = g.iymin + r;
-    unsigned short code;
-    if (iy >= 1 && iy <= nyu) {
-      code = lc[(long long)(ix - 1) * nyu + iy - 1];
-    } else {
-      const int iy0 = ext_row0(g, iy, nyu);
-      const double v = ufield_at(uf, qavg, ix, iy0, c) + g.bfac * (double)(iy - iy0);
-      code = (unsigned short)min(max(level_index(v, li), 0), 65535);
-    }
-    le[(long long)(ix - 1) * ld + r] = code;
+  const int yb = ext_row0(g, iy, nyu), iyy = (yb - 1) / 16;
+  const double add = g.bfac * (double)(iy - yb), pyf = cell_part(yb - 16 * iyy);
+  const double yn = uf.bnc != 0.0 ? uf.bnc * (c.ymin + c.glyu * (double)(yb - 1)) : 0.0;
+  const int ix0 = 1 + ixx, ix1 = 2 + ixx - n * (ix0 / n);
+  const int iy0 = 1 + iyy, iy1 = 2 + iyy - n * (iy0 / n);
+  const double *q0 = uf.qq + (long long)(ix0 - 1) * n, *q1 = uf.qq + (long long)(ix1 - 1) * n;
+  const double q00 = q0[iy0 - 1], q10 = q0[iy1 - 1], q01 = q1[iy0 - 1], q11 = q1[iy1 - 1];
+  const int *L = uf.L + 16LL * ixx * nyu + yb - 1;
+#pragma unroll 4
+  for (int k = 0; k < 16; k++) {
+    const int lv = uf.have ? L[(long long)k * nyu] : 0;
+    double v = ufield_elem(lv, cell_part(k + 1), pyf, q00, q10, q01, q11, uf.qjump, qavg, uf.have);
+    if (uf.bnc != 0.0) v = v + yn;
+    o[k * ld] = (unsigned short)level_code(v + add, li);
   }
 }
 
@@ -619,7 +671,7 @@ int recontour_dev(casl_handle *h, const double *qq) {
   int *Lu = ar.get<int>(NU);
   int *ljx = ar.get<int>(nxu);
   unsigned long long *lsum = ar.get<unsigned long long>(4);  // level sum; k_u_field's results
-  double *rmn = ar.get<double>(nyu), *rmx = ar.get<double>(nyu);
+  unsigned long long *rmn = ar.get<unsigned long long>(2 * nyu), *rmx = rmn + nyu;
   int *dtot = ar.get<int>(16);
   if (ar.failed) return CASL_ENOMEM;
   CASL_CUDA_TRY(cudaMemsetAsync(lsum, 0, 4 * sizeof(unsigned long long), st));
@@ -662,10 +714,16 @@ int recontour_dev(casl_handle *h, const double *qq) {
   // the host from the rows' minima and maxima
   ExtGrid eg{};
   if (econ) {
-    CASL_K(k_u_rowmm, nyu / 16, 256, 0, st)(uf, c, rmn, rmx);
+    const FillJob z[1] = {{rmn, 4LL * nyu, 0u}};
+    RC_TRY(fill_words(st, z, 1));
+    CASL_K(k_u_rowmm, dim3(nyu / 16, nxu / 512), 256, 0, st)(uf, c, rmn, rmx);
     std::vector<double> qqmin(nyu + 2), qqmax(nyu + 2);
-    RC_TRY(read_back(h, {{qqmin.data() + 1, rmn, nyu * sizeof(double)},
-                         {qqmax.data() + 1, rmx, nyu * sizeof(double)}}));
+    std::vector<unsigned long long> mm(2 * nyu);
+    RC_TRY(read_back(h, {{mm.data(), rmn, mm.size() * 8}}));
+    for (int iy = 0; iy < nyu; iy++) {
+      qqmin[iy + 1] = from_ordered(~mm[iy]);
+      qqmax[iy + 1] = from_ordered(mm[nyu + iy]);
+    }
     qqmin[nyu + 1] = qqmin[1] + ppvdif;
     qqmax[nyu + 1] = qqmax[1] + ppvdif;
     qamin = qqmin[1];
@@ -748,7 +806,7 @@ int recontour_dev(casl_handle *h, const double *qq) {
     tmpi = are.get<int>(scan_tmp_elems(nchunks) + 4);
     if (are.failed) return CASL_ENOMEM;
     cg.lc = le;
-    CASL_K(k_u_ext, gsz((long long)nxu * nye), 256, 0, st)(uf, eg, li, c, lc, cg.ld, le);
+    CASL_K(k_u_ext, dim3((nye + 255) / 256, c.nx), 256, 0, st)(uf, eg, li, c, lc, cg.ld, le);
   } else {
     ccnt = ar.get<int>(nchunks);
     coffs = ar.get<int>(nchunks + 1);
