@@ -579,11 +579,72 @@ struct C2GMembers {
   int cs;            // Scalars stride in 64-bit words (member m's csum = csum + m*cs)
 };
 
-// Per segment (i, nextq(i)): x fine-grid-line crossings and the crossing of
-// y = ymin, counted as +-1 PV jumps (contours.f90:232-270): J += sgn at
-// each (PACKED: into the row's 16-bit lane of JW), ljx the bottom-boundary
-// jumps.  The FP64 expressions are the reference's, evaluated in its order
-// without FMA, so every crossing lands in the same fine cell.
+// One segment, from (xi, yi) to (xa, ya): x fine-grid-line crossings and the
+// crossing of y = ymin, counted as +-1 PV jumps (contours.f90:232-270): J +=
+// sgn at each (PACKED: into the row's 16-bit lane of JW), ljx the
+// bottom-boundary jumps.  The FP64 expressions are the reference's, evaluated
+// in its order without FMA, so every crossing lands in the same fine cell.
+template <bool PACKED>
+__device__ __forceinline__ void c2g_segment(double xi, double yi, double xa, double ya,
+                                            int *__restrict__ J, unsigned long long *__restrict__ JW,
+                                            int *__restrict__ ljx, const Consts &c,
+                                            int *__restrict__ err) {
+  const int nf = c.nxf;
+  // both ends in the domain: an end outside it (or not finite) would give a
+  // crossing count without bound; the node itself is reported by its own lane
+  if (!(xi >= c.xmin && xi < c.xmax && yi >= c.ymin && yi < c.ymax) ||
+      !(xa >= c.xmin && xa < c.xmax && ya >= c.ymin && ya < c.ymax)) {
+    atomicExch(err, CASL_EDOMAIN);
+    return;
+  }
+  const int ixci = 1 + f_int(c.glxfi * (xi - c.xmin));
+  const int ixca = 1 + f_int(c.glxfi * (xa - c.xmin));
+  const double xx = xa - xi;
+  const double dx = xx - c.ellx * f_dint(xx * c.hlxi);
+  const double yy = ya - yi;
+  const double dy = yy - c.elly * f_dint(yy * c.hlyi);
+  const int ixdif = ixca - ixci;
+  // nxc = ixdif - nf*((2*ixdif)/nf): with |2*ixdif| < 2nf the truncated
+  // quotient is -1, 0 or 1
+  const int t2 = 2 * ixdif;
+  const int nxc = ixdif - nf * (t2 >= nf ? 1 : (t2 <= -nf ? -1 : 0));
+  if (fabs(yy) > c.hly) {
+    const double cc = f_sign1(dy);
+    const double p = -(yi - c.hly * cc) / (dy + c.small);
+    int ix = 1 + f_int(c.glxfi * fmod(c.ellx + c.hlx + xi + p * dx, c.ellx));
+    ix = ix < 1 ? 1 : (ix > nf ? nf : ix);
+    red_add_s32(&ljx[ix - 1], -(int)cc);
+  }
+  if (nxc == 0) return;
+  const int jump = f_isign1(nxc);
+  const int ixbeg = ixci + (jump - 1) / 2 + nf;
+  const int sgn = (int)f_sign1(dx);
+  const int cnt = nxc * jump;
+  // the crossings: fine lines ixbeg + k*jump, k < cnt (a few per segment; the
+  // lanes' loops diverge but need no exchange)
+  for (int k = 0; k < cnt; k++) {
+    // (ixbeg + k*jump) mod nf, the argument lying in (nf/2, 5nf/2)
+    int m = ixbeg + k * jump;
+    m -= m >= nf ? nf : 0;
+    m -= m >= nf ? nf : 0;
+    const int ix = 1 + m;
+    const double xgf = c.xmin + c.glxf * (double)(ix - 1);
+    const double x2 = xgf - xi;
+    const double px0 = (x2 - c.ellx * f_dint(x2 * c.hlxi)) / dx;
+    const double y2 = yi + px0 * dy;
+    const int iy = 2 + f_int(c.glyfi * (y2 - c.elly * f_dint(y2 * c.hlyi) - c.ymin));
+    if (iy >= 2 && iy <= c.nyf) {
+      if (PACKED) {
+        const int r = iy - 1;
+        red_add_u64(&JW[(long long)(ix - 1) * c.nx + (r >> 2)],
+                    (unsigned long long)((long long)sgn << (16 * (r & 3))));
+      } else
+        red_add_s32(&J[(long long)(ix - 1) * c.nyf + (iy - 1)], sgn);
+    }
+  }
+}
+
+// Every segment (i, nextq(i)) of the current contours.
 template <bool PACKED>
 __global__ void k_c2g_scatter(const double *__restrict__ xq, const double *__restrict__ yq,
                               const int *__restrict__ nextq, const Scalars *__restrict__ s,
@@ -596,13 +657,11 @@ __global__ void k_c2g_scatter(const double *__restrict__ xq, const double *__res
   if (blockIdx.x == 0)
     for (int m = threadIdx.x; m < mb.M; m += blockDim.x) csum[(long long)m * mb.cs] = 0;
   const unsigned FULL = 0xffffffffu;
-  const int npt = s->nptq, nf = c.nxf, lane = threadIdx.x & 31;
+  const int npt = s->nptq, lane = threadIdx.x & 31;
   const int wstride = gridDim.x * blockDim.x;
   // whole warps step through the nodes together (the shuffles below)
   for (int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < npt; base += wstride) {
     const int i = base + lane;
-    int cnt = 0, ixbeg = 0, jump = 0, sgn = 0;
-    double xi = 0.0, yi = 0.0, dx = 1.0, dy = 0.0;
     // the segment's far end is almost always the next node, which the next
     // lane has loaded: taken by shuffle, so the loads do not wait on nextq
     int ia = -1;
@@ -613,72 +672,15 @@ __global__ void k_c2g_scatter(const double *__restrict__ xq, const double *__res
       y1 = yq[i];
     }
     const double xs = __shfl_down_sync(FULL, x1, 1), ys = __shfl_down_sync(FULL, y1, 1);
-    int mi = 0;
-    if (i < npt) mi = member_of(mb.mnode, mb.M, i);
-    if (i < npt) {
-      if (ia < 0 || ia >= npt) {
-        atomicExch(err, CASL_EINVAL);
-      } else {
-        xi = x1;
-        yi = y1;
-        const bool nb = ia == i + 1 && lane < 31;
-        const double xa = nb ? xs : xq[ia], ya = nb ? ys : yq[ia];
-        // both ends in the domain: an end outside it (or not finite) would
-        // give a crossing count without bound; the node itself is reported
-        // by its own lane
-        if (!(xi >= c.xmin && xi < c.xmax && yi >= c.ymin && yi < c.ymax) ||
-            !(xa >= c.xmin && xa < c.xmax && ya >= c.ymin && ya < c.ymax)) {
-          atomicExch(err, CASL_EDOMAIN);
-        } else {
-          const int ixci = 1 + f_int(c.glxfi * (xi - c.xmin));
-          const int ixca = 1 + f_int(c.glxfi * (xa - c.xmin));
-          const double xx = xa - xi;
-          dx = xx - c.ellx * f_dint(xx * c.hlxi);
-          const double yy = ya - yi;
-          dy = yy - c.elly * f_dint(yy * c.hlyi);
-          const int ixdif = ixca - ixci;
-          // nxc = ixdif - nf*((2*ixdif)/nf): with |2*ixdif| < 2nf the
-          // truncated quotient is -1, 0 or 1
-          const int t2 = 2 * ixdif;
-          const int nxc = ixdif - nf * (t2 >= nf ? 1 : (t2 <= -nf ? -1 : 0));
-          if (fabs(yy) > c.hly) {
-            const double cc = f_sign1(dy);
-            const double p = -(yi - c.hly * cc) / (dy + c.small);
-            int ix = 1 + f_int(c.glxfi * fmod(c.ellx + c.hlx + xi + p * dx, c.ellx));
-            ix = ix < 1 ? 1 : (ix > nf ? nf : ix);
-            red_add_s32(&ljx[(long long)mi * mb.ljs + ix - 1], -(int)cc);
-          }
-          if (nxc != 0) {
-            jump = f_isign1(nxc);
-            ixbeg = ixci + (jump - 1) / 2 + nf;
-            sgn = (int)f_sign1(dx);
-            cnt = nxc * jump;
-          }
-        }
-      }
+    if (i >= npt) continue;
+    const int mi = member_of(mb.mnode, mb.M, i);
+    if (ia < 0 || ia >= npt) {
+      atomicExch(err, CASL_EINVAL);
+      continue;
     }
-    // this lane's own crossings: fine lines ixbeg + k*jump, k < cnt (a few
-    // per segment; the lanes' loops diverge but need no exchange)
-    for (int k = 0; k < cnt; k++) {
-      // (ixbeg + k*jump) mod nf, the argument lying in (nf/2, 5nf/2)
-      int m = ixbeg + k * jump;
-      m -= m >= nf ? nf : 0;
-      m -= m >= nf ? nf : 0;
-      const int ix = 1 + m;
-      const double xgf = c.xmin + c.glxf * (double)(ix - 1);
-      const double x2 = xgf - xi;
-      const double px0 = (x2 - c.ellx * f_dint(x2 * c.hlxi)) / dx;
-      const double y2 = yi + px0 * dy;
-      const int iy = 2 + f_int(c.glyfi * (y2 - c.elly * f_dint(y2 * c.hlyi) - c.ymin));
-      if (iy >= 2 && iy <= c.nyf) {
-        if (PACKED) {
-          const int r = iy - 1;
-          red_add_u64(&JW[(long long)mi * mb.jws + (long long)(ix - 1) * c.nx + (r >> 2)],
-                      (unsigned long long)((long long)sgn << (16 * (r & 3))));
-        } else
-          red_add_s32(&J[(long long)(ix - 1) * c.nyf + (iy - 1)], sgn);
-      }
-    }
+    const bool nb = ia == i + 1 && lane < 31;
+    c2g_segment<PACKED>(x1, y1, nb ? xs : xq[ia], nb ? ys : yq[ia], J,
+                        PACKED ? JW + (long long)mi * mb.jws : JW, ljx + (long long)mi * mb.ljs, c, err);
   }
 }
 
@@ -1031,33 +1033,43 @@ void c2g_sum32(cudaStream_t st, const int4 *J4, const int *ljx, int *C, unsigned
   c2g_sum<int4>(st, J4, ljx, C, csum, n, C2GMembers{nullptr, 1, 0, 0, 0}, nullptr);
 }
 
+// Whether con2grid counts in packed words: while the 16-bit counts cannot
+// overflow (one net crossing per level and fine edge: levels well below 32767).
+static bool c2g_packed(const casl_handle *h) {
+  return h->c.nxf == h->c.nyf && h->n % 32 == 0 && h->p.ncontq < 16384;
+}
+static C2GMembers c2g_members(const casl_handle *h) {
+  return C2GMembers{h->M > 1 ? h->mnode : nullptr, h->M, (long long)h->c.nxf * h->n, h->c.nxf,
+                    (int)(sizeof(Scalars) / 8)};
+}
+
 int con2grid_dev(casl_handle *h, bool want_levels) {
   const Consts &c = h->c;
   int *err = &h->scal->error;
   unsigned long long *csum = (unsigned long long *)&h->scal->csum;
   const int n = h->n;
-  const bool rows32 = n % 32 == 0;
-  // packed path while the 16-bit counts cannot overflow (one net crossing
-  // per level and fine edge: levels well below 32767)
   // an ensemble always takes the packed path (its scratch holds only that)
-  if (h->M > 1 && (want_levels || !rows32 || h->p.ncontq >= 16384)) return CASL_EUNSUPPORTED;
-  if (!want_levels && c.nxf == c.nyf && rows32 && h->p.ncontq < 16384) {
+  if (h->M > 1 && (want_levels || !c2g_packed(h))) return CASL_EUNSUPPORTED;
+  const bool counted = h->jw_counted && !want_levels;  // by the stage before (stage_t)
+  h->jw_counted = 0;
+  if (!want_levels && c2g_packed(h)) {
     // four fine rows of a column per 64-bit word, in the first half of the
     // fine-grid buffer (an ensemble: one such block per member)
     unsigned long long *JW = reinterpret_cast<unsigned long long *>(h->fineJ);
-    const C2GMembers mb{h->M > 1 ? h->mnode : nullptr, h->M, (long long)c.nxf * n, c.nxf,
-                        (int)(sizeof(Scalars) / 8)};
-    // zero words and bottom jumps: inside a step the stage that used them
-    // last has cleared them (k_fs_cols)
-    if (h->jw_dirty) {
-      const FillJob z[2] = {{JW, 2LL * c.nxf * n * h->M, 0u},
-                            {h->ljx, (long long)c.nxf * h->M, 0u}};
-      if (int rc = fill_words(h->stream, z, 2)) return rc;
+    const C2GMembers mb = c2g_members(h);
+    if (!counted) {
+      // zero words and bottom jumps: inside a step the stage that used them
+      // last has cleared them (k_fs_cols)
+      if (h->jw_dirty) {
+        const FillJob z[2] = {{JW, 2LL * c.nxf * n * h->M, 0u},
+                              {h->ljx, (long long)c.nxf * h->M, 0u}};
+        if (int rc = fill_words(h->stream, z, 2)) return rc;
+      }
+      h->jw_dirty = 1;
+      // with no nodes the scatter still runs (its first block clears the sums)
+      CASL_K(k_c2g_scatter<true>, grid_for(h->nptq > 0 ? h->nptq : 1), 256, 0, h->stream)(
+          h->xq, h->yq, h->nextq, h->scal, nullptr, JW, h->ljx, c, err, csum, mb);
     }
-    h->jw_dirty = 1;
-    // with no nodes the scatter still runs (its first block clears the sums)
-    CASL_K(k_c2g_scatter<true>, grid_for(h->nptq > 0 ? h->nptq : 1), 256, 0, h->stream)(
-        h->xq, h->yq, h->nextq, h->scal, nullptr, JW, h->ljx, c, err, csum, mb);
     // the learned closure's sub-cell levels, while it is attached (one simulation)
     c2g_sum<unsigned long long>(h->stream, JW, h->ljx, h->coarseC, csum, n, mb,
                                 h->M == 1 ? h->c2g_feat : nullptr);
@@ -1397,6 +1409,22 @@ struct NodeRkArgs {
   int M;
   const double *du, *dv;  // learned closure: correction at every node (nullable)
 };
+// The node update of an FP64 stage and con2grid's count of the moved contours'
+// crossings for the next stage (see move_nodes).
+struct NodeMoveArgs {
+  const double *x, *y;    // positions
+  const double *x0, *y0;  // at the start of the step (stage 1: x, y)
+  double *xn, *yn;        // moved: never x, y while jumps are counted
+  double *xf, *yf;        // RK4 sums
+  const double *uu, *vv;
+  const double *du, *dv;  // learned closure: correction at every node (nullable)
+  const int *nextq;
+  unsigned long long *JW; // packed jumps (nullptr: none are counted)
+  int *ljx;
+  unsigned long long *csum;
+  int *err;
+  C2GMembers mb;
+};
 // The end of an RK4 stage in the FP32-inversion mode, one launch: blocks below
 // nbn move the nodes (velint + node update), the rest update the spectral
 // fields; the two parts touch disjoint data and read only dt from the scalars.
@@ -1723,17 +1751,51 @@ static int stage_t(casl_handle *h) {
   a.emq = h->emq; a.epq = h->epq; a.qq = h->qq; a.pp = h->pp; a.qdiss = h->qdiss;
   a.rekman = h->p.rekman; a.kdsq = h->c.kdsq; a.therm = h->c.therm;
   a.heating = h->c.heating; a.friction = h->c.friction;
-  const NodeRkArgs<double> nd{h->xq, h->yq, h->xqi, h->yqi, h->xqf, h->yqf, h->uu, h->vv,
-                              M > 1 ? h->mnode : nullptr, M, du, dv};
   const long long npt = h->contex ? (h->nptq > 0 ? h->nptq : 1) : 0;
   // Nodes beyond what the row kernel's half occupancy holds at once move in a
   // launch of their own at full occupancy
   const bool apart = npt > FS_NODES_TOGETHER;
+  const bool count = STAGE < 4 && have && !apart && c2g_packed(h);
+  // Positions alternate between arrays, since a segment is counted from the
+  // moved positions of both its nodes while other warps still read the old
+  // ones: stage 1 leaves the step's start where it was, and the last stage
+  // writes over it, so that xq is the same array before and after a step.
+  NodeMoveArgs nd{};
+  nd.x = h->xq; nd.y = h->yq;
+  nd.x0 = FIRST ? h->xq : h->xqi; nd.y0 = FIRST ? h->yq : h->yqi;
+  nd.xn = STAGE == 4 ? h->xqi : h->uq; nd.yn = STAGE == 4 ? h->yqi : h->vq;
+  nd.xf = h->xqf; nd.yf = h->yqf;
+  nd.uu = h->uu; nd.vv = h->vv;
+  nd.du = du; nd.dv = dv;
+  nd.nextq = h->nextq;
+  nd.JW = count ? reinterpret_cast<unsigned long long *>(h->fineJ) : nullptr;
+  nd.ljx = h->ljx;
+  nd.csum = (unsigned long long *)&h->scal->csum;
+  nd.err = &h->scal->error;
+  nd.mb = c2g_members(h);
   if (apart)
     CASL_K(k_nodes_rk<STAGE>, grid_for(npt), 256, 0, h->stream)(nd, h->scal, h->c);
   const int nbn = apart || !npt ? 0 : grid_for(npt, E::NT);
-  return fs_launch<k_fs_end<LOGN, STAGE>>(h, "k_fs_end", dim3(E::ROWB * M + nbn), E::NT, E::smem,
-                                             0.0, a, nd, h->scal, h->c, nbn, (const double2 *)h->tw);
+  rc = fs_launch<k_fs_end<LOGN, STAGE>>(h, "k_fs_end", dim3(E::ROWB * M + nbn), E::NT, E::smem,
+                                        0.0, a, nd, h->scal, h->c, nbn, (const double2 *)h->tw);
+  if (rc || !npt) return rc;
+  // xq the moved positions, xqi the step's start, uq the array to write next
+  if (FIRST) {
+    std::swap(h->xq, h->xqi);
+    std::swap(h->yq, h->yqi);
+    std::swap(h->xq, h->uq);
+    std::swap(h->yq, h->vq);
+  } else if (STAGE < 4) {
+    std::swap(h->xq, h->uq);
+    std::swap(h->yq, h->vq);
+  } else {
+    std::swap(h->xq, h->xqi);
+    std::swap(h->yq, h->yqi);
+    std::swap(h->xqi, h->uq);
+    std::swap(h->yqi, h->vq);
+  }
+  if (count) h->jw_dirty = h->jw_counted = 1;
+  return CASL_OK;
 }
 template <int STAGE>
 static int stage_dispatch(casl_handle *h) {
@@ -1754,6 +1816,7 @@ static int stage_dispatch(casl_handle *h) {
 // advance (evolution.f90:166-326): four RK4 stages, each con2grid and the
 // stage's spectral work and updates
 static int advance_dev(casl_handle *h) {
+  h->jw_counted = 0;
   h->uv_fp32 = h->prec == CASL_PREC_FP32_INVERSION;
   Trace tr;
   tr.begin(h->stream, "advance");

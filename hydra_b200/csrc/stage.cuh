@@ -698,9 +698,79 @@ __device__ __forceinline__ void fs_rk_qd(const FsEndArgs &a, const Scalars &sm,
     }
   }
 }
+// The node update of a stage (evolution.f90:212-311), and (COUNT) the next
+// stage's con2grid count of the segments between the moved nodes, which is
+// otherwise a launch of its own.  A warp then moves 32 nodes and owns the first
+// 31 (the 32nd is the next warp's first again), so that a segment's far end,
+// almost always the next node, comes from the next lane; the last segment of a
+// contour moves its far end a second time.  Worth it while a launch costs its
+// latency (64^2, 10k nodes: a step 232 to 217 us); with the nodes in a launch of
+// their own it is not (1.4M nodes: 36 + 42 us apart, 76 together, at 46 and 70
+// registers).
+template <int STAGE>
+__device__ __forceinline__ double2 moved(const NodeMoveArgs &a, const Scalars *__restrict__ sc,
+                                         const Consts &c, int i, int m, double2 &u) {
+  const Scalars &sm = sc[m];
+  const long long nn = (long long)c.nx * c.ny;
+  const double x = a.x[i], y = a.y[i];
+  velint1(x, y, a.uu + m * nn, a.vv + m * nn, c, u.x, u.y);
+  if (a.du) {
+    u.x = u.x + a.du[i];
+    u.y = u.y + a.dv[i];
+  }
+  const double h = STAGE == 3 ? sm.dt : (STAGE == 4 ? sm.dt6 : sm.dt2);
+  const double bx = STAGE == 1 ? x : (STAGE == 4 ? a.xf[i] : a.x0[i]);
+  const double by = STAGE == 1 ? y : (STAGE == 4 ? a.yf[i] : a.y0[i]);
+  return make_double2(wrapp(bx + h * u.x, c.ellx, c.hlxi, c.oms),
+                      wrapp(by + h * u.y, c.elly, c.hlyi, c.oms));
+}
+template <int STAGE, bool COUNT>
+__device__ __forceinline__ void move_nodes(int bid, int nbk, const NodeMoveArgs &a,
+                                           const Scalars *__restrict__ sc, const Consts &c) {
+  constexpr int OWN = COUNT ? 31 : 32;
+  const unsigned FULL = 0xffffffffu;
+  const int npt = sc->nptq, lane = threadIdx.x & 31, nw = nbk * (blockDim.x >> 5);
+  if (COUNT && a.JW && bid == 0)  // the coarsening that follows accumulates here
+    for (int m = threadIdx.x; m < a.mb.M; m += blockDim.x) a.csum[(long long)m * a.mb.cs] = 0;
+  for (long long base = (long long)(bid * (blockDim.x >> 5) + (threadIdx.x >> 5)) * OWN; base < npt;
+       base += (long long)nw * OWN) {
+    const int i = (int)base + lane;
+    const bool own = lane < OWN && i < npt;
+    int ia = -1, m = 0;
+    double2 u, p = make_double2(0.0, 0.0);
+    if (i < npt) {
+      if (COUNT && a.JW && own) ia = a.nextq[i];
+      m = member_of(a.mb.mnode, a.mb.M, i);
+      p = moved<STAGE>(a, sc, c, i, m, u);
+    }
+    if (own) {
+      a.xn[i] = p.x;
+      a.yn[i] = p.y;
+      if (STAGE < 4) {
+        const double h = STAGE == 1 ? sc[m].dt6 : sc[m].dt3;
+        const double fx = STAGE == 1 ? a.x0[i] : a.xf[i], fy = STAGE == 1 ? a.y0[i] : a.yf[i];
+        a.xf[i] = wrapp(fx + h * u.x, c.ellx, c.hlxi, c.oms);
+        a.yf[i] = wrapp(fy + h * u.y, c.elly, c.hlyi, c.oms);
+      }
+    }
+    if (COUNT && a.JW) {
+      double2 q = make_double2(__shfl_down_sync(FULL, p.x, 1), __shfl_down_sync(FULL, p.y, 1));
+      if (own) {
+        if (ia < 0 || ia >= npt) {
+          atomicExch(a.err, CASL_EINVAL);
+        } else {
+          if (ia != i + 1) q = moved<STAGE>(a, sc, c, ia, m, u);
+          c2g_segment<true>(p.x, p.y, q.x, q.y, nullptr, a.JW + (long long)m * a.mb.jws,
+                            a.ljx + (long long)m * a.mb.ljs, c, a.err);
+        }
+      }
+    }
+  }
+}
+
 template <int LOGN, int STAGE>
 __global__ void __launch_bounds__(FsEnd<LOGN>::NT, 1024 / FsEnd<LOGN>::NT)
-    k_fs_end(FsEndArgs a, NodeRkArgs<double> nd, Scalars *__restrict__ sc, Consts c, int nbn,
+    k_fs_end(FsEndArgs a, NodeMoveArgs nd, Scalars *__restrict__ sc, Consts c, int nbn,
              const double2 *__restrict__ tw) {
   CASL_PDL_ENTRY();
   using Sh = FsEnd<LOGN>;
@@ -709,11 +779,10 @@ __global__ void __launch_bounds__(FsEnd<LOGN>::NT, 1024 / FsEnd<LOGN>::NT)
   // the half-step time advance that opens stages 2 and 4 (nothing reads t
   // in between)
   if ((STAGE == 1 || STAGE == 3) && blockIdx.x == 0)
-    for (int m = threadIdx.x; m < nd.M; m += blockDim.x) sc[m].t = sc[m].t + sc[m].dt2;
+    for (int m = threadIdx.x; m < nd.mb.M; m += blockDim.x) sc[m].t = sc[m].t + sc[m].dt2;
   const int nrow = gridDim.x - nbn;
   if ((int)blockIdx.x >= nrow) {
-    nodes_rk_body<STAGE, double>(blockIdx.x - nrow, nbn, nd.xq, nd.yq, nd.xqi, nd.yqi, nd.xqf, nd.yqf,
-                            nd.uu, nd.vv, sc, c, nd.mnode, nd.M, nd.du, nd.dv);
+    move_nodes<STAGE, (STAGE < 4)>(blockIdx.x - nrow, nbn, nd, sc, c);
     return;
   }
   extern __shared__ double2 smem[];
@@ -788,10 +857,9 @@ __global__ void __launch_bounds__(FsEnd<LOGN>::NT, 1024 / FsEnd<LOGN>::NT)
 #define FS_NODES_TOGETHER (148 * 1024)
 template <int STAGE>
 __global__ void __launch_bounds__(256)
-    k_nodes_rk(NodeRkArgs<double> nd, const Scalars *__restrict__ sc, Consts c) {
+    k_nodes_rk(NodeMoveArgs nd, const Scalars *__restrict__ sc, Consts c) {
   CASL_PDL_ENTRY();
-  nodes_rk_body<STAGE, double>(blockIdx.x, gridDim.x, nd.xq, nd.yq, nd.xqi, nd.yqi, nd.xqf, nd.yqf,
-                          nd.uu, nd.vv, sc, c, nd.mnode, nd.M, nd.du, nd.dv);
+  move_nodes<STAGE, false>(blockIdx.x, gridDim.x, nd, sc, c);
 }
 
 }  // namespace casl

@@ -55,6 +55,7 @@ struct casl_handle {
   int *fineJ;            // (nyf, nxf): row 0 = bottom level, rows 1.. = jump counts
   int *ljx;              // (nxf)
   int jw_dirty;          // the packed jumps (or ljx) are not zero: clear before a scatter
+  int jw_counted;        // they hold the current contours' jumps already (inside a step)
   int *coarseC;          // (n*n) coarse integer cells
   // reductions
   double *part;          // per-block partials
