@@ -3,7 +3,7 @@
 // The level codes at a box's four corners say for every level which of its
 // edges the level's contours enter and leave by, so a contour can be followed
 // from box to box without any table of crossings: a CTA stages the codes of
-// 32 x 32 boxes in shared memory and walks every contour piece of its tile
+// 128 x 64 boxes in shared memory and walks every contour piece of its tile
 // there.  A crossing's number is its edge's offset (the reference's edge order;
 // the offsets of 16-edge chunks come from a count and a scan, those inside a
 // chunk from the codes) plus its level's place on the edge, known to every CTA
@@ -18,9 +18,10 @@
 // order, and only contours (a few thousand) are sorted by level at the end.
 //
 // Measured (B200), contours plus residual at 1024^2, 25M crossings: the part
-// from the counts to the walk layout took 6.7 ms and takes 3.5 ms (k_cr_count
-// 0.31, k_tr_walk 1.40, ranking 0.45, k_tr_place 1.07), the whole recontouring
-// 13.3 and 9.5 ms; beta-plane from a field at 256^2 3.2 and 1.8 ms.
+// from the counts to the walk layout took 6.7 ms and takes 3.4 ms (k_cr_count
+// 0.24, k_tr_walk 1.37, ranking 0.45, k_tr_place 1.07), the whole recontouring
+// 13.3 and 9.5 ms (8.4 with later changes to the renode passes and the field);
+// beta-plane from a field at 256^2 3.2 and 1.8 ms (1.49).
 // k_tr_walk is bound by the latency of its walks (16k of a tile's 31k cycles:
 // 23 chains of 32 crossings, some 190 cycles a step, in one warp; the rest is
 // staging and the offsets), k_tr_place by issue (63 % of the slots).
@@ -47,6 +48,13 @@ struct CrGrid {
   const unsigned short *lc;
 };
 inline long long cr_chunks(const CrGrid &g) { return g.ncx + (long long)g.nyl * (g.nxu / 16); }
+
+// |a - b| of two pairs of unsigned 16-bit values: the halves' maxima less their
+// minima, which cannot borrow.  __vabsdiffu2 is several times the instructions
+// (k_cr_count at 1024^2 314 us with it, 241 so).
+__device__ __forceinline__ unsigned absdiff2(unsigned a, unsigned b) {
+  return __vmaxu2(a, b) - __vminu2(a, b);
+}
 
 // Crossings per chunk.  A thread takes 8 rows of 17 columns as 16-byte loads
 // (lanes along the rows: coalesced) and counts with packed 16-bit differences:
@@ -83,7 +91,7 @@ __global__ void __launch_bounds__(256, 2) k_cr_count(CrGrid g, int *__restrict__
       int s = 0;
 #pragma unroll
       for (int k = 0; k < 4; k++) {
-        const unsigned d = __vabsdiffu2(c[k], __funnelshift_r(c[k], c[k + 1], 16));
+        const unsigned d = absdiff2(c[k], __funnelshift_r(c[k], c[k + 1], 16));
         s += (2 * k < nv ? d & 0xffffu : 0u) + (2 * k + 1 < nv ? d >> 16 : 0u);
       }
       s += __shfl_down_sync(0xffffffffu, s, 1);
@@ -93,7 +101,7 @@ __global__ void __launch_bounds__(256, 2) k_cr_count(CrGrid g, int *__restrict__
     if (i > 0) {
 #pragma unroll
       for (int k = 0; k < 4; k++) {
-        const unsigned d = __vabsdiffu2(p[k], c[k]);
+        const unsigned d = absdiff2(p[k], c[k]);
         acc[2 * k] += d & 0xffffu;
         acc[2 * k + 1] += d >> 16;
       }
@@ -360,7 +368,7 @@ __global__ void __launch_bounds__(TR_NT, 4) k_tr_walk(TrArgs a) {
     unsigned w = word(p0), run = 0;
 #pragma unroll
     for (int k = 0; k < 8; k++) {
-      const unsigned n = word(p0 + 2 * k + 2), d = __vabsdiffu2(w, __funnelshift_r(w, n, 16));
+      const unsigned n = word(p0 + 2 * k + 2), d = absdiff2(w, __funnelshift_r(w, n, 16));
       const unsigned d0 = d & 0xffffu, d1 = d >> 16;
       *reinterpret_cast<unsigned *>(rel + p0 + 2 * k) = (run & 0xffffu) | (run + d0) << 16;
       if (inner) nodes += (r0 + 2 * k < th ? d0 : 0u) + (r0 + 2 * k + 1 < th ? d1 : 0u);
@@ -376,7 +384,7 @@ __global__ void __launch_bounds__(TR_NT, 4) k_tr_walk(TrArgs a) {
     for (int k = 0; k < 16; k++) {
       const unsigned n = word(p0 + (k + 1) * TS);
       *reinterpret_cast<unsigned *>(rel + TR_Y + p0 + k * TS) = run;
-      run = __vaddus2(run, __vabsdiffu2(w, n));
+      run = __vaddus2(run, absdiff2(w, n));
       w = n;
     }
     if (r > 0 && r < th) nodes += run & 0xffffu;
