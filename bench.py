@@ -147,11 +147,12 @@ def measured_peak():
         return 6650.0, "fallback"
 
 
-# DRAM bytes per launch of the transform pass at 1024^2, read off one ncu
-# capture of the bench workload (dram__bytes_read.sum + dram__bytes_write.sum
-# averaged over its k_rfft_r launches; profiles/rfft_pass_1024.md gives the
-# command).  A stated constant, not a measurement of this run.
-FFT_TRAFFIC_PER_LAUNCH_1024 = 30.7e6
+# DRAM bytes per launch of the transform kernels at 1024^2, read off one ncu
+# capture of steps of this size (dram__bytes_read.sum + dram__bytes_write.sum
+# averaged over its k_fs_cols, k_fs_rows and k_fs_prod launches;
+# profiles/stage_1024.md gives the command).  A stated constant, not a
+# measurement of this run.
+FFT_TRAFFIC_PER_LAUNCH_1024 = 41.4e6
 
 
 # ---------------------------------------------------------------------------
@@ -524,11 +525,12 @@ def run_gpu(a):
                     "steps": e2e["steps"]},
             "roofline": {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
                          "frac": ach / peak if peak else None, "traffic": traffic,
-                         "traffic_source": "constant: ncu DRAM bytes per k_rfft_r launch at "
-                                           "1024^2 (profiles/rfft_pass_1024.md)",
+                         "traffic_source": "constant: ncu DRAM bytes per transform launch at "
+                                           "1024^2 (profiles/stage_1024.md)",
                          "bytes_rule": "16 B per FP64 element per 2-D transform (one read, "
                                        "one write); a pass counts half",
-                         "kernel": "k_rfft (batched real-FFT pass, all variants)",
+                         "kernel": "k_fs_cols, k_fs_rows, k_fs_prod (a stage's transforms; "
+                                   "k_fs_end, whose transform shares the update, is not timed)",
                          "launches": fft_n, "kernel_ms_per_step": fft_ms / a.steps,
                          "peak_source": f"{peak_kind} hbm_gbs"},
             "cpu_baseline": cpu,

@@ -33,7 +33,10 @@ def ellipse(n, count):
 @pytest.mark.parametrize("n,opts,fp32,nodes", [
     (32, FULL, False, 40), (32, NONE, True, 257), (64, FULL, False, 1000), (128, NONE, False, 333),
     (256, FULL, True, 700), (256, NONE, False, 200_000), (512, FULL, False, 900),
-    (512, NONE, False, 0), (1024, FULL, False, 500), (2048, NONE, False, 500)])
+    (512, NONE, False, 0), (1024, FULL, False, 500), (2048, NONE, False, 500),
+    # the node update counts crossings 31 nodes a warp, up to 148 * 1024 nodes
+    (64, NONE, False, 31), (64, FULL, False, 62), (64, NONE, False, 63),
+    (256, NONE, False, 148 * 1024), (256, NONE, False, 148 * 1024 + 1)])
 def test_one_advance(oracle_mod, gpu_lib, n, opts, fp32, nodes):
     from hydra_b200.casl import CaslGPU
     kw = dict(ncontq=20, dtmax=0.05, npm=1 << 19, nm=1 << 12, **opts)
