@@ -601,7 +601,33 @@ static inline int gsz(long long work) {
   return (int)g;
 }
 
-int renode_batch(casl_handle *h, Arena &ar, const RenodeIn &in, RenodeOut &out, int mode) {
+// Steps of a density tile.
+static int rn_steps(long long N) {
+  // Tiles of one step while that leaves no more blocks than fit on the SMs at
+  // once (a tile's steps run one after the other: 10k nodes 16 us with 1, 33
+  // with 8); larger ones above, where each further tile costs its scans (1.4M
+  // nodes 170, 101, 78 and 73 us with 1, 3, 8 and 16; 75k nodes 23, 24, 35 with
+  // 1, 3 and 8; 1.0M nodes 86 and 91 with 8 and 16), 16 once two blocks an SM
+  // are left.
+  return N <= 148LL * 3 * RN_STEP       ? 1
+         : N <= 148LL * 3 * RN_STEP * 4 ? 3
+         : N <= 148LL * 2 * RN_STEP * 16 ? 8
+         : 16;
+}
+
+RenodeWords renode_words(Arena &ar, long long N, int C) {
+  const int step = rn_steps(N) * RN_STEP;
+  const long long nt = (N + step - 1) / step, ct = (C + 255LL) / 256;
+  RenodeWords w{};
+  w.ccnt = ar.get<int>(C);
+  w.nstat = ar.get<unsigned long long>(nt + ct + 2);  // then the contours' words, then the tickets
+  w.job[0] = {w.ccnt, C, 0u};
+  w.job[1] = {w.nstat, 2 * (nt + ct + 2), 0u};
+  return w;
+}
+
+int renode_batch(casl_handle *h, Arena &ar, const RenodeIn &in, RenodeOut &out, int mode,
+                 const RenodeWords *cleared) {
   cudaStream_t st = h->stream;
   const Consts &c = h->c;
   long long N = in.N;
@@ -616,20 +642,12 @@ int renode_batch(casl_handle *h, Arena &ar, const RenodeIn &in, RenodeOut &out, 
   s.S = ar.get<double>(N);
   s.cc = ar.get<int>(N);
   s.cornerpos = ar.get<int>(N + 1);
-  s.ccnt = ar.get<int>(C);
   s.poff = ar.get<int>(C);
-  // Tiles of one step while that leaves no more blocks than fit on the SMs at
-  // once (a tile's steps run one after the other: 10k nodes 16 us with 1, 33
-  // with 8); larger ones above, where each further tile costs its scans (1.4M
-  // nodes 170, 101, 78 and 73 us with 1, 3, 8 and 16; 75k nodes 23, 24, 35 with
-  // 1, 3 and 8; 1.0M nodes 86 and 91 with 8 and 16), 16 once two blocks an SM
-  // are left.
-  const int rnit = N <= 148LL * 3 * RN_STEP       ? 1
-                   : N <= 148LL * 3 * RN_STEP * 4 ? 3
-                   : N <= 148LL * 2 * RN_STEP * 16 ? 8
-                                                   : 16;
+  const int rnit = rn_steps(N);
   const long long nt = (N + rnit * RN_STEP - 1) / (rnit * RN_STEP), ct = (C + 255LL) / 256;
-  s.nstat = ar.get<unsigned long long>(nt + ct + 2);  // then the contours' words, then the tickets
+  const RenodeWords words = cleared ? *cleared : renode_words(ar, N, C);
+  s.ccnt = words.ccnt;
+  s.nstat = words.nstat;
   s.cstat = s.nstat + nt;
   s.tick = reinterpret_cast<int *>(s.cstat + ct);
   s.tilev = ar.get<double>(nt);
@@ -640,10 +658,8 @@ int renode_batch(casl_handle *h, Arena &ar, const RenodeIn &in, RenodeOut &out, 
   long long P = N + C;
   s.piece = ar.get<RnPiece>(P);
   if (ar.failed) return CASL_ENOMEM;
-  {
-    const FillJob z[2] = {{s.ccnt, C, 0u}, {s.nstat, 2 * (nt + ct + 2), 0u}};
-    if (int rc = fill_words(st, z, 2)) return rc;
-  }
+  if (!cleared)
+    if (int rc = fill_words(st, words.job, 2)) return rc;
   int g = gsz(N);
   if (!in.cid) CASL_K(k_rn_cid, g, 256, 0, st)(in, N, s.cid);
   if (rnit == 1)

@@ -116,6 +116,17 @@ struct RenodeScratch {
 // receives [kept contours, kept nodes, overflow flag]; on overflow (kept
 // nodes > out.cap) nothing is written to the output arrays and the caller
 // reports CASL_ECAPACITY when it reads the counts.
-int renode_batch(casl_handle *h, Arena &ar, const RenodeIn &in, RenodeOut &out, int mode);
+// The words a renode needs at zero (corner counts, tile words and tickets) are
+// cleared by renode_batch itself, or by a caller that clears other words
+// anyway: it allocates them (from the same arena, for the same N and C), clears
+// them with its own, and hands them over.
+struct RenodeWords {
+  int *ccnt;
+  unsigned long long *nstat;
+  FillJob job[2];
+};
+RenodeWords renode_words(Arena &ar, long long N, int C);
+int renode_batch(casl_handle *h, Arena &ar, const RenodeIn &in, RenodeOut &out, int mode,
+                 const RenodeWords *cleared = nullptr);
 
 }  // namespace casl

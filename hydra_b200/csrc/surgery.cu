@@ -782,9 +782,11 @@ static inline int gs(long long work) {
 
 // Walk-ordered contours of the current link array + renode + write back.
 // Issues no host synchronisation: every count stays in device memory and
-// every buffer is sized from the node count npt.
+// every buffer is sized from the node count npt.  stat (see surgery_dev) and
+// rw's words are zero.
 static int rebuild_and_renode(casl_handle *h, Arena &ar, int npt, const int *lvl,
-                              const LevelDesc *dlev) {
+                              const LevelDesc *dlev, unsigned long long *stat,
+                              const RenodeWords &rw) {
   cudaStream_t st = h->stream;
   int *rid = ar.get<int>(npt);
   int *dtot = ar.get<int>(8);
@@ -801,17 +803,10 @@ static int rebuild_and_renode(casl_handle *h, Arena &ar, int npt, const int *lvl
   int *ocs = ar.get<int>(npt), *olen = ar.get<int>(npt), *olev = ar.get<int>(npt);
   int *cnt = ar.get<int>(4);
   int *cidw = ar.get<int>(npt);
-  // status words of the runs' and the contours' tiles, then their tickets and
-  // the number of cut runs
   const int rt = (npt + RB_TILE - 1) / RB_TILE, ct = (npt + 255) / 256;
-  unsigned long long *stat = ar.get<unsigned long long>(rt + ct + 2);
   if (ar.failed) return CASL_ENOMEM;
   int *tick = reinterpret_cast<int *>(stat + rt + ct), *nmulti = tick + 2, *err = &h->scal->error;
   const int g = gs(npt);
-  {
-    const FillJob z[1] = {{stat, 2LL * (rt + ct + 2), 0u}};
-    if (int rc = fill_words(st, z, 1)) return rc;
-  }
   CASL_K(k_rb_runs, rt, 256, 0, st)(h->nextq, npt, tick, stat, rid, rs, re, dtot, err);  // dtot[0] = R
   CASL_K(k_rb_cycles_pre, g, 256, 0, st)(h->nextq, rid, rs, re, dtot, nr, lab, nrj, hr, val, ishead,
                                          multi, nmulti);
@@ -832,7 +827,7 @@ static int rebuild_and_renode(casl_handle *h, Arena &ar, int npt, const int *lvl
   out.ocs = ocs; out.olen = olen; out.olev = olev;
   out.cap = h->npm;
   out.d_counts = cnt;
-  rc = renode_batch(h, ar, in, out, RENODE_SURGERY);
+  rc = renode_batch(h, ar, in, out, RENODE_SURGERY, &rw);
   if (rc) return rc;
   CASL_K(k_rb_writeback, gs(h->npm < (1 << 24) ? h->npm : (1 << 24)), 256, 0, st)(
       cnt, h->npm, h->nm, ocs, olen, olev, h->xqi, h->yqi, h->xq, h->yq, h->nextq, h->i1q,
@@ -867,14 +862,23 @@ int surgery_dev(casl_handle *h) {
   unsigned int *wsum = ar.get<unsigned int>((npt >> 14) + 2);
   int *nbox_of = ar.get<int>(npt), *bhead = ar.get<int>(nbox_cap);
   BoxEntry *ent = ar.get<BoxEntry>(ne_cap);
+  // status words of the rebuild's run and contour tiles, then their tickets and
+  // the number of cut runs; and the renode's words
+  const long long nstat = (npt + RB_TILE - 1) / RB_TILE + (npt + 255) / 256 + 2;
+  unsigned long long *stat = ar.get<unsigned long long>(nstat);
+  const RenodeWords rw = renode_words(ar, npt, npt);
   if (ar.failed) return CASL_ENOMEM;
   const int g = gs(npt);
   {
-    const FillJob z[4] = {{endnext, npt, 0xffffffffu},
+    // everything the whole surgery needs cleared, in one launch
+    const FillJob z[7] = {{endnext, npt, 0xffffffffu},
                           {bhead, nbox_cap, 0xffffffffu},
                           {wsum, (npt >> 14) + 2, 0u},
-                          {dtot + 2, 5, 0u}};
-    if (int rc = fill_words(st, z, 4)) return rc;
+                          {dtot + 2, 5, 0u},
+                          {stat, 2 * nstat, 0u},
+                          rw.job[0],
+                          rw.job[1]};
+    if (int rc = fill_words(st, z, 7)) return rc;
   }
   CASL_K(k_lv_all, (nq + SCAN_BLOCK - 1) / SCAN_BLOCK, SCAN_BLOCK, 0, st)(
       h->i1q, h->i2q, h->indq, nq, npt, c, dlev, endnext, dtot, nbox_cap, err);
@@ -914,7 +918,7 @@ int surgery_dev(casl_handle *h) {
     fprintf(stderr, "[casl trace] replay: %d levels, pending %lld (max %d at level %d, %d surgeries there), surgeries %lld (max %d)\n",
             nlev, sp, mp, wl, hs[2 * wl + 1], ss, ms);
   }
-  rc = rebuild_and_renode(h, ar, npt, lvl, dlev);
+  rc = rebuild_and_renode(h, ar, npt, lvl, dlev, stat, rw);
   if (rc) return rc;
   tr.point("rebuild+renode");
   tr.flush("surgery");
