@@ -1816,7 +1816,13 @@ static int stage_dispatch(casl_handle *h) {
 // advance (evolution.f90:166-326): four RK4 stages, each con2grid and the
 // stage's spectral work and updates
 static int advance_dev(casl_handle *h) {
-  h->jw_counted = 0;
+  // A stage's counts serve the next stage of this step only: on every way out,
+  // the early ones included, none are left for a later con2grid of other
+  // contours (which finds the words dirty and clears them).
+  struct Uncount {
+    casl_handle *h;
+    ~Uncount() { h->jw_counted = 0; }
+  } uncount_at_exit{h};
   h->uv_fp32 = h->prec == CASL_PREC_FP32_INVERSION;
   Trace tr;
   tr.begin(h->stream, "advance");
