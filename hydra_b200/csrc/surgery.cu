@@ -57,6 +57,7 @@ struct SurgState {
   // one bit per window of 512 nodes (a word per 16384) set wherever a
   // pending flag is set, so the replay skips empty windows a word at a time
   unsigned int *wsum;
+  const int *err;  // set: lists may be incomplete, and nothing is tested or moved
 };
 
 __device__ __forceinline__ void set_pending(const SurgState &S, int x) {
@@ -250,7 +251,9 @@ __device__ __forceinline__ double4 ld_g0(const double4 *p) {
 // together, here one of 42; the replay, which now follows the links, went from
 // 26 to 42).  Entry q of segment ib is number q*npt + ib for q < SG_OWN;
 // further ones (a segment over more boxes than that) are taken from a running
-// total.  Past its capacity nothing is written (CASL_ECAPACITY is raised).
+// total, in 64 bits: some 80,000 segments that each span half the domain both
+// ways have more than 2^31.  Past its capacity nothing is written
+// (CASL_ECAPACITY is raised, and the kernels that read the lists return).
 // A box's nodes are found through the segments that start in it.  The box a
 // node is tested in and the first of its segment's are rounded apart, so a
 // node on a box's edge can be in neither: it gets an entry of its own.
@@ -259,7 +262,7 @@ __global__ void k_sg_link(const double4 *__restrict__ g0, const int *__restrict_
                           const int *__restrict__ lvl, const LevelDesc *__restrict__ lev, int npt,
                           long long ne_cap, int *__restrict__ bhead, BoxEntry *__restrict__ ent,
                           int *__restrict__ nbox_of,
-                          int *__restrict__ extra, Consts c, int *__restrict__ err) {
+                          unsigned long long *__restrict__ extra, Consts c, int *__restrict__ err) {
   CASL_PDL_ENTRY();
   for (int ib = blockIdx.x * blockDim.x + threadIdx.x; ib < npt; ib += gridDim.x * blockDim.x) {
     const LevelDesc L = lev[lvl[ib]];
@@ -273,7 +276,7 @@ __global__ void k_sg_link(const double4 *__restrict__ g0, const int *__restrict_
     long long far = 0;  // where this segment's entries beyond SG_OWN start
     bool own = false;    // the node's own box is among its segment's
     if (cnt > SG_OWN) {
-      far = (long long)SG_OWN * npt + atomicAdd(extra, cnt - SG_OWN);
+      far = (long long)SG_OWN * npt + (long long)atomicAdd(extra, (unsigned long long)(cnt - SG_OWN));
       if (far + cnt - SG_OWN > ne_cap) atomicExch(err, CASL_ECAPACITY);
     }
     int q = 0;
@@ -288,7 +291,7 @@ __global__ void k_sg_link(const double4 *__restrict__ g0, const int *__restrict_
       }
     }
     if (!own) {
-      const long long e = (long long)SG_OWN * npt + atomicAdd(extra, 1);
+      const long long e = (long long)SG_OWN * npt + (long long)atomicAdd(extra, 1ull);
       if (e < ne_cap)
         reinterpret_cast<int4 *>(ent)[e] = make_int4(atomicExch(&bhead[nb], (int)e), -2 - ib, i, 0);
       else
@@ -317,6 +320,7 @@ __device__ __forceinline__ bool surg_test(double xi, double yi, double xs, doubl
 __global__ void k_sg_candidates(SurgState S, const LevelDesc *__restrict__ lev, int npt,
                                 const int *__restrict__ nbox_of, Consts c) {
   CASL_PDL_ENTRY();
+  if (*S.err) return;
   for (int ib = blockIdx.x * blockDim.x + threadIdx.x; ib < npt; ib += gridDim.x * blockDim.x) {
     int i = S.nq0[ib];
     int mb = nbox_of[ib];
@@ -384,7 +388,7 @@ __global__ void k_sg_replay(SurgState S, const LevelDesc *__restrict__ lev,
   CASL_PDL_ENTRY();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (warp >= *nlev_dev) return;
+  if (warp >= *nlev_dev || *S.err) return;
   const LevelDesc L = lev[warp];
   // Every node, flag and box entry this warp reads or writes belongs to its
   // own level, so no other warp touches them: lane 0's updates reach the
@@ -852,7 +856,8 @@ int surgery_dev(casl_handle *h) {
   tr.begin(st, "start");
   // levels and boxes, on the device
   LevelDesc *dlev = ar.get<LevelDesc>(nq);
-  // [0] nlev, [1] nbox, [2] entries beyond the segments' own, [3] nsurg, [6] blocks done
+  // [0] nlev, [1] nbox, [2..3] entries beyond the segments' own (64 bits), [4] nsurg,
+  // [6] blocks done
   int *dtot = ar.get<int>(16);
   int *endnext = ar.get<int>(npt), *lvl = ar.get<int>(npt);
   double *dx = ar.get<double>(npt), *dy = ar.get<double>(npt);
@@ -884,20 +889,21 @@ int surgery_dev(casl_handle *h) {
       h->i1q, h->i2q, h->indq, nq, npt, c, dlev, endnext, dtot, nbox_cap, err);
   CASL_K(k_sg_init, g, 256, 0, st)(h->xq, h->yq, h->nextq, endnext, npt, dx, dy, g0, nq0, prev0,
                                    pending, dlev, dtot, lvl, c, err);
-  CASL_K(k_sg_link, g, 256, 0, st)(g0, nq0, lvl, dlev, npt, ne_cap, bhead, ent, nbox_of, dtot + 2, c,
-                                   err);
+  CASL_K(k_sg_link, g, 256, 0, st)(g0, nq0, lvl, dlev, npt, ne_cap, bhead, ent, nbox_of,
+                                   reinterpret_cast<unsigned long long *>(dtot + 2), c, err);
   SurgState S{};
   S.xq = h->xq; S.yq = h->yq; S.dx = dx; S.dy = dy; S.nextq = h->nextq;
   S.g0 = g0; S.nq0 = nq0; S.prev0 = prev0; S.lvl = lvl;
   S.bhead = bhead; S.ent = ent; S.nbox_of = nbox_of;
   S.pending = pending;
   S.wsum = wsum;
+  S.err = err;
   tr.point("binning");
   CASL_K(k_sg_candidates, g, 256, 0, st)(S, dlev, npt, nbox_of, c);
   tr.point("candidates");
   int *stats = tr.on ? ar.get<int>(2 * (size_t)nq) : nullptr;
   if (stats) CASL_CUDA_TRY(cudaMemsetAsync(stats, 0, 2 * (size_t)nq * sizeof(int), st));
-  CASL_K(k_sg_replay, (nq * 32 + 127) / 128, 128, 0, st)(S, dlev, dtot + 0, c, dtot + 3, stats);
+  CASL_K(k_sg_replay, (nq * 32 + 127) / 128, 128, 0, st)(S, dlev, dtot + 0, c, dtot + 4, stats);
   rc = check_launch(h);
   if (rc) return rc;
   tr.point("replay");
