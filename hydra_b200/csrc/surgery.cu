@@ -86,12 +86,14 @@ __device__ __forceinline__ void seg_boxes(double x, double y, double dx, double 
     mby1 = f_int(dnby + L.bwyi * (y + dy - c.ymin));
     mby2 = f_int(dnby + L.bwyi * (y - c.ymin));
   }
-  // a wrapped segment is shorter than half the domain; the clamps only guard
-  // the device against corrupt input
-  if (mbx2 - mbx1 + 1 > L.nbx) mbx2 = mbx1 + L.nbx - 1;
-  if (mby2 - mby1 + 1 > L.nby) mby2 = mby1 + L.nby - 1;
-  if (mbx2 < mbx1) mbx2 = mbx1;
-  if (mby2 < mby1) mby2 = mby1;
+  // a wrapped segment is shorter than half the domain, so its boxes lie in
+  // [nbx/2, 5/2 nbx] and it spans at most nbx/2 of them; the clamps keep nodes
+  // that a failed step left out of the domain, or not finite, inside the lists
+  // (the conversion of a NaN is the lowest int)
+  mbx1 = clampi(mbx1, 0, 3 * L.nbx);
+  mby1 = clampi(mby1, 0, 3 * L.nby);
+  mbx2 = clampi(mbx2, mbx1, mbx1 + L.nbx - 1);
+  mby2 = clampi(mby2, mby1, mby1 + L.nby - 1);
 }
 
 __device__ __forceinline__ int node_box(double x, double y, const LevelDesc &L, const Consts &c) {

@@ -4,7 +4,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-CASL_ECAPACITY = 2
+CASL_ECAPACITY, CASL_EDOMAIN = 2, 5
 
 
 def one_level(parts):
@@ -45,3 +45,31 @@ def test_more_entries_than_an_int_counts(gpu_lib):
     g.surgery()
     assert g.counts()[0] == 1
     g.close()
+
+
+def test_nodes_that_are_not_finite(gpu_lib):
+    """Surgery called on what a failed step left (nodes that are NaN have no
+    box) ends in the domain error and writes nowhere it should not: the next
+    state's surgery is that of a fresh handle."""
+    from hydra_b200.casl import CaslError, CaslGPU
+    from hydra_b200.synthetic import random_pv
+    kw = dict(ncontq=20, dtmax=0.05, npm=1 << 18, nm=1 << 14)
+    g, f = CaslGPU(64, **kw), CaslGPU(64, **kw)
+    for s in (g, f):
+        s.initialise(random_pv(64, 5.0, 3))
+    good = f.contours()
+    qs = g.field("qs")
+    qs[2, 3] = np.nan
+    g.set_field("qs", qs)
+    for call in (g.step, g.surgery):
+        with pytest.raises(CaslError) as e:
+            call()
+        assert e.value.code == CASL_EDOMAIN
+    for s in (g, f):
+        s.set_contours(good)
+        s.surgery()
+    cg, cf = g.contours(), f.contours()
+    for k in ("nq", "nptq", "xq", "yq", "nextq"):
+        assert np.array_equal(cg[k], cf[k]), k
+    g.close()
+    f.close()
