@@ -4,8 +4,9 @@
 // node positions and links as it goes, so later tests see earlier
 // reconnections.  The B200 version keeps that exact semantics:
 //   1. Box every segment of every level in parallel (the reference's
-//      nbx = nint(1.2 sqrt(N_lev)) boxes, its bwxi/bwyi scaling), as linked
-//      lists in any order: a scan takes the lowest list index that passes.
+//      nbx = nint(1.2 sqrt(N_lev)) boxes, its bwxi/bwyi scaling); a box's
+//      list is contiguous, in any order: a scan takes the lowest list index
+//      that passes.
 //   2. Test every node against the segments of its box in parallel on the
 //      unmodified state; nodes with a passing test are marked pending.
 //   3. One warp per level replays the reference loop in node order, but only
@@ -39,20 +40,16 @@ struct LevelDesc {
   double bwxi, bwyi;
 };
 
-// A segment in a box: the box's next entry, the segment's list index (the node
-// before its first) and its first node.  isb < 0: no segment, only the node of
-// list index -2 - isb, which lies in this box (see k_sg_link).
-struct __align__(16) BoxEntry {
-  int next, isb, is, pad;
-};
+// An entry of a box: x the list index (the node before the segment's first), ~x
+// where only the node lies in the box (see k_sg_place); y the first node, ~y
+// where it lies in this box.
 struct SurgState {
   double *xq, *yq, *dx, *dy;           // mutable
   int *nextq;                          // mutable
   const double4 *g0;                   // original x, y, dx, dy of every node
   const int *nq0, *prev0, *lvl;
-  const int *bhead;                    // segments listed per box: first entry (-1: none)
-  const BoxEntry *ent;
-  const int *nbox_of;                  // the box each list index's node lies in
+  const uint2 *range;                  // per box: its entries, first and end
+  const int2 *ent;
   unsigned char *pending;
   // one bit per window of 512 nodes (a word per 16384) set wherever a
   // pending flag is set, so the replay skips empty windows a word at a time
@@ -200,26 +197,53 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_lv_all(const int *__restrict__ i
   }
 }
 
+// Every box that lists the segment (x, y, dx, dy): f(box, true); then
+// f(own, false) where the first node's own box is not among them (the box a
+// node is tested in and the first of its segment's are rounded apart, so a node
+// on a box's edge can be in neither).  Nothing unless admit(number of boxes).
+template <class A, class F>
+__device__ __forceinline__ void for_boxes(double x, double y, double dx, double dy,
+                                          const LevelDesc &L, const Consts &c, int own, A admit, F f) {
+  int mbx1, mbx2, mby1, mby2;
+  seg_boxes(x, y, dx, dy, L, c, mbx1, mbx2, mby1, mby2);
+  if (!admit((mbx2 - mbx1 + 1) * (mby2 - mby1 + 1))) return;
+  bool met = false;
+  for (int mbx = mbx1; mbx <= mbx2; mbx++) {
+    const int b0 = L.boxbase + L.nby * (mbx % L.nbx);
+    for (int mby = mby1; mby <= mby2; mby++) {
+      const int gb = b0 + mby % L.nby;
+      met |= gb == own;
+      f(gb, true);
+    }
+  }
+  if (!met) f(own, false);
+}
+
 // work arrays dx, dy (contours.f90:397-415; dsq is dx*dx + dy*dy throughout)
-// and the original state, one 32-byte record per node
+// and the original state, one 32-byte record per node; the entries of every box
+// are counted (bcnt, zero on entry).  Segments of more than 64 boxes are also
+// added up in *far, and left out once those alone exceed the capacity: 90,000
+// segments over 29,000 boxes each would take seconds to count and then be
+// refused.
 __global__ void k_sg_init(const double *__restrict__ xq, const double *__restrict__ yq,
                           const int *__restrict__ nextq, const int *__restrict__ endnext, int npt,
                           double *dx, double *dy, double4 *g0, int *nq0, int *prev0,
                           unsigned char *pending,
                           const LevelDesc *__restrict__ lev, const int *__restrict__ nlev_dev,
-                          int *__restrict__ lvl, Consts c, int *err) {
+                          int *__restrict__ lvl, int *__restrict__ bcnt, long long nbox_cap,
+                          unsigned long long *__restrict__ far, unsigned int ne_cap, Consts c,
+                          int *err) {
   CASL_PDL_ENTRY();
-  const int nlev = *nlev_dev;
+  const int nlev = nlev_dev[0];
+  const bool fits = nlev_dev[1] <= nbox_cap;  // (else k_lv_all has raised CASL_ECAPACITY)
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npt; i += gridDim.x * blockDim.x) {
-    {
-      // the node's level: the last level starting at or below i
-      int lo = 0, hi = nlev - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (lev[mid].ibeg <= i) lo = mid; else hi = mid - 1;
-      }
-      lvl[i] = lo;
+    // the node's level: the last level starting at or below i
+    int lo = 0, hi = nlev - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (lev[mid].ibeg <= i) lo = mid; else hi = mid - 1;
     }
+    lvl[i] = lo;
     int a = endnext[i] >= 0 ? endnext[i] : i + 1;
     double xi = xq[i], yi = yq[i];
     if (!(xi >= c.xmin && xi < c.xmax && yi >= c.ymin && yi < c.ymax)) atomicExch(err, CASL_EDOMAIN);
@@ -238,6 +262,15 @@ __global__ void k_sg_init(const double *__restrict__ xq, const double *__restric
     nq0[i] = nx;
     prev0[nx] = i;
     pending[i] = 0;
+    const LevelDesc L = lev[lo];
+    auto admit = [&](int cnt) {
+      if (!fits) return false;
+      if (cnt <= 64 || atomicAdd(far, (unsigned long long)cnt) + cnt <= ne_cap) return true;
+      atomicExch(err, CASL_ECAPACITY);
+      return false;
+    };
+    for_boxes(xi, yi, ddx, ddy, L, c, node_box(xi, yi, L, c), admit,
+              [&](int gb, bool) { red_add_s32(&bcnt[gb], 1); });
   }
 }
 
@@ -246,59 +279,69 @@ __device__ __forceinline__ double4 ld_g0(const double4 *p) {
   return make_double4(a.x, a.y, b.x, b.y);
 }
 
-// Lists every segment in every box it spans, as linked lists: their order is
-// free (every box list is read as a set) and they hold about two entries, so
-// one exchange on the box's head per entry replaces
-// counting, allotting and placing (at 1.4M nodes five launches of 128 us
-// together, here one of 42; the replay, which now follows the links, went from
-// 26 to 42).  Entry q of segment ib is number q*npt + ib for q < SG_OWN;
-// further ones (a segment over more boxes than that) are taken from a running
-// total, in 64 bits: some 80,000 segments that each span half the domain both
-// ways have more than 2^31.  Past its capacity nothing is written
-// (CASL_ECAPACITY is raised, and the kernels that read the lists return).
-// A box's nodes are found through the segments that start in it.  The box a
-// node is tested in and the first of its segment's are rounded apart, so a
-// node on a box's edge can be in neither: it gets an entry of its own.
-constexpr int SG_OWN = 4;
-__global__ void k_sg_link(const double4 *__restrict__ g0, const int *__restrict__ nq0,
-                          const int *__restrict__ lvl, const LevelDesc *__restrict__ lev, int npt,
-                          long long ne_cap, int *__restrict__ bhead, BoxEntry *__restrict__ ent,
-                          int *__restrict__ nbox_of,
-                          unsigned long long *__restrict__ extra, Consts c, int *__restrict__ err) {
+// The boxes' ranges in the entry array: tiles of 1024 boxes, each taking its share
+// from a running total (the order of the boxes in memory is free).  The total
+// is kept in 64 bits: some 80,000 segments that each span half the domain both
+// ways have more than 2^31 entries.  Past the capacity (CASL_ECAPACITY is
+// raised, and the kernels that read the lists return) nothing is written.
+__global__ void __launch_bounds__(256) k_sg_alloc(const int *__restrict__ bcnt,
+                                                  const int *__restrict__ nbox_dev,
+                                                  long long nbox_cap, unsigned int ne_cap,
+                                                  uint2 *__restrict__ range,
+                                                  unsigned long long *__restrict__ total,
+                                                  int *__restrict__ err) {
   CASL_PDL_ENTRY();
+  __shared__ unsigned long long tot, base;
+  const long long nbox = *nbox_dev < nbox_cap ? (long long)*nbox_dev : nbox_cap;
+  for (long long t0 = blockIdx.x * 1024LL; t0 < nbox; t0 += gridDim.x * 1024LL) {
+    const long long b = t0 + 4 * threadIdx.x;
+    unsigned int n[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) n[k] = b + k < nbox ? (unsigned)bcnt[b + k] : 0u;
+    unsigned long long at = block_excl_scan_any<unsigned long long>(
+        (unsigned long long)n[0] + n[1] + n[2] + n[3], &tot);
+    if (threadIdx.x == 0) {
+      base = atomicAdd(total, tot);
+      if (base + tot > ne_cap) atomicExch(err, CASL_ECAPACITY);
+    }
+    __syncthreads();
+    at += base;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const unsigned int st = (unsigned)(at < ne_cap ? at : ne_cap);
+      if (b + k < nbox) range[b + k] = make_uint2(st, st);
+      at += n[k];
+    }
+    __syncthreads();
+  }
+}
+
+// The entries.  A box's list is contiguous so that the replay reads it 32 wide:
+// as links it was built in one pass, but a warp then waits for one load per
+// entry (a surgery of 40 patches of 500 nodes on one level, lists of thousands,
+// 124 ms, and 23 so; isolated vortices at 1024^2, 39k nodes, 1.6 ms a step, and
+// 1.1 so), and the short lists of a turbulent state gain by it as well (1.4M
+// nodes: this kernel, the counts and the ranges take 15 us more than the links
+// did, the replay went from 107 to 58 us).
+__global__ void k_sg_place(const double4 *__restrict__ g0, const int *__restrict__ nq0,
+                           const int *__restrict__ lvl, const LevelDesc *__restrict__ lev, int npt,
+                           unsigned int ne_cap, uint2 *__restrict__ range, int2 *__restrict__ ent,
+                           int *__restrict__ nbox_of, Consts c, int *__restrict__ err) {
+  CASL_PDL_ENTRY();
+  if (*reinterpret_cast<volatile int *>(err)) return;
   for (int ib = blockIdx.x * blockDim.x + threadIdx.x; ib < npt; ib += gridDim.x * blockDim.x) {
     const LevelDesc L = lev[lvl[ib]];
     const int i = nq0[ib];
     const double4 g = ld_g0(g0 + i);
-    int mbx1, mbx2, mby1, mby2;
-    seg_boxes(g.x, g.y, g.z, g.w, L, c, mbx1, mbx2, mby1, mby2);
-    const int cnt = (mbx2 - mbx1 + 1) * (mby2 - mby1 + 1);
     const int nb = node_box(g.x, g.y, L, c);
     nbox_of[ib] = nb;
-    long long far = 0;  // where this segment's entries beyond SG_OWN start
-    bool own = false;    // the node's own box is among its segment's
-    if (cnt > SG_OWN) {
-      far = (long long)SG_OWN * npt + (long long)atomicAdd(extra, (unsigned long long)(cnt - SG_OWN));
-      if (far + cnt - SG_OWN > ne_cap) atomicExch(err, CASL_ECAPACITY);
-    }
-    int q = 0;
-    for (int mbx = mbx1; mbx <= mbx2; mbx++) {
-      const int mmbx = mbx % L.nbx;
-      for (int mby = mby1; mby <= mby2; mby++, q++) {
-        const int gb = L.boxbase + L.nby * mmbx + mby % L.nby;
-        const long long e = q < SG_OWN ? (long long)q * npt + ib : far + q - SG_OWN;
-        own |= gb == nb;
-        if (e < ne_cap)
-          reinterpret_cast<int4 *>(ent)[e] = make_int4(atomicExch(&bhead[gb], (int)e), ib, i, 0);
-      }
-    }
-    if (!own) {
-      const long long e = (long long)SG_OWN * npt + (long long)atomicAdd(extra, 1ull);
+    for_boxes(g.x, g.y, g.z, g.w, L, c, nb, [](int) { return true; }, [&](int gb, bool segment) {
+      const unsigned int e = atomicAdd(&range[gb].y, 1u);
       if (e < ne_cap)
-        reinterpret_cast<int4 *>(ent)[e] = make_int4(atomicExch(&bhead[nb], (int)e), -2 - ib, i, 0);
+        ent[e] = make_int2(segment ? ib : ~ib, gb == nb ? ~i : i);
       else
         atomicExch(err, CASL_ECAPACITY);
-    }
+    });
   }
 }
 
@@ -329,16 +372,16 @@ __global__ void k_sg_candidates(SurgState S, const LevelDesc *__restrict__ lev, 
     const double2 xy = *reinterpret_cast<const double2 *>(S.g0 + i);
     const double xi = xy.x, yi = xy.y;
     bool hit = false;
-    // the next entry is loaded while this one is tested
-    int e = S.bhead[mb];
-    int4 r = e >= 0 ? reinterpret_cast<const int4 *>(S.ent)[e] : make_int4(-1, 0, 0, 0);
-    while (e >= 0 && !hit) {
-      const int is = r.y < 0 ? i : r.z;
-      e = r.x;
-      if (e >= 0) r = reinterpret_cast<const int4 *>(S.ent)[e];
-      if (is == ib || is == i) continue;
-      const double4 g = ld_g0(S.g0 + is);
-      hit = surg_test(xi, yi, g.x, g.y, g.z, g.w, g.z * g.z + g.w * g.w, c);
+    // two entries at a time: their loads and tests do not wait for each other
+    const uint2 r = S.range[mb];
+    for (unsigned int e = r.x; e < r.y && !hit; e += 2) {
+      const int2 v0 = S.ent[e], v1 = e + 1 < r.y ? S.ent[e + 1] : make_int2(~0, 0);
+      const int s0 = v0.x < 0 ? i : (v0.y < 0 ? ~v0.y : v0.y);
+      const int s1 = v1.x < 0 ? i : (v1.y < 0 ? ~v1.y : v1.y);
+      const double4 p = ld_g0(S.g0 + s0), q = ld_g0(S.g0 + s1);
+      const bool t0 = surg_test(xi, yi, p.x, p.y, p.z, p.w, p.z * p.z + p.w * p.w, c);
+      const bool t1 = surg_test(xi, yi, q.x, q.y, q.z, q.w, q.z * q.z + q.w * q.w, c);
+      hit = (t0 && s0 != ib && s0 != i) || (t1 && s1 != ib && s1 != i);
     }
     S.pending[ib] = hit ? 1 : 0;
     if (hit) atomicOr(&S.wsum[ib >> 14], 1u << ((ib >> 9) & 31));
@@ -366,17 +409,10 @@ __device__ void mark_affected(SurgState &S, const LevelDesc &L, int j, int ib, c
     for (int mbx = mbx1; mbx <= mbx2; mbx++) {
       int mmbx = mbx % L.nbx;
       for (int mby = mby1; mby <= mby2; mby++) {
-        // the nodes in this box are among the first nodes of its segments
-        const int gb = L.boxbase + L.nby * mmbx + mby % L.nby;
-        for (int e = S.bhead[gb]; e >= 0;) {  // 32 entries at a time, one per lane
-          int my = -1;
-          for (int k = 0; k < 32 && e >= 0; k++) {
-            const int2 r = *reinterpret_cast<const int2 *>(S.ent + e);
-            if (lane == k) my = r.y;
-            e = r.x;
-          }
-          if (my < -1) my = -2 - my;
-          if (my >= 0 && S.nbox_of[my] == gb) mark(S, my, ib, L.iend);
+        const uint2 r = S.range[L.boxbase + L.nby * mmbx + mby % L.nby];
+        for (unsigned int k = r.x + lane; k < r.y; k += 32) {
+          const int2 v = S.ent[k];
+          if (v.y < 0) mark(S, v.x < 0 ? ~v.x : v.x, ib, L.iend);  // a node in this box
         }
       }
     }
@@ -469,7 +505,7 @@ __global__ void k_sg_replay(SurgState S, const LevelDesc *__restrict__ lev,
     int i = nextq[ib];
     double xi = xq[i], yi = yq[i];
     int mb = node_box(xi, yi, L, c);
-    const int ehead = S.bhead[mb];
+    const uint2 list = S.range[mb];
     // The reference walks the box's segments in list order and continues
     // after each reconnection with the moved node.  The box list is stored
     // unordered, so each round takes the passing segment with the smallest
@@ -477,13 +513,8 @@ __global__ void k_sg_replay(SurgState S, const LevelDesc *__restrict__ lev,
     int thr = -1;
     while (true) {
       int best = INT_MAX;
-      for (int e = ehead; e >= 0;) {  // 32 entries of the list at a time, one per lane
-        int isb = -1;
-        for (int k = 0; k < 32 && e >= 0; k++) {
-          const int2 r = *reinterpret_cast<const int2 *>(S.ent + e);
-          if (lane == k) isb = r.y;
-          e = r.x;
-        }
+      for (unsigned int k = list.x + lane; k < list.y; k += 32) {
+        const int isb = S.ent[k].x;
         if (isb > thr && isb < best) {
           const int is = nextq[isb];
           if (!(is == ib || is == i)) {
@@ -847,9 +878,10 @@ int surgery_dev(casl_handle *h) {
   const Consts &c = h->c;
   const int nq = h->nq, npt = h->nptq;
   const long long nbox_cap = 2LL * npt + nq + 64;
-  const long long ne_cap = std::min((16LL + SG_OWN) * npt + 64, (long long)INT_MAX);
-  size_t need = (size_t)npt * 760 + (size_t)nq * 96 + (size_t)nbox_cap * 24 +
-                (size_t)ne_cap * 16 + ((size_t)64 << 20);
+  const unsigned int ne_cap = (unsigned)std::min(20LL * npt + 64, (long long)INT_MAX);
+  // (305 bytes a node beside the boxes and their entries)
+  size_t need = (size_t)npt * 400 + (size_t)nq * 96 + (size_t)nbox_cap * 12 +
+                (size_t)ne_cap * 8 + ((size_t)64 << 20);
   int rc = ensure_scratch(h, need);
   if (rc) return rc;
   Arena ar{(char *)h->sx, h->sx_bytes, 0};
@@ -858,8 +890,8 @@ int surgery_dev(casl_handle *h) {
   tr.begin(st, "start");
   // levels and boxes, on the device
   LevelDesc *dlev = ar.get<LevelDesc>(nq);
-  // [0] nlev, [1] nbox, [2..3] entries beyond the segments' own (64 bits), [4] nsurg,
-  // [6] blocks done
+  // [0] nlev, [1] nbox, [2..3] entries (64 bits), [4] nsurg, [6] blocks done,
+  // [8..9] entries of segments over many boxes (64 bits)
   int *dtot = ar.get<int>(16);
   int *endnext = ar.get<int>(npt), *lvl = ar.get<int>(npt);
   double *dx = ar.get<double>(npt), *dy = ar.get<double>(npt);
@@ -867,8 +899,9 @@ int surgery_dev(casl_handle *h) {
   int *nq0 = ar.get<int>(npt), *prev0 = ar.get<int>(npt);
   unsigned char *pending = ar.get<unsigned char>(npt + 16);
   unsigned int *wsum = ar.get<unsigned int>((npt >> 14) + 2);
-  int *nbox_of = ar.get<int>(npt), *bhead = ar.get<int>(nbox_cap);
-  BoxEntry *ent = ar.get<BoxEntry>(ne_cap);
+  int *nbox_of = ar.get<int>(npt), *bcnt = ar.get<int>(nbox_cap);
+  uint2 *range = ar.get<uint2>(nbox_cap);
+  int2 *ent = ar.get<int2>(ne_cap);
   // status words of the rebuild's run and contour tiles, then their tickets and
   // the number of cut runs; and the renode's words
   const long long nstat = (npt + RB_TILE - 1) / RB_TILE + (npt + 255) / 256 + 2;
@@ -879,9 +912,9 @@ int surgery_dev(casl_handle *h) {
   {
     // everything the whole surgery needs cleared, in one launch
     const FillJob z[7] = {{endnext, npt, 0xffffffffu},
-                          {bhead, nbox_cap, 0xffffffffu},
+                          {bcnt, nbox_cap, 0u},
                           {wsum, (npt >> 14) + 2, 0u},
-                          {dtot + 2, 5, 0u},
+                          {dtot + 2, 8, 0u},
                           {stat, 2 * nstat, 0u},
                           rw.job[0],
                           rw.job[1]};
@@ -890,13 +923,15 @@ int surgery_dev(casl_handle *h) {
   CASL_K(k_lv_all, (nq + SCAN_BLOCK - 1) / SCAN_BLOCK, SCAN_BLOCK, 0, st)(
       h->i1q, h->i2q, h->indq, nq, npt, c, dlev, endnext, dtot, nbox_cap, err);
   CASL_K(k_sg_init, g, 256, 0, st)(h->xq, h->yq, h->nextq, endnext, npt, dx, dy, g0, nq0, prev0,
-                                   pending, dlev, dtot, lvl, c, err);
-  CASL_K(k_sg_link, g, 256, 0, st)(g0, nq0, lvl, dlev, npt, ne_cap, bhead, ent, nbox_of,
-                                   reinterpret_cast<unsigned long long *>(dtot + 2), c, err);
+                                   pending, dlev, dtot, lvl, bcnt, nbox_cap,
+                                   reinterpret_cast<unsigned long long *>(dtot + 8), ne_cap, c, err);
+  CASL_K(k_sg_alloc, (int)std::min((nbox_cap + 1023) / 1024, 148LL * 8), 256, 0, st)(
+      bcnt, dtot + 1, nbox_cap, ne_cap, range, reinterpret_cast<unsigned long long *>(dtot + 2), err);
+  CASL_K(k_sg_place, g, 256, 0, st)(g0, nq0, lvl, dlev, npt, ne_cap, range, ent, nbox_of, c, err);
   SurgState S{};
   S.xq = h->xq; S.yq = h->yq; S.dx = dx; S.dy = dy; S.nextq = h->nextq;
   S.g0 = g0; S.nq0 = nq0; S.prev0 = prev0; S.lvl = lvl;
-  S.bhead = bhead; S.ent = ent; S.nbox_of = nbox_of;
+  S.range = range; S.ent = ent;
   S.pending = pending;
   S.wsum = wsum;
   S.err = err;

@@ -1,4 +1,9 @@
-"""Surgery's box lists where segments and boxes are unlike a smooth flow's."""
+"""Surgery's box lists where segments and boxes are unlike a smooth flow's.
+
+Bars: topology identical to the oracle's; nodes 1e-12 of the domain's half side,
+as in the surgery parity tests."""
+import time
+
 import numpy as np
 import pytest
 
@@ -47,6 +52,25 @@ def test_more_entries_than_an_int_counts(gpu_lib):
     g.close()
 
 
+def test_more_boxes_than_the_table(gpu_lib):
+    """A domain 16 times as long as wide gives a level of four nodes 10 boxes;
+    200 of them have more than the 2 a node that the table is sized for, which
+    is refused with nothing written behind it."""
+    from hydra_b200.casl import CaslError, CaslGPU
+    g = CaslGPU(64, ncontq=20, ellx=32 * np.pi, elly=2 * np.pi, npm=1 << 16, nm=1 << 12)
+    a = np.pi / 2 * np.arange(4)
+    c = one_level([(0.2 * k - 20 + 0.1 * np.cos(a), 0.1 * np.sin(a)) for k in range(200)])
+    g.set_contours(dict(c, indq=np.arange(1, 201, dtype=np.int32)))
+    with pytest.raises(CaslError) as e:
+        g.surgery()
+    assert e.value.code == CASL_ECAPACITY
+    a = 2 * np.pi * np.arange(300) / 300
+    g.set_contours(one_level([(5 * np.cos(a), np.sin(a))]))
+    g.surgery()
+    assert g.counts()[0] == 1
+    g.close()
+
+
 def test_nodes_that_are_not_finite(gpu_lib):
     """Surgery called on what a failed step left (nodes that are NaN have no
     box) ends in the domain error and writes nowhere it should not: the next
@@ -73,3 +97,65 @@ def test_nodes_that_are_not_finite(gpu_lib):
         assert np.array_equal(cg[k], cf[k]), k
     g.close()
     f.close()
+
+
+def ellipses(count, nodes, rx, ry, pitch, per_row):
+    a = 2 * np.pi * np.arange(nodes) / nodes
+    return [(-2 + pitch * (k % per_row) + rx * np.cos(a), -2 + pitch * (k // per_row) + ry * np.sin(a))
+            for k in range(count)]
+
+
+def spiral(nodes, turns, gap):
+    t = np.linspace(0, 2 * np.pi * turns, nodes // 2)
+    r = np.linspace(0.1, 0.5, nodes // 2)
+    out = [((r + s * gap) * np.cos(t), (r + s * gap) * np.sin(t)) for s in (0.5, -0.5)]
+    return [tuple(np.concatenate([out[0][k], out[1][k][::-1]]) for k in (0, 1))]
+
+
+# a box's list from a few entries to thousands (the whole level in a few boxes),
+# around the 32 lanes that read it, and boxes around the 1024 of a tile
+CLUSTERED = {
+    "one box": lambda: ellipses(3, 150, 0.02, 0.01, 0.0, 3),
+    "32 a box": lambda: ellipses(12, 100, 0.1, 0.08, 0.15, 4),
+    "patches": lambda: ellipses(40, 500, 0.05, 0.03, 0.1, 8),
+    "spiral": lambda: spiral(3000, 12, 0.004),
+    "tile of boxes": lambda: ellipses(8, 89, 0.3, 0.25, 0.7, 4),
+    "two tiles": lambda: ellipses(16, 90, 0.3, 0.25, 0.7, 4),
+}
+
+
+@pytest.mark.parametrize("case", list(CLUSTERED))
+def test_clustered_state(oracle_mod, gpu_lib, case):
+    from hydra_b200.casl import CaslGPU
+    n = 256
+    c = one_level(CLUSTERED[case]())
+    kw = dict(ncontq=20, npm=1 << 18, nm=1 << 14)
+    o, g = oracle_mod.Oracle(n, **kw), CaslGPU(n, **kw)
+    for s in (o, g):
+        s.set_contours(c)
+        s.surgery()
+    co, cg = o.contours(), g.contours()
+    assert (cg["nq"], cg["nptq"]) == (co["nq"], co["nptq"])
+    for k in ("npq", "i1q", "i2q", "indq", "nextq"):
+        assert np.array_equal(cg[k], co[k]), k
+    for k in ("xq", "yq"):
+        assert np.abs(cg[k] - co[k]).max() <= 1e-12 * np.pi, k
+    o.close()
+    g.close()
+
+
+def test_long_lists_are_read_in_parallel(gpu_lib):
+    """Thousands of entries a box, read by a level's warp at every pending node:
+    23 ms with 32 lanes on the list, 124 ms with a load after another.  The
+    best of five is to stay below 60 ms."""
+    from hydra_b200.casl import CaslGPU
+    g = CaslGPU(512, ncontq=60, npm=1 << 18, nm=1 << 14)
+    c = one_level(CLUSTERED["patches"]())
+    best = 1e9
+    for _ in range(5):
+        g.set_contours(c)
+        t = time.perf_counter()
+        g.surgery()
+        best = min(best, time.perf_counter() - t)
+    assert best < 60e-3, best
+    g.close()
