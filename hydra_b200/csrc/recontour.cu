@@ -898,6 +898,13 @@ int recontour_dev(casl_handle *h, const double *qq) {
     CASL_K(k_ch_jump2, gsS, 256, 0, st)(lA, S, lB, it, flag + MAXR);
     std::swap(lA, lB);
   }
+  if (tr.on) {
+    int f[2 * MAXR], ran[2] = {1, 1};
+    RC_TRY(read_back(h, {{f, flag, sizeof(f)}}));
+    for (int q = 0; q < 2; q++)
+      while (ran[q] < rounds && f[q * MAXR + ran[q] - 1]) ran[q]++;
+    fprintf(stderr, "[casl trace] ranking: %d and %d of %d launches\n", ran[0], ran[1], rounds);
+  }
   CASL_K(k_ch_heads, gsS, 256, 0, st)(head, jA, lA, ta.clev, S, key, slot, slen, cslot, dtot + 4);
   RC_TRY(check_launch(h));
   int C0 = 0;

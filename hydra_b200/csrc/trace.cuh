@@ -666,14 +666,16 @@ __global__ void __launch_bounds__(TR_NT) k_tr_place(PlArgs a) {
 // ---------------------------------------------------------------------------
 // Ranking over the chains
 // ---------------------------------------------------------------------------
-// Each chain's jump state is one 16-byte record (next, minimum, terminal flag,
-// last), so that a hop gathers two records (at next and at last).  A launch
-// makes three hops (windows grow fourfold): at a few hundred thousand chains
-// it is the launches and the gathers' latency that cost, not the bytes.  A
-// launch that changes no minimum, flag or last leaves none to change (a window
-// that does not cover its cycle has a chain whose minimum the next one
-// lowers), so the launches after it return at once: flag[it] says whether
-// launch it changed anything.
+// Each chain's jump state is one 16-byte record (next, minimum, terminal flag),
+// one gather a hop.  A launch makes three hops (windows grow fourfold): at a few
+// hundred thousand chains it is the launches and the gathers' latency that
+// cost, not the bytes.  The last chain of a list is its own next, so next ends
+// there in the launch that sets the flag; around a cycle it keeps turning and
+// says nothing.  A launch that changes no minimum and no flag leaves none to
+// change (a window that does not cover its cycle has a chain whose minimum the
+// next one lowers, one that does not reach its list's end a chain whose flag it
+// sets), so the launches after it return at once: flag[it] says whether launch
+// it changed anything.
 __global__ void k_ch_init(const int4 *__restrict__ chain, const int2 *__restrict__ own, int S,
                           int *__restrict__ nexts, int4 *__restrict__ J, int *__restrict__ err) {
   CASL_PDL_ENTRY();
@@ -685,7 +687,7 @@ __global__ void k_ch_init(const int4 *__restrict__ chain, const int2 *__restrict
       n = -1;
     }
     nexts[k] = n;
-    J[k] = make_int4(n < 0 ? k : n, c.z, n < 0, n < 0 ? k : n);
+    J[k] = make_int4(n < 0 ? k : n, c.z, n < 0, 0);
   }
 }
 __global__ void k_ch_jump1(const int4 *__restrict__ J, int S, int4 *__restrict__ J2, int it,
@@ -699,10 +701,10 @@ __global__ void k_ch_jump1(const int4 *__restrict__ J, int S, int4 *__restrict__
 #pragma unroll
     for (int h = 0; h < 3; h++) {
       const int4 b = J[r.x];
-      r = make_int4(b.x, min(r.y, b.y), r.z | b.z, J[r.w].w);
+      r = make_int4(b.x, min(r.y, b.y), r.z | b.z, 0);
     }
     J2[k] = r;
-    changed |= r.y != a.y || r.z != a.z || r.w != a.w;
+    changed |= r.y != a.y || r.z != a.z;
   }
   if (__syncthreads_or(changed) && threadIdx.x == 0 && __ldcg(flag + it) == 0) flag[it] = 1;
 }
@@ -777,12 +779,12 @@ __global__ void k_ch_query(const int *__restrict__ st, int m, const int2 *__rest
     const int2 o = own[st[q]];
     const int4 j = J[o.x];
     const int2 om = own[j.y];
-    out[q] = chain[j.w].w;
+    out[q] = chain[j.x].w;
     out[m + q] = (int)L[o.x].suf - o.y;
     out[2 * m + q] = j.y;
     out[3 * m + q] = (int)L[om.x].suf - om.y;
     out[4 * m + q] = clev[o.x];
-    out[5 * m + q] = j.w;
+    out[5 * m + q] = j.x;
   }
 }
 // Contours in order: lengths, levels, and each slot's place.
@@ -814,7 +816,7 @@ __global__ void k_ch_place(const int *__restrict__ head, const int4 *__restrict_
       const int c = place[cslot[h]], len = clen[c];
       R[k] = make_int4(len - suf - own[J[k].y].y, len, coff[c], c);
     } else {
-      const int q = listof ? listof[J[k].w] : -1;
+      const int q = listof ? listof[J[k].x] : -1;
       if (q < 0) {
         R[k] = make_int4(0, 0, 0, -1);
       } else {
