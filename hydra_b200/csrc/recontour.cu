@@ -849,7 +849,7 @@ int recontour_dev(casl_handle *h, const double *qq) {
     const FillJob z[1] = {{ta.nchain, 2, 0u}};
     RC_TRY(fill_words(st, z, 1));
   }
-  const int ntile = (nxu / TX) * ((cg.nbr + TY - 1) / TY);
+  const int ntile = (nxu / TX) * ((cg.nbr + TY - 1) / TY), nslice = tr_slices(ntile, ncr);
   {
     static std::atomic<unsigned long long> configured{0};  // a bit per device
     const unsigned long long bit = 1ULL << (h->device & 63);
@@ -859,7 +859,7 @@ int recontour_dev(casl_handle *h, const double *qq) {
       configured.fetch_or(bit);
     }
   }
-  CASL_K(k_tr_walk, ntile, TR_NT, sizeof(TrSmem), st)(ta);
+  CASL_K(k_tr_walk, dim3(ntile, nslice), TR_NT, sizeof(TrSmem), st)(ta);
   RC_TRY(check_launch(h));
   int cnts[2] = {0, 0};
   RC_TRY(read_back(h, {{cnts, ta.nchain, 2 * sizeof(int)}}));
@@ -1053,9 +1053,9 @@ int recontour_dev(casl_handle *h, const double *qq) {
                                       d_lslot, S, R);
   const PlArgs pl{cg, li, uf, eg, c, coffs, ta.own, R, xw, yw, cidw};
   if (econ)
-    CASL_K(k_tr_place<true>, ntile, TR_NT, 0, st)(pl);
+    CASL_K(k_tr_place<true>, dim3(ntile, nslice), TR_NT, 0, st)(pl);
   else
-    CASL_K(k_tr_place<false>, ntile, TR_NT, 0, st)(pl);
+    CASL_K(k_tr_place<false>, dim3(ntile, nslice), TR_NT, 0, st)(pl);
   RC_TRY(check_launch(h));
 
   tr.point("layout");

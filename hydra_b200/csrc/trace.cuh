@@ -134,7 +134,11 @@ constexpr int TCX = TY / 16, TCY = TX / 16;           // chunks per column, per 
 constexpr int TQX = (TX + 1) * TCX, TQY = (TY + 1) * TCY;  // x-line and y-line chunks met
 constexpr int TB = 32;             // chains end at every TB-th x-line and y-line
 constexpr int TR_NT = 256;        // threads per tile
-constexpr int TR_SCAP = 512, TR_GCAP = 2048;
+// Starts listed at once (2048 words leave room for the three CTAs an SM that 512
+// leave; 128^2, 2000 levels: k_tr_walk 845, 560, 405 us with 512, 1024, 2048),
+// crossings listed at once, and the crossings an edge from which edges are
+// listed instead (64^2, 1000 levels: k_tr_place 420 us from 4, 575 from 8 on).
+constexpr int TR_SCAP = 2048, TR_GCAP = 2048, TR_MANY = 4;
 // column of staged point m (m / TS for every m < (TX + 2) * TS)
 __device__ __forceinline__ int tr_col(int m) { return (m * 993) >> 16; }
 
@@ -330,20 +334,80 @@ __device__ __forceinline__ bool tr_least(const TrArgs &a, const TrTile &T, int m
   return false;
 }
 
+// The starts of a tile's chains: the crossings of every TB-th line that enter a
+// box of the tile, and the out-crossings of its saddle boxes on other lines.
+// line(m, y, c0, c1, which, last): an edge of such a line, from point m (y-line
+// when y) with codes c0, c1 at its ends, on line `which` of 0..last;
+// range(m, y, lo, hi): levels lo+1 .. hi that leave a saddle box by edge (m, y).
+template <class Line, class Range>
+__device__ __forceinline__ void tr_starts(const TrTile &T, Line line_f, Range range) {
+  const unsigned short *C = T.C;
+  const int tid = threadIdx.x, th = T.th;
+  auto word = [&](int p) { return *reinterpret_cast<const unsigned *>(C + p); };
+  constexpr int LX = (TX / TB + 1) * TY, LY = (TY / TB + 1) * TX;
+  for (int q = tid; q < LX + LY; q += TR_NT) {
+    const bool y = q >= LX;
+    const int line = y ? (q - LX) / TX * TB : q / TY * TB, at = y ? (q - LX) % TX : q % TY;
+    const int m = y ? at * TS + line : line * TS + at;
+    const bool ok = y ? line < th || (th == TY && line == TY) : at < th;
+    if (!ok || (y && ((line == 0 && T.open0) || (line == th && T.open1)))) continue;
+    line_f(m, (int)y, (int)C[m], (int)C[m + (y ? TS : 1)], line, y ? TY : TX);
+  }
+  // saddles, two rows of boxes at a time; a thread's boxes: half a column
+  const int bi = tid >> 1, bj0 = (TY / 2) * (tid & 1);
+  int m = bi * TS + bj0;
+  unsigned a0 = word(m), b0 = word(m + TS);
+  for (int j = bj0; j < bj0 + TY / 2; j += 2, m += 2) {
+    const unsigned a2 = word(m + 2), b2 = word(m + TS + 2);
+    const unsigned a1 = __funnelshift_r(a0, a2, 16), b1 = __funnelshift_r(b0, b2, 16);
+    const unsigned sd = __vcmpgtu2(__vminu2(a0, b1), __vmaxu2(b0, a1)) |
+                        __vcmpgtu2(__vminu2(b0, a1), __vmaxu2(a0, b1));
+    if (sd) {
+      for (int h = 0; h < 2; h++) {
+        const int jj = j + h, mm = m + h;
+        if (jj >= th) break;
+        const int c00 = C[mm], c10 = C[mm + TS], c01 = C[mm + 1], c11 = C[mm + TS + 1];
+        const int xl = max(c10, c01), xh = min(c00, c11), yl = max(c00, c11), yh = min(c10, c01);
+        if (xh > xl) {  // exits left and right
+          if (bi % TB) range(mm, 0, xl, xh);
+          if ((bi + 1) % TB) range(mm + TS, 0, xl, xh);
+        }
+        if (yh > yl) {  // exits bottom and top
+          if (jj % TB) range(mm, 1, yl, yh);
+          if ((jj + 1) % TB && jj + 1 < th) range(mm + 1, 1, yl, yh);
+        }
+      }
+    }
+    a0 = a2;
+    b0 = b2;
+  }
+}
+// The levels of a line's edge that start there: c1 high, to the right or down;
+// c0 high, to the left or up.  On the tile's own sides only those that enter it.
+template <class Range>
+__device__ __forceinline__ void tr_line_starts(int m, int y, int c0, int c1, int line, int last,
+                                               Range range) {
+  if ((y ? line > 0 : line < last) && c1 > c0) range(m, y, c0, c1);
+  if ((y ? line < last : line > 0) && c0 > c1) range(m, y, c1, c0);
+}
+
 struct TrSmem {
   unsigned short before[TS + 6];  // a step down or to the left of the tile reads here
   unsigned short C[TR_Y], rel[2 * TR_Y];
   int cb[TQX + TQY];
   unsigned int slist[TR_SCAP];
 };
-__global__ void __launch_bounds__(TR_NT, 4) k_tr_walk(TrArgs a) {
+// A tile is one CTA's (blockIdx.x), or several's when its crossings are many and
+// tiles few (blockIdx.y, tr_slices): each then stages the tile and takes its
+// share of the starts.
+__global__ void __launch_bounds__(TR_NT, 3) k_tr_walk(TrArgs a) {
   CASL_PDL_ENTRY();
   extern __shared__ __align__(16) unsigned char tr_smem[];
   TrSmem &sm = *reinterpret_cast<TrSmem *>(tr_smem);
   unsigned short *C = sm.C, *rel = sm.rel;
   int *cb = sm.cb;
   unsigned int *slist = sm.slist;
-  __shared__ int nstart, nvis, nnode, base;
+  __shared__ int nstart, nvis, nnode, base, total;
   const CrGrid &g = a.g;
   const int tid = threadIdx.x;
   const int ntx = g.nxu / TX;
@@ -393,94 +457,92 @@ __global__ void __launch_bounds__(TR_NT, 4) k_tr_walk(TrArgs a) {
   }
   if (big) atomicExch(a.err, CASL_ECAPACITY);  // beyond the 16-bit places
   __syncthreads();
-  // Chain starts: the crossings of every TB-th line that enter a box of the
-  // tile, and the out-crossings of its saddle boxes on other lines.  (A list
-  // that fills up leaves the rest to their threads.)
+  auto entry = [&](int m, int y, int l) { return (unsigned)(m << 1 | y) << 16 | (unsigned)l; };
+  // the walks of the list's first ns starts (consecutive lanes: a walking
+  // warp's cost is that of its longest walk)
   int mine = 0;
-  auto start = [&](int m, int y, int l) {
-    const int s = atomicAdd(&nstart, 1);
-    if (s < TR_SCAP) {
-      slist[s] = (unsigned)(m << 1 | y) << 16 | (unsigned)l;
-      return;
-    }
-    const int c = atomicAdd(a.nchain, 1);
-    if (c < a.cap) mine += tr_walk(a, T, m, y, l, c, false);
-    else atomicExch(a.err, CASL_ECAPACITY);
-  };
-  constexpr int LX = (TX / TB + 1) * TY, LY = (TY / TB + 1) * TX;
-  for (int q = tid; q < LX + LY; q += TR_NT) {
-    const bool y = q >= LX;
-    const int line = y ? (q - LX) / TX * TB : q / TY * TB, at = y ? (q - LX) % TX : q % TY;
-    const int m = y ? at * TS + line : line * TS + at;
-    const bool ok = y ? line < th || (th == TY && line == TY) : at < th;
-    if (!ok || (y && ((line == 0 && T.open0) || (line == th && T.open1)))) continue;
-    const int c0 = C[m], c1 = C[m + (y ? TS : 1)];
-    // c1 high: to the right or down; c0 high: to the left or up.  On the
-    // tile's own sides only those that enter it.
-    const int n = y ? TY : TX;
-    if (y ? line > 0 : line < n)
-      for (int l = c0 + 1; l <= c1; l++) start(m, y, l);
-    if (y ? line < n : line > 0)
-      for (int l = c1 + 1; l <= c0; l++) start(m, y, l);
-    if (line == 0) nodes += max(0, y ? c0 - c1 : c1 - c0);
-    if (line == n) nodes += max(0, y ? c1 - c0 : c0 - c1);
-  }
-  // saddles, two rows of boxes at a time; a thread's boxes: half a column
-  const int bi = tid >> 1, bj0 = (TY / 2) * (tid & 1);
-  {
-    int m = bi * TS + bj0;
-    unsigned a0 = word(m), b0 = word(m + TS);
-    for (int j = bj0; j < bj0 + TY / 2; j += 2, m += 2) {
-      const unsigned a2 = word(m + 2), b2 = word(m + TS + 2);
-      const unsigned a1 = __funnelshift_r(a0, a2, 16), b1 = __funnelshift_r(b0, b2, 16);
-      const unsigned sd = __vcmpgtu2(__vminu2(a0, b1), __vmaxu2(b0, a1)) |
-                          __vcmpgtu2(__vminu2(b0, a1), __vmaxu2(a0, b1));
-      if (sd) {
-        for (int h = 0; h < 2; h++) {
-          const int jj = j + h, mm = m + h;
-          if (jj >= th) break;
-          const int c00 = C[mm], c10 = C[mm + TS], c01 = C[mm + 1], c11 = C[mm + TS + 1];
-          const int xl = max(c10, c01), xh = min(c00, c11), yl = max(c00, c11), yh = min(c10, c01);
-          for (int l = xl + 1; l <= xh; l++) {  // exits left and right
-            if (bi % TB) start(mm, 0, l);
-            if ((bi + 1) % TB) start(mm + TS, 0, l);
-          }
-          for (int l = yl + 1; l <= yh; l++) {  // exits bottom and top
-            if (jj % TB) start(mm, 1, l);
-            if ((jj + 1) % TB && jj + 1 < th) start(mm + 1, 1, l);
-          }
-        }
-      }
-      a0 = a2;
-      b0 = b2;
-    }
-  }
-  if (nodes) atomicAdd(&nnode, nodes);
-  __syncthreads();
-  const int ns = min(nstart, TR_SCAP);
-  if (tid == 0) base = ns ? atomicAdd(a.nchain, ns) : 0;
-  __syncthreads();
-  // (consecutive lanes: a walking warp's cost is that of its longest walk)
-  for (int s = tid; s < ns; s += TR_NT) {
-    const int c = base + s;
-    const unsigned w = slist[s];
-    if (c < a.cap) mine += tr_walk(a, T, (int)(w >> 17), (int)(w >> 16) & 1, (int)(w & 0xffffu), c, false);
-    else atomicExch(a.err, CASL_ECAPACITY);
-  }
-  if (mine) atomicAdd(&nvis, mine);
-  __syncthreads();
-  if (nvis == nnode) return;
-  // contours that meet no line where chains end: the crossings no chain has
-  // taken
-  for (int j = bj0; j < min(bj0 + TY / 2, th); j++) {
-    const int m = (bi + 1) * TS + j;  // entered from the right
-    for (int l = (int)C[m + 1] + 1; l <= (int)C[m]; l++) {
-      if (!tr_least(a, T, m, l)) continue;
-      const int c = atomicAdd(a.nchain, 1);
-      if (c < a.cap) tr_walk(a, T, m, 0, l, c, true);
+  auto walk_list = [&](int ns) {
+    if (tid == 0) base = ns ? atomicAdd(a.nchain, ns) : 0;
+    __syncthreads();
+    for (int s = tid; s < ns; s += TR_NT) {
+      const int c = base + s;
+      const unsigned w = slist[s];
+      if (c < a.cap) mine += tr_walk(a, T, (int)(w >> 17), (int)(w >> 16) & 1, (int)(w & 0xffffu), c, false);
       else atomicExch(a.err, CASL_ECAPACITY);
     }
+  };
+  // What does not fit the list at once: numbered thread by thread by a count
+  // and a scan, then listed and taken window by window.  (Starts past the list
+  // walked where they were found, and contours that meet no line walked by the
+  // thread of their first box, left one thread with all levels of a steep edge:
+  // 32^2, 1000 levels: 735 us, noise 2220 us; 140 and 228 so.)
+  auto windows = [&](auto each, auto take) {
+    int n = 0;
+    each([&](int, int, int lo, int hi) { n += hi - lo; });
+    const int first = block_excl_scan_any<int>(n, &total);
+    const int tot = total;
+    for (int b = (int)blockIdx.y * TR_SCAP; b < tot; b += (int)gridDim.y * TR_SCAP) {
+      int run = first;
+      each([&](int m, int y, int lo, int hi) {
+        const int z = min(run + hi - lo, b + TR_SCAP);
+        for (int s = max(run, b); s < z; s++) slist[s - b] = entry(m, y, lo + 1 + s - run);
+        run += hi - lo;
+      });
+      __syncthreads();
+      take(min(TR_SCAP, tot - b));
+      __syncthreads();
+    }
+  };
+  auto starts = [&](auto range) {
+    tr_starts(T, [&](int m, int y, int c0, int c1, int line, int last) {
+      tr_line_starts(m, y, c0, c1, line, last, range);
+    }, range);
+  };
+  if (gridDim.y == 1) {
+    auto range = [&](int m, int y, int lo, int hi) {
+      int s = atomicAdd(&nstart, hi - lo);
+      for (int l = lo + 1; l <= hi && s < TR_SCAP; l++) slist[s++] = entry(m, y, l);
+    };
+    tr_starts(T, [&](int m, int y, int c0, int c1, int line, int last) {
+      tr_line_starts(m, y, c0, c1, line, last, range);
+      if (line == 0) nodes += max(0, y ? c0 - c1 : c1 - c0);
+      if (line == last) nodes += max(0, y ? c1 - c0 : c0 - c1);
+    }, range);
+    if (nodes) atomicAdd(&nnode, nodes);
+    __syncthreads();
+    if (nstart <= TR_SCAP) walk_list(nstart);
+    else windows(starts, walk_list);
+    if (mine) atomicAdd(&nvis, mine);
+    __syncthreads();
+    if (nvis == nnode) return;
+  } else {
+    windows(starts, walk_list);
   }
+  // contours that meet no line where chains end: the crossings no chain has
+  // taken.  Each is walked from the least of its crossings that move left.
+  windows(
+      [&](auto range) {
+        const int bi = tid >> 1, bj0 = (TY / 2) * (tid & 1);
+        for (int j = bj0; j < min(bj0 + TY / 2, th); j++) {
+          const int m = (bi + 1) * TS + j;  // entered from the right
+          if (C[m] > C[m + 1]) range(m, 0, (int)C[m + 1], (int)C[m]);
+        }
+      },
+      [&](int ns) {
+        for (int s = tid; s < ns; s += TR_NT) {
+          const int m = (int)(slist[s] >> 17), l = (int)(slist[s] & 0xffffu);
+          if (!tr_least(a, T, m, l)) continue;
+          const int c = atomicAdd(a.nchain, 1);
+          if (c < a.cap) tr_walk(a, T, m, 0, l, c, true);
+          else atomicExch(a.err, CASL_ECAPACITY);
+        }
+      });
+}
+// CTAs a tile: as many as leave each 4096 crossings, while the tiles alone are
+// fewer than the SMs hold.
+inline int tr_slices(int ntile, long long ncr) {
+  const long long room = 3LL * 148 / ntile, most = ncr / (4096LL * ntile);
+  return (int)(room < 2 || most < 2 ? 1 : (room < most ? room : most));
 }
 
 // ---------------------------------------------------------------------------
@@ -560,7 +622,7 @@ __global__ void __launch_bounds__(TR_NT) k_tr_place(PlArgs a) {
   CASL_PDL_ENTRY();
   __shared__ __align__(16) unsigned short C[(TX + 1) * TS];
   __shared__ uint2 glist[TR_GCAP];
-  __shared__ int wsum[TR_NT / 32];
+  __shared__ int wsum[TR_NT / 32], wedge[TR_NT / 32];
   const CrGrid &g = a.g;
   const int tid = threadIdx.x, lane = tid & 31;
   const int ntx = g.nxu / TX;
@@ -618,46 +680,96 @@ __global__ void __launch_bounds__(TR_NT) k_tr_place(PlArgs a) {
       if (!g.periodic && r + 1 >= g.ylo + g.nyl) mb = 0;
     }
   }
-  const int incl = warp_incl_scan(tot);
-  if (lane == 31) wsum[tid >> 5] = incl;
+  const int ne = __popc(ma) + __popc(mb);
+  const int incl = warp_incl_scan(tot), eincl = warp_incl_scan(ne);
+  if (lane == 31) {
+    wsum[tid >> 5] = incl;
+    wedge[tid >> 5] = eincl;
+  }
   __syncthreads();
-  int s0 = incl - tot, all = 0;
+  int s0 = incl - tot, all = 0, e0 = eincl - ne, edges = 0;
   for (int w = 0; w < TR_NT / 32; w++) {
-    if (w < tid >> 5) s0 += wsum[w];
+    if (w < tid >> 5) {
+      s0 += wsum[w];
+      e0 += wedge[w];
+    }
     all += wsum[w];
+    edges += wedge[w];
   }
   const double qavg = ufield_qavg(a.uf.lsum, a.uf.qjump, a.uf.have, a.c.nxu, a.c.nyu);
-  for (int b = 0; b < all; b += TR_GCAP) {
-    if (tot && s0 < b + TR_GCAP && s0 + tot > b) {
-      int s = s0, id = id0;
+  // the thread's edges in order: f(point, first number, lower code, crossings)
+  auto each_edge = [&](auto f) {
+    int id = id0;
 #pragma unroll
-      for (int h = 0; h < 2; h++) {
-        if (!xl && h) id = id1;
-        for (unsigned m = h ? mb : ma; m; m &= m - 1) {
-          const int k = __ffs(m) - 1;
-          const int p = xl ? p0 + 32 * h + k : p0 + h + k * TS;
-          const int c0 = C[p], c1 = C[p + (xl ? 1 : TS)];
-          for (int l = min(c0, c1) + 1; l <= max(c0, c1); l++, s++, id++)
-            if (s >= b && s < b + TR_GCAP)
-              glist[s - b] = make_uint2((unsigned)(p << 1 | !xl) << 16 | (unsigned)l, (unsigned)id);
-        }
+    for (int h = 0; h < 2; h++) {
+      if (!xl && h) id = id1;
+      for (unsigned m = h ? mb : ma; m; m &= m - 1) {
+        const int k = __ffs(m) - 1;
+        const int p = xl ? p0 + 32 * h + k : p0 + h + k * TS;
+        const int c0 = C[p], c1 = C[p + (xl ? 1 : TS)], n = abs(c1 - c0);
+        f((unsigned)(p << 1 | !xl) << 16, id, min(c0, c1), n);
+        id += n;
       }
     }
+  };
+  auto put = [&](unsigned e, int id) {  // edge << 16 | level
+    const int2 o = __ldg(&a.own[id]);
+    const int4 R = __ldg(&a.R[o.x]);
+    const int m = (int)(e >> 17), cx = tr_col(m), cy = m - cx * TS;
+    const double2 v = tr_place<ECON>(a, qavg, ix0 + cx + 1, j0 + cy, (e >> 16) & 1u, (int)(e & 0xffffu));
+    if (R.w < 0) return;
+    int rp = R.x + o.y;
+    if (rp < 0) rp += R.y;
+    const long long pos = (long long)R.z + rp;
+    a.xw[pos] = v.x;
+    a.yw[pos] = v.y;
+    a.cidw[pos] = R.w;  // the contour of every walk position, for the first renode
+  };
+  if (all <= TR_MANY * edges) {
+    for (int b = (int)blockIdx.y * TR_GCAP; b < all; b += (int)gridDim.y * TR_GCAP) {
+      if (tot && s0 < b + TR_GCAP && s0 + tot > b) {
+        int s = s0;
+        each_edge([&](unsigned e, int id, int lo, int n) {
+          for (int l = lo + 1; l <= lo + n; l++, s++, id++)
+            if (s >= b && s < b + TR_GCAP) glist[s - b] = make_uint2(e | (unsigned)l, (unsigned)id);
+        });
+      }
+      __syncthreads();
+      for (int s = tid; s < min(TR_GCAP, all - b); s += TR_NT) put(glist[s].x, (int)glist[s].y);
+      __syncthreads();
+    }
+    return;
+  }
+  // Many levels an edge: the edges are listed, with the places of their first
+  // crossings, and a crossing finds its edge by search.  (A thread that lists
+  // its crossings one by one fills whole batches alone: 32^2, 1000 levels, with
+  // a CTA a tile, 2.0 ms, and 0.2 so.)
+  constexpr int EC = TR_GCAP / 2;
+  int *gst = reinterpret_cast<int *>(glist + EC);  // EC + 1 of them
+  for (int b = 0; b < edges; b += EC - 1) {
+    const int nl = min(EC - 1, edges - b);
+    if (ne && e0 < b + nl && e0 + ne > b) {
+      int s = s0, q = e0 - b;
+      each_edge([&](unsigned e, int id, int lo, int n) {
+        if (q >= 0 && q < nl) {
+          glist[q] = make_uint2(e | (unsigned)lo, (unsigned)id);
+          gst[q] = s;
+          if (q == nl - 1) gst[nl] = s + n;
+        }
+        s += n;
+        q++;
+      });
+    }
     __syncthreads();
-    for (int s = tid; s < min(TR_GCAP, all - b); s += TR_NT) {
-      const uint2 e = glist[s];
-      const int2 o = __ldg(&a.own[e.y]);
-      const int4 R = __ldg(&a.R[o.x]);
-      const int m = (int)(e.x >> 17), cx = tr_col(m), cy = m - cx * TS;
-      const double2 v = tr_place<ECON>(a, qavg, ix0 + cx + 1, j0 + cy, (e.x >> 16) & 1u,
-                                       (int)(e.x & 0xffffu));
-      if (R.w < 0) continue;
-      int rp = R.x + o.y;
-      if (rp < 0) rp += R.y;
-      const long long pos = (long long)R.z + rp;
-      a.xw[pos] = v.x;
-      a.yw[pos] = v.y;
-      a.cidw[pos] = R.w;  // the contour of every walk position, for the first renode
+    const int end = gst[nl];
+    for (int s = gst[0] + (int)blockIdx.y * TR_NT + tid; s < end; s += (int)gridDim.y * TR_NT) {
+      int lo = 0, hi = nl;  // gst[lo] <= s < gst[hi]
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (gst[mid] <= s) lo = mid; else hi = mid;
+      }
+      const int k = s - gst[lo];
+      put(glist[lo].x + 1u + (unsigned)k, (int)glist[lo].y + k);
     }
     __syncthreads();
   }
