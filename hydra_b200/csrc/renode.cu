@@ -327,91 +327,139 @@ __device__ double seq_sum(const double *__restrict__ e, long long cs, long long 
   return t;
 }
 
-// Per contour: node count and pieces (contours.f90:799-809, 813-930), and where
-// its nodes go in the output: tiles of 256 contours, whose kept nodes and
-// contours are scanned by looking back (packed as nodes * 2^31 + contours).
-// Pieces are stored block by block from a running total; their order is free.
+// A contour's pieces (contours.f90:799-809, 813-930): its nodes, corners, density
+// total, first corner and first piece.
+struct RnContour {
+  long long cs, L;
+  double total;
+  int nc, np, cfirst, p0;
+};
+// Piece q of it, stored; its new nodes.
+__device__ __forceinline__ int rn_piece(const RenodeScratch &s, const Consts &c, const RnContour &a,
+                                        int q) {
+  long long st, pl;
+  double sum;
+  int n;
+  if (a.nc <= 1) {
+    st = a.nc == 0 ? a.cs : s.cornerpos[a.cfirst];
+    pl = a.L;
+    sum = a.total;
+    n = nint_d(a.total) + 1;
+  } else {
+    st = s.cornerpos[a.cfirst + q];
+    const long long en = s.cornerpos[a.cfirst + (q + 1) % a.nc];
+    pl = en - st;  // both corners lie in [cs, cs+L)
+    if (pl < 0) pl += a.L;
+    sum = sumrange(s.S, a.cs, a.L, st, pl);
+    if (near_half(sum)) sum = seq_sum(s.e, a.cs, a.L, st, pl);
+    n = sum > c.small ? nint_d(sum) + 1 : 0;
+  }
+  const double preA = st == a.cs ? 0.0 : s.S[st - 1];
+  s.piece[a.p0 + q] = RnPiece{(int)st, (int)pl, n, 0, n > 0 ? (double)n / sum : 0.0,
+                              preA, s.S[a.cs + a.L - 1] - preA, 0.0};
+  return n;
+}
+
+// Per contour: node count and pieces, and where its nodes go in the output:
+// tiles of 256 contours, whose kept nodes and contours are scanned by looking
+// back (packed as nodes * 2^31 + contours).  Pieces are stored block by block
+// from a running total; their order is free.  Contours of more than RN_MANY
+// pieces are taken by the whole block: a thread alone needs half a
+// microsecond a corner, which the tiles behind it wait for (one contour of
+// 200,000 corners 107 ms, 1.8 so; from two million on those waits ran out).
+constexpr int RN_MANY = 64;
 __global__ void __launch_bounds__(256) k_rn_contours(RenodeIn in, RenodeScratch s, RenodeOut out,
                                                      Consts c, int mode) {
   CASL_PDL_ENTRY();
-  __shared__ int ptot, pbase;
+  __shared__ int ptot, pbase, nmany;
   __shared__ unsigned long long ntot, nbefore;
-  const int Ce = contours_in(in), ntile = (Ce + 255) / 256;
+  __shared__ int many[256], mn[256];  // the tile's long contours; their new nodes, then outputs
+  __shared__ RnContour mc[256];
+  const int Ce = contours_in(in), ntile = (Ce + 255) / 256, tid = threadIdx.x;
   while (true) {
     const int tile = lb_ticket(&s.tick[1]);
     if (tile >= ntile) {
-      if (ntile == 0 && tile == 0 && threadIdx.x < 3) out.d_counts[threadIdx.x] = 0;
+      if (ntile == 0 && tile == 0 && tid < 3) out.d_counts[tid] = 0;
       return;
     }
-    const int k = tile * 256 + threadIdx.x;
-    int np = 0, nc = 0;
-    long long cs = 0, L = 0;
-    double total = 0.0;
+    if (tid == 0) nmany = 0;
+    const int k = tile * 256 + tid;
+    RnContour a{};
     if (k < Ce) {
-      cs = in.cs[k];
-      L = in.len[k];
-      nc = s.ccnt[k];
-      total = s.S[cs + L - 1];
-      if (near_half(total)) total = seq_sum(s.e, cs, L, cs, L);
-      if (!(mode == RENODE_SURGERY && L <= 3)) {
-        int npr0 = nint_d(total) + 1;
-        if (npr0 >= 3) np = nc > 1 ? nc : 1;
+      a.cs = in.cs[k];
+      a.L = in.len[k];
+      a.nc = s.ccnt[k];
+      a.total = s.S[a.cs + a.L - 1];
+      if (near_half(a.total)) a.total = seq_sum(s.e, a.cs, a.L, a.cs, a.L);
+      if (!(mode == RENODE_SURGERY && a.L <= 3)) {
+        int npr0 = nint_d(a.total) + 1;
+        if (npr0 >= 3) a.np = a.nc > 1 ? a.nc : 1;
       }
     }
-    const int ex = block_excl_scan_any<int>(np, &ptot);
-    if (threadIdx.x == 0) pbase = ptot ? atomicAdd(&s.tick[2], ptot) : 0;
+    const int ex = block_excl_scan_any<int>(a.np, &ptot);
+    if (tid == 0) pbase = ptot ? atomicAdd(&s.tick[2], ptot) : 0;
     __syncthreads();
-    const int p0 = pbase + ex;
+    a.p0 = pbase + ex;
+    a.cfirst = a.np ? s.cc[a.cs] >> 1 : 0;
     int npr = 0;
-    const int cfirst = np ? s.cc[cs] >> 1 : 0;
-    for (int q = 0; q < np; q++) {
-      const int p = p0 + q;
-      long long st, pl;
-      double sum;
-      int n;
-      if (nc <= 1) {
-        st = nc == 0 ? cs : s.cornerpos[cfirst];
-        pl = L;
-        sum = total;
-        n = nint_d(total) + 1;
-      } else {
-        st = s.cornerpos[cfirst + q];
-        long long en = s.cornerpos[cfirst + (q + 1) % nc];
-        pl = en - st;  // both corners lie in [cs, cs+L)
-        if (pl < 0) pl += L;
-        sum = sumrange(s.S, cs, L, st, pl);
-        if (near_half(sum)) sum = seq_sum(s.e, cs, L, st, pl);
-        n = sum > c.small ? nint_d(sum) + 1 : 0;
-      }
-      const double preA = st == cs ? 0.0 : s.S[st - 1];
-      s.piece[p] = RnPiece{(int)st, (int)pl, n, 0, n > 0 ? (double)n / sum : 0.0,
-                           preA, s.S[cs + L - 1] - preA, 0.0};
-      npr += n;
+    if (a.np > RN_MANY) {
+      many[atomicAdd(&nmany, 1)] = tid;
+      mc[tid] = a;
+    } else {
+      for (int q = 0; q < a.np; q++) npr += rn_piece(s, c, a, q);
+    }
+    __syncthreads();
+    for (int m = 0; m < nmany; m++) {
+      const RnContour b = mc[many[m]];
+      int n = 0;
+      for (int q = tid; q < b.np; q += 256) n += rn_piece(s, c, b, q);
+      block_excl_scan_any<int>(n, &ptot);
+      if (tid == many[m]) npr = ptot;
+      __syncthreads();
     }
     const bool keep = k < Ce && (mode == RENODE_SURGERY ? npr > 3 : npr > 0);
     const unsigned long long mine = keep ? ((unsigned long long)npr << 31) + 1ull : 0ull;
     unsigned long long at = block_excl_scan_any<unsigned long long>(mine, &ntot);
-    if (threadIdx.x < 32) {
+    if (tid < 32) {
       const unsigned long long pre = lb_prefix(s.cstat, tile, ntot, s.err);
-      if (threadIdx.x == 0) nbefore = pre;
+      if (tid == 0) nbefore = pre;
     }
     __syncthreads();
     at += nbefore;
+    mn[tid] = -1;
     if (k < Ce) {
-      s.poff[k] = keep ? p0 : -1;
+      s.poff[k] = keep ? a.p0 : -1;
       if (keep) {
         int base = (int)(at >> 31);
         const int j = (int)(at & 0x7fffffffull);
         out.ocs[j] = base;
         out.olen[j] = npr;
         out.olev[j] = in.levt ? in.levt[k] : 0;
-        for (int q = 0; q < np; q++) {
-          s.piece[p0 + q].out = base;
-          base += s.piece[p0 + q].n;
+        if (a.np > RN_MANY) {
+          mn[tid] = base;
+        } else {
+          for (int q = 0; q < a.np; q++) {
+            s.piece[a.p0 + q].out = base;
+            base += s.piece[a.p0 + q].n;
+          }
         }
       }
     }
-    if (tile == ntile - 1 && threadIdx.x == 0) {
+    __syncthreads();
+    for (int m = 0; m < nmany; m++) {
+      int base = mn[many[m]];
+      if (base < 0) continue;
+      const int np = mc[many[m]].np;
+      RnPiece *p = s.piece + mc[many[m]].p0;
+      for (int q0 = 0; q0 < np; q0 += 256) {
+        const int q = q0 + tid;
+        const int off = block_excl_scan_any<int>(q < np ? p[q].n : 0, &ptot);
+        if (q < np) p[q].out = base + off;
+        base += ptot;
+        __syncthreads();
+      }
+    }
+    if (tile == ntile - 1 && tid == 0) {
       const unsigned long long all = nbefore + ntot;
       const long long nodes = (long long)(all >> 31);
       out.d_counts[0] = (int)(all & 0x7fffffffull);
