@@ -612,6 +612,19 @@ static int l1_host(casl_handle *h, const double *qq, double *l1) {
   return CASL_OK;
 }
 
+template <class Rel>
+static int launch_walk(casl_handle *h, const TrArgs &ta, int ntile, int nslice) {
+  static std::atomic<unsigned long long> configured{0};  // a bit per device
+  const unsigned long long bit = 1ULL << (h->device & 63);
+  if (!(configured.load() & bit)) {
+    CASL_CUDA_TRY(cudaFuncSetAttribute(k_tr_walk<Rel>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)sizeof(TrSmem<Rel>)));
+    configured.fetch_or(bit);
+  }
+  CASL_K(k_tr_walk<Rel>, dim3(ntile, nslice), TR_NT, sizeof(TrSmem<Rel>), h->stream)(ta);
+  return CASL_OK;
+}
+
 int recontour_dev(casl_handle *h, const double *qq) {
   cudaStream_t st = h->stream;
   const Consts &c = h->c;
@@ -670,11 +683,12 @@ int recontour_dev(casl_handle *h, const double *qq) {
   unsigned short *lc = ar.get<unsigned short>(NU);
   int *Lu = ar.get<int>(NU);
   int *ljx = ar.get<int>(nxu);
-  unsigned long long *lsum = ar.get<unsigned long long>(4);  // level sum; k_u_field's results
+  // level sum; k_u_field's results; k_cr_count's word
+  unsigned long long *lsum = ar.get<unsigned long long>(5);
   unsigned long long *rmn = ar.get<unsigned long long>(2 * nyu), *rmx = rmn + nyu;
   int *dtot = ar.get<int>(16);
   if (ar.failed) return CASL_ENOMEM;
-  CASL_CUDA_TRY(cudaMemsetAsync(lsum, 0, 4 * sizeof(unsigned long long), st));
+  CASL_CUDA_TRY(cudaMemsetAsync(lsum, 0, 5 * sizeof(unsigned long long), st));
   if (have) {
     CASL_CUDA_TRY(cudaMemsetAsync(Lu, 0, (size_t)NU * sizeof(int), st));
     CASL_CUDA_TRY(cudaMemsetAsync(ljx, 0, (size_t)nxu * sizeof(int), st));
@@ -813,13 +827,14 @@ int recontour_dev(casl_handle *h, const double *qq) {
     tmpi = ar.get<int>(scan_tmp_elems(nchunks) + 4);
     if (ar.failed) return CASL_ENOMEM;
   }
-  CASL_K(k_cr_count, (int)((nxu / 128) * (cg.ld / 256)), 256, 0, st)(cg, ccnt);
+  CASL_K(k_cr_count, (int)((nxu / 128) * (cg.ld / 256)), 256, 0, st)(
+      cg, ccnt, reinterpret_cast<int *>(lsum + 4));
   tr.point("cr_count");
   exclusive_scan<int>(st, ccnt, coffs, nchunks, tmpi, dtot);
   // the offset after the last chunk
   CASL_CUDA_TRY(cudaMemcpyAsync(coffs + nchunks, dtot, sizeof(int), cudaMemcpyDeviceToDevice, st));
-  int ncr_i = 0;
-  RC_TRY(read_back(h, {{&ncr_i, dtot, sizeof(int)}}));
+  int ncr_i = 0, wide = 0;
+  RC_TRY(read_back(h, {{&ncr_i, dtot, sizeof(int)}, {&wide, lsum + 4, sizeof(int)}}));
   const long long ncr = ncr_i;
   if (tr.on) fprintf(stderr, "[casl trace] recontour: %lld crossings on %d levels\n", ncr, nlev);
   if (ncr == 0) return set_empty();
@@ -850,16 +865,8 @@ int recontour_dev(casl_handle *h, const double *qq) {
     RC_TRY(fill_words(st, z, 1));
   }
   const int ntile = (nxu / TX) * ((cg.nbr + TY - 1) / TY), nslice = tr_slices(ntile, ncr);
-  {
-    static std::atomic<unsigned long long> configured{0};  // a bit per device
-    const unsigned long long bit = 1ULL << (h->device & 63);
-    if (!(configured.load() & bit)) {
-      CASL_CUDA_TRY(cudaFuncSetAttribute(k_tr_walk, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)sizeof(TrSmem)));
-      configured.fetch_or(bit);
-    }
-  }
-  CASL_K(k_tr_walk, dim3(ntile, nslice), TR_NT, sizeof(TrSmem), st)(ta);
+  RC_TRY(wide ? launch_walk<unsigned int>(h, ta, ntile, nslice)
+              : launch_walk<unsigned short>(h, ta, ntile, nslice));
   RC_TRY(check_launch(h));
   int cnts[2] = {0, 0};
   RC_TRY(read_back(h, {{cnts, ta.nchain, 2 * sizeof(int)}}));

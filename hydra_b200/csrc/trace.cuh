@@ -59,8 +59,11 @@ __device__ __forceinline__ unsigned absdiff2(unsigned a, unsigned b) {
 // Crossings per chunk.  A thread takes 8 rows of 17 columns as 16-byte loads
 // (lanes along the rows: coalesced) and counts with packed 16-bit differences:
 // both kinds of chunk from one read of the codes.  8 warps cover 128 columns,
-// so that the y-line counts of a row are written as whole sectors.
-__global__ void __launch_bounds__(256, 2) k_cr_count(CrGrid g, int *__restrict__ cnt) {
+// so that the y-line counts of a row are written as whole sectors.  *wide (zero on
+// entry) is set when a chunk has more than 16-bit places can number.
+constexpr int TR_NARROW = 65534;
+__global__ void __launch_bounds__(256, 2) k_cr_count(CrGrid g, int *__restrict__ cnt,
+                                                     int *__restrict__ wide) {
   CASL_PDL_ENTRY();
   __shared__ int Y[256][9];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -96,7 +99,10 @@ __global__ void __launch_bounds__(256, 2) k_cr_count(CrGrid g, int *__restrict__
       }
       s += __shfl_down_sync(0xffffffffu, s, 1);
       const int seg = r0 >> 4;
-      if (!(lane & 1) && seg < g.nseg) cnt[(long long)ix * g.nseg + seg] = s;
+      if (!(lane & 1) && seg < g.nseg) {
+        cnt[(long long)ix * g.nseg + seg] = s;
+        if (s > TR_NARROW) *wide = 1;
+      }
     }
     if (i > 0) {
 #pragma unroll
@@ -118,6 +124,10 @@ __global__ void __launch_bounds__(256, 2) k_cr_count(CrGrid g, int *__restrict__
     int4 *o = reinterpret_cast<int4 *>(cnt + g.ncx + (long long)(row - g.ylo) * (g.nxu / 16) + bx * 8);
     o[0] = make_int4(y[0], y[1], y[2], y[3]);
     o[1] = make_int4(y[4], y[5], y[6], y[7]);
+    int most = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) most = max(most, y[k]);
+    if (most > TR_NARROW) *wide = 1;
   }
 }
 
@@ -208,9 +218,10 @@ __device__ __forceinline__ long long tr_ychunk(const CrGrid &g, int ix0, int j0,
 }
 
 constexpr int TR_Y = (TX + 1) * TS;  // y-lines' places follow the x-lines'
+template <class Rel>
 struct TrTile {
   const unsigned short *C;    // codes, [column][row], row length TS
-  const unsigned short *rel;  // by an edge's first point: crossings of its chunk before it
+  const Rel *rel;             // by an edge's first point: crossings of its chunk before it
   const int *cb;              // chunk offsets: x-lines [column][TCX], y-lines [row][TCY]
   int th;                     // box rows of the tile (TY but at an open top)
   bool open0, open1;          // no boxes below / above the tile (a grid open in y)
@@ -222,7 +233,8 @@ struct TrTile {
 struct TrPos {
   int P, Q, v, lo;
 };
-__device__ __forceinline__ TrPos tr_at(const TrTile &T, int m, int y, int l) {
+template <class Rel>
+__device__ __forceinline__ TrPos tr_at(const TrTile<Rel> &T, int m, int y, int l) {
   const int n = m + (y ? TS : 1);
   const bool fwd = (int)T.C[m] >= l;
   TrPos p;
@@ -238,7 +250,8 @@ struct TrEdge {
   int q, r;
   bool line, open;  // open: a first or last row that no level reaches
 };
-__device__ __forceinline__ TrEdge tr_edge(const TrTile &T, const TrPos &p) {
+template <class Rel>
+__device__ __forceinline__ TrEdge tr_edge(const TrTile<Rel> &T, const TrPos &p) {
   const int m = min(p.P, p.Q), col = tr_col(m), row = m - col * TS;
   const bool y = p.v == 1 || p.v == -1;
   TrEdge e;
@@ -248,7 +261,8 @@ __device__ __forceinline__ TrEdge tr_edge(const TrTile &T, const TrPos &p) {
   e.open = y && ((row == 0 && T.open0) || (row == T.th && T.open1));
   return e;
 }
-__device__ __forceinline__ int tr_id(const TrTile &T, const TrPos &p, int l) {
+template <class Rel>
+__device__ __forceinline__ int tr_id(const TrTile<Rel> &T, const TrPos &p, int l) {
   const TrEdge e = tr_edge(T, p);
   return T.cb[e.q] + (int)T.rel[e.r] + l - p.lo - 1;
 }
@@ -269,7 +283,8 @@ __device__ __forceinline__ void tr_step(TrPos &p, int l, int cl, int cr) {
 // of shared memory are issued together: the crossing's number and the two
 // points ahead (which lie outside the staged codes, but inside the block's
 // shared memory, where the walk ends).
-__device__ __forceinline__ int tr_walk(const TrArgs &a, const TrTile &T, int m, int y, int l, int c,
+template <class Rel>
+__device__ __forceinline__ int tr_walk(const TrArgs &a, const TrTile<Rel> &T, int m, int y, int l, int c,
                                        bool loop) {
   TrPos p = tr_at(T, m, y, l);
   int first = -1, last = -1, mn = 0x7fffffff, k = 0, nxt = -1;
@@ -314,7 +329,8 @@ __device__ __forceinline__ int tr_walk(const TrArgs &a, const TrTile &T, int m, 
 // Whether level l's crossing of x-line edge m, which moves to the left, is the
 // least such one of a contour that meets no line where chains end (most walks
 // end after a step or two, at the next x-line to the left).
-__device__ __forceinline__ bool tr_least(const TrArgs &a, const TrTile &T, int m, int l) {
+template <class Rel>
+__device__ __forceinline__ bool tr_least(const TrArgs &a, const TrTile<Rel> &T, int m, int l) {
   TrPos p = tr_at(T, m, 0, l);
   int first = -1;
   for (int guard = 0; guard <= (1 << 20); guard++) {
@@ -339,8 +355,8 @@ __device__ __forceinline__ bool tr_least(const TrArgs &a, const TrTile &T, int m
 // line(m, y, c0, c1, which, last): an edge of such a line, from point m (y-line
 // when y) with codes c0, c1 at its ends, on line `which` of 0..last;
 // range(m, y, lo, hi): levels lo+1 .. hi that leave a saddle box by edge (m, y).
-template <class Line, class Range>
-__device__ __forceinline__ void tr_starts(const TrTile &T, Line line_f, Range range) {
+template <class Rel, class Line, class Range>
+__device__ __forceinline__ void tr_starts(const TrTile<Rel> &T, Line line_f, Range range) {
   const unsigned short *C = T.C;
   const int tid = threadIdx.x, th = T.th;
   auto word = [&](int p) { return *reinterpret_cast<const unsigned *>(C + p); };
@@ -391,20 +407,27 @@ __device__ __forceinline__ void tr_line_starts(int m, int y, int c0, int c1, int
   if ((y ? line < last : line > 0) && c0 > c1) range(m, y, c1, c0);
 }
 
+template <class Rel>
 struct TrSmem {
   unsigned short before[TS + 6];  // a step down or to the left of the tile reads here
-  unsigned short C[TR_Y], rel[2 * TR_Y];
+  unsigned short C[TR_Y];
+  alignas(4) Rel rel[2 * TR_Y];
   int cb[TQX + TQY];
   unsigned int slist[TR_SCAP];
 };
 // A tile is one CTA's (blockIdx.x), or several's when its crossings are many and
 // tiles few (blockIdx.y, tr_slices): each then stages the tile and takes its
 // share of the starts.
-__global__ void __launch_bounds__(TR_NT, 3) k_tr_walk(TrArgs a) {
+// Rel: places inside a chunk in 16 bits, or in 32 where some chunk has more
+// crossings (3 CTAs an SM and 2; 2 CTAs for every grid would cost a third of
+// this kernel's speed, which is latency).
+template <class Rel>
+__global__ void __launch_bounds__(TR_NT, sizeof(Rel) == 2 ? 3 : 2) k_tr_walk(TrArgs a) {
   CASL_PDL_ENTRY();
   extern __shared__ __align__(16) unsigned char tr_smem[];
-  TrSmem &sm = *reinterpret_cast<TrSmem *>(tr_smem);
-  unsigned short *C = sm.C, *rel = sm.rel;
+  TrSmem<Rel> &sm = *reinterpret_cast<TrSmem<Rel> *>(tr_smem);
+  unsigned short *C = sm.C;
+  Rel *rel = sm.rel;
   int *cb = sm.cb;
   unsigned int *slist = sm.slist;
   __shared__ int nstart, nvis, nnode, base, total;
@@ -420,12 +443,14 @@ __global__ void __launch_bounds__(TR_NT, 3) k_tr_walk(TrArgs a) {
   }
   if (!tr_stage(g, ix0, j0, C)) return;
   const int th = min(TY, g.nbr - j0);
-  const TrTile T{C, rel, cb, th, !g.periodic && j0 == 0, !g.periodic && j0 + th == g.nbr};
+  const TrTile<Rel> T{C, rel, cb, th, !g.periodic && j0 == 0, !g.periodic && j0 + th == g.nbr};
   // Places inside the chunks: prefix sums of the codes' differences, two rows
   // at a time (16-bit halves), and the crossings of the edges between two of
-  // the tile's boxes, all of which enter one of them.
+  // the tile's boxes, all of which enter one of them.  (Rows of a grid open in y
+  // past its last have codes of any kind, and sums that nothing reads.)
   auto word = [&](int p) { return *reinterpret_cast<const unsigned *>(C + p); };
-  int nodes = 0, big = 0;
+  constexpr bool WIDE = sizeof(Rel) == 4;
+  int nodes = 0;
   for (int q = tid; q < TQX; q += TR_NT) {
     const int col = q / TCX, r0 = 16 * (q % TCX), p0 = col * TS + r0;
     const bool inner = col > 0 && col < TX;
@@ -434,28 +459,37 @@ __global__ void __launch_bounds__(TR_NT, 3) k_tr_walk(TrArgs a) {
     for (int k = 0; k < 8; k++) {
       const unsigned n = word(p0 + 2 * k + 2), d = absdiff2(w, __funnelshift_r(w, n, 16));
       const unsigned d0 = d & 0xffffu, d1 = d >> 16;
-      *reinterpret_cast<unsigned *>(rel + p0 + 2 * k) = (run & 0xffffu) | (run + d0) << 16;
+      if constexpr (WIDE) {
+        rel[p0 + 2 * k] = run;
+        rel[p0 + 2 * k + 1] = run + d0;
+      } else {
+        *reinterpret_cast<unsigned *>(rel + p0 + 2 * k) = (run & 0xffffu) | (run + d0) << 16;
+      }
       if (inner) nodes += (r0 + 2 * k < th ? d0 : 0u) + (r0 + 2 * k + 1 < th ? d1 : 0u);
       run += d0 + d1;
       w = n;
     }
-    big |= run > 0xffffu && r0 + 16 <= th;
   }
   for (int q = tid; q < (TY / 2 + 1) * TCY; q += TR_NT) {
     const int r = 2 * (q / TCY), p0 = 16 * (q % TCY) * TS + r;
-    unsigned w = word(p0), run = 0;
+    unsigned w = word(p0), lo = 0, hi = 0;  // (16 bits: both rows' sums in lo)
 #pragma unroll
     for (int k = 0; k < 16; k++) {
-      const unsigned n = word(p0 + (k + 1) * TS);
-      *reinterpret_cast<unsigned *>(rel + TR_Y + p0 + k * TS) = run;
-      run = __vaddus2(run, absdiff2(w, n));
+      const unsigned n = word(p0 + (k + 1) * TS), d = absdiff2(w, n);
+      if constexpr (WIDE) {
+        rel[TR_Y + p0 + k * TS] = lo;
+        rel[TR_Y + p0 + k * TS + 1] = hi;
+        lo += d & 0xffffu;
+        hi += d >> 16;
+      } else {
+        *reinterpret_cast<unsigned *>(rel + TR_Y + p0 + k * TS) = lo;
+        lo = __vadd2(lo, d);
+      }
       w = n;
     }
-    if (r > 0 && r < th) nodes += run & 0xffffu;
-    if (r + 1 < th) nodes += run >> 16;
-    big |= (r + 1 < th) && ((run & 0xffffu) == 0xffffu || run >> 16 == 0xffffu);
+    if (r > 0 && r < th) nodes += WIDE ? lo : lo & 0xffffu;
+    if (r + 1 < th) nodes += WIDE ? hi : lo >> 16;
   }
-  if (big) atomicExch(a.err, CASL_ECAPACITY);  // beyond the 16-bit places
   __syncthreads();
   auto entry = [&](int m, int y, int l) { return (unsigned)(m << 1 | y) << 16 | (unsigned)l; };
   // the walks of the list's first ns starts (consecutive lanes: a walking
