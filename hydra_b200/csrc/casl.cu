@@ -1456,10 +1456,6 @@ __global__ void k_stage_rk(NodeRkArgs<float> a, SpecRkArgs b, Scalars *__restric
 
 namespace casl {
 
-__global__ void k_twist_sub(Scalars *s, double twistmax, int M) {
-  CASL_PDL_ENTRY();
-  for (int m = threadIdx.x; m < M; m += blockDim.x) s[m].twist = s[m].twist - twistmax;
-}
 __global__ void k_twist_zero(Scalars *s, int M) {
   CASL_PDL_ENTRY();
   for (int m = threadIdx.x; m < M; m += blockDim.x) s[m].twist = 0.0;
@@ -3153,16 +3149,14 @@ int casl_step(casl_handle *h, int nsteps) {
         h->ireg = 0;
         if (force) {
           h->ireg = 1;
-          if ((rc = surgery_dev(h))) return rc;
+          if ((rc = surgery_dev(h, h->p.twistmax))) return rc;
           if ((rc = debug_check(h, "surgery after recontouring"))) return rc;
           if (h->M > 1 && (rc = member_ranges(h))) return rc;
-          CASL_K(k_twist_sub, 1, 256, 0, h->stream)(h->scal, h->p.twistmax, h->M);
         }
       } else {
-        if ((rc = surgery_dev(h))) return rc;
+        if ((rc = surgery_dev(h, h->p.twistmax))) return rc;
         if ((rc = debug_check(h, "surgery"))) return rc;
         if (h->M > 1 && (rc = member_ranges(h))) return rc;
-        CASL_K(k_twist_sub, 1, 256, 0, h->stream)(h->scal, h->p.twistmax, h->M);
       }
     }
     if ((rc = saves_before_advance(h))) return rc;

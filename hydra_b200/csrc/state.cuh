@@ -121,7 +121,7 @@ int con2grid_dev(casl_handle *h, bool want_levels);  // -> coarseC, scal->csum
 int con2grid_to_spec(casl_handle *h, double *spec); // con2grid + ptospc fused load
 int con2grid_to_phys(casl_handle *h, double *phys, bool want_levels);  // -> qc(ny,nx)
 
-int surgery_dev(casl_handle *h);
+int surgery_dev(casl_handle *h, double twist = 0.0);  // takes twist off every member's twist
 int recontour_dev(casl_handle *h, const double *qq_dev);
 int renode_host(casl_handle *h, const double *xd, const double *yd, int npd, double *xr,
                 double *yr, int cap, int *npr);

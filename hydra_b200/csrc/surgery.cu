@@ -782,9 +782,11 @@ __global__ void k_rb_writeback(const int *__restrict__ cnt, long long npm, long 
                                double *__restrict__ yq, int *__restrict__ nextq,
                                int *__restrict__ i1q, int *__restrict__ i2q,
                                int *__restrict__ npq, int *__restrict__ indq,
-                               Scalars *__restrict__ s) {
+                               Scalars *__restrict__ s, int M, double twist) {
   CASL_PDL_ENTRY();
   const int nq = cnt[0], npt = cnt[1];
+  if (blockIdx.x == 0)  // (a launch of its own took 2 us of a step)
+    for (int m = threadIdx.x; m < M; m += blockDim.x) s[m].twist = s[m].twist - twist;
   if (cnt[2] || npt > npm || nq > nm) {
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicExch(&s->error, CASL_ECAPACITY);
     return;
@@ -810,6 +812,11 @@ __global__ void k_rb_writeback(const int *__restrict__ cnt, long long npm, long 
   }
 }
 
+__global__ void k_twist_sub(Scalars *s, int M, double twist) {
+  CASL_PDL_ENTRY();
+  for (int m = threadIdx.x; m < M; m += blockDim.x) s[m].twist = s[m].twist - twist;
+}
+
 static inline int gs(long long work) {
   long long g = (work + 255) / 256;
   if (g < 1) g = 1;
@@ -823,7 +830,7 @@ static inline int gs(long long work) {
 // rw's words are zero.
 static int rebuild_and_renode(casl_handle *h, Arena &ar, int npt, const int *lvl,
                               const LevelDesc *dlev, unsigned long long *stat,
-                              const RenodeWords &rw) {
+                              const RenodeWords &rw, double twist) {
   cudaStream_t st = h->stream;
   int *rid = ar.get<int>(npt);
   int *dtot = ar.get<int>(8);
@@ -868,13 +875,16 @@ static int rebuild_and_renode(casl_handle *h, Arena &ar, int npt, const int *lvl
   if (rc) return rc;
   CASL_K(k_rb_writeback, gs(h->npm < (1 << 24) ? h->npm : (1 << 24)), 256, 0, st)(
       cnt, h->npm, h->nm, ocs, olen, olev, h->xqi, h->yqi, h->xq, h->yq, h->nextq, h->i1q,
-      h->i2q, h->npq, h->indq, h->scal);
+      h->i2q, h->npq, h->indq, h->scal, h->M, twist);
   return check_launch(h);
 }
 
-int surgery_dev(casl_handle *h) {
-  if (h->nq == 0 || h->nptq == 0) return CASL_OK;
+int surgery_dev(casl_handle *h, double twist) {
   cudaStream_t st = h->stream;
+  if (h->nq == 0 || h->nptq == 0) {
+    if (twist != 0.0) CASL_K(k_twist_sub, 1, 256, 0, st)(h->scal, h->M, twist);
+    return check_launch(h);
+  }
   const Consts &c = h->c;
   const int nq = h->nq, npt = h->nptq;
   const long long nbox_cap = 2LL * npt + nq + 64;
@@ -961,7 +971,7 @@ int surgery_dev(casl_handle *h) {
     fprintf(stderr, "[casl trace] replay: %d levels, pending %lld (max %d at level %d, %d surgeries there), surgeries %lld (max %d)\n",
             nlev, sp, mp, wl, hs[2 * wl + 1], ss, ms);
   }
-  rc = rebuild_and_renode(h, ar, npt, lvl, dlev, stat, rw);
+  rc = rebuild_and_renode(h, ar, npt, lvl, dlev, stat, rw, twist);
   if (rc) return rc;
   tr.point("rebuild+renode");
   tr.flush("surgery");
