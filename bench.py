@@ -149,9 +149,8 @@ def measured_peak():
 
 # DRAM bytes per launch of the transform kernels at 1024^2, read off one ncu
 # capture of steps of this size (dram__bytes_read.sum + dram__bytes_write.sum
-# averaged over its k_fs_cols, k_fs_rows and k_fs_prod launches;
-# profiles/stage_1024.md gives the command).  A stated constant, not a
-# measurement of this run.
+# averaged over its k_fs_cols, k_fs_rows and k_fs_prod launches, from cold
+# caches).  A stated constant, not a measurement of this run.
 FFT_TRAFFIC_PER_LAUNCH_1024 = 41.4e6
 
 
@@ -523,12 +522,16 @@ def run_gpu(a):
             "e2e": {"value": e2e_ns / (e2e_ms * 1e-3), "unit": UNIT,
                     "h2d_bytes_per_step": e2e["h2d"], "d2h_bytes_per_step": e2e["d2h"],
                     "steps": e2e["steps"]},
-            "roofline": {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
-                         "frac": ach / peak if peak else None, "traffic": traffic,
+            # bound by the exchanges in shared memory (60 % of the cycles; DRAM
+            # 13 %), so frac is what the bytes a transform cannot do without
+            # would take at the HBM rate, not HBM traffic
+            "roofline": {"bound": "shared-memory wavefronts", "achieved": ach, "peak": peak,
+                         "unit": "GB/s", "frac": ach / peak if peak else None, "traffic": traffic,
                          "traffic_source": "constant: ncu DRAM bytes per transform launch at "
-                                           "1024^2 (profiles/stage_1024.md)",
-                         "bytes_rule": "16 B per FP64 element per 2-D transform (one read, "
-                                       "one write); a pass counts half",
+                                           "1024^2, cold caches",
+                         "bytes_rule": "algorithmic: 16 B per FP64 element per 2-D transform "
+                                       "(one read, one write), half for each axis, whether or "
+                                       "not fused away",
                          "kernel": "k_fs_cols, k_fs_rows, k_fs_prod (a stage's transforms; "
                                    "k_fs_end, whose transform shares the update, is not timed)",
                          "launches": fft_n, "kernel_ms_per_step": fft_ms / a.steps,

@@ -1543,8 +1543,10 @@ int inversion_dev(casl_handle *h) {
 // operations, rather than stage.cuh's.  Rounding the inverse transforms'
 // intermediate to FP32 turns a difference in the last FP64 bit into one of
 // 6e-8 wherever a value lies next to a rounding boundary; over five steps at
-// 2048^2 stage.cuh's order moved qd by 2.5e-9 (and the FP64 mode's by 1e-14),
-// so runs in this mode keep the order they have been made with.
+// 2048^2 stage.cuh's order moved qd by 2.5e-9 (and the FP64 mode's by 1e-14).
+// That is below the mode's own distance from FP64 (8e-9 in qd, 5e-8 in
+// velocity): the old order is kept so that runs repeat, not because the new one
+// would be worse.
 // main_invert and the four gradients of source (evolution.f90:432-490,
 // spectral.f90:304-366) as one batch-6 inverse transform pair with FP32
 // storage (CASL_PREC_FP32_INVERSION): u, v from green*qq and the x/y

@@ -57,7 +57,7 @@ Launch<F> launch_of(F f, dim3 grid, dim3 block, size_t smem = 0, cudaStream_t st
   return Launch<F>{f, grid, block, smem, st};
 }
 
-// Clears or fills up to six word arrays in one kernel launch: in-stream like
+// Clears or fills up to eight word arrays in one kernel launch: in-stream like
 // cudaMemsetAsync, but a kernel, so the launches around it keep the
 // programmatic overlap.  p is 4-byte aligned, words counts 32-bit words.
 struct FillJob {

@@ -770,7 +770,9 @@ int recontour_dev(casl_handle *h, const double *qq) {
     eg.iymax = iy;
     eg.nby = 1 - eg.iymin / nyu;
     eg.bfac = bfac;
-    // box numbers of the extended grid are 32-bit
+    // extended grids of 2^32 points and more are refused, as they were when
+    // boxes had 32-bit numbers (10 GB of codes and counts; crossings are
+    // counted in an int)
     if ((long long)nxu * (eg.iymax - eg.iymin + 2) >= (1LL << 32)) return CASL_ECAPACITY;
   }
   // --- 2. levels (congen.f90:156-173; econgen.f90:131-134) -------------------

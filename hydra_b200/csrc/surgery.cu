@@ -320,9 +320,9 @@ __global__ void __launch_bounds__(256) k_sg_alloc(const int *__restrict__ bcnt,
 // as links it was built in one pass, but a warp then waits for one load per
 // entry (a surgery of 40 patches of 500 nodes on one level, lists of thousands,
 // 124 ms, and 23 so; isolated vortices at 1024^2, 39k nodes, 1.6 ms a step, and
-// 1.1 so), and the short lists of a turbulent state gain by it as well (1.4M
-// nodes: this kernel, the counts and the ranges take 15 us more than the links
-// did, the replay went from 107 to 58 us).
+// 1.1 so).  A turbulent state of 1.4M nodes: this kernel, the counts and the
+// ranges take 15 us more than the links did, the candidate search 7 less, and
+// the replay 3 to 50 less, as there are few or many nodes to replay.
 __global__ void k_sg_place(const double4 *__restrict__ g0, const int *__restrict__ nq0,
                            const int *__restrict__ lvl, const LevelDesc *__restrict__ lev, int npt,
                            unsigned int ne_cap, uint2 *__restrict__ range, int2 *__restrict__ ent,

@@ -18,10 +18,10 @@
 // order, and only contours (a few thousand) are sorted by level at the end.
 //
 // Measured (B200), contours plus residual at 1024^2, 25M crossings: the part
-// from the counts to the walk layout took 6.7 ms and takes 3.4 ms (k_cr_count
-// 0.24, k_tr_walk 1.37, ranking 0.45, k_tr_place 1.07), the whole recontouring
-// 13.3 and 9.5 ms (8.4 with later changes to the renode passes and the field);
-// beta-plane from a field at 256^2 3.2 and 1.8 ms (1.49).
+// from the counts to the walk layout took 6.7 ms and takes 3.3 ms (k_cr_count
+// 0.24, k_tr_walk 1.35, ranking 0.41, k_tr_place 1.09), the whole recontouring
+// 13.3 and 9.5 ms (8.5 with later changes to the renode passes and the field);
+// beta-plane from a field at 256^2 3.2 and 1.8 ms (1.50).
 // k_tr_walk is bound by the latency of its walks (16k of a tile's 31k cycles:
 // 23 chains of 32 crossings, some 190 cycles a step, in one warp; the rest is
 // staging and the offsets), k_tr_place by issue (63 % of the slots).
@@ -419,8 +419,8 @@ struct TrSmem {
 // tiles few (blockIdx.y, tr_slices): each then stages the tile and takes its
 // share of the starts.
 // Rel: places inside a chunk in 16 bits, or in 32 where some chunk has more
-// crossings (3 CTAs an SM and 2; 2 CTAs for every grid would cost a third of
-// this kernel's speed, which is latency).
+// crossings: 98 KB of shared memory for 64, 2 CTAs an SM for 3 (25M crossings at
+// 1024^2: 2.12 ms with 32 bits, 1.35 with 16).
 template <class Rel>
 __global__ void __launch_bounds__(TR_NT, sizeof(Rel) == 2 ? 3 : 2) k_tr_walk(TrArgs a) {
   CASL_PDL_ENTRY();
